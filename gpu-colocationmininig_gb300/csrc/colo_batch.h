@@ -64,19 +64,23 @@ struct Batch {
     DevBuf<uint8_t> qfirst;      // per cell: bit q set when it is the first occupied cell of its quad q
     // runs
     DevBuf<uint32_t> rfeat, rstart, rcnt, rcell;
-    // neighbourhood run lists: for cell c, the runs of its adjacent cells
-    // ordered by (feature, cell), entries above the cell's lowest own feature:
-    // nrl_ent[nrl_off[c] .. nrl_off[c+1]), each the run's (first sorted
-    // position, point count)
-    DevBuf<uint64_t> nrl_off;
+    // neighbourhood run lists: for each cell with targets, the runs of its
+    // adjacent cells ordered by (feature, cell), entries above the cell's lowest
+    // own feature, each the run's (first sorted position, point count); the
+    // lists are in no particular order
     DevBuf<uint2> nrl_ent;
     uint64_t nrl_total = 0;
-    // per run: first entry of its cell's list with a higher feature (absolute
-    // index), the entries from there to the list's end (run_qn), and the
-    // number of target points in them; run_sfx and run_qn are set where run_L > 0
+    // per own run of those cells: first entry of its cell's list with a higher
+    // feature (absolute index), the entries from there to the list's end, and
+    // the number of target points in them
     DevBuf<uint64_t> run_sfx;
     DevBuf<uint32_t> run_qn;
     DevBuf<uint32_t> run_L;
+    // the join's anchors (points of runs with targets), in no particular order:
+    // act = (sorted position, entries qn, first entry sfx low and high word), and
+    // act_base = the anchor's start in the single-pass layout
+    DevBuf<uint4> act;
+    DevBuf<uint64_t> act_base;
     // neighbour lists N+(a) = nb[nb_beg[a] .. nb_beg[a] + nb_cnt[a]), each in
     // (feature, neighbour cell, id) order; nb_beg[a] is set only where nb_cnt[a] > 0
     DevBuf<uint64_t> nb_beg;

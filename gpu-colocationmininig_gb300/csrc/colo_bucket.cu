@@ -541,45 +541,26 @@ __device__ __forceinline__ int adjacent_cells(uint64_t c, const uint64_t* ckey, 
 // lowest own feature: the join reads a list from an own run's suffix on, and
 // the lowest own run's suffix starts past every entry of feature <= its own.
 // Most lists are then empty; the cells whose 3x3 mask allows one were queued
-// by k_quad_masks (nrl_len is zero for the others).  Grid-stride over the queue.
-__global__ void k_nrl_count(const uint32_t* __restrict__ listq, const uint32_t* __restrict__ nlistq,
-                            const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob,
-                            const JobGrid* __restrict__ grids, const int32_t* __restrict__ nb9,
-                            const uint32_t* __restrict__ crun, const uint32_t* __restrict__ rfeat,
-                            uint32_t* __restrict__ nrl_len) {
-    const uint32_t n = *nlistq;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint64_t c = listq[i];
-        const uint32_t fmin = rfeat[crun[c]];
-        int32_t adj[9];
-        const int na = adjacent_cells(c, ckey, cjob, grids, nb9, adj);
-        uint32_t nr = 0;
-        for (int t = 0; t < na; ++t) {
-            const uint64_t q0 = crun[adj[t]], q1 = crun[adj[t] + 1];
-            nr += (uint32_t)(q1 - lower_bound_dev(rfeat, q0, q1, fmin + 1));
-        }
-        nrl_len[c] = nr;
-    }
-}
+// by k_quad_masks.
 
-// The list of cell c (lanes l = 0..G-1 of a group share it).  In the full
-// (feature, slot) order a run of feature f in adjacent slot s is at the sum
-// over slots of (#runs with feature < f) plus the number of earlier slots
-// that also hold f; the kept list drops the off0 entries of feature <= the
-// cell's lowest own feature.  Per own run of the cell: the first entry with a
-// higher feature and the number of target points from there on (the points
-// of each adjacent cell past its runs of features <= f), both from one binary
-// search per slot.
-template <int G>
-__device__ __forceinline__ void nrl_cell(uint64_t c, int l, const uint64_t* __restrict__ ckey,
-                                         const uint32_t* __restrict__ cjob, const JobGrid* __restrict__ grids,
-                                         const int32_t* __restrict__ nb9, const uint32_t* __restrict__ cstart,
-                                         const uint32_t* __restrict__ crun, const uint32_t* __restrict__ rfeat,
-                                         const uint32_t* __restrict__ rstart, const uint32_t* __restrict__ cmask,
-                                         const uint32_t* __restrict__ rcnt, uint32_t W,
-                                         const uint64_t* __restrict__ nrl_off, uint2* __restrict__ nrl_ent,
-                                         uint64_t* __restrict__ run_sfx, uint32_t* __restrict__ run_qn,
-                                         uint32_t* __restrict__ run_L) {
+constexpr uint32_t kBigList = 64;        // cells with longer lists are merged by their whole warp
+constexpr uint32_t kHeavyAnchors = 32;   // cells with more anchors are listed by their whole warp
+
+// The list of cell c by a whole warp.  In the full (feature, slot) order a run
+// of feature f in adjacent slot s is at the sum over slots of (#runs with
+// feature < f) plus the number of earlier slots that also hold f; the kept
+// list (from entry `first` on) drops the entries of feature <= the cell's
+// lowest own feature.  Per own run of the cell: the first entry with a higher
+// feature, the entries from there on, and the number of target points in them
+// (the points of each adjacent cell past its runs of features <= f), from one
+// binary search per slot.
+__device__ __forceinline__ void nrl_cell_warp(uint64_t c, int l, uint64_t first, uint32_t kept,
+                                              const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob,
+                                              const JobGrid* __restrict__ grids, const int32_t* __restrict__ nb9,
+                                              const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ crun,
+                                              const uint32_t* __restrict__ rfeat, const uint32_t* __restrict__ rstart,
+                                              const uint32_t* __restrict__ rcnt, uint2* __restrict__ nrl_ent,
+                                              uint64_t* run_sfx, uint32_t* run_qn, uint32_t* run_L) {
     int32_t adj[9];
     const int na = adjacent_cells(c, ckey, cjob, grids, nb9, adj);
     const uint32_t fmin = rfeat[crun[c]];
@@ -597,8 +578,8 @@ __device__ __forceinline__ void nrl_cell(uint64_t c, int l, const uint64_t* __re
         }
         pre[t + 1] = pre[t] + (q1[t] - q0[t]);
     }
-    const uint64_t base = nrl_off[c] - off0;   // where entry 0 of the full order would be
-    for (uint32_t e = l; e < pre[9]; e += G) {
+    const uint64_t base = first - off0;   // where entry 0 of the full order would be
+    for (uint32_t e = l; e < pre[9]; e += 32) {
         int sl = 0;
         uint32_t r = 0;
 #pragma unroll
@@ -620,7 +601,7 @@ __device__ __forceinline__ void nrl_cell(uint64_t c, int l, const uint64_t* __re
         }
         nrl_ent[base + pos] = make_uint2(rstart[r], rcnt[r]);
     }
-    for (uint32_t r = crun[c] + l; r < crun[c + 1]; r += G) {
+    for (uint32_t r = crun[c] + l; r < crun[c + 1]; r += 32) {
         const uint32_t f = rfeat[r];
         uint64_t sfx = base;
         uint32_t L = 0;
@@ -633,131 +614,193 @@ __device__ __forceinline__ void nrl_cell(uint64_t c, int l, const uint64_t* __re
             }
         }
         run_sfx[r] = sfx;
-        run_qn[r] = (uint32_t)(nrl_off[c + 1] - sfx);
+        run_qn[r] = (uint32_t)(first + kept - sfx);
         run_L[r] = L;
     }
 }
 
-constexpr uint32_t kBigList = 512;   // cells with longer lists get a warp each
-
-// One thread per cell: the list is the 9-way merge, by (feature, slot), of
-// the adjacent cells' runs above the lowest own feature (each slot ascending
-// by feature).  The running point count P gives the suffix counts: the
-// cell's own run of feature f gets sfx = the first position after every
-// entry of feature <= f and L = (points in the list) - P(sfx).  Cells with
-// lists longer than kBigList are queued for k_nrl_fill_big.
-__device__ __forceinline__ void nrl_fill_cell(uint64_t c, const uint64_t* __restrict__ ckey,
-                                              const uint32_t* __restrict__ cjob, const JobGrid* __restrict__ grids,
-                                              const int32_t* __restrict__ nb9, const uint32_t* __restrict__ crun,
-                                              const uint32_t* __restrict__ rfeat, const uint32_t* __restrict__ rstart,
-                                              const uint32_t* __restrict__ rcnt, const uint64_t* __restrict__ nrl_off,
-                                              uint2* __restrict__ nrl_ent, uint64_t* __restrict__ run_sfx,
-                                              uint32_t* __restrict__ run_qn, uint32_t* __restrict__ run_L,
-                                              uint32_t* __restrict__ big, uint32_t* __restrict__ nbig) {
-    const uint64_t base = nrl_off[c], kept = nrl_off[c + 1] - base;
-    if (kept == 0) return;   // no own run has targets (run_L is zero)
-    const uint32_t r0 = crun[c], r1 = crun[c + 1];
-    if (kept > kBigList) {   // the merge below is serial in the list
-        big[atomicAdd(nbig, 1u)] = (uint32_t)c;
-        return;
-    }
-    int32_t adj[9];
-    const int na = adjacent_cells(c, ckey, cjob, grids, nb9, adj);
-    const uint32_t fmin = rfeat[r0];
-    // each slot's cursor starts at its first run above the lowest own feature
-    uint32_t h[9], e[9], f[9];
-    int own = 0;
+// Neighbourhood run lists and the join's anchors in one pass over the queued
+// cells.  A thread takes a cell: its list is the 9-way merge, by (feature,
+// slot), of the adjacent cells' runs above the lowest own feature (each slot
+// ascending by feature).  The running point count P gives the suffix counts:
+// the cell's own run of feature f gets sfx = the first position after every
+// entry of feature <= f and L = (points in the list) - P(sfx).  Then every
+// point of an own run with targets (L > 0) is listed as an anchor: act =
+// (sorted position, list entries qn, first entry sfx) and act_base, its start
+// in the single-pass layout, where it owns L entries.
+//
+// Bound by the merge's chain of dependent loads.  The lists, anchors and
+// capacities are not in cell order: a warp reserves its 32 cells' room with one
+// atomic on each of the three totals (tot: list entries, anchors, capacity), so
+// nothing is counted or scanned over the cells and runs beforehand (the order
+// within a list is all that a result depends on).  This replaces a count
+// kernel, a scan over the cells, the list fill, a second kernel for long lists
+// and a scan over the runs, with a clear of two arrays: 413 us of kernels (64 count, 149 fill, 200
+// scans) became 164 us on the 20M workload, one host wait fewer; the 200,000-point dense one, whose
+// few long lists share a neighbourhood, 327 became 137 us.
+// Lists past `cap` entries are not written; the host sees it in tot[0] and runs
+// the kernel again with room for all.
+__global__ void __launch_bounds__(128) k_neighbour_lists(
+    const uint32_t* __restrict__ listq, const uint32_t* __restrict__ nlistq, const uint64_t* __restrict__ ckey,
+    const uint32_t* __restrict__ cjob, const JobGrid* __restrict__ grids, const int32_t* __restrict__ nb9,
+    const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ crun, const uint32_t* __restrict__ rfeat,
+    const uint32_t* __restrict__ rstart, const uint32_t* __restrict__ rcnt, uint64_t cap, uint2* __restrict__ nrl_ent,
+    uint64_t* run_sfx, uint32_t* run_qn, uint32_t* run_L, uint4* __restrict__ act, uint64_t* __restrict__ act_base,
+    unsigned long long* __restrict__ tot) {
+    const uint32_t n = *nlistq;
+    const int lane = threadIdx.x & 31;
+    const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5), w = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    // A queue of 32 cells a warp or more is taken 32 consecutive cells at a time.  A shorter one is
+    // dealt out evenly, one cell after the other to warp after warp: long lists sit next to each
+    // other in the queue, and the merge's latency then runs in as many warps as there are.
+    const bool deal = n < 32 * nw;
+    const uint64_t per = deal ? (n + nw - 1) / nw : 32;
+    for (uint64_t i0 = deal ? w : 32 * w; i0 < n; i0 += 32 * nw) {
+        const uint64_t i = deal ? i0 + (uint64_t)lane * nw : i0 + lane;
+        const bool in = (uint64_t)lane < per && i < n;
+        uint32_t c = 0, r0 = 0, r1 = 0, kept = 0;
+        // each slot's cursor starts at its first run above the lowest own feature
+        uint32_t h[9], e[9], f[9];
+        int own = 0;
 #pragma unroll
-    for (int t = 0; t < 9; ++t) {
-        if (t < na) {
-            e[t] = crun[adj[t] + 1];
-            h[t] = (uint32_t)lower_bound_dev(rfeat, (uint64_t)crun[adj[t]], (uint64_t)e[t], fmin + 1);
-            f[t] = h[t] < e[t] ? rfeat[h[t]] : 0xffffffffu;
-            if ((uint64_t)adj[t] == c) own = t;
-        } else {
+        for (int t = 0; t < 9; ++t) {
             h[t] = e[t] = 0;
             f[t] = 0xffffffffu;
         }
-    }
-    // the lowest own run's suffix is the whole list
-    const uint64_t end = base + kept;
-    run_sfx[r0] = base;
-    run_qn[r0] = (uint32_t)kept;
-    run_L[r0] = 0;
-    uint64_t pos = base;
-    uint32_t P = 0, pend_r = 0, pend_f = 0;
-    bool pend = false;
-    for (;;) {
-        int ts = 0;
-        uint32_t fm = f[0];
+        if (in) {
+            c = listq[i];
+            r0 = crun[c];
+            r1 = crun[c + 1];
+            const uint32_t fmin = rfeat[r0];
+            int32_t adj[9];
+            const int na = adjacent_cells(c, ckey, cjob, grids, nb9, adj);
 #pragma unroll
-        for (int t = 1; t < 9; ++t)
-            if (f[t] < fm) {
-                fm = f[t];
-                ts = t;
-            }
-        if (fm == 0xffffffffu) break;
-        if (pend && pend_f < fm) {
-            run_sfx[pend_r] = pos;
-            run_qn[pend_r] = (uint32_t)(end - pos);
-            run_L[pend_r] = P;
-            pend = false;
+            for (int t = 0; t < 9; ++t)
+                if (t < na) {
+                    e[t] = crun[adj[t] + 1];
+                    h[t] = (uint32_t)lower_bound_dev(rfeat, (uint64_t)crun[adj[t]], (uint64_t)e[t], fmin + 1);
+                    f[t] = h[t] < e[t] ? rfeat[h[t]] : 0xffffffffu;
+                    kept += e[t] - h[t];
+                    if ((uint32_t)adj[t] == c) own = t;
+                }
         }
-        uint32_t r = 0;
+        const uint32_t kincl = warp_incl_scan(kept);
+        const uint32_t ktot = __shfl_sync(0xffffffffu, kincl, 31);
+        if (ktot == 0) continue;
+        unsigned long long kb = 0;
+        if (lane == 0) kb = atomicAdd(&tot[0], (unsigned long long)ktot);
+        kb = __shfl_sync(0xffffffffu, kb, 0);
+        if (kb + ktot > cap) continue;   // no room: the host runs the kernel again
+        const uint64_t first = kb + (kincl - kept);
+        const bool big = kept > kBigList;
+        if (kept && !big) {
+            // the lowest own run's suffix is the whole list
+            const uint64_t end = first + kept;
+            run_sfx[r0] = first;
+            run_qn[r0] = kept;
+            run_L[r0] = 0;
+            for (uint32_t r = r0 + 1; r < r1; ++r) run_L[r] = 0;
+            uint64_t pos = first;
+            uint32_t P = 0, pend_r = 0, pend_f = 0;
+            bool pend = false;
+            for (;;) {
+                int ts = 0;
+                uint32_t fm = f[0];
 #pragma unroll
-        for (int t = 0; t < 9; ++t)
-            if (t == ts) {
-                r = h[t]++;
-                f[t] = h[t] < e[t] ? rfeat[h[t]] : 0xffffffffu;
+                for (int t = 1; t < 9; ++t)
+                    if (f[t] < fm) {
+                        fm = f[t];
+                        ts = t;
+                    }
+                if (fm == 0xffffffffu) break;
+                if (pend && pend_f < fm) {
+                    run_sfx[pend_r] = pos;
+                    run_qn[pend_r] = (uint32_t)(end - pos);
+                    run_L[pend_r] = P;
+                    pend = false;
+                }
+                uint32_t r = 0;
+#pragma unroll
+                for (int t = 0; t < 9; ++t)
+                    if (t == ts) {
+                        r = h[t]++;
+                        f[t] = h[t] < e[t] ? rfeat[h[t]] : 0xffffffffu;
+                    }
+                const uint32_t rc = rcnt[r];
+                nrl_ent[pos++] = make_uint2(rstart[r], rc);
+                P += rc;
+                if (ts == own) {
+                    pend = true;
+                    pend_r = r;
+                    pend_f = fm;
+                }
             }
-        const uint32_t rc = rcnt[r];
-        nrl_ent[pos++] = make_uint2(rstart[r], rc);
-        P += rc;
-        if (ts == own) {
-            pend = true;
-            pend_r = r;
-            pend_f = fm;
+            if (pend) {
+                run_sfx[pend_r] = pos;
+                run_qn[pend_r] = 0;
+                run_L[pend_r] = P;
+            }
+            for (uint32_t r = r0; r < r1; ++r) run_L[r] = P - run_L[r];
+        }
+        for (uint32_t m = __ballot_sync(0xffffffffu, big); m; m &= m - 1) {   // the merge above is serial in the list
+            const int j = __ffs(m) - 1;
+            nrl_cell_warp(__shfl_sync(0xffffffffu, c, j), lane, __shfl_sync(0xffffffffu, first, j),
+                          __shfl_sync(0xffffffffu, kept, j), ckey, cjob, grids, nb9, cstart, crun, rfeat, rstart, rcnt,
+                          nrl_ent, run_sfx, run_qn, run_L);
+        }
+        __syncwarp();
+        // anchors: the points of own runs with targets
+        uint32_t na = 0;
+        uint64_t nu = 0;
+        if (kept)
+            for (uint32_t r = r0; r < r1; ++r) {
+                const uint32_t L = run_L[r];
+                if (!L) continue;
+                const uint32_t rc = rcnt[r];
+                na += rc;
+                nu += (uint64_t)rc * L;
+            }
+        const uint32_t aincl = warp_incl_scan(na);
+        const uint64_t uincl = warp_incl_scan(nu);
+        unsigned long long ab = 0, ub = 0;
+        if (lane == 31 && aincl) {
+            ab = atomicAdd(&tot[1], (unsigned long long)aincl);
+            ub = atomicAdd(&tot[2], (unsigned long long)uincl);
+        }
+        uint64_t o = __shfl_sync(0xffffffffu, ab, 31) + (aincl - na);
+        uint64_t u = __shfl_sync(0xffffffffu, ub, 31) + (uincl - nu);
+        const bool heavy = na > kHeavyAnchors;
+        if (na && !heavy)
+            for (uint32_t r = r0; r < r1; ++r) {
+                const uint32_t L = run_L[r];
+                if (!L) continue;
+                const uint32_t st = rstart[r], rc = rcnt[r], qn = run_qn[r];
+                const uint64_t sfx = run_sfx[r];
+                for (uint32_t q = 0; q < rc; ++q) {
+                    act[o] = make_uint4(st + q, qn, (uint32_t)sfx, (uint32_t)(sfx >> 32));
+                    act_base[o] = u;
+                    ++o;
+                    u += L;
+                }
+            }
+        for (uint32_t m = __ballot_sync(0xffffffffu, heavy); m; m &= m - 1) {   // the loop above is serial in the points
+            const int j = __ffs(m) - 1;
+            const uint32_t s0 = __shfl_sync(0xffffffffu, r0, j), s1 = __shfl_sync(0xffffffffu, r1, j);
+            uint64_t oj = __shfl_sync(0xffffffffu, o, j), uj = __shfl_sync(0xffffffffu, u, j);
+            for (uint32_t r = s0; r < s1; ++r) {   // the whole warp reads the run
+                const uint32_t L = run_L[r];
+                if (!L) continue;
+                const uint32_t st = rstart[r], rc = rcnt[r], qn = run_qn[r];
+                const uint64_t sfx = run_sfx[r];
+                for (uint32_t q = lane; q < rc; q += 32) {
+                    act[oj + q] = make_uint4(st + q, qn, (uint32_t)sfx, (uint32_t)(sfx >> 32));
+                    act_base[oj + q] = uj + (uint64_t)q * L;
+                }
+                oj += rc;
+                uj += (uint64_t)rc * L;
+            }
         }
     }
-    if (pend) {
-        run_sfx[pend_r] = pos;
-        run_qn[pend_r] = 0;
-        run_L[pend_r] = P;
-    }
-    for (uint32_t r = r0; r < r1; ++r) run_L[r] = P - run_L[r];
-}
-
-// Grid-stride over the queued cells; run_L is zero for every run of the
-// others, and run_sfx is read only where run_L > 0.
-__global__ void k_nrl_fill(const uint32_t* __restrict__ work, const uint32_t* __restrict__ nwork,
-                           const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob,
-                           const JobGrid* __restrict__ grids, const int32_t* __restrict__ nb9,
-                           const uint32_t* __restrict__ crun, const uint32_t* __restrict__ rfeat,
-                           const uint32_t* __restrict__ rstart, const uint32_t* __restrict__ rcnt,
-                           const uint64_t* __restrict__ nrl_off, uint2* __restrict__ nrl_ent,
-                           uint64_t* __restrict__ run_sfx, uint32_t* __restrict__ run_qn,
-                           uint32_t* __restrict__ run_L, uint32_t* __restrict__ big, uint32_t* __restrict__ nbig) {
-    const uint32_t n = *nwork;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        nrl_fill_cell(work[i], ckey, cjob, grids, nb9, crun, rfeat, rstart, rcnt, nrl_off, nrl_ent, run_sfx, run_qn,
-                      run_L, big, nbig);
-}
-
-// A warp per queued cell (grid-stride over the queue).
-__global__ void k_nrl_fill_big(const uint32_t* __restrict__ big, const uint32_t* __restrict__ nbig,
-                               const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob,
-                               const JobGrid* __restrict__ grids, const int32_t* __restrict__ nb9,
-                               const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ crun,
-                               const uint32_t* __restrict__ rfeat, const uint32_t* __restrict__ rstart,
-                               const uint32_t* __restrict__ cmask, uint32_t W,
-                               const uint32_t* __restrict__ rcnt, const uint64_t* __restrict__ nrl_off,
-                               uint2* __restrict__ nrl_ent, uint64_t* __restrict__ run_sfx,
-                               uint32_t* __restrict__ run_qn, uint32_t* __restrict__ run_L) {
-    const uint32_t n = *nbig;
-    const int lane = threadIdx.x & 31;
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5)
-        nrl_cell<32>(big[i], lane, ckey, cjob, grids, nb9, cstart, crun, rfeat, rstart, cmask, rcnt, W, nrl_off,
-                     nrl_ent, run_sfx, run_qn, run_L);
 }
 
 inline unsigned grid_for(uint64_t n, int threads) {
@@ -963,46 +1006,39 @@ void bucket_points(Batch& b) {
 void build_neighborhoods(Batch& b) {
     cudaStream_t s = b.s;
     const uint64_t M = b.M;
-    DevBuf<uint32_t> nrl_len;
-    nrl_len.alloc(M ? M : 1, s);
-    nrl_len.zero(s);
-    const unsigned qgrid = (unsigned)std::min<uint64_t>(grid_for(M, 128), (uint64_t)b.sms * 16);
-    {
-        KScope ks("nrl_count");
-        k_nrl_count<<<qgrid, 128, 0, s>>>(b.listq.get(), b.nlistq.get(), b.ckey.get(), b.cjob.get(), b.grids.get(),
-                                          b.nb9.get(), b.crun.get(), b.rfeat.get(), nrl_len.get());
-        COLO_LAUNCH_CHECK();
-        count_launch();
-    }
-    b.nrl_off.alloc(M + 1, s);
-    uint64_t tr = 0;
-    scan_u32_to_u64(nrl_len.get(), b.nrl_off.get(), M, s, &tr);
-    COLO_CUDA(cudaMemcpyAsync(b.nrl_off.get() + M, &tr, 8, cudaMemcpyHostToDevice, s));
-    b.nrl_total = tr;
-    b.nrl_ent.alloc(tr ? tr : 1, s);
     b.run_sfx.alloc(b.Rn, s);
     b.run_qn.alloc(b.Rn, s);
     b.run_L.alloc(b.Rn, s);
-    {
-        KScope ks("nrl_fill");
-        DevBuf<uint32_t> big, nbig;
-        big.alloc(M ? M : 1, s);
-        nbig.alloc(1, s);
-        nbig.zero(s);
-        COLO_CUDA(cudaMemsetAsync(b.run_L.get(), 0, b.Rn * 4, s));
-        k_nrl_fill<<<qgrid, 128, 0, s>>>(
-            b.listq.get(), b.nlistq.get(), b.ckey.get(), b.cjob.get(), b.grids.get(), b.nb9.get(), b.crun.get(),
-            b.rfeat.get(), b.rstart.get(), b.rcnt.get(), b.nrl_off.get(), b.nrl_ent.get(), b.run_sfx.get(),
-            b.run_qn.get(), b.run_L.get(), big.get(), nbig.get());
-        COLO_LAUNCH_CHECK();
-        k_nrl_fill_big<<<(unsigned)(b.sms * 8), 256, 0, s>>>(big.get(), nbig.get(), b.ckey.get(), b.cjob.get(),
-                                                             b.grids.get(), b.nb9.get(), b.cstart.get(), b.crun.get(),
-                                                             b.rfeat.get(), b.rstart.get(), b.cmask.get(), b.W,
-                                                             b.rcnt.get(), b.nrl_off.get(), b.nrl_ent.get(),
-                                                             b.run_sfx.get(), b.run_qn.get(), b.run_L.get());
-        COLO_LAUNCH_CHECK();
-        count_launch(2);
+    b.act.alloc(b.N ? b.N : 1, s);
+    b.act_base.alloc(b.N ? b.N : 1, s);
+    DevBuf<unsigned long long> tot;
+    tot.alloc(3, s);
+    const unsigned qgrid = (unsigned)std::min<uint64_t>(grid_for(M, 128), (uint64_t)b.sms * 16);
+    // room for four list entries per run (0.2 on the 20M workload, 3.4 on a batch of many small
+    // jobs; nine at most: a run is adjacent to nine cells); lists that need more are built again
+    // with the counted room
+    uint64_t cap = std::min<uint64_t>(9 * b.Rn, 4 * b.Rn + 65536);
+    unsigned long long h[3] = {0, 0, 0};
+    for (;;) {
+        b.nrl_ent.alloc(cap ? cap : 1, s);
+        tot.zero(s);
+        {
+            KScope ks("neighbour_lists");
+            k_neighbour_lists<<<qgrid, 128, 0, s>>>(
+                b.listq.get(), b.nlistq.get(), b.ckey.get(), b.cjob.get(), b.grids.get(), b.nb9.get(), b.cstart.get(),
+                b.crun.get(), b.rfeat.get(), b.rstart.get(), b.rcnt.get(), cap, b.nrl_ent.get(), b.run_sfx.get(),
+                b.run_qn.get(), b.run_L.get(), b.act.get(), b.act_base.get(), tot.get());
+            COLO_LAUNCH_CHECK();
+            count_launch();
+        }
+        COLO_CUDA(cudaMemcpyAsync(h, tot.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+        stream_wait(s);
+        if (h[0] <= cap) break;
+        cap = h[0];
     }
+    b.nrl_total = h[0];
+    b.active_anchors = h[1];
+    b.join_pairs = h[2];
 }
 
 }  // namespace colo

@@ -13,10 +13,12 @@
 //               qmask[M*4*W] (masks of the 4 quads containing the cell)
 //   runs        (cell, feature) runs rfeat/rstart/rcnt/rcell[Rn], cell-major;
 //               runs per feature on the host (h_frun_off prefix)
-//   NRL         per cell, the runs of its adjacent cells with a feature above
-//               the cell's lowest own feature, ordered by (feature, cell):
-//               nrl_off[M+1], nrl_ent (start, count); per run the start of its
-//               higher-feature suffix run_sfx and its size run_L
+//   NRL         per cell with targets, the runs of its adjacent cells with a
+//               feature above the cell's lowest own feature, ordered by
+//               (feature, cell): nrl_ent (start, count); per run the start of
+//               its higher-feature suffix run_sfx and its size run_L
+//   anchors     act[A], act_base[A]: the points of runs with targets, with
+//               their list slices and their starts in the single-pass layout
 //   neighbours  N+(a) = nb[nb_beg[a] .. nb_beg[a] + nb_cnt[a]) by point id
 #pragma once
 #include <cuda_runtime.h>
@@ -320,16 +322,6 @@ void scan_u32_to_u32(const uint32_t* in, uint32_t* out, uint64_t n, cudaStream_t
                      uint32_t* total_host, uint32_t* total_dev = nullptr);
 void scan_u64_to_u64(const uint64_t* in, uint64_t* out, uint64_t n, cudaStream_t s,
                      uint64_t* total_host, uint64_t* total_dev = nullptr);
-// The join's run scans in one pass: act_r = rcnt[r] if run_L[r] > 0 else 0 and
-// cap_r = act_r * run_L[r].  The active anchors are listed in run order:
-// act_pos (sorted positions rstart[r] .. rstart[r] + act_r - 1), act_run (r)
-// and act_base (the exclusive scan of cap over the runs before r, plus the
-// anchor's index in its run times run_L[r]: its list start in the single-pass
-// layout); they need room for the sum of act_r.  The totals (sum of act_r,
-// sum of cap_r) land in device memory (no wait).
-void run_scans(const uint32_t* rcnt, const uint32_t* run_L, const uint32_t* rstart, uint32_t* act_pos,
-               uint32_t* act_run, uint64_t* act_base, uint64_t Rn, cudaStream_t s, uint32_t* act_total,
-               uint64_t* cap_total);
 // Digit split of a radix sort: pass p sorts width[p] (<= 8) bits from shift[p].
 constexpr int kRadixDigits = 256;
 constexpr int kRadixMaxPasses = 8;

@@ -33,23 +33,22 @@ constexpr int kEntrySlots = 64, kEntryStride = 16;
 // One anchor's neighbour list, by its group of T lanes; returns the list length.
 template <int T, int MODE>
 __device__ __forceinline__ uint32_t join_anchor(
-    uint64_t i, const uint32_t* __restrict__ act_pos, const uint32_t* __restrict__ act_run,
-    const uint32_t* __restrict__ sid, const uint32_t* __restrict__ sfeat, const float2* __restrict__ sxy,
-    const uint64_t* __restrict__ run_sfx, const uint32_t* __restrict__ run_qn, const uint64_t* __restrict__ act_base,
+    uint64_t i, const uint4* __restrict__ act, const uint32_t* __restrict__ sid, const uint32_t* __restrict__ sfeat,
+    const float2* __restrict__ sxy, const uint64_t* __restrict__ act_base,
     const uint2* __restrict__ nrl_ent, const uint32_t* __restrict__ fjob, const JobGrid* __restrict__ grids,
     uint64_t* __restrict__ nb_beg, uint32_t* __restrict__ nb_cnt, uint32_t* __restrict__ nb) {
     const int lane = threadIdx.x & 31;
     const int gl = lane % T;
     const int gbase = lane - gl;
     const uint32_t gmask = (T == 32) ? 0xffffffffu : (((1u << T) - 1u) << gbase);
-    const uint32_t p = act_pos[i];
-    const uint32_t r = act_run[i];
+    const uint4 an = act[i];   // position and list slice in one load: the list's first entry waits on this one alone
+    const uint32_t p = an.x;
     const uint32_t a = sid[p];
     const float2 pa = sxy[p];
     const float xa = pa.x, ya = pa.y;
     const JobGrid& g = grids[fjob ? fjob[sfeat[p]] : 0u];   // fjob is null for one-job batches
     const float R2 = g.R2, hu = g.R2hu;
-    const uint64_t q0 = run_sfx[r], qend = q0 + run_qn[r];
+    const uint64_t q0 = (uint64_t)an.w << 32 | an.z, qend = q0 + an.y;
     uint64_t base = 0;
     if (MODE == J_SINGLE) base = act_base[i];
     if (MODE == J_FILL) base = nb_beg[a];
@@ -92,9 +91,8 @@ __device__ __forceinline__ uint32_t join_anchor(
 // measured 0.398 -> 0.377 ms per step on the 20M workload.
 template <int T, int MODE>
 __global__ void __launch_bounds__(256, 6) k_join(
-    uint64_t A, const uint32_t* __restrict__ act_pos, const uint32_t* __restrict__ act_run,
-    const uint32_t* __restrict__ sid, const uint32_t* __restrict__ sfeat, const float2* __restrict__ sxy,
-    const uint64_t* __restrict__ run_sfx, const uint32_t* __restrict__ run_qn, const uint64_t* __restrict__ act_base,
+    uint64_t A, const uint4* __restrict__ act, const uint32_t* __restrict__ sid, const uint32_t* __restrict__ sfeat,
+    const float2* __restrict__ sxy, const uint64_t* __restrict__ act_base,
     const uint2* __restrict__ nrl_ent, const uint32_t* __restrict__ fjob, const JobGrid* __restrict__ grids,
     uint64_t* __restrict__ nb_beg, uint32_t* __restrict__ nb_cnt, uint32_t* __restrict__ nb,
     unsigned long long* __restrict__ total) {
@@ -102,8 +100,7 @@ __global__ void __launch_bounds__(256, 6) k_join(
     const int gl = lane % T;
     const uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / T;
     // groups past the last anchor (whole groups) count nothing but stay for the block sum
-    const uint32_t k = i < A ? join_anchor<T, MODE>(i, act_pos, act_run, sid, sfeat, sxy, run_sfx, run_qn, act_base,
-                                                     nrl_ent, fjob, grids, nb_beg, nb_cnt, nb)
+    const uint32_t k = i < A ? join_anchor<T, MODE>(i, act, sid, sfeat, sxy, act_base, nrl_ent, fjob, grids, nb_beg, nb_cnt, nb)
                              : 0u;
     if (MODE == J_SINGLE) {
         // the entries of the warp's anchors (each group's count once), one atomic per warp into
@@ -119,15 +116,15 @@ __global__ void __launch_bounds__(256, 6) k_join(
 }
 
 template <int T>
-void run_join(Batch& b, int mode, uint64_t A, const uint32_t* act_pos, const uint32_t* act_run,
-              const uint64_t* act_base) {
+void run_join(Batch& b, int mode) {
+    const uint64_t A = b.active_anchors;
     if (A == 0) return;
     uint64_t threads = A * T;
     unsigned grid = (unsigned)((threads + 255) / 256);
     KScope ks(mode == J_SINGLE ? "join" : mode == J_COUNT ? "join_count" : "join_fill");
 #define COLO_JOIN(MD)                                                                                        \
-    k_join<T, MD><<<grid, 256, 0, b.s>>>(A, act_pos, act_run, b.sid.get(), b.sfeat.get(), b.sxy.get(),       \
-                                         b.run_sfx.get(), b.run_qn.get(), act_base, b.nrl_ent.get(),            \
+    k_join<T, MD><<<grid, 256, 0, b.s>>>(A, b.act.get(), b.sid.get(), b.sfeat.get(), b.sxy.get(),               \
+                                         b.act_base.get(), b.nrl_ent.get(),                                     \
                                          b.J > 1 ? b.fjob.get() : nullptr,                                      \
                                          b.grids.get(), b.nb_beg.get(), b.nb_cnt.get(), b.nb.get(), b.dE.get())
     if (mode == J_SINGLE) COLO_JOIN(J_SINGLE);
@@ -138,15 +135,14 @@ void run_join(Batch& b, int mode, uint64_t A, const uint32_t* act_pos, const uin
     count_launch();
 }
 
-void dispatch_join(Batch& b, int mode, uint64_t A, const uint32_t* act_pos, const uint32_t* act_run,
-                   const uint64_t* act_base) {
+void dispatch_join(Batch& b, int mode) {
     switch (b.join_group) {
-        case 1: run_join<1>(b, mode, A, act_pos, act_run, act_base); break;
-        case 2: run_join<2>(b, mode, A, act_pos, act_run, act_base); break;
-        case 4: run_join<4>(b, mode, A, act_pos, act_run, act_base); break;
-        case 16: run_join<16>(b, mode, A, act_pos, act_run, act_base); break;
-        case 32: run_join<32>(b, mode, A, act_pos, act_run, act_base); break;
-        default: run_join<8>(b, mode, A, act_pos, act_run, act_base); break;
+        case 1: run_join<1>(b, mode); break;
+        case 2: run_join<2>(b, mode); break;
+        case 4: run_join<4>(b, mode); break;
+        case 16: run_join<16>(b, mode); break;
+        case 32: run_join<32>(b, mode); break;
+        default: run_join<8>(b, mode); break;
     }
 }
 
@@ -167,28 +163,7 @@ static const uint64_t kSinglePassCap = 1ull << 30;
 
 void join_neighbors(Batch& b) {
     cudaStream_t s = b.s;
-    const uint64_t Rn = b.Rn;
-    // the active anchors (the points of runs with targets, by run) are listed by the
-    // scan itself, into arrays sized for every point
-    DevBuf<uint32_t> act_pos, act_run;
-    DevBuf<uint64_t> act_base;
-    act_pos.alloc(b.N ? b.N : 1, s);
-    act_run.alloc(b.N ? b.N : 1, s);
-    act_base.alloc(b.N ? b.N : 1, s);
-    // per run: active anchors (its points, when it has targets) and the single-pass layout's
-    // capacity (points x targets), both scanned in one pass; the totals A and U (= pair
-    // evaluations) come back together with one wait
-    DevBuf<uint64_t> totals;
-    totals.alloc(2, s);
-    run_scans(b.rcnt.get(), b.run_L.get(), b.rstart.get(), act_pos.get(), act_run.get(), act_base.get(), Rn, s,
-              reinterpret_cast<uint32_t*>(totals.get()), totals.get() + 1);
-    uint64_t ht[2] = {0, 0};
-    COLO_CUDA(cudaMemcpyAsync(ht, totals.get(), 16, cudaMemcpyDeviceToHost, s));
-    stream_wait(s);
-    const uint32_t A = (uint32_t)ht[0];
-    const uint64_t U = ht[1];
-    b.active_anchors = A;
-    b.join_pairs = U;
+    const uint64_t U = b.join_pairs;
     // a point without targets keeps a zero count; its list start is never read (every
     // reader takes nb_cnt first), so only the counts are cleared
     b.nb_beg.alloc(b.N ? b.N : 1, s);
@@ -201,15 +176,15 @@ void join_neighbors(Batch& b) {
         b.nb_cap = U;
         b.nb.alloc(U ? U : 1, s);
         b.dE.zero(s);
-        dispatch_join(b, J_SINGLE, A, act_pos.get(), act_run.get(), act_base.get());
+        dispatch_join(b, J_SINGLE);
         b.E = UINT64_MAX;
     } else {
-        dispatch_join(b, J_COUNT, A, act_pos.get(), act_run.get(), nullptr);
+        dispatch_join(b, J_COUNT);
         uint64_t E = 0;
         scan_u32_to_u64(b.nb_cnt.get(), b.nb_beg.get(), b.N, s, &E);
         b.nb_cap = E;
         b.nb.alloc(E ? E : 1, s);
-        dispatch_join(b, J_FILL, A, act_pos.get(), act_run.get(), nullptr);
+        dispatch_join(b, J_FILL);
         b.E = E;
     }
 }

@@ -623,6 +623,8 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
     double t_bucket = ms_since(t0);
     t0 = Clock::now();
     if (N > 0) join_neighbors(b);
+    b.act.release();
+    b.act_base.release();
     double t_join = ms_since(t0);   // host time: the level loop's first wait absorbs the join's tail
 
     double t_filter = 0, t_refine = 0, t_fill = 0, t_apriori = 0;

@@ -147,116 +147,6 @@ __global__ void __launch_bounds__(kScanThreads, 5) k_scan_1p(const Tin* __restri
     if (total && threadIdx.x == 0 && (uint64_t)(tile + 1) * kScan1Tile >= n) *total = (Tout)s_prefix + tot;
 }
 
-// The join's two run scans in one pass: per run r the active anchors
-// act_r = rcnt[r] when the run has targets (run_L[r] > 0) and the single-pass
-// layout's capacity cap_r = rcnt[r] * run_L[r] (both 0 otherwise), scanned
-// exclusively, with the totals; warps 0 and 1 look back for the two scans at
-// once.  Tiles of 2048 runs (two values per run in registers).  The anchors
-// are listed in the same pass: the active anchors of a warp's 32 runs fill one
-// contiguous range of act_pos / act_run / act_base (their sorted positions,
-// runs and single-pass list starts: the run's capacity offset plus the
-// anchor's index in the run times run_L), which the warp writes 32 entries at
-// a time, each lane finding its entry's run by a binary search over the
-// warp's inclusive counts.
-constexpr int kRunItems = 8;
-constexpr int kRunTile = kScanThreads * kRunItems;
-
-// Six blocks per SM (40 registers, a few spilled): the scan waits on its look-back at the
-// barrier, so more resident tiles help -- the scans of the 20M workload took 0.316 ms per
-// step against 0.342 ms at four blocks (62 registers).
-__global__ void __launch_bounds__(kScanThreads, 6) k_run_scans(uint64_t Rn, const uint32_t* __restrict__ rcnt,
-                                                            const uint32_t* __restrict__ run_L,
-                                                            const uint32_t* __restrict__ rstart,
-                                                            uint32_t* __restrict__ act_pos, uint32_t* __restrict__ act_run,
-                                                            uint64_t* __restrict__ act_base,
-                                                            unsigned long long* __restrict__ status,
-                                                            uint32_t* __restrict__ ticket, uint32_t* __restrict__ act_total,
-                                                            uint64_t* __restrict__ cap_total) {
-    __shared__ uint32_t s_tile;
-    __shared__ unsigned long long s_prefix[2];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
-    __syncthreads();
-    const uint32_t tile = s_tile;
-    const uint64_t ntiles = (Rn + kRunTile - 1) / kRunTile;
-    unsigned long long* st_act = status;
-    unsigned long long* st_cap = status + ntiles;
-    const uint64_t seg = (uint64_t)tile * kRunTile + (uint64_t)w * (32 * kRunItems);
-    uint32_t a[kRunItems], L[kRunItems];
-    uint32_t asum = 0;
-    uint64_t csum = 0;
-#pragma unroll
-    for (int i = 0; i < kRunItems; ++i) {
-        const uint64_t p = seg + (uint64_t)i * 32 + lane;
-        const uint32_t l = p < Rn ? run_L[p] : 0u;
-        a[i] = l ? rcnt[p] : 0u;
-        L[i] = l;
-        asum += a[i];
-        csum += (uint64_t)a[i] * l;
-    }
-    uint32_t atot;
-    uint64_t ctot;
-    const uint32_t aex = block_excl_scan<uint32_t>(asum, &atot);
-    const uint64_t cex = block_excl_scan<uint64_t>(csum, &ctot);
-    if (w < 2) {
-        unsigned long long* st = w == 0 ? st_act : st_cap;
-        const unsigned long long agg = w == 0 ? (unsigned long long)atot : (unsigned long long)ctot;
-        unsigned long long prefix;
-        if (!warp_lookback(st, tile, agg, prefix)) {   // the predecessors' runs, summed here
-            unsigned long long add = 0;
-            for (uint64_t p = lane; p < (uint64_t)tile * kRunTile; p += 32) {
-                const uint32_t l = run_L[p];
-                const uint64_t av = l ? rcnt[p] : 0u;
-                add += w == 0 ? av : av * l;
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
-            prefix = add;
-            lookback_publish(st, tile, prefix + agg);
-        }
-        if (lane == 0) s_prefix[w] = prefix;
-    }
-    __syncthreads();
-    uint32_t acarry = __shfl_sync(0xffffffffu, aex, 0) + (uint32_t)s_prefix[0];
-    uint64_t ccarry = __shfl_sync(0xffffffffu, cex, 0) + (uint64_t)s_prefix[1];
-#pragma unroll
-    for (int i = 0; i < kRunItems; ++i) {
-        const uint64_t cv = (uint64_t)a[i] * L[i];
-        const uint32_t ainc = warp_incl_scan(a[i]);
-        const uint64_t cinc = warp_incl_scan(cv);
-        const uint64_t p = seg + (uint64_t)i * 32 + lane;
-        const uint32_t wa = __shfl_sync(0xffffffffu, ainc, 31);   // the warp's anchors this round
-        if (wa) {
-            const uint32_t st = a[i] ? rstart[p] : 0u;
-            const uint32_t aex = ainc - a[i];
-            const uint64_t cex = ccarry + cinc - cv;
-            for (uint32_t t0 = 0; t0 < wa; t0 += 32) {
-                const uint32_t t = t0 + lane;
-                // j = the number of runs whose inclusive count is <= t: the run of entry t
-                uint32_t j = 0;
-#pragma unroll
-                for (uint32_t step = 16; step > 0; step >>= 1)
-                    if (__shfl_sync(0xffffffffu, ainc, j + step - 1) <= t) j += step;
-                const uint32_t jst = __shfl_sync(0xffffffffu, st, j);
-                const uint32_t jex = __shfl_sync(0xffffffffu, aex, j);
-                const uint32_t jL = __shfl_sync(0xffffffffu, L[i], j);
-                const uint64_t jcex = __shfl_sync(0xffffffffu, cex, j);
-                if (t < wa) {
-                    act_pos[acarry + t] = jst + (t - jex);
-                    act_run[acarry + t] = (uint32_t)(seg + (uint64_t)i * 32 + j);
-                    act_base[acarry + t] = jcex + (uint64_t)(t - jex) * jL;
-                }
-            }
-        }
-        acarry += wa;
-        ccarry += __shfl_sync(0xffffffffu, cinc, 31);
-    }
-    if (threadIdx.x == 0 && (uint64_t)(tile + 1) * kRunTile >= Rn) {
-        *act_total = (uint32_t)s_prefix[0] + atot;
-        *cap_total = (uint64_t)s_prefix[1] + ctot;
-    }
-}
-
 template <class Tin, class Tout>
 void scan_impl(const Tin* in, Tout* out, uint64_t n, cudaStream_t s, Tout* total_host, Tout* total_dev) {
     KScope ks("scan");
@@ -583,27 +473,6 @@ void scan_partials_u64(uint64_t* partial, uint64_t m, cudaStream_t s, uint64_t* 
         COLO_CUDA(cudaMemcpyAsync(total_host, partial + m, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
         stream_wait(s);
     }
-}
-
-void run_scans(const uint32_t* rcnt, const uint32_t* run_L, const uint32_t* rstart, uint32_t* act_pos,
-               uint32_t* act_run, uint64_t* act_base, uint64_t Rn, cudaStream_t s, uint32_t* act_total,
-               uint64_t* cap_total) {
-    KScope ks("scan");
-    const uint64_t tiles = Rn ? (Rn + kRunTile - 1) / kRunTile : 0;
-    if (tiles >= (1ull << 31)) throw StatusError{COLO_ERR_CAPACITY, "scan supports < 2^31 tiles"};
-    DevBuf<unsigned long long> st;   // two status words per tile, then the tile counter
-    st.alloc(2 * tiles + 1, s);
-    st.zero(s);
-    if (!tiles) {
-        COLO_CUDA(cudaMemsetAsync(act_total, 0, 4, s));
-        COLO_CUDA(cudaMemsetAsync(cap_total, 0, 8, s));
-        return;
-    }
-    k_run_scans<<<(unsigned)tiles, kScanThreads, 0, s>>>(Rn, rcnt, run_L, rstart, act_pos, act_run, act_base, st.get(),
-                                                          reinterpret_cast<uint32_t*>(st.get() + 2 * tiles), act_total,
-                                                          cap_total);
-    COLO_LAUNCH_CHECK();
-    count_launch();
 }
 
 void scan_u32_to_u64(const uint32_t* in, uint64_t* out, uint64_t n, cudaStream_t s,

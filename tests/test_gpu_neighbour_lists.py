@@ -1,0 +1,49 @@
+"""The one-pass neighbourhood lists at the edges of their paths: cells whose anchors are listed by one
+thread (up to 32) or by the whole warp, lists merged by one thread (up to 64 entries) or by the warp, and
+more entries than the first allocation holds (four a run plus 65,536), which builds the lists again.  The
+neighbour lists equal the oracle's exactly."""
+import numpy as np
+import pytest
+
+import colo
+import oracle
+from helpers import resolve_ambiguous
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(x, y, fid, bounds, R):
+    ctx = colo.Context(0)
+    ds = colo.Dataset.from_arrays(ctx, x, y, fid, bounds)
+    offs, nbr = ctx.stage_neighbors(ds, R)
+    res = resolve_ambiguous(ctx, x, y, fid, R)
+    o_offs, o_nbr, unres = oracle.neighbors(x, y, fid, bounds, R, res=res)
+    assert unres == 0
+    assert np.array_equal(offs, o_offs)
+    assert np.array_equal(nbr, o_nbr)
+    assert nbr.size > 0
+
+
+@pytest.mark.parametrize("per", [1, 15, 16, 17, 40])
+@pytest.mark.parametrize("cells", [1, 31, 33])
+def test_anchors_per_cell(per, cells):
+    """`cells` separate cells with `per` points of each of three features: 2 * per anchors a cell."""
+    rng = np.random.default_rng(per * 100 + cells)
+    x = np.concatenate([np.concatenate([30.0 * c + rng.uniform(0.0, 10.0, per) for c in range(cells)])
+                        for _ in range(3)]).astype(np.float32)
+    y = rng.uniform(0.0, 10.0, len(x)).astype(np.float32)
+    fid = np.repeat(np.arange(3, dtype=np.int32), per * cells)
+    _check(x, y, fid, np.array([0.0, 0.0, 30.0 * cells + 20.0, 40.0], np.float32), 10.0)
+
+
+@pytest.mark.parametrize("features,side", [(40, 45), (8, 20), (9, 20), (3, 330)])
+def test_list_lengths(features, side):
+    """Every cell of a side x side grid holds one point of every feature: nine times (features - 1) entries an
+    inner cell (63 and 72: both sides of the long-list limit).  40 features on 45 x 45 cells need more than four
+    entries a run; 330 x 330 cells are more than the grid's warps take one each."""
+    rng = np.random.default_rng(features)
+    gx, gy = np.meshgrid(np.arange(side), np.arange(side))
+    x = np.concatenate([(gx.ravel() + rng.uniform(0.01, 0.99, side * side)) * 10.0 for _ in range(features)])
+    y = np.concatenate([(gy.ravel() + rng.uniform(0.01, 0.99, side * side)) * 10.0 for _ in range(features)])
+    fid = np.repeat(np.arange(features, dtype=np.int32), side * side)
+    _check(x.astype(np.float32), y.astype(np.float32), fid, np.array([0, 0, 10 * side, 10 * side], np.float32), 10.0)
