@@ -15,6 +15,22 @@ struct JobHost {
     uint64_t p0 = 0, np = 0;     // point range
 };
 
+// A counter that many warps add to at once, on a 128-byte line of its own: atomics on one
+// address are taken one after another, those on different lines side by side.
+struct alignas(128) LineCounter {
+    unsigned long long v;
+};
+
+// Totals of a batch on the device: cleared before bucketing, filled by its
+// kernels, and read back once (settle).  dcnt, frun and ub2 follow it directly.
+struct alignas(128) BatchCtrl {
+    DevFlags flags;
+    uint32_t M, Rn;              // occupied cells, runs
+    uint32_t keys_done;          // blocks of the cell-key pass that have added their histograms
+    LineCounter nlistq;          // cells queued for a neighbourhood run list
+    LineCounter entries, anchors, capacity;   // of the lists; capacity of the single-pass layout = pair evaluations
+};
+
 struct Batch {
     cudaStream_t s = 0;
     int sms = 148;
@@ -24,35 +40,59 @@ struct Batch {
     uint32_t J = 0;              // jobs
     uint32_t W = 1;              // mask words per cell (max local feature count / 32)
     uint32_t Fmax_local = 0;
-    uint64_t M = 0;              // occupied cells
-    uint64_t Rn = 0;             // (cell, feature) runs
+    uint64_t M = 0;              // occupied cells (known after settle, or earlier when not bounded)
+    uint64_t Rn = 0;             // (cell, feature) runs (the same)
     uint64_t key_bits = 1;
+    // Sizes that bucketing finds are kept on the device, and arrays over cells, runs, list
+    // entries and neighbours are laid out for an upper bound (capM, capR, nrl_cap, nb_cap), so
+    // that everything up to the pairs' bounds is queued without a host wait.  Batches whose
+    // bounds are too large a reservation wait for the sizes instead (bounded = false).
+    bool bounded = true;
+    uint64_t capM = 0, capR = 0;
+    uint64_t device_bytes = 0;   // the device's memory
     // host copies of small arrays
     std::vector<JobHost> jobs;
     std::vector<uint32_t> h_fstart, h_fcount, h_fjob;
+    std::vector<uint64_t> h_job_off;    // pairs' bounds of job j start at h_job_off[j] (J + 1 entries)
     std::vector<uint32_t> h_frun_off;   // prefix of the number of runs (occupied cells) per feature
+    // one allocation: feature and job tables (uploaded with one copy), then the cleared words:
+    // the totals with the per-feature counts and the pairs' bounds, and the kernels' counters
+    DevBuf<unsigned char> mem0;
+    Span<uint32_t> fstart, fcount, fjob;
+    Span<JobGrid> grids;
+    Span<uint64_t> job_off;
+    Span<BatchCtrl> ctrl;        // followed by dcnt[F], frun[F], ub2[job_off[J]]
+    uint64_t ctrl_bytes = 0;     // of all four
+    Span<unsigned long long> dE; // neighbour entries, spread over counters
+    Span<unsigned long long> hist, head_status, sort_status;
+    Span<uint32_t> tickets;      // one per digit pass, then the head kernel's
+    RadixPlan plan{};
+    bool sort_shared = false;    // one pass's look-back words, cleared per pass
+    uint32_t* dcnt() const { return reinterpret_cast<uint32_t*>(ctrl.get() + 1); }
+    uint32_t* frun() const { return dcnt() + F; }
+    uint32_t* ub2() const { return frun() + F; }
+    DevFlags* flags() const { return &ctrl.get()->flags; }
     // points (by id)
     const float* x = nullptr;    // borrowed (dataset device copy)
     const float* y = nullptr;
-    DevBuf<uint32_t> fstart, fcount, fjob;
-    DevBuf<JobGrid> grids;
-    DevBuf<DevFlags> flags;
+    DevBuf<unsigned char> mem_points, mem_heads, mem_cells, mem_lists, mem_act, mem_nb;
+    Span<float2> xy;             // coordinates by id, packed (built by the cell-key pass)
     // bucketed (sorted by cell key, then id)
-    DevBuf<float2> xy;           // coordinates by id, packed (built by the cell-key pass)
-    DevBuf<uint32_t> sid, sfeat, scell;   // scell (cell of each sorted point) only when keep_scell
+    Span<uint32_t> sid, sfeat, scell;     // scell (cell of each sorted point) only when keep_scell
     bool keep_scell = false;              // colo_stage_cells reports each point's cell
-    DevBuf<float2> sxy;          // coordinates in cell-sorted order
+    Span<float2> sxy;            // coordinates in cell-sorted order
     // cells
-    DevBuf<uint64_t> ckey;
-    DevBuf<uint32_t> cstart, crun, cjob;
+    Span<uint64_t> ckey;
+    Span<uint32_t> cstart, crun, cjob;    // cstart, crun with an end entry
     uint64_t h2d_points = 0;     // bytes of point data copied to the device for this batch
     uint64_t rows = 0;           // grid rows of all jobs (row table size - 1)
-    DevBuf<uint32_t> rowstart;   // per grid row: first occupied cell at or after the row (empty when too large)
-    DevBuf<int32_t> nb9;
-    DevBuf<uint32_t> cmask;
-    DevBuf<uint32_t> nbmask;     // per cell: feature mask of its geometric 3x3 block
-    DevBuf<uint32_t> listq, nlistq;   // cells whose 3x3 block has a feature above their lowest own one
-    DevBuf<uint32_t> qmask;      // per cell: masks of the 4 quads containing it ([M][4][W])
+    bool row_table = false;
+    Span<uint32_t> rowstart;     // per grid row: first occupied cell at or after the row (unless too large)
+    Span<int32_t> nb9;
+    Span<uint32_t> cmask;
+    Span<uint32_t> nbmask;       // per cell: feature mask of its geometric 3x3 block
+    Span<uint32_t> listq;        // cells whose 3x3 block has a feature above their lowest own one
+    Span<uint32_t> qmask;        // per cell: masks of the 4 quads containing it ([M][4][W])
     // driver lists: for global feature f, the cells whose 3x3 block holds f
     // (nbmask bit), dlist[doff[f] .. doff[f+1]), in no particular order; the
     // level filters test exactly these cells for the candidates f drives
@@ -61,36 +101,34 @@ struct Batch {
     std::vector<uint64_t> h_dcnt;    // cells per feature's list (every feature)
     std::vector<uint64_t> h_doff;    // offsets of the lists filled (features in dlist_have; others empty)
     std::vector<uint8_t> dlist_have; // features whose lists are filled (by the level filters, on demand)
-    DevBuf<uint8_t> qfirst;      // per cell: bit q set when it is the first occupied cell of its quad q
-    // runs
-    DevBuf<uint32_t> rfeat, rstart, rcnt, rcell;
+    Span<uint8_t> qfirst;        // per cell: bit q set when it is the first occupied cell of its quad q
+    // runs: run r's points are sorted positions rstart[r] .. rstart[r+1] (rstart has an end entry)
+    Span<uint32_t> rfeat, rstart, rcell;
     // neighbourhood run lists: for each cell with targets, the runs of its
     // adjacent cells ordered by (feature, cell), entries above the cell's lowest
     // own feature, each the run's (first sorted position, point count); the
     // lists are in no particular order
-    DevBuf<uint2> nrl_ent;
-    uint64_t nrl_total = 0;
+    Span<uint2> nrl_ent;
+    uint64_t nrl_cap = 0, nrl_total = 0;
     // per own run of those cells: first entry of its cell's list with a higher
     // feature (absolute index), the entries from there to the list's end, and
     // the number of target points in them
-    DevBuf<uint64_t> run_sfx;
-    DevBuf<uint32_t> run_qn;
-    DevBuf<uint32_t> run_L;
+    Span<uint64_t> run_sfx;
+    Span<uint32_t> run_qn;
+    Span<uint32_t> run_L;
     // the join's anchors (points of runs with targets), in no particular order:
-    // act = (sorted position, entries qn, first entry sfx low and high word), and
-    // act_base = the anchor's start in the single-pass layout
-    DevBuf<uint4> act;
-    DevBuf<uint64_t> act_base;
+    // sorted position, start in the single-pass layout, first entry of the list
+    // slice (40 bits) and its entries (24 bits)
+    Span<uint4> act;
     // neighbour lists N+(a) = nb[nb_beg[a] .. nb_beg[a] + nb_cnt[a]), each in
     // (feature, neighbour cell, id) order; nb_beg[a] is set only where nb_cnt[a] > 0
-    DevBuf<uint64_t> nb_beg;
-    DevBuf<uint32_t> nb_cnt, nb;
+    Span<uint64_t> nb_beg;
+    Span<uint32_t> nb_cnt, nb;
     uint64_t E = 0;              // neighbour entries (UINT64_MAX: still on the device in dE)
-    DevBuf<unsigned long long> dE;
     uint64_t nb_cap = 0;         // allocated entries (upper bound in single-pass mode)
     uint64_t join_pairs = 0;     // pair distance evaluations
     uint64_t active_anchors = 0; // anchors whose cell has higher-feature neighbours
-    bool join_single = true;     // single pass into per-run upper-bound regions
+    bool lists_built = false, join_queued = false;
     int join_group = 8;          // lanes per anchor in the join (autotuned)
     int filter_unit = 32;        // candidates per warp unit in the level filter (autotuned: 8, 16, 32)
     int level_block = 256;       // threads per block of the level kernels (autotuned: 64, 128, 256)
@@ -100,10 +138,15 @@ struct Batch {
 };
 
 // colo_bucket.cu
-void bucket_points(Batch& b);            // cells, runs, masks, nb9, runs per feature
-void build_neighborhoods(Batch& b);      // NRL / NPL
+void bucket_layout(Batch& b, Carver& c); // the cleared words of mem0 that bucketing uses, after the upload
+void bucket_points(Batch& b);            // cells, runs, masks, nb9, runs per feature (launches; see bounded)
+void build_neighborhoods(Batch& b);      // neighbourhood lists and anchors (launches)
 // colo_join.cu
-void join_neighbors(Batch& b);           // neighbour CSR
+constexpr int kEntrySlots = 64, kEntryStride = 16;   // dE: counters on separate 128-byte lines
+constexpr uint64_t kSinglePassCap = 1ull << 30;      // largest single-pass layout (entries)
+void join_queue(Batch& b);               // single-pass join into nb_cap entries, skipped on the device when they
+                                         // or the lists did not fit (bounded batches, before settle)
+void join_neighbors(Batch& b);           // neighbour CSR (after settle)
 uint64_t neighbor_entries(Batch& b);     // E (waits for the device sum once)
 // Level-k candidates of every job from its prevalent (k-1)-patterns (km1
 // features each, lexicographic), with each candidate's prefix pattern index;
@@ -115,10 +158,10 @@ void apriori_device(cudaStream_t s, const std::vector<const std::vector<uint32_t
 // themselves are filled by the level filters for the drivers of their
 // candidates (a level whose drivers are not all filled yet fills the union of
 // the old and new ones).
-// Level-2 upper bounds of every pair of every job: ub2[job_off[j] + lf*Fj + lg] is the
-// bound of feature lf's side of pair {lf, lg}.  job_off has J+1 entries.
-// Runs on stream s (no wait at the end).
-void filter_pairs(Batch& b, DevBuf<uint32_t>& ub2, std::vector<uint64_t>& job_off, cudaStream_t s);
+// Level-2 upper bounds of every pair of every job into the batch's ub2:
+// ub2[job_off[j] + lf*Fj + lg] is the bound of feature lf's side of pair {lf, lg}
+// (launch only).
+void filter_pairs(Batch& b);
 // Level-k upper bounds for host candidates cand[c*k + j] (global features) of
 // jobs job[c]: d_ub[c*k + j] (zeroed by the caller).  d_stats (optional,
 // zeroed, 2 per candidate): full quads and cells of U_c.

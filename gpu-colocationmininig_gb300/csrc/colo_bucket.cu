@@ -7,24 +7,28 @@
 // kernel_CountCellFeatures (Codes/DeviceProcess_Kernel.h:629-647): instead of
 // dense totalCells x F count/start arrays, only occupied cells and runs are
 // stored, so grids of 10^10 cells cost nothing.
+#include <algorithm>
+
 #include "colo_batch.h"
 #include "colo_device.cuh"
 
 namespace colo {
 namespace {
 
-// Cell keys, packed coordinates and (vals non-null) point ids, and the digit
-// histograms of every radix pass over the keys (block-private counts added to
-// hist once per block), so the sort does not read the keys again to count
-// them.  When the sort runs a pass its first pass generates the ids itself.
-
+// Cell keys, packed coordinates, cleared neighbour counts and (vals non-null)
+// point ids, and the digit starts of every radix pass over the keys
+// (block-private counts added to hist once per block; the last block to finish
+// scans them in place), so the sort does not read the keys again to count
+// them.  When the sort runs a pass its first pass makes the ids itself.
 template <class KT>
 __global__ void __launch_bounds__(256) k_cell_keys(
     uint64_t n, const float* __restrict__ x, const float* __restrict__ y, uint32_t F,
     const uint32_t* __restrict__ fstart, const uint32_t* __restrict__ fjob, const JobGrid* __restrict__ grids,
-    KT* __restrict__ keys, uint32_t* __restrict__ vals, float2* __restrict__ xy, DevFlags* flags, RadixPlan plan,
-    unsigned long long* __restrict__ hist) {
+    KT* __restrict__ keys, uint32_t* __restrict__ vals, float2* __restrict__ xy, uint32_t* __restrict__ nb_cnt,
+    BatchCtrl* __restrict__ ctrl, RadixPlan plan, unsigned long long* __restrict__ hist) {
+    static_assert(kRadixDigits == 256, "one digit a thread in the scan");
     __shared__ uint32_t h[kRadixMaxPasses * kRadixDigits];
+    __shared__ bool s_last;
     for (int i = threadIdx.x; i < plan.n * kRadixDigits; i += blockDim.x) h[i] = 0;
     __syncthreads();
     // each block takes one contiguous range of points (coalesced, and a
@@ -42,9 +46,10 @@ __global__ void __launch_bounds__(256) k_cell_keys(
         const JobGrid g = grids[fjob[f]];
         const float xi = x[i], yi = y[i];
         xy[i] = make_float2(xi, yi);
+        nb_cnt[i] = 0;
         uint64_t c = ref_cell(g, xi, yi);
         if (c >= g.total) {
-            atomicAdd(&flags->out_of_grid, 1u);
+            atomicAdd(&ctrl->flags.out_of_grid, 1u);
             c = g.total - 1;
         }
         const KT key = (KT)(g.key_base + c);
@@ -58,191 +63,211 @@ __global__ void __launch_bounds__(256) k_cell_keys(
         const uint32_t v = h[i];
         if (v) atomicAdd(&hist[i], (unsigned long long)v);
     }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&ctrl->keys_done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int p = 0; p < plan.n; ++p) {
+        unsigned long long* hp = hist + p * kRadixDigits + threadIdx.x;
+        unsigned long long tot;
+        const unsigned long long v = __ldcg(hp);
+        *hp = block_excl_scan<unsigned long long>(v, &tot);
+    }
 }
 
-// Cell and run heads in the sorted order, counted and compacted in two
-// passes over the keys (no flag arrays).  A 2048-point tile is eight warp
-// segments of 256 points; a warp reads its segment 32 consecutive points at a
-// time (coalesced) and ranks heads with ballots.  Pass 1 stores per tile the
-// number of cell heads (high 32 bits) and run heads (low 32 bits); pass 2
-// writes each point's cell and the head arrays at the tile's scanned base.
+// Sorted copies, cells and runs in one pass over the sorted keys.  A block
+// takes a 2048-point tile (eight warp segments of 256 points, 32 consecutive
+// points at a time): per point its coordinates (one 8-byte gather) and its
+// feature (from the feature start table, points being grouped by feature; it
+// stays in L1); a cell starts where the key changes, a run where the key or
+// the feature does (a point's predecessor comes from the lane before it, lane 0
+// reads it).  The tile's head counts go through a decoupled look-back (warp 0
+// for cells, warp 1 for runs), and the heads are written at the offsets found,
+// as far as the arrays reach (capM, capR: a launch with no room counts them).
+// The last tile records the totals and the end entries.
+//
+// Bound by the gather (an 8-byte load by a sorted id moves a whole DRAM
+// sector).  One kernel instead of four (gather and count, scan of the tile
+// counts, compaction, run lengths): the tile's keys and features are read once,
+// and no host wait is needed for the totals (20M points: 0.50 ms against 0.32 + 0.21; a few
+// thousand points: 14 us against 64 us with the wait).
+//
+// After a sort that timed out the keys are not a sorted permutation: nothing
+// is written, the totals stay zero and every later kernel finds no cells.  A
+// look-back that waits too long counts the heads before its tile itself.
 constexpr int kHeadThreads = 256, kHeadRounds = 8, kHeadTile = kHeadThreads * kHeadRounds;
 constexpr int kHeadWarps = kHeadThreads / 32;
 
 template <class KT>
-__device__ __forceinline__ void head_flags(uint64_t p, uint64_t n, const KT* __restrict__ keys,
-                                           const uint32_t* __restrict__ sfeat, bool& ch, bool& rh) {
-    ch = rh = false;
-    if (p >= n) return;
-    ch = p == 0 || keys[p - 1] != keys[p];
-    rh = ch || sfeat[p - 1] != sfeat[p];
-}
-
-// Ballots of the cell and run heads of the calling warp's segment.
-template <class KT>
-__device__ __forceinline__ void head_ballots(uint64_t seg, uint64_t n, const KT* __restrict__ keys,
-                                             const uint32_t* __restrict__ sfeat, int lane,
-                                             uint32_t (&chb)[kHeadRounds], uint32_t (&rhb)[kHeadRounds]) {
-#pragma unroll
-    for (int r = 0; r < kHeadRounds; ++r) {
-        bool ch, rh;
-        head_flags(seg + (uint64_t)r * 32 + lane, n, keys, sfeat, ch, rh);
-        chb[r] = __ballot_sync(0xffffffffu, ch);
-        rhb[r] = __ballot_sync(0xffffffffu, rh);
-    }
-}
-
-// Sorted copies and pass 1 of the heads in one pass: per point its
-// coordinates (one 8-byte gather) and feature (from the feature start table,
-// points being grouped by feature; it stays in L1), and per tile the cell
-// and run head counts.  A point's predecessor comes from the lane before it
-// (lane 0 reads it).  An id outside the points (only after a sort that timed
-// out; the host then stops the mine) reads point 0.
-template <class KT>
-__global__ void __launch_bounds__(kHeadThreads, 8) k_gather_heads(uint64_t n, uint32_t F, const KT* __restrict__ keys,
-                                                              const uint32_t* __restrict__ sid,
-                                                              const float2* __restrict__ xy,
-                                                              const uint32_t* __restrict__ fstart,
-                                                              float2* __restrict__ sxy, uint32_t* __restrict__ sfeat,
-                                                              uint64_t* __restrict__ partial) {
-    __shared__ uint64_t s_tot[kHeadWarps];
+__global__ void __launch_bounds__(kHeadThreads, 6) k_heads(
+    uint64_t n, uint32_t F, const KT* __restrict__ keys, const uint32_t* __restrict__ sid,
+    const float2* __restrict__ xy, const uint32_t* __restrict__ fstart, const uint32_t* __restrict__ fjob,
+    float2* __restrict__ sxy, uint32_t* __restrict__ sfeat, uint64_t* __restrict__ ckey, uint32_t* __restrict__ cstart,
+    uint32_t* __restrict__ crun, uint32_t* __restrict__ cjob, uint32_t* __restrict__ rfeat,
+    uint32_t* __restrict__ rstart, uint32_t* __restrict__ rcell, uint32_t* __restrict__ scell, uint64_t capM,
+    uint64_t capR, unsigned long long* __restrict__ status, uint32_t* __restrict__ ticket,
+    BatchCtrl* __restrict__ ctrl) {
+    __shared__ uint32_t s_tile, s_heads[2][kHeadWarps];
+    __shared__ unsigned long long s_prefix[2];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint64_t seg = (uint64_t)blockIdx.x * kHeadTile + (uint64_t)w * (32 * kHeadRounds);
-    uint64_t v = 0;
+    if (threadIdx.x == 0) s_tile = ctrl->flags.timeout ? 0xffffffffu : atomicAdd(ticket, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    if (tile == 0xffffffffu) return;
+    const uint64_t seg = (uint64_t)tile * kHeadTile + (uint64_t)w * (32 * kHeadRounds);
+    KT key[kHeadRounds];
+    uint32_t f[kHeadRounds], chm = 0, rhm = 0;   // the lane's own head bits, one a round
+    uint32_t cc = 0, rc = 0;
 #pragma unroll
     for (int r = 0; r < kHeadRounds; ++r) {
         const uint64_t p = seg + (uint64_t)r * 32 + lane;
         const bool in = p < n;
-        KT key = 0;
-        uint32_t f = 0;
+        key[r] = 0;
+        f[r] = 0;
         if (in) {
-            uint32_t id = sid[p];
-            if (id >= n) id = 0;
+            const uint32_t id = sid[p];
             sxy[p] = xy[id];
-            f = feature_of(id, F, fstart);
-            sfeat[p] = f;
-            key = keys[p];
+            f[r] = feature_of(id, F, fstart);
+            sfeat[p] = f[r];
+            key[r] = keys[p];
         }
-        KT pkey = __shfl_up_sync(0xffffffffu, key, 1);
-        uint32_t pf = __shfl_up_sync(0xffffffffu, f, 1);
+        KT pkey = __shfl_up_sync(0xffffffffu, key[r], 1);
+        uint32_t pf = __shfl_up_sync(0xffffffffu, f[r], 1);
         if (lane == 0 && in && p > 0) {
-            uint32_t pid = sid[p - 1];
-            if (pid >= n) pid = 0;
             pkey = keys[p - 1];
-            pf = feature_of(pid, F, fstart);
+            pf = feature_of(sid[p - 1], F, fstart);
         }
-        const bool ch = in && (p == 0 || pkey != key);
-        const bool rh = ch || (in && pf != f);
-        v += ((uint64_t)__popc(__ballot_sync(0xffffffffu, ch)) << 32) + (uint64_t)__popc(__ballot_sync(0xffffffffu, rh));
+        const bool ch = in && (p == 0 || pkey != key[r]);
+        const bool rh = ch || (in && pf != f[r]);
+        chm |= (ch ? 1u : 0u) << r;
+        rhm |= (rh ? 1u : 0u) << r;
+        cc += __popc(__ballot_sync(0xffffffffu, ch));
+        rc += __popc(__ballot_sync(0xffffffffu, rh));
     }
-    if (lane == 0) s_tot[w] = v;
+    if (lane == 0) {
+        s_heads[0][w] = cc;
+        s_heads[1][w] = rc;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint64_t t = 0;
-        for (int i = 0; i < kHeadWarps; ++i) t += s_tot[i];
-        partial[blockIdx.x] = t;
-    }
-}
-
-template <class KT>
-__global__ void __launch_bounds__(kHeadThreads, 8) k_head_compact(
-    uint64_t n, const KT* __restrict__ keys, const uint32_t* __restrict__ sfeat, const uint32_t* __restrict__ fjob,
-    const uint64_t* __restrict__ partial, uint64_t* __restrict__ ckey, uint32_t* __restrict__ cstart,
-    uint32_t* __restrict__ crun, uint32_t* __restrict__ cjob, uint32_t* __restrict__ rfeat,
-    uint32_t* __restrict__ rstart, uint32_t* __restrict__ rcell, uint32_t* __restrict__ scell) {
-    __shared__ uint64_t s_tot[kHeadWarps];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint64_t seg = (uint64_t)blockIdx.x * kHeadTile + (uint64_t)w * (32 * kHeadRounds);
-    uint32_t chb[kHeadRounds], rhb[kHeadRounds];
-    head_ballots(seg, n, keys, sfeat, lane, chb, rhb);
-    uint64_t v = 0;
+    if (w < 2) {
+        uint32_t agg = 0;
+        for (int i = 0; i < kHeadWarps; ++i) agg += s_heads[w][i];
+        unsigned long long* st = status + (w == 0 ? 0 : gridDim.x);
+        unsigned long long prefix;
+        if (!warp_lookback(st, tile, agg, prefix)) {   // the heads before this tile, counted here
+            unsigned long long add = 0;
+            for (uint64_t p = lane; p < (uint64_t)tile * kHeadTile; p += 32) {
+                const bool ch = p == 0 || keys[p - 1] != keys[p];
+                add += ch || (w == 1 && feature_of(sid[p - 1], F, fstart) != feature_of(sid[p], F, fstart));
+            }
 #pragma unroll
-    for (int r = 0; r < kHeadRounds; ++r) v += ((uint64_t)__popc(chb[r]) << 32) + (uint64_t)__popc(rhb[r]);
-    if (lane == 0) s_tot[w] = v;
+            for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+            prefix = add;
+            lookback_publish(st, tile, prefix + agg);
+        }
+        if (lane == 0) s_prefix[w] = prefix;
+    }
     __syncthreads();
-    uint64_t ex = partial[blockIdx.x];
-    for (int i = 0; i < w; ++i) ex += s_tot[i];
-    uint32_t cb = (uint32_t)(ex >> 32), rb = (uint32_t)ex;   // heads before this round
+    uint32_t cb = (uint32_t)s_prefix[0], rb = (uint32_t)s_prefix[1];   // heads before this round
+    for (int i = 0; i < w; ++i) {
+        cb += s_heads[0][i];
+        rb += s_heads[1][i];
+    }
     const uint32_t lt = (1u << lane) - 1u;
 #pragma unroll
     for (int r = 0; r < kHeadRounds; ++r) {
         const uint64_t p = seg + (uint64_t)r * 32 + lane;
-        const bool ch = chb[r] >> lane & 1u, rh = rhb[r] >> lane & 1u;
-        const uint32_t c = cb + __popc(chb[r] & lt) + (ch ? 1u : 0u) - 1u;   // the cell of p
-        const uint32_t ri = rb + __popc(rhb[r] & lt);
-        if (p < n) {
-            if (scell) scell[p] = c;
-            if (ch) {
-                ckey[c] = keys[p];
-                cstart[c] = (uint32_t)p;
-                crun[c] = ri;
-                cjob[c] = fjob[sfeat[p]];
-            }
-            if (rh) {
-                rfeat[ri] = sfeat[p];
-                rstart[ri] = (uint32_t)p;
-                rcell[ri] = c;
-            }
+        const bool ch = chm >> r & 1u, rh = rhm >> r & 1u;
+        const uint32_t chb = __ballot_sync(0xffffffffu, ch), rhb = __ballot_sync(0xffffffffu, rh);
+        const uint32_t c = cb + __popc(chb & lt) + (ch ? 1u : 0u) - 1u;   // the cell of p
+        const uint32_t ri = rb + __popc(rhb & lt);
+        if (scell && p < n) scell[p] = c;
+        if (ch && c < capM) {
+            ckey[c] = key[r];
+            cstart[c] = (uint32_t)p;
+            crun[c] = ri;
+            cjob[c] = fjob[f[r]];
         }
-        cb += __popc(chb[r]);
-        rb += __popc(rhb[r]);
+        if (rh && ri < capR) {
+            rfeat[ri] = f[r];
+            rstart[ri] = (uint32_t)p;
+            rcell[ri] = c;
+        }
+        cb += __popc(chb);
+        rb += __popc(rhb);
     }
-}
-
-__global__ void k_run_tail(uint64_t Rn, uint64_t M, uint64_t n, const uint32_t* __restrict__ rstart,
-                           uint32_t* __restrict__ rcnt, uint32_t* __restrict__ cstart,
-                           uint32_t* __restrict__ crun) {
-    uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < Rn) rcnt[r] = (r + 1 < Rn ? rstart[r + 1] : (uint32_t)n) - rstart[r];
-    if (r == 0) {
-        cstart[M] = (uint32_t)n;
-        crun[M] = (uint32_t)Rn;
+    // the warp of the last point ends with every head counted
+    if (lane == 0 && seg < n && n - seg <= 32 * kHeadRounds) {
+        ctrl->M = cb;
+        ctrl->Rn = rb;
+        if (cb <= capM && rb <= capR) {
+            cstart[cb] = (uint32_t)n;
+            crun[cb] = rb;
+            rstart[rb] = (uint32_t)n;
+        }
     }
 }
 
 // Per cell its feature mask (bit lf of word lf / 32 for each of its runs' local
 // features): a thread walks the cell's runs, which ascend by feature, and writes
-// every word of the row (no clearing pass, no atomics).
-__global__ void k_cell_masks(uint64_t M, const uint32_t* __restrict__ crun, const uint32_t* __restrict__ rfeat,
-                             const uint32_t* __restrict__ cjob, const JobGrid* __restrict__ grids, uint32_t W,
-                             uint32_t* __restrict__ cmask) {
-    const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= M) return;
-    const uint32_t f0 = grids[cjob[c]].f0;
-    uint32_t r = crun[c];
-    const uint32_t r1 = crun[c + 1];
-    uint32_t* row = cmask + c * W;
-    for (uint32_t w = 0; w < W; ++w) {
-        uint32_t bits = 0;
-        for (; r < r1; ++r) {
-            const uint32_t lf = rfeat[r] - f0;
-            if ((lf >> 5) != w) break;
-            bits |= 1u << (lf & 31);
-        }
-        row[w] = bits;
-    }
-}
+// every word of the row (no clearing pass, no atomics).  The row table comes
+// with it (rows > 0): rowstart[Y] = first occupied cell whose key is at or after
+// the first key of grid row Y (rows of all jobs, job j's row y at Y = row_base_j
+// + y), rowstart[rows] = M.  The runs per feature (frun) are counted in the same walk, in a
+// block histogram when the features fit (a kernel of its own over the runs, with its copies and
+// its wait, took 72 us on the 20M workload).
+constexpr uint32_t kRunHist = 8192;
 
-// rowstart[Y] = first occupied cell whose key is at or after the first key of
-// grid row Y (rows of all jobs, job j's row y at Y = row_base_j + y);
-// rowstart[rows] = M.
-__global__ void k_row_starts(uint64_t rows, uint32_t J, uint64_t M, const uint64_t* __restrict__ ckey,
-                             const JobGrid* __restrict__ grids, uint32_t* __restrict__ rowstart) {
-    const uint64_t Y = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (Y > rows) return;
-    if (Y == rows) {
-        rowstart[Y] = (uint32_t)M;
-        return;
+__global__ void k_cell_masks(const BatchCtrl* __restrict__ ctrl, const uint64_t* __restrict__ ckey,
+                             const uint32_t* __restrict__ crun, const uint32_t* __restrict__ rfeat,
+                             const uint32_t* __restrict__ cjob, const JobGrid* __restrict__ grids, uint32_t W,
+                             uint32_t* __restrict__ cmask, uint64_t rows, uint32_t J, uint32_t* __restrict__ rowstart,
+                             uint32_t F, uint32_t* __restrict__ frun) {
+    extern __shared__ uint32_t s_run[];   // F counters (F <= kRunHist)
+    const bool local = F <= kRunHist;
+    const uint64_t M = ctrl->M;
+    if (local)
+        for (uint32_t i = threadIdx.x; i < F; i += blockDim.x) s_run[i] = 0;
+    __syncthreads();
+    const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t c = t0; c < M; c += step) {
+        const uint32_t f0 = grids[cjob[c]].f0;
+        uint32_t r = crun[c];
+        const uint32_t r1 = crun[c + 1];
+        uint32_t* row = cmask + c * W;
+        for (uint32_t w = 0; w < W; ++w) {
+            uint32_t bits = 0;
+            for (; r < r1; ++r) {
+                const uint32_t f = rfeat[r], lf = f - f0;
+                if ((lf >> 5) != w) break;
+                bits |= 1u << (lf & 31);
+                atomicAdd(local ? &s_run[f] : &frun[f], 1u);
+            }
+            row[w] = bits;
+        }
     }
-    uint32_t lo = 0, hi = J;   // last job whose first row is <= Y
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (grids[mid].row_base <= Y) lo = mid;
-        else hi = mid;
+    __syncthreads();
+    if (local)
+        for (uint32_t i = threadIdx.x; i < F; i += blockDim.x)
+            if (s_run[i]) atomicAdd(&frun[i], s_run[i]);
+    if (!rows) return;
+    for (uint64_t Y = t0; Y <= rows; Y += step) {
+        if (Y == rows) {
+            rowstart[Y] = (uint32_t)M;
+            break;
+        }
+        uint32_t lo = 0, hi = J;   // last job whose first row is <= Y
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (grids[mid].row_base <= Y) lo = mid;
+            else hi = mid;
+        }
+        const JobGrid g = grids[lo];
+        const uint64_t key = g.key_base + (Y - g.row_base) * g.gx;
+        rowstart[Y] = (uint32_t)lower_bound_dev(ckey, (uint64_t)0, M, key);
     }
-    const JobGrid g = grids[lo];
-    const uint64_t key = g.key_base + (Y - g.row_base) * g.gx;
-    rowstart[Y] = (uint32_t)lower_bound_dev(ckey, (uint64_t)0, M, key);
 }
 
 // nb9[c*9 + (dy+1)*3 + (dx+1)] = occupied index of the geometric neighbour
@@ -257,11 +282,12 @@ __global__ void k_row_starts(uint64_t rows, uint32_t J, uint64_t M, const uint64
 // 0 <= by <= gy-2 are never full and get no bit.
 // rowstart (optional, rows + 1 entries) bounds the search of a row to the
 // cells of that row.
-__global__ void __launch_bounds__(128, 16) k_nb9(uint64_t M, const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob,
+__global__ void __launch_bounds__(128, 16) k_nb9(const BatchCtrl* __restrict__ ctrl,
+                      const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob,
                       const JobGrid* __restrict__ grids, const uint32_t* __restrict__ rowstart,
                       int32_t* __restrict__ nb9, uint8_t* __restrict__ qfirst) {
-    uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= M) return;
+    const uint64_t M = ctrl->M;
+    for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < M; c += (uint64_t)gridDim.x * blockDim.x) {
     const JobGrid g = grids[cjob[c]];
     const uint64_t key = ckey[c];
     uint64_t ucx, ucy;
@@ -321,6 +347,7 @@ __global__ void __launch_bounds__(128, 16) k_nb9(uint64_t M, const uint64_t* __r
         if (first) qf |= 1u << q;
     }
     qfirst[c] = (uint8_t)qf;
+    }   // cells
 }
 
 // Per cell: the feature masks of the four quads (2x2 cell blocks) containing
@@ -368,26 +395,40 @@ constexpr uint32_t kQuadHist = 1024;
 
 // Per cell: the four quad masks and the 3x3 mask (nbmask), the queue of cells
 // that need a neighbourhood run list, and the driver-list sizes: dcnt[f] =
-// cells whose 3x3 mask holds f.  A block walks 128 cells at a time over a
-// strided range and keeps one histogram for all of them (one global atomic per
+// cells whose 3x3 mask holds f.  A block walks spans of consecutive cells (so that
+// queued cells stay near each other: the list kernel reads their neighbourhoods)
+// and keeps one histogram for all of them (one global atomic per
 // feature per block at the end); a warp's 32 cells are counted by a bit
 // transpose (lane b holds feature b's column of the warp's cell x feature
-// matrix and adds its popcount).
+// matrix and adds its popcount).  Cells for the list queue collect in a small
+// buffer of their warp, which is written out 32 at a time (one global atomic per
+// 32 queued cells and no block barrier; an atomic and three barriers per 128
+// cells made every warp wait for the atomic's round trip: 0.29 ms became 0.26 ms,
+// 20M points).
 template <int WT>
 __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
-    uint64_t M, const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob,
+    BatchCtrl* __restrict__ ctrl, const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob,
     const JobGrid* __restrict__ grids, const int32_t* __restrict__ nb9, const uint32_t* __restrict__ cmask,
-    uint32_t* __restrict__ qmask, uint32_t* __restrict__ nbmask, uint32_t* __restrict__ listq,
-    uint32_t* __restrict__ nlistq, uint32_t F, uint32_t* __restrict__ dcnt) {
+    uint32_t* __restrict__ qmask, uint32_t* __restrict__ nbmask, uint32_t* __restrict__ listq, uint32_t F,
+    uint32_t* __restrict__ dcnt) {
+    const uint64_t M = ctrl->M;
     __shared__ uint32_t s_hist[kQuadHist];
-    __shared__ uint32_t s_cnt[kQuadThreads / 32], s_base;
+    __shared__ uint32_t s_queue[kQuadThreads / 32][64];
     const bool local_hist = F <= kQuadHist;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (local_hist)
         for (uint32_t i = threadIdx.x; i < F; i += blockDim.x) s_hist[i] = 0;
     __syncthreads();
-    for (uint64_t c0 = (uint64_t)blockIdx.x * kQuadThreads; c0 < M; c0 += (uint64_t)gridDim.x * kQuadThreads) {
-        const uint64_t c = c0 + threadIdx.x;
+    uint32_t* queue = s_queue[wid];
+    uint32_t queued = 0;   // cells in the warp's buffer (below 32 between rounds)
+    // A warp takes 128 consecutive cells, 32 at a time, next to the block's other warps (32 when
+    // there are too few for every block): its queued cells stay together, and blocks that run at
+    // the same time read neighbouring rows (one far-apart range per block: 297 us, 20M points).
+    const uint32_t rounds = M >= (uint64_t)gridDim.x * (4 * kQuadThreads) ? 4u : 1u;
+    const uint64_t span = (uint64_t)rounds * kQuadThreads;
+    for (uint64_t q0 = (uint64_t)blockIdx.x * span; q0 < M; q0 += (uint64_t)gridDim.x * span)
+    for (uint32_t round = 0; round < rounds; ++round) {
+        const uint64_t c = q0 + ((uint64_t)wid * rounds + round) * 32 + lane;
         bool above = false;
         uint32_t all[WT];
 #pragma unroll
@@ -453,9 +494,9 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
 #pragma unroll
                 for (int w = 0; w < WT; ++w) {
                     if (!__any_sync(0xffffffffu, all[w])) continue;
+                    const uint32_t f = fl + (uint32_t)w * 32 + (uint32_t)lane;
                     const uint32_t n = __popc(warp_transpose32(all[w]));
                     if (n) {
-                        const uint32_t f = fl + (uint32_t)w * 32 + (uint32_t)lane;
                         if (local_hist) atomicAdd(&s_hist[f], n);
                         else atomicAdd(&dcnt[f], n);
                     }
@@ -467,47 +508,32 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
                         atomicAdd(&dcnt[f0 + (uint32_t)w * 32 + (uint32_t)(__ffs(bits) - 1)], 1u);
             }
         }
-        // one atomic per block and round for the queue
         const uint32_t has = __ballot_sync(0xffffffffu, above);
-        if (lane == 0) s_cnt[wid] = (uint32_t)__popc(has);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t t = 0;
-            for (int w = 0; w < kQuadThreads / 32; ++w) {
-                const uint32_t v = s_cnt[w];
-                s_cnt[w] = t;
-                t += v;
-            }
-            s_base = t ? atomicAdd(nlistq, t) : 0u;
+        if (above) queue[queued + __popc(has & ((1u << lane) - 1u))] = (uint32_t)c;
+        queued += __popc(has);
+        if (queued >= 32) {
+            __syncwarp();
+            unsigned long long at = 0;
+            if (lane == 0) at = atomicAdd(&ctrl->nlistq.v, 32ull);
+            listq[__shfl_sync(0xffffffffu, at, 0) + lane] = queue[lane];
+            queued -= 32;
+            const uint32_t rest = (uint32_t)lane < queued ? queue[32 + lane] : 0u;
+            __syncwarp();
+            if ((uint32_t)lane < queued) queue[lane] = rest;
         }
-        __syncthreads();
-        if (above) listq[s_base + s_cnt[wid] + __popc(has & ((1u << lane) - 1u))] = (uint32_t)c;
-        __syncthreads();   // s_cnt and s_base are rewritten by the next round
+        __syncwarp();
+    }
+    if (queued) {
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(&ctrl->nlistq.v, (unsigned long long)queued);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if ((uint32_t)lane < queued) listq[at + lane] = queue[lane];
     }
     if (local_hist) {
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < F; i += blockDim.x)
             if (s_hist[i]) atomicAdd(&dcnt[i], s_hist[i]);
     }
-}
-
-// Runs per feature: a block-local histogram (F <= kHistMax), else global atomics.
-constexpr uint32_t kHistMax = 12288;
-
-__global__ void k_feature_runs(uint64_t Rn, uint32_t F, const uint32_t* __restrict__ rfeat, uint32_t* __restrict__ cnt) {
-    extern __shared__ uint32_t h[];
-    const bool local = F <= kHistMax;
-    if (local)
-        for (uint32_t i = threadIdx.x; i < F; i += blockDim.x) h[i] = 0;
-    __syncthreads();
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < Rn; r += (uint64_t)gridDim.x * blockDim.x) {
-        if (local) atomicAdd(&h[rfeat[r]], 1u);
-        else atomicAdd(&cnt[rfeat[r]], 1u);
-    }
-    __syncthreads();
-    if (local)
-        for (uint32_t i = threadIdx.x; i < F; i += blockDim.x)
-            if (h[i]) atomicAdd(&cnt[i], h[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -543,7 +569,7 @@ __device__ __forceinline__ int adjacent_cells(uint64_t c, const uint64_t* ckey, 
 // Most lists are then empty; the cells whose 3x3 mask allows one were queued
 // by k_quad_masks.
 
-constexpr uint32_t kBigList = 64;        // cells with longer lists are merged by their whole warp
+constexpr uint32_t kBigList = 128;       // cells with longer lists are merged by their whole warp
 constexpr uint32_t kHeavyAnchors = 32;   // cells with more anchors are listed by their whole warp
 
 // The list of cell c by a whole warp.  In the full (feature, slot) order a run
@@ -559,8 +585,8 @@ __device__ __forceinline__ void nrl_cell_warp(uint64_t c, int l, uint64_t first,
                                               const JobGrid* __restrict__ grids, const int32_t* __restrict__ nb9,
                                               const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ crun,
                                               const uint32_t* __restrict__ rfeat, const uint32_t* __restrict__ rstart,
-                                              const uint32_t* __restrict__ rcnt, uint2* __restrict__ nrl_ent,
-                                              uint64_t* run_sfx, uint32_t* run_qn, uint32_t* run_L) {
+                                              uint2* __restrict__ nrl_ent, uint64_t* run_sfx,
+                                              uint32_t* run_qn, uint32_t* run_L) {
     int32_t adj[9];
     const int na = adjacent_cells(c, ckey, cjob, grids, nb9, adj);
     const uint32_t fmin = rfeat[crun[c]];
@@ -599,7 +625,7 @@ __device__ __forceinline__ void nrl_cell_warp(uint64_t c, int l, uint64_t first,
                 if (t < sl && lb < q1[t] && rfeat[lb] == f) pos += 1;
             }
         }
-        nrl_ent[base + pos] = make_uint2(rstart[r], rcnt[r]);
+        nrl_ent[base + pos] = make_uint2(rstart[r], rstart[r + 1] - rstart[r]);
     }
     for (uint32_t r = crun[c] + l; r < crun[c + 1]; r += 32) {
         const uint32_t f = rfeat[r];
@@ -625,39 +651,41 @@ __device__ __forceinline__ void nrl_cell_warp(uint64_t c, int l, uint64_t first,
 // ascending by feature).  The running point count P gives the suffix counts:
 // the cell's own run of feature f gets sfx = the first position after every
 // entry of feature <= f and L = (points in the list) - P(sfx).  Then every
-// point of an own run with targets (L > 0) is listed as an anchor: act =
-// (sorted position, list entries qn, first entry sfx) and act_base, its start
-// in the single-pass layout, where it owns L entries.
+// point of an own run with targets (L > 0) is listed as an anchor with its
+// sorted position, its start in the single-pass layout, where it owns L entries
+// (32 bits: a layout of more than 2^30 entries is not used), and its list slice
+// (first entry sfx, entries qn), in one 16-byte word.
 //
 // Bound by the merge's chain of dependent loads.  The lists, anchors and
 // capacities are not in cell order: a warp reserves its 32 cells' room with one
-// atomic on each of the three totals (tot: list entries, anchors, capacity), so
+// atomic on each of the three totals (list entries, anchors, capacity), so
 // nothing is counted or scanned over the cells and runs beforehand (the order
 // within a list is all that a result depends on).  This replaces a count
 // kernel, a scan over the cells, the list fill, a second kernel for long lists
 // and a scan over the runs, with a clear of two arrays: 413 us of kernels (64 count, 149 fill, 200
-// scans) became 164 us on the 20M workload, one host wait fewer; the 200,000-point dense one, whose
-// few long lists share a neighbourhood, 327 became 137 us.
-// Lists past `cap` entries are not written; the host sees it in tot[0] and runs
+// scans) became 154 us on the 20M workload; the 200,000-point dense one, whose few long lists
+// share a neighbourhood, 327 became 135 us.  Eight blocks an SM (64 registers) hide more of the
+// chain than the six that the compiler's choice of registers left: 172 us at 20M points.
+// Lists past `cap` entries are not written; the host sees it in the total and runs
 // the kernel again with room for all.
-__global__ void __launch_bounds__(128) k_neighbour_lists(
-    const uint32_t* __restrict__ listq, const uint32_t* __restrict__ nlistq, const uint64_t* __restrict__ ckey,
+__global__ void __launch_bounds__(128, 8) k_neighbour_lists(
+    const uint32_t* __restrict__ listq, BatchCtrl* __restrict__ ctrl, const uint64_t* __restrict__ ckey,
     const uint32_t* __restrict__ cjob, const JobGrid* __restrict__ grids, const int32_t* __restrict__ nb9,
     const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ crun, const uint32_t* __restrict__ rfeat,
-    const uint32_t* __restrict__ rstart, const uint32_t* __restrict__ rcnt, uint64_t cap, uint2* __restrict__ nrl_ent,
-    uint64_t* run_sfx, uint32_t* run_qn, uint32_t* run_L, uint4* __restrict__ act, uint64_t* __restrict__ act_base,
-    unsigned long long* __restrict__ tot) {
-    const uint32_t n = *nlistq;
+    const uint32_t* __restrict__ rstart, uint64_t cap, uint2* __restrict__ nrl_ent, uint64_t* run_sfx,
+    uint32_t* run_qn, uint32_t* run_L, uint4* __restrict__ act) {
+    const uint32_t n = (uint32_t)ctrl->nlistq.v;
     const int lane = threadIdx.x & 31;
     const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5), w = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    // A queue of 32 cells a warp or more is taken 32 consecutive cells at a time.  A shorter one is
-    // dealt out evenly, one cell after the other to warp after warp: long lists sit next to each
-    // other in the queue, and the merge's latency then runs in as many warps as there are.
-    const bool deal = n < 32 * nw;
-    const uint64_t per = deal ? (n + nw - 1) / nw : 32;
-    for (uint64_t i0 = deal ? w : 32 * w; i0 < n; i0 += 32 * nw) {
-        const uint64_t i = deal ? i0 + (uint64_t)lane * nw : i0 + lane;
-        const bool in = (uint64_t)lane < per && i < n;
+    // Consecutive cells share their neighbours, so a warp takes 32 consecutive ones.  A queue of
+    // fewer than four cells a warp is dealt out one by one to as many warps as take 16 each: long
+    // lists sit next to each other in it, and their merges then run side by side
+    // (dense 200,000 points: 135 us against 353 us; lists elsewhere cost the same either way).
+    const bool deal = n < 4 * nw;
+    const uint64_t dealt = deal ? (n + 15) / 16 : 0;
+    for (uint64_t i0 = deal ? w : w * 32; i0 < (deal ? dealt : n); i0 += nw * 32) {
+        const uint64_t i = deal ? i0 + (uint64_t)lane * dealt : i0 + lane;
+        const bool in = i < n && (!deal || lane < 16);
         uint32_t c = 0, r0 = 0, r1 = 0, kept = 0;
         // each slot's cursor starts at its first run above the lowest own feature
         uint32_t h[9], e[9], f[9];
@@ -688,7 +716,7 @@ __global__ void __launch_bounds__(128) k_neighbour_lists(
         const uint32_t ktot = __shfl_sync(0xffffffffu, kincl, 31);
         if (ktot == 0) continue;
         unsigned long long kb = 0;
-        if (lane == 0) kb = atomicAdd(&tot[0], (unsigned long long)ktot);
+        if (lane == 0) kb = atomicAdd(&ctrl->entries.v, (unsigned long long)ktot);
         kb = __shfl_sync(0xffffffffu, kb, 0);
         if (kb + ktot > cap) continue;   // no room: the host runs the kernel again
         const uint64_t first = kb + (kincl - kept);
@@ -726,8 +754,8 @@ __global__ void __launch_bounds__(128) k_neighbour_lists(
                         r = h[t]++;
                         f[t] = h[t] < e[t] ? rfeat[h[t]] : 0xffffffffu;
                     }
-                const uint32_t rc = rcnt[r];
-                nrl_ent[pos++] = make_uint2(rstart[r], rc);
+                const uint32_t st = rstart[r], rc = rstart[r + 1] - st;
+                nrl_ent[pos++] = make_uint2(st, rc);
                 P += rc;
                 if (ts == own) {
                     pend = true;
@@ -745,8 +773,8 @@ __global__ void __launch_bounds__(128) k_neighbour_lists(
         for (uint32_t m = __ballot_sync(0xffffffffu, big); m; m &= m - 1) {   // the merge above is serial in the list
             const int j = __ffs(m) - 1;
             nrl_cell_warp(__shfl_sync(0xffffffffu, c, j), lane, __shfl_sync(0xffffffffu, first, j),
-                          __shfl_sync(0xffffffffu, kept, j), ckey, cjob, grids, nb9, cstart, crun, rfeat, rstart, rcnt,
-                          nrl_ent, run_sfx, run_qn, run_L);
+                          __shfl_sync(0xffffffffu, kept, j), ckey, cjob, grids, nb9, cstart, crun, rfeat, rstart, nrl_ent,
+                          run_sfx, run_qn, run_L);
         }
         __syncwarp();
         // anchors: the points of own runs with targets
@@ -756,7 +784,7 @@ __global__ void __launch_bounds__(128) k_neighbour_lists(
             for (uint32_t r = r0; r < r1; ++r) {
                 const uint32_t L = run_L[r];
                 if (!L) continue;
-                const uint32_t rc = rcnt[r];
+                const uint32_t rc = rstart[r + 1] - rstart[r];
                 na += rc;
                 nu += (uint64_t)rc * L;
             }
@@ -764,8 +792,8 @@ __global__ void __launch_bounds__(128) k_neighbour_lists(
         const uint64_t uincl = warp_incl_scan(nu);
         unsigned long long ab = 0, ub = 0;
         if (lane == 31 && aincl) {
-            ab = atomicAdd(&tot[1], (unsigned long long)aincl);
-            ub = atomicAdd(&tot[2], (unsigned long long)uincl);
+            ab = atomicAdd(&ctrl->anchors.v, (unsigned long long)aincl);
+            ub = atomicAdd(&ctrl->capacity.v, (unsigned long long)uincl);
         }
         uint64_t o = __shfl_sync(0xffffffffu, ab, 31) + (aincl - na);
         uint64_t u = __shfl_sync(0xffffffffu, ub, 31) + (uincl - nu);
@@ -774,12 +802,11 @@ __global__ void __launch_bounds__(128) k_neighbour_lists(
             for (uint32_t r = r0; r < r1; ++r) {
                 const uint32_t L = run_L[r];
                 if (!L) continue;
-                const uint32_t st = rstart[r], rc = rcnt[r], qn = run_qn[r];
+                const uint32_t st = rstart[r], rc = rstart[r + 1] - st;
                 const uint64_t sfx = run_sfx[r];
+                const uint32_t hi = run_qn[r] << 8 | (uint32_t)(sfx >> 32);
                 for (uint32_t q = 0; q < rc; ++q) {
-                    act[o] = make_uint4(st + q, qn, (uint32_t)sfx, (uint32_t)(sfx >> 32));
-                    act_base[o] = u;
-                    ++o;
+                    act[o++] = make_uint4(st + q, (uint32_t)u, (uint32_t)sfx, hi);
                     u += L;
                 }
             }
@@ -790,12 +817,11 @@ __global__ void __launch_bounds__(128) k_neighbour_lists(
             for (uint32_t r = s0; r < s1; ++r) {   // the whole warp reads the run
                 const uint32_t L = run_L[r];
                 if (!L) continue;
-                const uint32_t st = rstart[r], rc = rcnt[r], qn = run_qn[r];
+                const uint32_t st = rstart[r], rc = rstart[r + 1] - st;
                 const uint64_t sfx = run_sfx[r];
-                for (uint32_t q = lane; q < rc; q += 32) {
-                    act[oj + q] = make_uint4(st + q, qn, (uint32_t)sfx, (uint32_t)(sfx >> 32));
-                    act_base[oj + q] = uj + (uint64_t)q * L;
-                }
+                const uint32_t hi = run_qn[r] << 8 | (uint32_t)(sfx >> 32);
+                for (uint32_t q = lane; q < rc; q += 32)
+                    act[oj + q] = make_uint4(st + q, (uint32_t)(uj + (uint64_t)q * L), (uint32_t)sfx, hi);
                 oj += rc;
                 uj += (uint64_t)rc * L;
             }
@@ -810,130 +836,207 @@ inline unsigned grid_for(uint64_t n, int threads) {
 
 }  // namespace
 
-// Cell keys, the stable sort by key, the sorted point copies and the cell /
-// run compaction, with KT = 32-bit keys when every key fits (less traffic per
-// radix pass), else 64-bit.
+// Bounded batches reserve at most this much for arrays laid out by bounds (and no more than
+// a sixteenth of the device); the 20M-point workload takes 5 GB.  Larger ones wait for the
+// number of cells and runs before their per-cell arrays are laid out.
+constexpr uint64_t kBoundBytes = 8ull << 30;
+// Look-back words of all digit passes in one clear, up to this much (above 100 million points
+// one pass's words are cleared before each pass).
+constexpr uint64_t kSortStatusBytes = 256ull << 20;
+// Room for list entries and neighbours before their numbers are known: four entries per run
+// (0.2 on the 20M workload, 3.4 on a batch of many small jobs; nine at most: a run is adjacent
+// to nine cells) and eight neighbours per point (0.14 on the 20M workload, 16 on that batch,
+// 30 in dense clusters).  What does not fit is built again with the counted room.
+inline uint64_t list_room(uint64_t runs) { return std::min<uint64_t>(9 * runs, 4 * runs + 65536); }
+inline uint64_t neighbour_room(uint64_t n) { return std::min<uint64_t>(kSinglePassCap, 8 * n + 65536); }
+
+namespace {
+
+void lay_points(Batch& b, Carver& c) {
+    c.add(b.xy, b.N);
+    c.add(b.sxy, b.N);
+    c.add(b.sfeat, b.N);
+    c.add(b.sid, b.N);
+    c.add(b.nb_beg, b.N);
+    c.add(b.nb_cnt, b.N);
+}
+void lay_heads(Batch& b, Carver& c, uint64_t M, uint64_t R) {
+    c.add(b.ckey, M);
+    c.add(b.cstart, M + 1);
+    c.add(b.crun, M + 1);
+    c.add(b.cjob, M);
+    c.add(b.rfeat, R);
+    c.add(b.rstart, R + 1);
+    c.add(b.rcell, R);
+    if (b.keep_scell) c.add(b.scell, b.N);
+}
+void lay_cells(Batch& b, Carver& c, uint64_t M, uint64_t R) {
+    c.add(b.cmask, M * b.W);
+    c.add(b.nbmask, M * b.W);
+    c.add(b.qmask, M * 4 * b.W);
+    c.add(b.nb9, M * 9);
+    c.add(b.qfirst, M);
+    c.add(b.listq, M);
+    c.add(b.run_sfx, R);
+    c.add(b.run_qn, R);
+    c.add(b.run_L, R);
+    if (b.row_table) c.add(b.rowstart, b.rows + 1);
+}
+void lay_lists(Batch& b, Carver& c) { c.add(b.nrl_ent, b.nrl_cap); }
+void lay_act(Batch& b, Carver& c) { c.add(b.act, b.N); }
+
+// The row table when it is not much larger than the cell list.
+bool wants_row_table(const Batch& b, uint64_t cells) {
+    return b.rows < (1ull << 31) && b.rows <= 4 * cells + (1u << 20);
+}
+
+template <class KT>
+void launch_heads(Batch& b, const KT* keys, uint64_t capM, uint64_t capR) {
+    const uint64_t tiles = (b.N + kHeadTile - 1) / kHeadTile;
+    KScope ks("gather_sorted");
+    k_heads<KT><<<(unsigned)tiles, kHeadThreads, 0, b.s>>>(
+        b.N, b.F, keys, b.sid.get(), b.xy.get(), b.fstart.get(), b.fjob.get(), b.sxy.get(), b.sfeat.get(),
+        b.ckey.get(), b.cstart.get(), b.crun.get(), b.cjob.get(), b.rfeat.get(), b.rstart.get(), b.rcell.get(),
+        capM ? b.scell.get() : nullptr, capM, capR, b.head_status.get(), b.tickets.get() + b.plan.n, b.ctrl.get());
+    COLO_LAUNCH_CHECK();
+    count_launch();
+}
+
+// Waits for the totals of the sort and the heads.
+void read_sizes(Batch& b) {
+    BatchCtrl h;
+    COLO_CUDA(cudaMemcpyAsync(&h, b.ctrl.get(), sizeof(h), cudaMemcpyDeviceToHost, b.s));
+    stream_wait(b.s);
+    if (h.flags.timeout) throw StatusError{COLO_ERR_TIMEOUT, "radix sort: a tile waited too long for its predecessors"};
+    b.M = h.M;
+    b.Rn = h.Rn;
+}
+
+// Cell keys, the stable sort by key, and the sorted point copies with the cells and runs,
+// with KT = 32-bit keys when every key fits (less traffic per radix pass), else 64-bit.
 template <class KT>
 void sort_and_compact(Batch& b) {
     cudaStream_t s = b.s;
     const uint64_t n = b.N;
-    DevBuf<KT> keys;
-    keys.alloc(n, s);
-    b.sid.alloc(n, s);
-    const int bits = sizeof(KT) == 4 && b.key_bits > 32 ? 32 : (int)b.key_bits;
-    const RadixPlan plan = radix_plan(bits);
-    DevBuf<unsigned long long> hist;
-    hist.alloc((uint64_t)(plan.n > 0 ? plan.n : 1) * kRadixDigits, s);
-    hist.zero(s);
+    const bool sorts = n > 1 && b.plan.n > 0;
+    // the sort's buffers: the ids end in b.sid, whichever of the two the last pass writes
+    DevBuf<unsigned char> mem;
+    Span<KT> ka, kb;
+    Span<uint32_t> other;
+    Carver::place(mem, s, [&](Carver& c) {
+        c.add(ka, n);
+        c.add(kb, n);
+        c.add(other, n);
+        if (b.sort_shared) c.add(b.sort_status, radix_status_words(n));
+    });
     {
-    KScope ks("cell_keys");
-    b.xy.alloc(n, s);
-    const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, (uint64_t)b.sms * 8);
-    // the ids are written here only when the sort runs no pass (its first pass makes them)
-    const bool sorted_ids = n > 1 && bits > 0;
-    k_cell_keys<KT><<<(unsigned)(blocks ? blocks : 1), 256, 0, s>>>(n, b.x, b.y, b.F, b.fstart.get(), b.fjob.get(), b.grids.get(),
-                                                                    keys.get(), sorted_ids ? nullptr : b.sid.get(),
-                                                                    b.xy.get(), b.flags.get(), plan, hist.get());
-    COLO_LAUNCH_CHECK();
-    count_launch();
+        KScope ks("cell_keys");
+        const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, (uint64_t)b.sms * 8);
+        // the ids are written here only when the sort runs no pass (its first pass makes them)
+        k_cell_keys<KT><<<(unsigned)(blocks ? blocks : 1), 256, 0, s>>>(
+            n, b.x, b.y, b.F, b.fstart.get(), b.fjob.get(), b.grids.get(), ka.get(), sorts ? nullptr : b.sid.get(),
+            b.xy.get(), b.nb_cnt.get(), b.ctrl.get(), b.plan, b.hist.get());
+        COLO_LAUNCH_CHECK();
+        count_launch();
     }
-    // a look-back timeout lands in the batch's flags, read with the compaction totals
-    radix_sort(keys, b.sid, n, bits, s, "radix_sort", hist.get(), &b.flags.get()->timeout, b.test_spin, true);
+    const KT* keys = ka.get();
+    if (sorts) {
+        const bool odd = (b.plan.n & 1) != 0;
+        RadixBufs<KT> bufs{ka.get(), kb.get(), odd ? other.get() : b.sid.get(), odd ? b.sid.get() : other.get()};
+        radix_sort(bufs, n, b.plan, s, b.hist.get(), b.sort_status.get(), b.sort_shared, b.tickets.get(),
+                   &b.flags()->timeout, b.test_spin);
+        keys = bufs.ka;
+    }
+    if (b.bounded) {
+        launch_heads<KT>(b, keys, b.capM, b.capR);
+        return;
+    }
+    // heads laid out for every point when that is small against the device, else counted first
+    const size_t all = Carver::bytes([&](Carver& c) { lay_heads(b, c, n, n); });
+    if (all <= b.device_bytes / 16) {
+        Carver::place(b.mem_heads, s, [&](Carver& c) { lay_heads(b, c, n, n); });
+        launch_heads<KT>(b, keys, n, n);
+        read_sizes(b);
+    } else {
+        launch_heads<KT>(b, keys, 0, 0);
+        read_sizes(b);
+        Carver::place(b.mem_heads, s, [&](Carver& c) { lay_heads(b, c, b.M, b.Rn); });
+        const uint64_t tiles = (n + kHeadTile - 1) / kHeadTile;
+        COLO_CUDA(cudaMemsetAsync(b.head_status.get(), 0, 2 * tiles * 8, s));
+        COLO_CUDA(cudaMemsetAsync(b.tickets.get() + b.plan.n, 0, 4, s));
+        launch_heads<KT>(b, keys, b.M, b.Rn);
+    }
+    b.capM = b.M;
+    b.capR = b.Rn;
+}
 
-    b.sxy.alloc(n, s);
-    b.sfeat.alloc(n, s);
-    const uint64_t tiles = (n + kHeadTile - 1) / kHeadTile;
-    DevBuf<uint64_t> part;
-    part.alloc(tiles + 1, s);
-    uint64_t totals = 0;
-    {
-        KScope ks("gather_sorted");
-        k_gather_heads<KT><<<(unsigned)tiles, kHeadThreads, 0, s>>>(n, b.F, keys.get(), b.sid.get(), b.xy.get(),
-                                                                   b.fstart.get(), b.sxy.get(), b.sfeat.get(),
-                                                                   part.get());
-        COLO_LAUNCH_CHECK();
-        count_launch();
-    }
-    {
-        KScope ks("cell_compact");
-        // the sort's timeout word comes back with the totals: after a timeout the keys are not
-        // a sorted permutation, and nothing past this point may read them
-        uint32_t sort_err = 0;
-        COLO_CUDA(cudaMemcpyAsync(&sort_err, &b.flags.get()->timeout, 4, cudaMemcpyDeviceToHost, s));
-        scan_partials_u64(part.get(), tiles, s, &totals);
-        if (sort_err) throw StatusError{COLO_ERR_TIMEOUT, "radix sort: a tile waited too long for its predecessors"};
-    }
-    const uint32_t M = (uint32_t)(totals >> 32), Rn = (uint32_t)totals;
-    b.M = M;
-    b.Rn = Rn;
-    b.ckey.alloc(M, s);
-    b.cstart.alloc(M + 1, s);
-    b.crun.alloc(M + 1, s);
-    b.cjob.alloc(M, s);
-    b.rfeat.alloc(Rn, s);
-    b.rstart.alloc(Rn, s);
-    b.rcnt.alloc(Rn, s);
-    b.rcell.alloc(Rn, s);
-    if (b.keep_scell) b.scell.alloc(n, s);
-    {
-        KScope ks("cell_compact");
-        k_head_compact<KT><<<(unsigned)tiles, kHeadThreads, 0, s>>>(
-            n, keys.get(), b.sfeat.get(), b.fjob.get(), part.get(), b.ckey.get(), b.cstart.get(), b.crun.get(),
-            b.cjob.get(), b.rfeat.get(), b.rstart.get(), b.rcell.get(), b.keep_scell ? b.scell.get() : nullptr);
-        COLO_LAUNCH_CHECK();
-        count_launch();
-    }
-    {
-        KScope ks("cell_compact");
-        k_run_tail<<<grid_for(Rn, 256), 256, 0, s>>>(Rn, M, n, b.rstart.get(), b.rcnt.get(), b.cstart.get(),
-                                                      b.crun.get());
-        COLO_LAUNCH_CHECK();
-        count_launch();
-    }
+}  // namespace
+
+void bucket_layout(Batch& b, Carver& c) {
+    const uint64_t tiles = (b.N + kHeadTile - 1) / kHeadTile, sw = b.N ? radix_status_words(b.N) : 0;
+    b.sort_shared = sw * 8 * (uint64_t)b.plan.n > kSortStatusBytes;
+    c.add(b.hist, (uint64_t)std::max(b.plan.n, 1) * kRadixDigits);
+    c.add(b.tickets, (uint64_t)b.plan.n + 1);
+    c.add(b.head_status, 2 * tiles);
+    if (!b.sort_shared) c.add(b.sort_status, sw * (uint64_t)b.plan.n);
 }
 
 void bucket_points(Batch& b) {
     cudaStream_t s = b.s;
+    const uint64_t n = b.N;
+    // everything up to the pairs' bounds in one block laid out by bounds, when that is small
+    // enough to reserve; a device that has no such block left takes the other way
+    b.capM = b.capR = n;
+    b.nrl_cap = list_room(n);
+    b.nb_cap = neighbour_room(n);
+    b.row_table = wants_row_table(b, n);
+    auto bounds = [&](Carver& c) {
+        lay_points(b, c);
+        lay_heads(b, c, n, n);
+        lay_cells(b, c, n, n);
+        lay_lists(b, c);
+        lay_act(b, c);
+        c.add(b.nb, b.nb_cap);
+    };
+    b.bounded = Carver::bytes(bounds) <= std::min<uint64_t>(kBoundBytes, b.device_bytes / 16);
+    if (b.bounded) {
+        try {
+            Carver::place(b.mem_points, s, bounds);
+        } catch (const StatusError& e) {
+            if (e.st != COLO_ERR_NOMEM) throw;
+            b.bounded = false;
+        }
+    }
+    if (!b.bounded) {
+        b.nb_cap = 0;
+        b.nb = Span<uint32_t>();
+        Carver::place(b.mem_points, s, [&](Carver& c) { lay_points(b, c); });
+    }
     if (b.key_bits <= 32) sort_and_compact<uint32_t>(b);
     else sort_and_compact<uint64_t>(b);
-    const uint64_t M = b.M, Rn = b.Rn;
-
-    b.cmask.alloc((uint64_t)M * b.W, s);
+    if (!b.bounded) {
+        b.row_table = wants_row_table(b, b.M);
+        Carver::place(b.mem_cells, s, [&](Carver& c) { lay_cells(b, c, b.M, b.Rn); });
+    }
+    const uint64_t capM = b.capM;
     {
         KScope ks("cell_masks");
-        k_cell_masks<<<grid_for(M, 256), 256, 0, s>>>(M, b.crun.get(), b.rfeat.get(), b.cjob.get(), b.grids.get(),
-                                                       b.W, b.cmask.get());
+        const uint64_t items = std::max<uint64_t>(capM, b.row_table ? b.rows + 1 : 0);
+        const unsigned grid = (unsigned)std::min<uint64_t>(grid_for(items, 256), (uint64_t)b.sms * 8);
+        k_cell_masks<<<grid, 256, b.F <= kRunHist ? b.F * 4 : 0, s>>>(
+            b.ctrl.get(), b.ckey.get(), b.crun.get(), b.rfeat.get(), b.cjob.get(), b.grids.get(), b.W, b.cmask.get(),
+            b.row_table ? b.rows : 0, b.J, b.rowstart.get(), b.F, b.frun());
         COLO_LAUNCH_CHECK();
         count_launch();
     }
-    b.nb9.alloc((uint64_t)M * 9, s);
-    b.qfirst.alloc(M, s);
     {
         KScope ks("cell_neighbours");
-        // the row table when it is not much larger than the cell list
-        const bool table = b.rows < (1ull << 31) && b.rows <= 4 * (uint64_t)M + (1u << 20);
-        b.rowstart.release();
-        if (table) {
-            b.rowstart.alloc(b.rows + 1, s);
-            k_row_starts<<<grid_for(b.rows + 1, 256), 256, 0, s>>>(b.rows, b.J, M, b.ckey.get(), b.grids.get(),
-                                                                  b.rowstart.get());
-            COLO_LAUNCH_CHECK();
-            count_launch();
-        }
-        k_nb9<<<grid_for(M, 128), 128, 0, s>>>(M, b.ckey.get(), b.cjob.get(), b.grids.get(),
-                                               table ? b.rowstart.get() : nullptr, b.nb9.get(), b.qfirst.get());
+        const unsigned grid = (unsigned)std::min<uint64_t>(grid_for(capM, 128), (uint64_t)b.sms * 64);
+        k_nb9<<<grid, 128, 0, s>>>(b.ctrl.get(), b.ckey.get(), b.cjob.get(), b.grids.get(),
+                                   b.row_table ? b.rowstart.get() : nullptr, b.nb9.get(), b.qfirst.get());
         COLO_LAUNCH_CHECK();
         count_launch();
     }
-    b.nbmask.alloc((uint64_t)M * b.W, s);
-    b.qmask.alloc((uint64_t)M * 4 * b.W, s);
-    b.listq.alloc(M ? M : 1, s);
-    b.nlistq.alloc(1, s);
-    b.nlistq.zero(s);
-    // cells per driver list (3x3 blocks holding each feature), counted with the masks
-    DevBuf<uint32_t> dcnt;
-    dcnt.alloc(b.F ? b.F : 1, s);
-    dcnt.zero(s);
     {
         KScope ks("quad_masks");
         // one wave of resident blocks (each keeps one histogram for all its cells)
@@ -942,10 +1045,10 @@ void bucket_points(Batch& b) {
         int per_sm = 1;                                                                                      \
         COLO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_quad_masks<WW>, kQuadThreads, 0)); \
         const unsigned qblocks = (unsigned)std::max<uint64_t>(                                               \
-            1, std::min<uint64_t>(grid_for(M, kQuadThreads), (uint64_t)b.sms * (uint64_t)std::max(per_sm, 1))); \
+            1, std::min<uint64_t>(grid_for(capM, kQuadThreads), (uint64_t)b.sms * (uint64_t)std::max(per_sm, 1))); \
         k_quad_masks<WW><<<qblocks, kQuadThreads, 0, s>>>(                                                   \
-            M, b.ckey.get(), b.cjob.get(), b.grids.get(), b.nb9.get(), b.cmask.get(), b.qmask.get(),         \
-            b.nbmask.get(), b.listq.get(), b.nlistq.get(), b.F, dcnt.get());                                 \
+            b.ctrl.get(), b.ckey.get(), b.cjob.get(), b.grids.get(), b.nb9.get(), b.cmask.get(),             \
+            b.qmask.get(), b.nbmask.get(), b.listq.get(), b.F, b.dcnt());                          \
     } while (0)
         switch (b.W) {
             case 1: COLO_QM(1); break;
@@ -966,79 +1069,29 @@ void bucket_points(Batch& b) {
         COLO_LAUNCH_CHECK();
         count_launch();
     }
-
-    // runs per feature
-    {
-        KScope ks("run_index");
-        DevBuf<uint32_t> cnt;
-        cnt.alloc(b.F ? b.F : 1, s);
-        cnt.zero(s);
-        const uint64_t blocks = std::min<uint64_t>((Rn + 255) / 256, (uint64_t)b.sms * 4);
-        const size_t smem = b.F <= kHistMax ? (size_t)b.F * 4 : 0;
-        if (smem > 48 * 1024)
-            COLO_CUDA(cudaFuncSetAttribute(k_feature_runs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (Rn) {
-            k_feature_runs<<<(unsigned)(blocks ? blocks : 1), 256, smem, s>>>(Rn, b.F, b.rfeat.get(), cnt.get());
-            COLO_LAUNCH_CHECK();
-            count_launch();
-        }
-        // the run counts, list sizes and error flags come back with one wait
-        std::vector<uint32_t> hc(b.F), hd(b.F);
-        DevFlags hf;
-        if (b.F) {
-            COLO_CUDA(cudaMemcpyAsync(hc.data(), cnt.get(), b.F * 4, cudaMemcpyDeviceToHost, s));
-            COLO_CUDA(cudaMemcpyAsync(hd.data(), dcnt.get(), b.F * 4, cudaMemcpyDeviceToHost, s));
-        }
-        COLO_CUDA(cudaMemcpyAsync(&hf, b.flags.get(), sizeof(hf), cudaMemcpyDeviceToHost, s));
-        stream_wait(s);
-        b.h_frun_off.assign(b.F + 1, 0);
-        for (uint32_t f = 0; f < b.F; ++f) b.h_frun_off[f + 1] = b.h_frun_off[f] + hc[f];
-        b.h_dcnt.assign(hd.begin(), hd.end());
-        b.h_doff.assign(b.F + 1, 0);
-        b.dlist_have.assign(b.F, 0);
-        if (hf.timeout) throw StatusError{COLO_ERR_TIMEOUT, "radix sort: a tile waited too long for its predecessors"};
-        if (hf.out_of_grid)
-            throw StatusError{COLO_ERR_INPUT, std::to_string(hf.out_of_grid) +
-                                                  " point(s) fall outside the grid derived from the bounds line"};
-    }
 }
 
 void build_neighborhoods(Batch& b) {
     cudaStream_t s = b.s;
-    const uint64_t M = b.M;
-    b.run_sfx.alloc(b.Rn, s);
-    b.run_qn.alloc(b.Rn, s);
-    b.run_L.alloc(b.Rn, s);
-    b.act.alloc(b.N ? b.N : 1, s);
-    b.act_base.alloc(b.N ? b.N : 1, s);
-    DevBuf<unsigned long long> tot;
-    tot.alloc(3, s);
-    const unsigned qgrid = (unsigned)std::min<uint64_t>(grid_for(M, 128), (uint64_t)b.sms * 16);
-    // room for four list entries per run (0.2 on the 20M workload, 3.4 on a batch of many small
-    // jobs; nine at most: a run is adjacent to nine cells); lists that need more are built again
-    // with the counted room
-    uint64_t cap = std::min<uint64_t>(9 * b.Rn, 4 * b.Rn + 65536);
-    unsigned long long h[3] = {0, 0, 0};
-    for (;;) {
-        b.nrl_ent.alloc(cap ? cap : 1, s);
-        tot.zero(s);
-        {
-            KScope ks("neighbour_lists");
-            k_neighbour_lists<<<qgrid, 128, 0, s>>>(
-                b.listq.get(), b.nlistq.get(), b.ckey.get(), b.cjob.get(), b.grids.get(), b.nb9.get(), b.cstart.get(),
-                b.crun.get(), b.rfeat.get(), b.rstart.get(), b.rcnt.get(), cap, b.nrl_ent.get(), b.run_sfx.get(),
-                b.run_qn.get(), b.run_L.get(), b.act.get(), b.act_base.get(), tot.get());
-            COLO_LAUNCH_CHECK();
-            count_launch();
-        }
-        COLO_CUDA(cudaMemcpyAsync(h, tot.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
-        stream_wait(s);
-        if (h[0] <= cap) break;
-        cap = h[0];
+    if (!b.bounded && !b.act.get()) {
+        Carver::place(b.mem_act, s, [&](Carver& c) { lay_act(b, c); });
+        b.nrl_cap = list_room(b.Rn);
+        Carver::place(b.mem_lists, s, [&](Carver& c) { lay_lists(b, c); });
     }
-    b.nrl_total = h[0];
-    b.active_anchors = h[1];
-    b.join_pairs = h[2];
+    if (b.lists_built) {   // the lists did not fit: room for all of them, and the totals from zero
+        b.nrl_cap = b.nrl_total;
+        Carver::place(b.mem_lists, s, [&](Carver& c) { lay_lists(b, c); });
+        COLO_CUDA(cudaMemsetAsync(&b.ctrl.get()->entries, 0, 3 * sizeof(LineCounter), s));
+    }
+    b.lists_built = true;
+    const unsigned qgrid = (unsigned)std::min<uint64_t>(grid_for(b.capM, 128), (uint64_t)b.sms * 16);
+    KScope ks("neighbour_lists");
+    k_neighbour_lists<<<qgrid, 128, 0, s>>>(b.listq.get(), b.ctrl.get(), b.ckey.get(), b.cjob.get(), b.grids.get(),
+                                            b.nb9.get(), b.cstart.get(), b.crun.get(), b.rfeat.get(), b.rstart.get(),
+                                            b.nrl_cap, b.nrl_ent.get(), b.run_sfx.get(), b.run_qn.get(),
+                                            b.run_L.get(), b.act.get());
+    COLO_LAUNCH_CHECK();
+    count_launch();
 }
 
 }  // namespace colo

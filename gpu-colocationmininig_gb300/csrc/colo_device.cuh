@@ -164,4 +164,56 @@ __device__ __forceinline__ T block_excl_scan(T v, T* total) {
     return res;
 }
 
+// ---- decoupled look-back --------------------------------------------------
+constexpr unsigned long long kScanA = 1ull << 62;   // tile sum published
+constexpr unsigned long long kScanP = 2ull << 62;   // inclusive prefix published
+constexpr unsigned long long kScanVal = (1ull << 62) - 1;
+constexpr uint32_t kScanSpin = 1u << 20;
+
+// Decoupled look-back by one full warp for tile `tile` of a single-pass scan:
+// publishes the tile's sum `agg`, reads the predecessors' words 32 at a time
+// back to the nearest inclusive prefix, publishes the tile's own inclusive
+// prefix and returns the exclusive one.  Past the poll limit it returns false
+// and publishes nothing more; the caller then computes the prefix itself and
+// publishes it with lookback_publish.
+__device__ __forceinline__ bool warp_lookback(unsigned long long* status, uint32_t tile, unsigned long long agg,
+                                              unsigned long long& prefix) {
+    const int lane = threadIdx.x & 31;
+    prefix = 0;
+    volatile unsigned long long* st = status + tile;
+    if (tile == 0) {
+        if (lane == 0) *st = kScanP | agg;
+        return true;
+    }
+    if (lane == 0) *st = kScanA | agg;
+    int64_t base = (int64_t)tile - 1;
+    uint32_t spins = 0;
+    while (true) {
+        const int64_t t = base - lane;
+        const unsigned long long sv = t >= 0 ? *(volatile const unsigned long long*)(status + t) : kScanP;
+        const unsigned long long flag = sv & ~kScanVal;
+        const uint32_t pm = __ballot_sync(0xffffffffu, flag == kScanP);
+        const uint32_t zm = __ballot_sync(0xffffffffu, flag == 0);
+        const int fp = pm ? __ffs(pm) - 1 : 32;   // nearest inclusive prefix
+        const uint32_t upto = fp == 32 ? 0xffffffffu : ((2u << fp) - 1u);
+        if (zm & upto) {   // a predecessor has not published yet
+            if (++spins > kScanSpin) return false;
+            __nanosleep(32);
+            continue;
+        }
+        unsigned long long add = ((upto >> lane) & 1u) ? (sv & kScanVal) : 0ull;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+        prefix += add;
+        if (fp < 32) break;
+        base -= 32;
+    }
+    if (lane == 0) *st = kScanP | (prefix + agg);
+    return true;
+}
+
+__device__ __forceinline__ void lookback_publish(unsigned long long* status, uint32_t tile, unsigned long long incl) {
+    if ((threadIdx.x & 31) == 0) *(volatile unsigned long long*)(status + tile) = kScanP | incl;
+}
+
 }  // namespace colo

@@ -39,17 +39,20 @@ constexpr uint64_t kAccMax = 16384;   // block-private level sums (64 KB of shar
 // null for a one-job batch (job 0 everywhere): the mask load then waits on one
 // dependent load (the run's cell) instead of three.
 __global__ void __launch_bounds__(kFilterThreads) k_filter_pairs(
-    uint64_t Rn, const uint32_t* __restrict__ rcell, const uint32_t* __restrict__ cjob,
+    const BatchCtrl* __restrict__ ctrl, const uint32_t* __restrict__ rcell, const uint32_t* __restrict__ cjob,
     const JobGrid* __restrict__ grids, const uint32_t* __restrict__ nbmask,
-    uint32_t W, const uint32_t* __restrict__ rfeat, const uint32_t* __restrict__ rcnt,
-    const uint64_t* __restrict__ job_off, uint32_t* __restrict__ ub2, uint32_t acc_dim, uint64_t runs_per_block) {
+    uint32_t W, const uint32_t* __restrict__ rfeat, const uint32_t* __restrict__ rstart,
+    const uint64_t* __restrict__ job_off, uint32_t* __restrict__ ub2, uint32_t acc_dim) {
     extern __shared__ uint32_t acc[];   // acc_dim x acc_dim (acc_dim = 0: no privatisation)
     __shared__ int32_t cur_job;
-    const uint64_t r0 = (uint64_t)blockIdx.x * runs_per_block;
-    const uint64_t r1 = r0 + runs_per_block < Rn ? r0 + runs_per_block : Rn;
+    const uint64_t Rn = ctrl->Rn;
+    const uint64_t per = ((Rn + gridDim.x - 1) / gridDim.x + blockDim.x - 1) / blockDim.x * blockDim.x;
+    const uint64_t r0 = (uint64_t)blockIdx.x * per;
+    const uint64_t r1 = r0 + per < Rn ? r0 + per : Rn;
+    if (r0 >= r1) return;
     const uint32_t accn = acc_dim * acc_dim;
     for (uint32_t i = threadIdx.x; i < accn; i += blockDim.x) acc[i] = 0;
-    if (threadIdx.x == 0) cur_job = r0 < Rn ? (cjob ? (int32_t)cjob[rcell[r0]] : 0) : -1;
+    if (threadIdx.x == 0) cur_job = cjob ? (int32_t)cjob[rcell[r0]] : 0;
     __syncthreads();
     for (uint64_t base = r0; base < r1; base += blockDim.x) {
         const int32_t jb = cjob ? (int32_t)cjob[rcell[base]] : 0;
@@ -72,7 +75,7 @@ __global__ void __launch_bounds__(kFilterThreads) k_filter_pairs(
             const JobGrid g = grids[job];
             if (g.gx >= 2 && g.gy >= 2) {
                 const bool priv = acc_dim && (int32_t)job == cur_job && g.nf <= acc_dim;
-                const uint32_t lf = rfeat[r] - g.f0, cnt = rcnt[r];
+                const uint32_t lf = rfeat[r] - g.f0, cnt = rstart[r + 1] - rstart[r];
                 for (uint32_t w = 0; w < W; ++w) {
                     uint32_t bits = nbmask[(uint64_t)c * W + w];
                     while (bits) {
@@ -88,7 +91,7 @@ __global__ void __launch_bounds__(kFilterThreads) k_filter_pairs(
         }
     }
     __syncthreads();
-    if (cur_job >= 0 && acc_dim) {
+    if (acc_dim) {
         uint32_t nf = grids[cur_job].nf;
         for (uint32_t i = threadIdx.x; i < nf * nf; i += blockDim.x) {
             uint32_t v = acc[(i / nf) * acc_dim + (i % nf)];
@@ -266,7 +269,7 @@ __global__ void __launch_bounds__(256, (WT <= 4 ? 5 : (WT <= 6 ? 4 : (WT <= 8 ? 
     const uint32_t* __restrict__ dlist, const uint32_t* __restrict__ order, const uint32_t* __restrict__ need_all,
     const uint32_t* __restrict__ lmem, uint32_t k, const uint32_t* __restrict__ qmask,
     const uint32_t* __restrict__ cmask, const uint32_t* __restrict__ crun, const uint8_t* __restrict__ qfirst,
-    const uint32_t* __restrict__ rcnt, uint32_t* __restrict__ ub, unsigned long long* __restrict__ stats,
+    const uint32_t* __restrict__ rstart, uint32_t* __restrict__ ub, unsigned long long* __restrict__ stats,
     uint32_t acc_n, uint32_t cu) {
     constexpr uint32_t W = WT;
     constexpr bool kCacheQuads = WT <= 8;
@@ -342,7 +345,8 @@ __global__ void __launch_bounds__(256, (WT <= 4 ? 5 : (WT <= 6 ? 4 : (WT <= 8 ? 
                     if ((uint32_t)w == wq) word = cm[w];
                 }
                 if (word >> (lf & 31) & 1u) {
-                    const uint32_t v = rcnt[q0 + rk + __popc(word & ((1u << (lf & 31)) - 1u))];
+                    const uint32_t ri = q0 + rk + __popc(word & ((1u << (lf & 31)) - 1u));
+                    const uint32_t v = rstart[ri + 1] - rstart[ri];
                     if (acc_n) atomicAdd(&acc[c * stride + jj], v);
                     else atomicAdd(&ub[(uint64_t)c * k + jj], v);
                 }
@@ -438,17 +442,9 @@ void driver_lists_fill(Batch& b, const std::vector<uint8_t>& need) {
 
 }  // namespace
 
-void filter_pairs(Batch& b, DevBuf<uint32_t>& ub2, std::vector<uint64_t>& job_off, cudaStream_t s) {
-    job_off.assign(b.J + 1, 0);
-    for (uint32_t j = 0; j < b.J; ++j)
-        job_off[j + 1] = job_off[j] + (uint64_t)b.jobs[j].grid.nf * b.jobs[j].grid.nf;
-    ub2.alloc(job_off[b.J] ? job_off[b.J] : 1, s);
-    ub2.zero(s);
-    if (b.M == 0) return;
+void filter_pairs(Batch& b) {
+    cudaStream_t s = b.s;
     if (b.W > kMaxW) throw StatusError{COLO_ERR_CAPACITY, "the filter handles at most 1024 features per job"};
-    DevBuf<uint64_t> d_job_off;
-    d_job_off.alloc(b.J + 1, s);
-    COLO_CUDA(cudaMemcpyAsync(d_job_off.get(), job_off.data(), (b.J + 1) * 8, cudaMemcpyHostToDevice, s));
     uint32_t acc_dim = b.Fmax_local;
     size_t smem = (size_t)acc_dim * acc_dim * 4;
     if (smem > 200 * 1024) {
@@ -457,18 +453,16 @@ void filter_pairs(Batch& b, DevBuf<uint32_t>& ub2, std::vector<uint64_t>& job_of
     }
     if (smem > 48 * 1024)
         COLO_CUDA(cudaFuncSetAttribute(k_filter_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // as many resident blocks per SM as the accumulator allows (at most 8)
+    // as many resident blocks per SM as the accumulator allows (at most 8), each with its share of the runs
     uint64_t per_sm = smem ? (200 * 1024) / smem : 8;
     if (per_sm < 1) per_sm = 1;
     if (per_sm > 8) per_sm = 8;
-    uint64_t blocks = (uint64_t)b.sms * per_sm;
-    uint64_t per = (b.Rn + blocks - 1) / blocks;
-    per = (per + kFilterThreads - 1) / kFilterThreads * kFilterThreads;
-    blocks = (b.Rn + per - 1) / per;
+    const uint64_t blocks = std::min<uint64_t>((uint64_t)b.sms * per_sm, (b.capR + kFilterThreads - 1) / kFilterThreads);
+    if (!blocks) return;
     KScope ks("filter_pairs");
     k_filter_pairs<<<(unsigned)blocks, kFilterThreads, smem, s>>>(
-        b.Rn, b.rcell.get(), b.J > 1 ? b.cjob.get() : nullptr, b.grids.get(), b.nbmask.get(), b.W, b.rfeat.get(),
-        b.rcnt.get(), d_job_off.get(), ub2.get(), acc_dim, per);
+        b.ctrl.get(), b.rcell.get(), b.J > 1 ? b.cjob.get() : nullptr, b.grids.get(), b.nbmask.get(), b.W,
+        b.rfeat.get(), b.rstart.get(), b.job_off.get(), b.ub2(), acc_dim);
     COLO_LAUNCH_CHECK();
     count_launch();
 }
@@ -580,7 +574,7 @@ void filter_level(Batch& b, const uint32_t* h_cand, const uint32_t* h_job, uint6
 #define COLO_FL(WW)                                                                                             \
     k_filter_drv<WW><<<grid((const void*)k_filter_drv<WW>), 256, smem, s>>>(                                    \
         nunits, ngroups, d_uoff, d_gfeat, d_gstart, d_gcount, b.doff.get(), b.dlist.get(), d_order, d_need,       \
-        d_lmem, k, b.qmask.get(), b.cmask.get(), b.crun.get(), b.qfirst.get(), b.rcnt.get(), d_ub, d_stats, acc_n, cu)
+        d_lmem, k, b.qmask.get(), b.cmask.get(), b.crun.get(), b.qfirst.get(), b.rstart.get(), d_ub, d_stats, acc_n, cu)
     COLO_W_SWITCH(b.W, COLO_FL)
 #undef COLO_FL
     COLO_LAUNCH_CHECK();

@@ -86,6 +86,7 @@ struct colo_ctx {
     int device = 0;
     cudaStream_t s = nullptr;
     int sms = 0;
+    uint64_t device_bytes = 0;  // the device's memory
     std::string err;
     int refs = 1;          // the owner plus one per live dataset (freed at zero)
     std::vector<float> model;   // cost-model parameters for LEARNED mines (empty: none)
@@ -131,4 +132,8 @@ uint64_t upload_dataset(colo_dataset* ds, cudaStream_t s);   // bytes copied (0 
 // `own` keeps the concatenated device copies of multi-job batches alive.
 void setup_batch(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params* pv, uint32_t J, Batch& b,
                  std::vector<DevBuf<float>>& ownf, double* t_upload);
+// Waits for the batch's totals, per-feature counts and (ub2 non-null) the pairs' bounds, one copy
+// for all; reports the errors that bucketing recorded, and builds the neighbour lists and their
+// join again, with room, when they were queued and did not fit.
+void settle(colo_ctx* ctx, Batch& b, std::vector<uint32_t>* ub2);
 }  // namespace colo

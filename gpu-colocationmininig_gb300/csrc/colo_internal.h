@@ -123,6 +123,42 @@ struct DevBuf {
     size_t bytes() const { return n * sizeof(T); }
 };
 
+// A typed part of a larger device allocation.
+template <class T>
+struct Span {
+    T* p = nullptr;
+    T* get() const { return p; }
+};
+
+// Lays out spans in one allocation, each on a 256-byte boundary: `layout` names
+// them with add(span, count), once to size the block and once to place them.
+struct Carver {
+    unsigned char* base = nullptr;
+    size_t off = 0;
+    template <class T>
+    void add(Span<T>& sp, uint64_t count) {
+        off = (off + 255) & ~(size_t)255;
+        sp.p = base ? reinterpret_cast<T*>(base + off) : nullptr;
+        off += (size_t)(count * sizeof(T));
+    }
+    template <class Fn>
+    static size_t place(DevBuf<unsigned char>& mem, cudaStream_t st, Fn&& layout) {
+        Carver size;
+        layout(size);
+        mem.alloc(size.off ? size.off : 256, st);
+        Carver at;
+        at.base = mem.get();
+        layout(at);
+        return size.off;
+    }
+    template <class Fn>
+    static size_t bytes(Fn&& layout) {
+        Carver size;
+        layout(size);
+        return size.off;
+    }
+};
+
 // Instance-table storage: device memory, or pinned host memory mapped into
 // the device's address space when asked for or when the device allocation
 // fails (on Grace the kernels then read and write them over NVLink-C2C).
@@ -311,15 +347,10 @@ struct KScope {
 // Primitives (colo_prims.cu)
 // ---------------------------------------------------------------------------
 
-// In place: exclusive scan of partial[0..m), partial[m] = total (read back
-// when total_host != nullptr).
-void scan_partials_u64(uint64_t* partial, uint64_t m, cudaStream_t s, uint64_t* total_host);
 // out[i] = sum(in[0..i)).  The total is read back (with a wait) when
 // total_host is given, and copied to device memory (no wait) when total_dev is.
 void scan_u32_to_u64(const uint32_t* in, uint64_t* out, uint64_t n, cudaStream_t s,
                      uint64_t* total_host, uint64_t* total_dev = nullptr);
-void scan_u32_to_u32(const uint32_t* in, uint32_t* out, uint64_t n, cudaStream_t s,
-                     uint32_t* total_host, uint32_t* total_dev = nullptr);
 void scan_u64_to_u64(const uint64_t* in, uint64_t* out, uint64_t n, cudaStream_t s,
                      uint64_t* total_host, uint64_t* total_dev = nullptr);
 // Digit split of a radix sort: pass p sorts width[p] (<= 8) bits from shift[p].
@@ -331,26 +362,30 @@ struct RadixPlan {
     int width[kRadixMaxPasses];
 };
 RadixPlan radix_plan(int bits);
-// Stable LSD radix sort of (key, val) pairs by the low `bits` bits of key.
-// The sorted pairs are in keys/vals on return (the buffers may have been
-// exchanged for the sort's second buffers, which avoids a copy back).
-// hist, when given, holds every pass's digit counts of the keys
-// (hist[p * kRadixDigits + d], radix_plan(bits) passes), counted by the
-// caller while it wrote the keys; the sort then skips its own count.
-// err_dev, when given, receives the timeout flag of a look-back wait (the
-// caller checks it at its next wait); otherwise the sort waits and throws.
-// test_spin != 0 (tests of the timeout path only): the look-back gives up
-// after test_spin polls, and in the first pass tile 0 withholds its counts,
-// so tile 1's wait runs out; every wait stays bounded and the sort ends with
-// the timeout flag set (its output is discarded by the caller).
-// iota_vals: the values are the positions 0 .. n-1, which the first pass
-// generates instead of reading (vals must still hold n items).  With no pass
-// (n <= 1 or bits <= 0) vals is left as given, so the caller writes them then.
-void radix_sort(DevBuf<uint64_t>& keys, DevBuf<uint32_t>& vals, uint64_t n, int bits, cudaStream_t s,
-                const char* name = "radix_sort", unsigned long long* hist = nullptr, uint32_t* err_dev = nullptr,
-                uint32_t test_spin = 0, bool iota_vals = false);
-void radix_sort(DevBuf<uint32_t>& keys, DevBuf<uint32_t>& vals, uint64_t n, int bits, cudaStream_t s,
-                const char* name = "radix_sort", unsigned long long* hist = nullptr, uint32_t* err_dev = nullptr,
-                uint32_t test_spin = 0, bool iota_vals = false);
+// Stable LSD radix sort of (key, id) pairs by the plan's digits, the ids being
+// the positions 0 .. n-1 (the first pass makes them).  The keys are in ka; each
+// pass writes the other pair of buffers, and ka / va name the sorted ones on
+// return.  Launches only.
+//   hist      every pass's digit starts (hist[p * kRadixDigits + d])
+//   status    look-back words, radix_status_words(n) per pass, all cleared when
+//             `shared` is false; with `shared` one pass's words, cleared here
+//   tickets   one cleared word per pass
+//   err       receives a look-back wait that ran out (the failed pass + 1): the
+//             output is then not a permutation, later passes write nothing, and
+//             no kernel may index by it
+// test_spin != 0 (tests of the timeout path only): the look-back gives up after
+// test_spin polls, and in the first pass tile 0 withholds its counts.
+template <class KT>
+struct RadixBufs {
+    KT *ka, *kb;
+    uint32_t *va, *vb;
+};
+uint64_t radix_status_words(uint64_t n);
+void radix_sort(RadixBufs<uint32_t>& bufs, uint64_t n, const RadixPlan& plan, cudaStream_t s,
+                const unsigned long long* hist, unsigned long long* status, bool shared, uint32_t* tickets,
+                uint32_t* err, uint32_t test_spin);
+void radix_sort(RadixBufs<uint64_t>& bufs, uint64_t n, const RadixPlan& plan, cudaStream_t s,
+                const unsigned long long* hist, unsigned long long* status, bool shared, uint32_t* tickets,
+                uint32_t* err, uint32_t test_spin);
 
 }  // namespace colo

@@ -15,6 +15,7 @@
 // number of target points) and writes its hits there, so no counting pass is
 // needed; when the upper bounds would not fit, a count pass + scan + fill
 // pass produces a compact layout instead.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -26,31 +27,30 @@ namespace {
 
 enum { J_SINGLE = 0, J_COUNT = 1, J_FILL = 2 };
 
-// The single pass sums the list total into kEntrySlots counters kEntryStride
-// words apart (one 128-byte line each), added up when the total is read.
-constexpr int kEntrySlots = 64, kEntryStride = 16;
+constexpr uint64_t kJoinWaves = 8;   // waves of resident blocks at most (the groups take anchors grid-stride)
 
 // One anchor's neighbour list, by its group of T lanes; returns the list length.
 template <int T, int MODE>
 __device__ __forceinline__ uint32_t join_anchor(
     uint64_t i, const uint4* __restrict__ act, const uint32_t* __restrict__ sid, const uint32_t* __restrict__ sfeat,
-    const float2* __restrict__ sxy, const uint64_t* __restrict__ act_base,
-    const uint2* __restrict__ nrl_ent, const uint32_t* __restrict__ fjob, const JobGrid* __restrict__ grids,
-    uint64_t* __restrict__ nb_beg, uint32_t* __restrict__ nb_cnt, uint32_t* __restrict__ nb) {
+    const float2* __restrict__ sxy, const uint2* __restrict__ nrl_ent, const uint32_t* __restrict__ fjob,
+    const JobGrid* __restrict__ grids, uint64_t* __restrict__ nb_beg, uint32_t* __restrict__ nb_cnt,
+    uint32_t* __restrict__ nb) {
     const int lane = threadIdx.x & 31;
     const int gl = lane % T;
     const int gbase = lane - gl;
     const uint32_t gmask = (T == 32) ? 0xffffffffu : (((1u << T) - 1u) << gbase);
-    const uint4 an = act[i];   // position and list slice in one load: the list's first entry waits on this one alone
+    // position, list start and list slice in one load: the slice's first entry waits on this one alone
+    const uint4 an = act[i];
     const uint32_t p = an.x;
     const uint32_t a = sid[p];
     const float2 pa = sxy[p];
     const float xa = pa.x, ya = pa.y;
     const JobGrid& g = grids[fjob ? fjob[sfeat[p]] : 0u];   // fjob is null for one-job batches
     const float R2 = g.R2, hu = g.R2hu;
-    const uint64_t q0 = (uint64_t)an.w << 32 | an.z, qend = q0 + an.y;
+    const uint64_t q0 = (uint64_t)(an.w & 0xffu) << 32 | an.z, qend = q0 + (an.w >> 8);
     uint64_t base = 0;
-    if (MODE == J_SINGLE) base = act_base[i];
+    if (MODE == J_SINGLE) base = an.y;
     if (MODE == J_FILL) base = nb_beg[a];
     uint32_t k = 0;
     for (uint64_t q = q0; q < qend; ++q) {
@@ -88,43 +88,49 @@ __device__ __forceinline__ uint32_t join_anchor(
 
 
 // Six blocks per SM (40 registers): the join is latency-bound, and the sixth block
-// measured 0.398 -> 0.377 ms per step on the 20M workload.
+// measured 0.398 -> 0.377 ms per step on the 20M workload.  The anchors are counted on the
+// device; the groups take them grid-stride.  Lists or a layout that did not fit their room
+// are left to a later launch with room.
 template <int T, int MODE>
 __global__ void __launch_bounds__(256, 6) k_join(
-    uint64_t A, const uint4* __restrict__ act, const uint32_t* __restrict__ sid, const uint32_t* __restrict__ sfeat,
-    const float2* __restrict__ sxy, const uint64_t* __restrict__ act_base,
+    const BatchCtrl* __restrict__ ctrl, uint64_t nrl_cap, uint64_t nb_cap, const uint4* __restrict__ act,
+    const uint32_t* __restrict__ sid, const uint32_t* __restrict__ sfeat, const float2* __restrict__ sxy,
     const uint2* __restrict__ nrl_ent, const uint32_t* __restrict__ fjob, const JobGrid* __restrict__ grids,
     uint64_t* __restrict__ nb_beg, uint32_t* __restrict__ nb_cnt, uint32_t* __restrict__ nb,
     unsigned long long* __restrict__ total) {
+    if (ctrl->entries.v > nrl_cap || (MODE == J_SINGLE && ctrl->capacity.v > nb_cap)) return;
+    const uint64_t A = ctrl->anchors.v;
     const int lane = threadIdx.x & 31;
     const int gl = lane % T;
-    const uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / T;
-    // groups past the last anchor (whole groups) count nothing but stay for the block sum
-    const uint32_t k = i < A ? join_anchor<T, MODE>(i, act, sid, sfeat, sxy, act_base, nrl_ent, fjob, grids, nb_beg, nb_cnt, nb)
-                             : 0u;
+    const uint64_t thread = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long v = 0;
+    for (uint64_t i = thread / T; i < A; i += (uint64_t)gridDim.x * blockDim.x / T) {
+        const uint32_t k = join_anchor<T, MODE>(i, act, sid, sfeat, sxy, nrl_ent, fjob, grids, nb_beg, nb_cnt, nb);
+        if (gl == 0) v += k;
+    }
     if (MODE == J_SINGLE) {
         // the entries of the warp's anchors (each group's count once), one atomic per warp into
         // one of kEntrySlots counters on separate lines: the list total without another pass
         // over the counts, and no block barrier (one made every warp wait for its block's
         // longest list: the 512-job batch's join ran 10.96 ms against 9.38 ms)
-        unsigned long long v = gl == 0 ? k : 0u;
+        __syncwarp();
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-        if (lane == 0 && v) atomicAdd(total + (warp % kEntrySlots) * kEntryStride, v);
+        if (lane == 0 && v) atomicAdd(total + ((thread >> 5) % kEntrySlots) * kEntryStride, v);
     }
 }
 
+// `anchors`: as many as there are, or a bound.
 template <int T>
-void run_join(Batch& b, int mode) {
-    const uint64_t A = b.active_anchors;
-    if (A == 0) return;
-    uint64_t threads = A * T;
-    unsigned grid = (unsigned)((threads + 255) / 256);
+void run_join(Batch& b, int mode, uint64_t anchors) {
+    const uint64_t nrl_cap = b.nrl_cap, nb_cap = b.nb_cap;
+    uint64_t grid = (anchors * T + 255) / 256;
+    grid = std::min<uint64_t>(grid, (uint64_t)b.sms * 6 * kJoinWaves);
+    if (grid == 0) return;
     KScope ks(mode == J_SINGLE ? "join" : mode == J_COUNT ? "join_count" : "join_fill");
 #define COLO_JOIN(MD)                                                                                        \
-    k_join<T, MD><<<grid, 256, 0, b.s>>>(A, b.act.get(), b.sid.get(), b.sfeat.get(), b.sxy.get(),               \
-                                         b.act_base.get(), b.nrl_ent.get(),                                     \
+    k_join<T, MD><<<(unsigned)grid, 256, 0, b.s>>>(b.ctrl.get(), nrl_cap, nb_cap, b.act.get(), b.sid.get(), \
+                                         b.sfeat.get(), b.sxy.get(), b.nrl_ent.get(),                           \
                                          b.J > 1 ? b.fjob.get() : nullptr,                                      \
                                          b.grids.get(), b.nb_beg.get(), b.nb_cnt.get(), b.nb.get(), b.dE.get())
     if (mode == J_SINGLE) COLO_JOIN(J_SINGLE);
@@ -135,14 +141,14 @@ void run_join(Batch& b, int mode) {
     count_launch();
 }
 
-void dispatch_join(Batch& b, int mode) {
+void dispatch_join(Batch& b, int mode, uint64_t anchors) {
     switch (b.join_group) {
-        case 1: run_join<1>(b, mode); break;
-        case 2: run_join<2>(b, mode); break;
-        case 4: run_join<4>(b, mode); break;
-        case 16: run_join<16>(b, mode); break;
-        case 32: run_join<32>(b, mode); break;
-        default: run_join<8>(b, mode); break;
+        case 1: run_join<1>(b, mode, anchors); break;
+        case 2: run_join<2>(b, mode, anchors); break;
+        case 4: run_join<4>(b, mode, anchors); break;
+        case 16: run_join<16>(b, mode, anchors); break;
+        case 32: run_join<32>(b, mode, anchors); break;
+        default: run_join<8>(b, mode, anchors); break;
     }
 }
 
@@ -157,34 +163,36 @@ __global__ void k_sqdist(const float* __restrict__ x1, const float* __restrict__
 
 }  // namespace
 
-// Upper bound of the single-pass layout above which the compact two-pass
-// layout is used instead (entries).
-static const uint64_t kSinglePassCap = 1ull << 30;
+void join_queue(Batch& b) {
+    b.join_queued = true;
+    dispatch_join(b, J_SINGLE, b.N);
+    b.E = UINT64_MAX;
+}
 
+// A point without targets keeps the zero count that the cell-key pass gave it; its list
+// start is never read (every reader takes nb_cnt first).
 void join_neighbors(Batch& b) {
     cudaStream_t s = b.s;
-    const uint64_t U = b.join_pairs;
-    // a point without targets keeps a zero count; its list start is never read (every
-    // reader takes nb_cnt first), so only the counts are cleared
-    b.nb_beg.alloc(b.N ? b.N : 1, s);
-    b.nb_cnt.alloc(b.N ? b.N : 1, s);
-    b.nb_cnt.zero(s);
-    b.dE.alloc(kEntrySlots * kEntryStride, s);
-    b.join_single = U <= kSinglePassCap;
-    if (b.join_single) {
+    const uint64_t A = b.active_anchors, U = b.join_pairs;
+    b.join_queued = false;
+    // layouts above kSinglePassCap entries are counted first and then compact
+    const bool single = U <= kSinglePassCap;
+    auto room = [&](uint64_t n) {
+        b.nb_cap = n;
+        Carver::place(b.mem_nb, s, [&](Carver& c) { c.add(b.nb, std::max<uint64_t>(n, 1)); });
+    };
+    if (single) {
         // total entries: summed by the join's warps and read at the mine's next wait
-        b.nb_cap = U;
-        b.nb.alloc(U ? U : 1, s);
-        b.dE.zero(s);
-        dispatch_join(b, J_SINGLE);
+        if (U > b.nb_cap || !b.nb.get()) room(U);
+        COLO_CUDA(cudaMemsetAsync(b.dE.get(), 0, kEntrySlots * kEntryStride * 8, s));
+        dispatch_join(b, J_SINGLE, A);
         b.E = UINT64_MAX;
     } else {
-        dispatch_join(b, J_COUNT);
+        dispatch_join(b, J_COUNT, A);
         uint64_t E = 0;
         scan_u32_to_u64(b.nb_cnt.get(), b.nb_beg.get(), b.N, s, &E);
-        b.nb_cap = E;
-        b.nb.alloc(E ? E : 1, s);
-        dispatch_join(b, J_FILL);
+        room(E);
+        dispatch_join(b, J_FILL, A);
         b.E = E;
     }
 }

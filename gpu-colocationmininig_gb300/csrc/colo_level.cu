@@ -422,7 +422,7 @@ void launch_level(Batch& b, const LevelWork& w, uint32_t k, uint32_t* ovf) {
     k_level<KK, MODE><<<grid, block, 0, b.s>>>(w.cands, w.chunk_off, w.ncand, w.nchunks, b.nb_beg.get(), b.nb_cnt.get(), \
                                             b.nb.get(), b.xy.get(), b.fstart.get(), b.fcount.get(),  \
                                             b.grids.get(), ovf, w.items, w.chunk_status, w.ticket,    \
-                                            &b.flags.get()->timeout, persistent)
+                                            &b.flags()->timeout, persistent)
     switch (k) {
         case 2: COLO_LVL(2); break;
         case 3: COLO_LVL(3); break;

@@ -515,21 +515,77 @@ void setup_batch(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params* pv,
     b.key_bits = 1;
     while (b.key_bits < 64 && (1ull << b.key_bits) < key_base) b.key_bits++;
     b.rows = row_base;
-    b.fstart.alloc(b.F ? b.F : 1, s);
-    b.fcount.alloc(b.F ? b.F : 1, s);
-    b.fjob.alloc(b.F ? b.F : 1, s);
-    b.grids.alloc(J, s);
-    b.flags.alloc(1, s);
-    b.flags.zero(s);
-    std::vector<JobGrid> hg(J);
-    for (uint32_t j = 0; j < J; ++j) hg[j] = b.jobs[j].grid;
-    if (b.F) {
-        COLO_CUDA(cudaMemcpyAsync(b.fstart.get(), b.h_fstart.data(), b.F * 4, cudaMemcpyHostToDevice, s));
-        COLO_CUDA(cudaMemcpyAsync(b.fcount.get(), b.h_fcount.data(), b.F * 4, cudaMemcpyHostToDevice, s));
-        COLO_CUDA(cudaMemcpyAsync(b.fjob.get(), b.h_fjob.data(), b.F * 4, cudaMemcpyHostToDevice, s));
+    b.device_bytes = ctx->device_bytes;
+    b.plan = radix_plan(b.key_bits <= 32 ? (int)b.key_bits : (int)std::min<uint64_t>(b.key_bits, 64));
+    b.h_job_off.assign(J + 1, 0);
+    for (uint32_t j = 0; j < J; ++j)
+        b.h_job_off[j + 1] = b.h_job_off[j] + (uint64_t)b.jobs[j].grid.nf * b.jobs[j].grid.nf;
+    // the tables (one upload from page-locked staging) and the cleared words (one clear)
+    const uint64_t F1 = std::max<uint32_t>(b.F, 1);
+    b.ctrl_bytes = sizeof(BatchCtrl) + 4 * (2 * (uint64_t)b.F + b.h_job_off[J]);
+    Span<unsigned char> ctrl;
+    const size_t total = Carver::place(b.mem0, s, [&](Carver& c) {
+        c.add(b.fstart, F1);
+        c.add(b.fcount, F1);
+        c.add(b.fjob, F1);
+        c.add(b.grids, J);
+        c.add(b.job_off, J + 1);
+        c.add(ctrl, b.ctrl_bytes);
+        c.add(b.dE, kEntrySlots * kEntryStride);
+        bucket_layout(b, c);
+    });
+    b.ctrl.p = reinterpret_cast<BatchCtrl*>(ctrl.get());
+    const size_t up = (size_t)(ctrl.get() - b.mem0.get());
+    unsigned char* h = upload_area(ctx, s, up);
+    auto put = [&](const void* dst, const void* src, size_t bytes) {
+        if (bytes) std::memcpy(h + (static_cast<const unsigned char*>(dst) - b.mem0.get()), src, bytes);
+    };
+    put(b.fstart.get(), b.h_fstart.data(), b.F * 4);
+    put(b.fcount.get(), b.h_fcount.data(), b.F * 4);
+    put(b.fjob.get(), b.h_fjob.data(), b.F * 4);
+    for (uint32_t j = 0; j < J; ++j) put(b.grids.get() + j, &b.jobs[j].grid, sizeof(JobGrid));
+    put(b.job_off.get(), b.h_job_off.data(), (J + 1) * 8);
+    upload_from(s, b.mem0.get(), h, up);
+    COLO_CUDA(cudaMemsetAsync(ctrl.get(), 0, total - up, s));
+}
+
+void settle(colo_ctx* ctx, Batch& b, std::vector<uint32_t>* ub2) {
+    const size_t bytes = ub2 ? b.ctrl_bytes : sizeof(BatchCtrl) + 8 * (size_t)b.F;
+    std::vector<unsigned char> back(bytes);
+    BatchCtrl h;
+    {
+        Readback rb(ctx, b.s, bytes);
+        rb.copy(back.data(), b.ctrl.get(), bytes);
+        rb.finish();
     }
-    // (copies from pageable memory return once the source is staged: no wait is needed)
-    COLO_CUDA(cudaMemcpyAsync(b.grids.get(), hg.data(), J * sizeof(JobGrid), cudaMemcpyHostToDevice, s));
+    std::memcpy(&h, back.data(), sizeof(h));
+    if (h.flags.timeout) throw StatusError{COLO_ERR_TIMEOUT, "radix sort: a tile waited too long for its predecessors"};
+    if (h.flags.out_of_grid)
+        throw StatusError{COLO_ERR_INPUT, std::to_string(h.flags.out_of_grid) +
+                                              " point(s) fall outside the grid derived from the bounds line"};
+    b.M = h.M;
+    b.Rn = h.Rn;
+    const uint32_t* counts = reinterpret_cast<const uint32_t*>(back.data() + sizeof(BatchCtrl));
+    b.h_dcnt.assign(counts, counts + b.F);
+    b.h_frun_off.assign(b.F + 1, 0);
+    for (uint32_t f = 0; f < b.F; ++f) b.h_frun_off[f + 1] = b.h_frun_off[f] + counts[b.F + f];
+    b.h_doff.assign(b.F + 1, 0);
+    b.dlist_have.assign(b.F, 0);
+    if (ub2) ub2->assign(counts + 2 * b.F, counts + 2 * b.F + b.h_job_off[b.J]);
+    if (!b.lists_built) return;
+    b.nrl_total = h.entries.v;
+    bool again = false;
+    while (b.nrl_total > b.nrl_cap) {
+        again = true;
+        build_neighborhoods(b);
+        Readback rb(ctx, b.s, sizeof(h));
+        rb.copy(&h, b.ctrl.get(), sizeof(h));
+        rb.finish();
+        b.nrl_total = h.entries.v;
+    }
+    b.active_anchors = h.anchors.v;
+    b.join_pairs = h.capacity.v;
+    if (b.join_queued && (again || b.join_pairs > b.nb_cap)) join_neighbors(b);
 }
 
 // The stream-ordered pool keeps what it has mapped (its release threshold is
@@ -622,10 +678,16 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
     }
     double t_bucket = ms_since(t0);
     t0 = Clock::now();
-    if (N > 0) join_neighbors(b);
-    b.act.release();
-    b.act_base.release();
-    double t_join = ms_since(t0);   // host time: the level loop's first wait absorbs the join's tail
+    // bounded batches join into the room they have; the others when the sizes are known (settle)
+    if (N > 0 && b.bounded) join_queue(b);
+    double t_join = ms_since(t0);   // host time: the level loop's first wait absorbs the rest
+    bool settled = N == 0;
+    auto settle_and_join = [&](std::vector<uint32_t>* ub2) {
+        settle(ctx, b, ub2);
+        settled = true;
+        if (!b.bounded) join_neighbors(b);
+        b.mem_act.release();
+    };
 
     double t_filter = 0, t_refine = 0, t_fill = 0, t_apriori = 0;
     uint64_t rows_written = 0;
@@ -639,6 +701,9 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
                 js[j].cands.push_back(js[j].f0 + c);
             }
     }
+    bool pairs = false;
+    for (const auto& st : js) pairs |= st.active && !st.cands.empty();
+    if (!settled && !pairs) settle_and_join(nullptr);   // no level asks for the totals
     std::unique_ptr<TableBuf> tables_prev, tables_cur, single_prev;
     // level tables go to pinned host memory when forced (reserved[0] bit 3)
     // or when their device allocation fails
@@ -678,20 +743,20 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         bool force_single_any = false;
         for (uint32_t j = 0; j < J; ++j) force_single_any |= (pv[j].reserved[0] & 16) != 0;
         if (k == 2) {
-            DevBuf<uint32_t> ub2;
-            std::vector<uint64_t> job_off;
-            filter_pairs(b, ub2, job_off, s);
-            std::vector<uint32_t> h(job_off[J]);
-            if (!h.empty()) COLO_CUDA(cudaMemcpyAsync(h.data(), ub2.get(), h.size() * 4, cudaMemcpyDeviceToHost, s));
-            stream_wait(s);
+            // the mine's first wait: sizes, counts and the pairs' bounds
+            std::vector<uint32_t> h;
+            filter_pairs(b);
+            kt.mark("bucketing launches");
+            settle_and_join(&h);
+            kt.mark("bucketing wait");
             for (uint32_t j = 0; j < J; ++j) {
                 if (!tr[j]) continue;
                 LevelTrace& L = *tr[j];
                 uint32_t nf = js[j].nf;
                 for (size_t c = 0; c < L.cand.size() / 2; ++c) {
                     uint32_t l0 = L.cand[2 * c] - js[j].f0, l1 = L.cand[2 * c + 1] - js[j].f0;
-                    L.ub[2 * c] = h[job_off[j] + (uint64_t)l0 * nf + l1];
-                    L.ub[2 * c + 1] = h[job_off[j] + (uint64_t)l1 * nf + l0];
+                    L.ub[2 * c] = h[b.h_job_off[j] + (uint64_t)l0 * nf + l1];
+                    L.ub[2 * c + 1] = h[b.h_job_off[j] + (uint64_t)l1 * nf + l0];
                     L.pass[c] = filter_pass(&L.ub[2 * c], &L.cand[2 * c], 2, b.h_fcount, js[j].thr);
                 }
             }
@@ -1072,7 +1137,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         std::vector<unsigned char> hout(ar.out_bytes);
         if (ar.out_bytes) rb.copy(hout.data(), ar.out, ar.out_bytes);
         DevFlags hflags{};
-        if (ns) rb.copy(&hflags, b.flags.get(), sizeof(hflags));
+        if (ns) rb.copy(&hflags, b.flags(), sizeof(hflags));
         kt.mark("refine launches");
         rb.finish();
         kt.mark("refine wait");
@@ -1445,6 +1510,9 @@ colo_status colo_create(colo_ctx** out, int device) {
         cudaEventCreateWithFlags(&c->ev_scanned, cudaEventDisableTiming) != cudaSuccess)
         return COLO_ERR_CUDA;
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return COLO_ERR_CUDA;
+    c->device_bytes = total_b;
     // keep freed blocks in the stream-ordered pool between calls
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {

@@ -12,33 +12,6 @@ thread_local KTimer* g_ktimer = nullptr;
 namespace {
 
 constexpr int kScanThreads = 256;
-constexpr int kScanItems = 8;   // per thread in the one-block partials scan
-
-// Single block: exclusive scan of partial[0..m) in place; partial[m] = total.
-template <class T>
-__global__ void k_scan_partials(T* partial, uint64_t m) {
-    T carry = 0;
-    for (uint64_t base = 0; base < m; base += (uint64_t)blockDim.x * kScanItems) {
-        uint64_t i0 = base + (uint64_t)threadIdx.x * kScanItems;
-        T v[kScanItems];
-        T s = 0;
-#pragma unroll
-        for (int i = 0; i < kScanItems; ++i) {
-            v[i] = (i0 + i < m) ? partial[i0 + i] : T(0);
-            s += v[i];
-        }
-        T tot;
-        T ex = block_excl_scan<T>(s, &tot) + carry;
-#pragma unroll
-        for (int i = 0; i < kScanItems; ++i) {
-            if (i0 + i < m) partial[i0 + i] = ex;
-            ex += v[i];
-        }
-        carry += tot;
-    }
-    if (threadIdx.x == 0) partial[m] = carry;
-}
-
 // Single-pass scan (decoupled look-back): a block takes the next tile number
 // from a counter, sums its 4096 items, publishes the sum, and warp 0 reads its
 // predecessors' published words 32 at a time, back to the nearest inclusive
@@ -50,57 +23,6 @@ __global__ void k_scan_partials(T* partial, uint64_t m) {
 // items per round (coalesced loads and stores).
 constexpr int kScan1Items = 16;
 constexpr int kScan1Tile = kScanThreads * kScan1Items;
-constexpr unsigned long long kScanA = 1ull << 62;   // tile sum published
-constexpr unsigned long long kScanP = 2ull << 62;   // inclusive prefix published
-constexpr unsigned long long kScanVal = (1ull << 62) - 1;
-constexpr uint32_t kScanSpin = 1u << 20;
-
-// Decoupled look-back by one full warp for tile `tile` of a single-pass scan:
-// publishes the tile's sum `agg`, reads the predecessors' words 32 at a time
-// back to the nearest inclusive prefix, publishes the tile's own inclusive
-// prefix and returns the exclusive one.  Past the poll limit it returns false
-// and publishes nothing more; the caller then computes the prefix itself and
-// publishes it with lookback_publish.
-__device__ __forceinline__ bool warp_lookback(unsigned long long* status, uint32_t tile, unsigned long long agg,
-                                              unsigned long long& prefix) {
-    const int lane = threadIdx.x & 31;
-    prefix = 0;
-    volatile unsigned long long* st = status + tile;
-    if (tile == 0) {
-        if (lane == 0) *st = kScanP | agg;
-        return true;
-    }
-    if (lane == 0) *st = kScanA | agg;
-    int64_t base = (int64_t)tile - 1;
-    uint32_t spins = 0;
-    while (true) {
-        const int64_t t = base - lane;
-        const unsigned long long sv = t >= 0 ? *(volatile const unsigned long long*)(status + t) : kScanP;
-        const unsigned long long flag = sv & ~kScanVal;
-        const uint32_t pm = __ballot_sync(0xffffffffu, flag == kScanP);
-        const uint32_t zm = __ballot_sync(0xffffffffu, flag == 0);
-        const int fp = pm ? __ffs(pm) - 1 : 32;   // nearest inclusive prefix
-        const uint32_t upto = fp == 32 ? 0xffffffffu : ((2u << fp) - 1u);
-        if (zm & upto) {   // a predecessor has not published yet
-            if (++spins > kScanSpin) return false;
-            __nanosleep(32);
-            continue;
-        }
-        unsigned long long add = ((upto >> lane) & 1u) ? (sv & kScanVal) : 0ull;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
-        prefix += add;
-        if (fp < 32) break;
-        base -= 32;
-    }
-    if (lane == 0) *st = kScanP | (prefix + agg);
-    return true;
-}
-
-__device__ __forceinline__ void lookback_publish(unsigned long long* status, uint32_t tile, unsigned long long incl) {
-    if ((threadIdx.x & 31) == 0) *(volatile unsigned long long*)(status + tile) = kScanP | incl;
-}
-
 template <class Tin, class Tout>
 __global__ void __launch_bounds__(kScanThreads, 5) k_scan_1p(const Tin* __restrict__ in, Tout* __restrict__ out,
                                                           uint64_t n, unsigned long long* __restrict__ status,
@@ -210,8 +132,8 @@ struct SortSmem {
 
 
 // ---------------------------------------------------------------------------
-// One-sweep LSD radix sort: the digit histograms of every pass from one read
-// of the keys, then one kernel per pass.  A block takes the next tile number
+// One-sweep LSD radix sort: the digit histograms of every pass come with the
+// keys (k_cell_keys), then one kernel per pass.  A block takes the next tile number
 // from a counter, ranks its keys stably, publishes its per-digit counts, and
 // looks back over the preceding tiles' published counts (a tile that has
 // finished its own look-back publishes its inclusive prefix, which ends the
@@ -228,42 +150,6 @@ constexpr unsigned long long kFlagA = 1ull << 62;   // tile count published
 constexpr unsigned long long kFlagP = 2ull << 62;   // inclusive prefix published
 constexpr unsigned long long kValMask = (1ull << 62) - 1;
 constexpr uint32_t kSpinLimit = 1u << 22;
-
-template <class KT>
-__global__ void k_digit_hist(const KT* __restrict__ keys, uint64_t n, RadixPlan plan,
-                             unsigned long long* __restrict__ ghist) {
-    __shared__ uint32_t h[kMaxPasses * kMaxRadix];
-    for (int i = threadIdx.x; i < plan.n * kMaxRadix; i += blockDim.x) h[i] = 0;
-    __syncthreads();
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const KT k = keys[i];
-        for (int p = 0; p < plan.n; ++p)
-            atomicAdd(&h[p * kMaxRadix + ((uint32_t)(k >> plan.shift[p]) & ((1u << plan.width[p]) - 1u))], 1u);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < plan.n * kMaxRadix; i += blockDim.x) {
-        const uint32_t v = h[i];
-        if (v) atomicAdd(&ghist[i], (unsigned long long)v);
-    }
-}
-
-// Exclusive scan of each pass's counters in place (one block of kMaxRadix).
-__global__ void k_digit_scan(unsigned long long* __restrict__ ghist, int passes) {
-    __shared__ unsigned long long sh[kMaxRadix];
-    for (int p = 0; p < passes; ++p) {
-        const unsigned long long v = ghist[p * kMaxRadix + threadIdx.x];
-        sh[threadIdx.x] = v;
-        __syncthreads();
-        for (int o = 1; o < kMaxRadix; o <<= 1) {
-            unsigned long long t = threadIdx.x >= (unsigned)o ? sh[threadIdx.x - o] : 0ull;
-            __syncthreads();
-            sh[threadIdx.x] += t;
-            __syncthreads();
-        }
-        ghist[p * kMaxRadix + threadIdx.x] = sh[threadIdx.x] - v;
-        __syncthreads();
-    }
-}
 
 // Bulk (TMA engine) copy of a full tile from global to shared memory,
 // completing on an mbarrier: one thread issues it, every thread waits.
@@ -465,24 +351,9 @@ __global__ void __launch_bounds__(kSortThreads, SortShape<KT>::min_blocks) k_one
 
 }  // namespace
 
-void scan_partials_u64(uint64_t* partial, uint64_t m, cudaStream_t s, uint64_t* total_host) {
-    k_scan_partials<uint64_t><<<1, 1024, 0, s>>>(partial, m);
-    COLO_LAUNCH_CHECK();
-    count_launch();
-    if (total_host) {
-        COLO_CUDA(cudaMemcpyAsync(total_host, partial + m, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-        stream_wait(s);
-    }
-}
-
 void scan_u32_to_u64(const uint32_t* in, uint64_t* out, uint64_t n, cudaStream_t s,
                      uint64_t* total_host, uint64_t* total_dev) {
     scan_impl<uint32_t, uint64_t>(in, out, n, s, total_host, total_dev);
-}
-
-void scan_u32_to_u32(const uint32_t* in, uint32_t* out, uint64_t n, cudaStream_t s,
-                     uint32_t* total_host, uint32_t* total_dev) {
-    scan_impl<uint32_t, uint32_t>(in, out, n, s, total_host, total_dev);
 }
 
 void scan_u64_to_u64(const uint64_t* in, uint64_t* out, uint64_t n, cudaStream_t s,
@@ -493,85 +364,45 @@ void scan_u64_to_u64(const uint64_t* in, uint64_t* out, uint64_t n, cudaStream_t
 namespace {
 
 template <class KT>
-void radix_sort_impl(DevBuf<KT>& keys, DevBuf<uint32_t>& vals, uint64_t n, int bits, cudaStream_t s,
-                     const char* name, unsigned long long* hist_in, uint32_t* err_dev, uint32_t test_spin,
-                     bool iota_vals) {
-    if (n <= 1 || bits <= 0) return;   // no pass: vals is left as given, iota_vals or not
+void radix_sort_impl(RadixBufs<KT>& bufs, uint64_t n, const RadixPlan& plan, cudaStream_t s,
+                     const unsigned long long* hist, unsigned long long* status, bool shared, uint32_t* tickets,
+                     uint32_t* err, uint32_t test_spin) {
     if (n >= (1ull << 32)) throw StatusError{COLO_ERR_CAPACITY, "radix sort supports < 2^32 items"};
-    const RadixPlan plan = radix_plan(bits);
     using SM = SortSmem<KT, kMaxRadixBits>;
     const uint32_t ntiles = (uint32_t)((n + SM::tile - 1) / SM::tile);
-    DevBuf<KT> k2;
-    DevBuf<uint32_t> v2, tickets, err;
-    DevBuf<unsigned long long> ghist, status;
-    k2.alloc(n, s);
-    v2.alloc(n, s);
-    if (!hist_in) ghist.alloc((uint64_t)plan.n * kMaxRadix, s);
-    unsigned long long* hist = hist_in ? hist_in : ghist.get();
-    status.alloc((uint64_t)ntiles * kMaxRadix, s);
-    tickets.alloc(plan.n, s);
-    tickets.zero(s);
-    if (!err_dev) {
-        err.alloc(1, s);
-        err.zero(s);
-    }
-    uint32_t* errp = err_dev ? err_dev : err.get();
-    {
-        KScope ks("radix_hist");
-        if (!hist_in) {
-            ghist.zero(s);
-            uint64_t blocks = (n + 255) / 256;
-            if (blocks > 1024) blocks = 1024;
-            k_digit_hist<KT><<<(unsigned)blocks, 256, 0, s>>>(keys.get(), n, plan, hist);
-            COLO_LAUNCH_CHECK();
-            count_launch();
-        }
-        k_digit_scan<<<1, kMaxRadix, 0, s>>>(hist, plan.n);
-        COLO_LAUNCH_CHECK();
-        count_launch();
-    }
-    KT* ka = keys.get();
-    uint32_t* va = vals.get();
-    KT* kb = k2.get();
-    uint32_t* vb = v2.get();
     // several blocks per SM: ask for the largest shared-memory carveout
     COLO_CUDA(cudaFuncSetAttribute((const void*)k_onesweep<KT, kMaxRadixBits>,
                                    cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     COLO_CUDA(cudaFuncSetAttribute((const void*)k_onesweep<KT, kMaxRadixBits>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM::bytes));
     for (int p = 0; p < plan.n; ++p) {
-        KScope ks(name);   // one timed launch per digit pass
+        KScope ks("radix_sort");   // one timed launch per digit pass
         const uint32_t dm = (1u << plan.width[p]) - 1u;
-        // the words of the digits in use are cleared for every pass (a pitched clear:
+        // shared words: those of the digits in use are cleared for every pass (a pitched clear:
         // a tile's words stay kMaxRadix apart, which spreads the polled lines over L2)
-        COLO_CUDA(cudaMemset2DAsync(status.get(), kMaxRadix * 8, 0, ((size_t)1 << plan.width[p]) * 8, ntiles, s));
-        const int bulk = ((uintptr_t)ka % 16 == 0 && (uintptr_t)va % 16 == 0) ? 1 : 0;
-        // the first pass of a sort of positions generates them (no read)
-        const uint32_t* vin = (iota_vals && p == 0) ? nullptr : va;
-        k_onesweep<KT, kMaxRadixBits><<<ntiles, SM::T, SM::bytes, s>>>(ka, vin, kb, vb, n, plan.shift[p], dm,
-                                                                     hist + p * kMaxRadix, status.get(),
-                                                                     tickets.get() + p, errp, bulk,
+        unsigned long long* st = status + (shared ? 0 : (uint64_t)p * ntiles * kMaxRadix);
+        if (shared)
+            COLO_CUDA(cudaMemset2DAsync(st, kMaxRadix * 8, 0, ((size_t)1 << plan.width[p]) * 8, ntiles, s));
+        const int bulk = ((uintptr_t)bufs.ka % 16 == 0 && (uintptr_t)bufs.va % 16 == 0) ? 1 : 0;
+        const uint32_t* vin = p == 0 ? nullptr : bufs.va;   // the first pass makes the ids (no read)
+        k_onesweep<KT, kMaxRadixBits><<<ntiles, SM::T, SM::bytes, s>>>(bufs.ka, vin, bufs.kb, bufs.vb, n, plan.shift[p], dm,
+                                                                     hist + p * kMaxRadix, st, tickets + p, err, bulk,
                                                                      test_spin ? test_spin : kSpinLimit,
                                                                      test_spin && p == 0 ? 1 : 0, p);
         COLO_LAUNCH_CHECK();
         count_launch();
-        std::swap(ka, kb);
-        std::swap(va, vb);
+        std::swap(bufs.ka, bufs.kb);
+        std::swap(bufs.va, bufs.vb);
     }
-    if (ka != keys.get()) {   // an odd number of passes: the result is in the second buffers
-        keys.swap(k2);
-        vals.swap(v2);
-    }
-    // the caller reads the error word at its next wait; until then its kernels read the
-    // output with ids checked against n (a timed-out pass leaves ids unwritten)
-    if (err_dev) return;
-    uint32_t herr = 0;
-    COLO_CUDA(cudaMemcpyAsync(&herr, err.get(), 4, cudaMemcpyDeviceToHost, s));
-    stream_wait(s);
-    if (herr) throw StatusError{COLO_ERR_TIMEOUT, "radix sort: a tile waited too long for its predecessors"};
 }
 
 }  // namespace
+
+uint64_t radix_status_words(uint64_t n) {
+    static_assert(SortSmem<uint32_t, kMaxRadixBits>::tile == SortSmem<uint64_t, kMaxRadixBits>::tile, "one tile size");
+    const uint64_t tile = SortSmem<uint32_t, kMaxRadixBits>::tile;
+    return (n + tile - 1) / tile * kMaxRadix;
+}
 
 RadixPlan radix_plan(int bits) {
     // fewest passes of at most 8 bits, widths as even as possible (25 bits: 7 + 6 + 6 + 6)
@@ -586,14 +417,16 @@ RadixPlan radix_plan(int bits) {
     return plan;
 }
 
-void radix_sort(DevBuf<uint64_t>& keys, DevBuf<uint32_t>& vals, uint64_t n, int bits, cudaStream_t s,
-                const char* name, unsigned long long* hist, uint32_t* err_dev, uint32_t test_spin, bool iota_vals) {
-    radix_sort_impl<uint64_t>(keys, vals, n, bits, s, name, hist, err_dev, test_spin, iota_vals);
+void radix_sort(RadixBufs<uint32_t>& bufs, uint64_t n, const RadixPlan& plan, cudaStream_t s,
+                const unsigned long long* hist, unsigned long long* status, bool shared, uint32_t* tickets,
+                uint32_t* err, uint32_t test_spin) {
+    radix_sort_impl<uint32_t>(bufs, n, plan, s, hist, status, shared, tickets, err, test_spin);
 }
 
-void radix_sort(DevBuf<uint32_t>& keys, DevBuf<uint32_t>& vals, uint64_t n, int bits, cudaStream_t s,
-                const char* name, unsigned long long* hist, uint32_t* err_dev, uint32_t test_spin, bool iota_vals) {
-    radix_sort_impl<uint32_t>(keys, vals, n, bits > 32 ? 32 : bits, s, name, hist, err_dev, test_spin, iota_vals);
+void radix_sort(RadixBufs<uint64_t>& bufs, uint64_t n, const RadixPlan& plan, cudaStream_t s,
+                const unsigned long long* hist, unsigned long long* status, bool shared, uint32_t* tickets,
+                uint32_t* err, uint32_t test_spin) {
+    radix_sort_impl<uint64_t>(bufs, n, plan, s, hist, status, shared, tickets, err, test_spin);
 }
 
 }  // namespace colo

@@ -37,7 +37,10 @@ colo_status colo_stage_cells(colo_ctx* ctx, colo_dataset* ds, float R, uint64_t*
         colo_dataset* dsv[1] = {ds};
         setup_batch(ctx, dsv, &p, 1, b, of, nullptr);
         b.keep_scell = cell_of != nullptr;
-        if (b.N) bucket_points(b);
+        if (b.N) {
+            bucket_points(b);
+            settle(ctx, b, nullptr);
+        }
         cudaStream_t s = ctx->s;
         uint64_t cap = *nruns;
         *nruns = b.Rn;
@@ -53,17 +56,17 @@ colo_status colo_stage_cells(colo_ctx* ctx, colo_dataset* ds, float R, uint64_t*
         }
         if ((run_cell || run_feat || run_count) && b.Rn) {
             if (cap < b.Rn) return COLO_ERR_CAPACITY;
-            std::vector<uint32_t> rf(b.Rn), rc(b.Rn), rcell(b.Rn);
+            std::vector<uint32_t> rf(b.Rn), rs(b.Rn + 1), rcell(b.Rn);
             std::vector<uint64_t> ckey(b.M);
             COLO_CUDA(cudaMemcpyAsync(rf.data(), b.rfeat.get(), b.Rn * 4, cudaMemcpyDeviceToHost, s));
-            COLO_CUDA(cudaMemcpyAsync(rc.data(), b.rcnt.get(), b.Rn * 4, cudaMemcpyDeviceToHost, s));
+            COLO_CUDA(cudaMemcpyAsync(rs.data(), b.rstart.get(), (b.Rn + 1) * 4, cudaMemcpyDeviceToHost, s));
             COLO_CUDA(cudaMemcpyAsync(rcell.data(), b.rcell.get(), b.Rn * 4, cudaMemcpyDeviceToHost, s));
             COLO_CUDA(cudaMemcpyAsync(ckey.data(), b.ckey.get(), b.M * 8, cudaMemcpyDeviceToHost, s));
             COLO_CUDA(cudaStreamSynchronize(s));
             for (uint64_t r = 0; r < b.Rn; ++r) {
                 if (run_cell) run_cell[r] = ckey[rcell[r]];
                 if (run_feat) run_feat[r] = rf[r];
-                if (run_count) run_count[r] = rc[r];
+                if (run_count) run_count[r] = rs[r + 1] - rs[r];
             }
         }
         return COLO_OK;
@@ -83,6 +86,7 @@ colo_status colo_stage_neighbors(colo_ctx* ctx, colo_dataset* ds, float R, uint6
         if (b.N) {
             bucket_points(b);
             build_neighborhoods(b);
+            settle(ctx, b, nullptr);
             join_neighbors(b);
         }
         *total = neighbor_entries(b);
@@ -120,19 +124,18 @@ colo_status colo_stage_filter(colo_ctx* ctx, colo_dataset* ds, float R, float th
         std::vector<DevBuf<float>> of;
         colo_dataset* dsv[1] = {ds};
         setup_batch(ctx, dsv, &p, 1, b, of, nullptr);
-        if (b.N) bucket_points(b);
+        std::vector<uint32_t> h;
+        if (b.N) {
+            bucket_points(b);
+            if (k == 2 && ncand) filter_pairs(b);
+            settle(ctx, b, &h);
+        }
         for (uint64_t c = 0; c < ncand * k; ++c)
             if (cand[c] >= b.F) return COLO_ERR_ARG;
         cudaStream_t s = ctx->s;
         std::vector<uint64_t> hub(ncand * k, 0);
         if (b.N && ncand) {
             if (k == 2) {
-                DevBuf<uint32_t> ub2;
-                std::vector<uint64_t> job_off;
-                filter_pairs(b, ub2, job_off, s);
-                COLO_CUDA(cudaStreamSynchronize(s));
-                std::vector<uint32_t> h(job_off[1]);
-                COLO_CUDA(cudaMemcpy(h.data(), ub2.get(), h.size() * 4, cudaMemcpyDeviceToHost));
                 uint32_t nf = b.F;
                 for (uint64_t c = 0; c < ncand; ++c) {
                     uint32_t a = cand[2 * c], bb = cand[2 * c + 1];
@@ -260,6 +263,7 @@ colo_status colo_autotune(colo_ctx* ctx, colo_dataset* ds, const colo_params* p,
         if (b.N) {
             bucket_points(b);
             build_neighborhoods(b);
+            settle(ctx, b, nullptr);
             cudaEvent_t e0, e1;
             COLO_CUDA(cudaEventCreate(&e0));
             COLO_CUDA(cudaEventCreate(&e1));
@@ -397,7 +401,10 @@ colo_status colo_autotune_all(colo_ctx* ctx, colo_dataset* ds, const colo_params
         std::vector<DevBuf<float>> of;
         colo_dataset* dsv[1] = {ds};
         setup_batch(ctx, dsv, p, 1, b, of, nullptr);
-        if (b.N) bucket_points(b);
+        if (b.N) {
+            bucket_points(b);
+            settle(ctx, b, nullptr);
+        }
         key.m = b.M;
         return COLO_OK;
     });

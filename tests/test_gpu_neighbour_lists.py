@@ -1,5 +1,5 @@
 """The one-pass neighbourhood lists at the edges of their paths: cells whose anchors are listed by one
-thread (up to 32) or by the whole warp, lists merged by one thread (up to 64 entries) or by the warp, and
+thread (up to 32) or by the whole warp, lists merged by one thread (up to 128 entries) or by the warp, and
 more entries than the first allocation holds (four a run plus 65,536), which builds the lists again.  The
 neighbour lists equal the oracle's exactly."""
 import numpy as np
@@ -36,10 +36,10 @@ def test_anchors_per_cell(per, cells):
     _check(x, y, fid, np.array([0.0, 0.0, 30.0 * cells + 20.0, 40.0], np.float32), 10.0)
 
 
-@pytest.mark.parametrize("features,side", [(40, 45), (8, 20), (9, 20), (3, 330)])
+@pytest.mark.parametrize("features,side", [(40, 45), (15, 20), (16, 20), (3, 330)])
 def test_list_lengths(features, side):
     """Every cell of a side x side grid holds one point of every feature: nine times (features - 1) entries an
-    inner cell (63 and 72: both sides of the long-list limit).  40 features on 45 x 45 cells need more than four
+    inner cell (126 and 135: both sides of the long-list limit).  40 features on 45 x 45 cells need more than four
     entries a run; 330 x 330 cells are more than the grid's warps take one each."""
     rng = np.random.default_rng(features)
     gx, gy = np.meshgrid(np.arange(side), np.arange(side))
