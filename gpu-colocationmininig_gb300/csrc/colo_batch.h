@@ -170,20 +170,29 @@ void filter_level(Batch& b, const uint32_t* h_cand, const uint32_t* h_job, uint6
                   uint32_t* d_ub, unsigned long long* d_stats, const uint32_t* d_cand = nullptr);
 
 // colo_level.cu --------------------------------------------------------------
-// One candidate's view for the level kernels.
+// One member of a candidate: its feature's first point id and instances, and where its
+// participation bitmap starts (words from the candidate's bm_base).
+struct alignas(16) MemberInfo {
+    uint32_t start, n, off, feature;
+};
+
+// One candidate's view for the level kernels.  What a kernel needs first (the last member's
+// id range, the threshold) is written out, so that it waits on one load.
 struct CandDesc {
     const uint32_t* parent;      // column-major parent table (k-1 columns); nullptr: implicit (k=2)
     uint64_t prow;               // parent rows (k=2: anchors of member 0)
     uint64_t pstride;            // parent column stride (>= prow)
-    uint32_t m[kMaxK];           // member features
-    uint32_t* slots;             // per parent row counts (count pass output)
-    const uint64_t* offs;        // per parent row output offsets (fill pass input)
+    const MemberInfo* mem;       // its k members
+    uint32_t* chunk_rows;        // rows per chunk of 32 parent rows (count pass output)
+    const uint64_t* offs;        // the level's scan of them from this candidate's first chunk on (fill pass input)
     uint32_t* out;               // column-major output table (k columns, rows = total)
     uint64_t out_rows;           // rows of the output table (column stride)
     uint64_t out_cap;            // capacity (single-pass mode; also its column stride)
     unsigned long long* rows;    // count pass: rows of this candidate (atomic sum)
-    uint32_t* bitmap;            // member bitmaps: member j's words start at bm_base plus
-    uint64_t bm_base;            // the sum over i < j of ceil(fcount[m[i]] / 32)
+    uint32_t* bitmap;            // the level's bitmap words; this candidate's members' start at
+    uint64_t bm_base;            // bm_base + their off
+    uint32_t last_start, last_end, last_off;   // the last member's point ids and bitmap offset
+    float R2, R2hu;              // the job's threshold (JobGrid)
     uint32_t job;
     uint32_t k;
 };
@@ -198,10 +207,25 @@ struct LevelWork {
     unsigned long long* ticket = nullptr;         // single pass: chunk ticket counter, zeroed
 };
 
-// count pass: slots + bitmaps; fill pass: rows; single pass: slots +
-// bitmaps + rows at their count-and-fill positions (overflow recorded per
+// The count pass's candidates in groups that share a parent table: group g is candidates
+// gstart[g] .. gstart[g+1] (at most kGroupMax), neighbours in the candidate order, and its chunks
+// of parent rows start at gchunk[g].
+constexpr uint32_t kGroupMax = 32;
+struct CountWork {
+    const CandDesc* cands;       // device arrays
+    const uint32_t* gstart;
+    const uint64_t* gchunk;
+    uint64_t ngroups;
+    uint64_t nchunks;            // of all groups
+    unsigned long long* items;   // optional: sum of candidate-slice lengths examined
+    unsigned long long* ticket;  // chunk tickets of the persistent queue, zeroed
+    uint64_t chunk0 = 0;         // gchunk[0]
+};
+
+// count pass: rows per chunk + bitmaps; fill pass: rows; single pass: rows per
+// chunk + bitmaps + rows at their count-and-fill positions (overflow recorded per
 // candidate; a look-back that waits too long sets the batch's timeout flag).
-void level_count(Batch& b, const LevelWork& w, uint32_t k);
+void level_count(Batch& b, const CountWork& w, uint32_t k);
 void level_fill(Batch& b, const LevelWork& w, uint32_t k);
 void level_single(Batch& b, const LevelWork& w, uint32_t k, uint32_t* d_overflow);
 // Participation statistics per candidate and member: [A, last, first, full]

@@ -71,6 +71,15 @@ __device__ __forceinline__ uint64_t lower_bound_dev(const T* a, uint64_t lo, uin
     return lo;
 }
 
+__device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* __restrict__ a, uint32_t lo, uint32_t hi, uint32_t v) {
+    while (lo < hi) {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        if (a[mid] < v) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
 // Number of set bits of the W-word mask m below bit b.  A cell's runs ascend
 // by feature and its mask has one bit per feature present, so for local
 // feature b the run index in the cell is crun + mask_rank(mask, b).

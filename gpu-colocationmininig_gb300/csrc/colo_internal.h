@@ -334,6 +334,10 @@ inline void stream_wait(cudaStream_t s) {
     COLO_CUDA(cudaStreamSynchronize(s));
     if (g_ktimer) g_ktimer->note_wait();
 }
+inline void event_wait(cudaEvent_t e) {
+    COLO_CUDA(cudaEventSynchronize(e));
+    if (g_ktimer) g_ktimer->note_wait();
+}
 struct KScope {
     explicit KScope(const char* name) {
         if (g_ktimer) g_ktimer->begin(name);
@@ -353,6 +357,9 @@ void scan_u32_to_u64(const uint32_t* in, uint64_t* out, uint64_t n, cudaStream_t
                      uint64_t* total_host, uint64_t* total_dev = nullptr);
 void scan_u64_to_u64(const uint64_t* in, uint64_t* out, uint64_t n, cudaStream_t s,
                      uint64_t* total_host, uint64_t* total_dev = nullptr);
+// The same with the caller's cleared look-back words (scan_words(n)); no total, launch only.
+uint64_t scan_words(uint64_t n);
+void scan_u32_to_u64(const uint32_t* in, uint64_t* out, uint64_t n, unsigned long long* words, cudaStream_t s);
 // Digit split of a radix sort: pass p sorts width[p] (<= 8) bits from shift[p].
 constexpr int kRadixDigits = 256;
 constexpr int kRadixMaxPasses = 8;

@@ -105,12 +105,7 @@ void ctx_release(colo_ctx* ctx) {
         cudaStreamSynchronize(ctx->s);
         cudaStreamDestroy(ctx->s);
     }
-    if (ctx->s2) {
-        cudaStreamSynchronize(ctx->s2);
-        cudaStreamDestroy(ctx->s2);
-    }
     if (ctx->ev_counted) cudaEventDestroy(ctx->ev_counted);
-    if (ctx->ev_scanned) cudaEventDestroy(ctx->ev_scanned);
     if (ctx->stage) cudaFreeHost(ctx->stage);
     if (ctx->ustage) cudaFreeHost(ctx->ustage);
     delete ctx;
@@ -293,12 +288,14 @@ struct Readback {
         items.push_back({dst, off, bytes});
         off += bytes;
     }
-    void finish() {
-        stream_wait(s);
+    // `ev`: an event recorded after the last copy (work queued behind it is not waited for)
+    void finish(cudaEvent_t ev = nullptr) {
+        if (ev) event_wait(ev);
+        else stream_wait(s);
         for (const Item& it : items) std::memcpy(it.dst, static_cast<char*>(ctx->stage) + it.off, it.bytes);
         items.clear();
         off = 0;
-        ctx->ustage_off = 0;   // the stream has drained: every upload staged so far has landed
+        ctx->ustage_off = 0;   // every upload staged so far has landed
     }
 };
 
@@ -346,28 +343,34 @@ struct ArenaSpan {
 };
 
 // The refinement's per-level device buffers, carved from one stream-ordered
-// allocation with the zero-initialised ones (bitmap, rows, chunk status, overflow)
+// allocation with the zero-initialised ones (bitmap, rows, look-back words, overflow)
 // adjacent, so that a level costs one allocation, one clear and one free
 // instead of nine, four and nine.  Parts start on 256-byte boundaries.
 struct LevelArena {
-    DevBuf<unsigned char> mem;
+    DevBuf<unsigned char> block;
     ArenaSpan<uint32_t> bitmap;
     ArenaSpan<unsigned long long> rows;
     ArenaSpan<unsigned long long> items;    // candidate-slice entries examined (work counter)
     ArenaSpan<unsigned long long> status;   // single pass: per chunk look-back word, then the chunk ticket
     ArenaSpan<unsigned long long> tickets;  // chunk tickets of the count and fill launches (persistent queue)
     ArenaSpan<uint32_t> overflow;           // single pass: 1 when the table outgrew its capacity
-    ArenaSpan<uint32_t> slots;
+    ArenaSpan<unsigned long long> words;    // look-back words of the chunk scan
+    ArenaSpan<uint32_t> chunk_rows;         // rows per chunk of 32 parent rows, single pass first
+    ArenaSpan<uint64_t> offs;               // their scan: the fill's output offsets
     ArenaSpan<CandDesc> descs;
     ArenaSpan<uint64_t> chunk_off;
+    ArenaSpan<uint64_t> gchunk;
+    ArenaSpan<uint32_t> gstart;
+    ArenaSpan<MemberInfo> mem;
     ArenaSpan<uint64_t> stats;
     // the refine's results (rows | items | overflow | stats) and inputs (descs | chunk
-    // prefixes) are each one contiguous block: one copy back, one copy in
-    size_t out_bytes = 0, in_bytes = 0, chunk_at = 0;
+    // prefixes | groups | members) are each one contiguous block: one copy back, one copy in
+    size_t out_bytes = 0, in_bytes = 0, chunk_at = 0, gchunk_at = 0, gstart_at = 0, mem_at = 0;
     unsigned char* out = nullptr;
     unsigned char* in = nullptr;
 
-    void init(uint64_t nslots, uint64_t nwords, uint64_t ncand, uint64_t nchunks, uint32_t k, bool single,
+    // nchunks: the single pass's; nall: all chunks
+    void init(uint64_t nall, uint64_t nwords, uint64_t ncand, uint64_t nchunks, uint32_t k, bool single,
               cudaStream_t s) {
         size_t off = 0;
         auto take = [&](uint64_t bytes) {
@@ -381,13 +384,18 @@ struct LevelArena {
         const size_t o_status = single ? take((nchunks + 1) * 8) : 0;
         const size_t o_tickets = take(2 * 8);
         const size_t o_bitmap = take(std::max<uint64_t>(nwords, 1) * 4);
+        const size_t o_words = take(scan_words(nall) * 8);
         const size_t zeroed = off;
-        const size_t o_slots = take(std::max<uint64_t>(nslots, 1) * 4);
+        const size_t o_rows = take(std::max<uint64_t>(nall, 1) * 4);
+        const size_t o_offs = take(std::max<uint64_t>(nall, 1) * 8);
         chunk_at = (std::max<uint64_t>(ncand, 1) * sizeof(CandDesc) + 15) & ~(size_t)15;
-        in_bytes = chunk_at + (ncand + 2) * 8;
+        gchunk_at = chunk_at + (ncand + 2) * 8;
+        gstart_at = gchunk_at + (ncand + 1) * 8;
+        mem_at = (gstart_at + (ncand + 1) * 4 + 15) & ~(size_t)15;
+        in_bytes = mem_at + ncand * k * sizeof(MemberInfo);
         const size_t o_in = take(in_bytes);
-        mem.alloc(off, s);
-        unsigned char* b = mem.get();
+        block.alloc(off, s);
+        unsigned char* b = block.get();
         out = b + o_out;
         in = b + o_in;
         rows.p = reinterpret_cast<unsigned long long*>(out);
@@ -397,16 +405,26 @@ struct LevelArena {
         status.p = single ? reinterpret_cast<unsigned long long*>(b + o_status) : nullptr;
         tickets.p = reinterpret_cast<unsigned long long*>(b + o_tickets);
         bitmap.p = reinterpret_cast<uint32_t*>(b + o_bitmap);
-        slots.p = reinterpret_cast<uint32_t*>(b + o_slots);
+        words.p = reinterpret_cast<unsigned long long*>(b + o_words);
+        chunk_rows.p = reinterpret_cast<uint32_t*>(b + o_rows);
+        offs.p = reinterpret_cast<uint64_t*>(b + o_offs);
         descs.p = reinterpret_cast<CandDesc*>(in);
         chunk_off.p = reinterpret_cast<uint64_t*>(in + chunk_at);
+        gchunk.p = reinterpret_cast<uint64_t*>(in + gchunk_at);
+        gstart.p = reinterpret_cast<uint32_t*>(in + gstart_at);
+        mem.p = reinterpret_cast<MemberInfo*>(in + mem_at);
         COLO_CUDA(cudaMemsetAsync(b, 0, zeroed, s));
     }
-    // descs and chunk prefixes in one upload
-    void put_inputs(colo_ctx* ctx, cudaStream_t s, const std::vector<CandDesc>& hd, const std::vector<uint64_t>& ch) {
+    // descs, chunk prefixes, groups and members (written by `put_members` in the staging) in one upload
+    template <class Fn>
+    void put_inputs(colo_ctx* ctx, cudaStream_t s, const std::vector<CandDesc>& hd, const std::vector<uint64_t>& ch,
+                    const std::vector<uint64_t>& gc, const std::vector<uint32_t>& gs, Fn&& put_members) {
         unsigned char* h = upload_area(ctx, s, in_bytes);
         std::memcpy(h, hd.data(), hd.size() * sizeof(CandDesc));
-        std::memcpy(h + chunk_at, ch.data(), std::min<size_t>(ch.size() * 8, in_bytes - chunk_at));
+        std::memcpy(h + chunk_at, ch.data(), std::min<size_t>(ch.size() * 8, gchunk_at - chunk_at));
+        std::memcpy(h + gchunk_at, gc.data(), gc.size() * 8);
+        std::memcpy(h + gstart_at, gs.data(), gs.size() * 4);
+        put_members(reinterpret_cast<MemberInfo*>(h + mem_at));
         upload_from(s, in, h, in_bytes);
     }
 };
@@ -925,17 +943,16 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         t0 = Clock::now();
         std::vector<CandDesc> hd;
         std::vector<std::pair<uint32_t, size_t>> owner;
-        std::vector<uint64_t> slot_base, chunk_off(1, 0);
+        std::vector<uint64_t> chunk_off(1, 0);
         {
             size_t most = 0;   // every candidate of the level passes at most
             for (uint32_t j = 0; j < J; ++j)
                 if (tr[j]) most += tr[j]->cand.size() / k;
             hd.reserve(most);
             owner.reserve(most);
-            slot_base.reserve(most);
             chunk_off.reserve(most + 1);
         }
-        uint64_t nslots = 0, nwords = 0;
+        uint64_t nwords = 0;
         for (uint32_t j = 0; j < J; ++j) {
             if (!tr[j]) continue;
             LevelTrace& L = *tr[j];
@@ -955,15 +972,19 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
                     d.prow = pt.rows;
                     d.pstride = pt.stride;
                 }
-                for (uint32_t t = 0; t < k; ++t) d.m[t] = mem[t];
                 d.job = j;
                 d.k = k;
+                d.R2 = b.jobs[j].grid.R2;
+                d.R2hu = b.jobs[j].grid.R2hu;
+                d.last_start = b.h_fstart[mem[k - 1]];
+                d.last_end = d.last_start + b.h_fcount[mem[k - 1]];
                 uint64_t w = 0;
-                for (uint32_t t = 0; t < k; ++t) w += (b.h_fcount[mem[t]] + 31) / 32;
+                for (uint32_t t = 0; t < k; ++t) {
+                    if (t + 1 == k) d.last_off = (uint32_t)w;
+                    w += (b.h_fcount[mem[t]] + 31) / 32;
+                }
                 d.bm_base = nwords;
                 nwords += w;
-                slot_base.push_back(nslots);
-                nslots += d.prow;
                 chunk_off.push_back(chunk_off.back() + (d.prow + 31) / 32);
                 hd.push_back(d);
                 owner.push_back({j, c});
@@ -984,7 +1005,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
             pc.resize(ncand);
             uint64_t words = 0;
             for (uint64_t q = 0; q < ncand; ++q) {
-                const uint64_t most = hd[q].prow * (uint64_t)b.h_fcount[hd[q].m[k - 1]];
+                const uint64_t most = hd[q].prow * (uint64_t)(hd[q].last_end - hd[q].last_start);
                 pc[q] = std::min(presize_rows(y[q]), std::max<uint64_t>(most, 1));
                 words += pc[q] * k;
             }
@@ -1013,19 +1034,16 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
             std::stable_sort(perm.begin(), mid, [&](uint64_t a, uint64_t c) { return pc[a] > pc[c]; });
             std::vector<CandDesc> hd2(ncand);
             std::vector<std::pair<uint32_t, size_t>> own2(ncand);
-            std::vector<uint64_t> sb2(ncand);
             cap.resize(ncand);
             chunk_off.assign(1, 0);
             for (uint64_t i = 0; i < ncand; ++i) {
                 hd2[i] = hd[perm[i]];
                 own2[i] = owner[perm[i]];
-                sb2[i] = slot_base[perm[i]];
                 cap[i] = pc[perm[i]];
                 chunk_off.push_back(chunk_off.back() + (hd2[i].prow + 31) / 32);
             }
             hd.swap(hd2);
             owner.swap(own2);
-            slot_base.swap(sb2);
         }
         // the single pass writes a table while counting it; it pays for tables predicted large
         // (a fill pass would walk them again), small ones are counted and the needed ones filled
@@ -1041,20 +1059,30 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         }
         if (ns == ncand) chunk_all.push_back(0);
         const uint64_t nch_single = chunk_all[ns], nch_count = chunk_all.back();
+        auto members = [&](uint64_t q) { return &tr[owner[q].first]->cand[owner[q].second * k]; };
+        // the counted candidates that share a parent table, counted together (the plain form counts
+        // one candidate at a time, as the reference refines)
+        std::vector<uint32_t> gstart;
+        std::vector<uint64_t> gchunk;
+        uint64_t gchunks = 0;
+        for (uint64_t q = ns; q < ncand; ++q) {
+            const bool same = !plain && !gstart.empty() && q - gstart.back() < kGroupMax &&
+                              owner[q].first == owner[q - 1].first &&
+                              std::equal(members(q), members(q) + (k - 1), members(q - 1));
+            if (same) continue;
+            gstart.push_back((uint32_t)q);
+            gchunk.push_back(gchunks);
+            gchunks += (hd[q].prow + 31) / 32;
+        }
+        const uint64_t ngroups = gstart.size();
+        gstart.push_back((uint32_t)ncand);
+        gchunk.push_back(gchunks);
         kt.mark("refine presize");
         LevelArena ar;
-        DevBuf<uint64_t> G;   // the fill's output offsets: the scan of every parent row's count
-        // the side stream's scan reads the arena and writes G: the main stream waits for it
-        // before either is freed, also when the level ends by an error
-        struct SideScan {
-            cudaStream_t s;
-            cudaEvent_t ev;
-            bool pending = false;
-            ~SideScan() {
-                if (pending) cudaStreamWaitEvent(s, ev, 0);
-            }
-        } side{s, ctx->ev_scanned};
-        ar.init(nslots, nwords, ncand, nch_single, k, ns > 0, s);
+        const uint64_t nch_all = nch_single + nch_count;
+        // candidate q's first chunk among all (the single pass's chunks come first)
+        auto first_chunk = [&](uint64_t q) { return q < ns ? chunk_all[q] : nch_single + chunk_all[q + 1]; };
+        ar.init(nch_all, nwords, ncand, nch_single, k, ns > 0, s);
         std::unique_ptr<TableBuf> single_cur;
         uint64_t single_words = 0;
         if (ns) {
@@ -1064,8 +1092,9 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
             if (single_cur->on_host()) cnt_host_table_bytes += single_words * 4;
         }
         for (uint64_t q = 0, o = 0; q < ncand; ++q) {
-            hd[q].slots = ar.slots.get() + slot_base[q];
+            hd[q].chunk_rows = ar.chunk_rows.get() + first_chunk(q);
             hd[q].bitmap = ar.bitmap.get();
+            hd[q].mem = ar.mem.get() + q * k;
             hd[q].rows = ar.rows.get() + q;
             if (q < ns) {
                 hd[q].out = single_cur->get() + o;
@@ -1081,20 +1110,22 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         cnt_bmw += nwords;
         for (uint64_t q = 0; q < ncand; ++q) cnt_parent += (uint64_t)(k - 1) * hd[q].prow;
         if (ncand) {
-            ar.put_inputs(ctx, s, hd, chunk_all);
+            ar.put_inputs(ctx, s, hd, chunk_all, gchunk, gstart, [&](MemberInfo* out) {
+                for (uint64_t q = 0; q < ncand; ++q) {
+                    const uint32_t* mem = members(q);
+                    uint32_t off = 0;
+                    for (uint32_t t = 0; t < k; ++t) {
+                        const uint32_t n = b.h_fcount[mem[t]];
+                        *out++ = MemberInfo{b.h_fstart[mem[t]], n, off, mem[t]};
+                        off += (n + 31) / 32;
+                    }
+                }
+            });
             if (plain) {
                 // per candidate, as the reference refines (one candidate at a time)
-                DevBuf<uint64_t> one_off;
-                one_off.alloc(2 * ncand, s);
-                std::vector<uint64_t> hoff(2 * ncand);
                 for (uint64_t q = 0; q < ncand; ++q) {
-                    hoff[2 * q] = 0;
-                    hoff[2 * q + 1] = chunk_off[q + 1] - chunk_off[q];
-                }
-                COLO_CUDA(cudaMemcpyAsync(one_off.get(), hoff.data(), 2 * ncand * 8, cudaMemcpyHostToDevice, s));
-                for (uint64_t q = 0; q < ncand; ++q) {
-                    LevelWork w{ar.descs.get() + q, one_off.get() + 2 * q, 1, hoff[2 * q + 1], ar.items.get()};
-                    level_count(b, w, k);
+                    level_count(b, CountWork{ar.descs.get(), ar.gstart.get() + q, ar.gchunk.get() + q, 1,
+                                             gchunk[q + 1] - gchunk[q], ar.items.get(), nullptr, gchunk[q]}, k);
                     level_pi(b, ar.descs.get() + q, 1, k, ar.stats.get() + q * k * 4);
                     COLO_CUDA(cudaMemcpyAsync(hstats.data() + q * k * 4, ar.stats.get() + q * k * 4, k * 4 * 8,
                                               cudaMemcpyDeviceToHost, s));
@@ -1108,24 +1139,8 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
                     level_single(b, w, k, ar.overflow.get());
                 }
                 if (ns < ncand) {
-                    LevelWork w{ar.descs.get() + ns, ar.chunk_off.get() + ns + 1, ncand - ns, nch_count, ar.items.get()};
-                    w.ticket = ar.tickets.get();
-                    level_count(b, w, k);
-                }
-                // the fill's output offsets (the scan of every row's count) on the side stream,
-                // during the participation kernel, the wait and the host's Apriori; the profiled
-                // pass keeps it on the main stream so that its timers see it
-                if (nslots) {
-                    G.alloc(nslots, s);
-                    if (!kt.on) {
-                        COLO_CUDA(cudaEventRecord(ctx->ev_counted, s));
-                        COLO_CUDA(cudaStreamWaitEvent(ctx->s2, ctx->ev_counted, 0));
-                        scan_u32_to_u64(ar.slots.get(), G.get(), nslots, ctx->s2, nullptr);
-                        COLO_CUDA(cudaEventRecord(ctx->ev_scanned, ctx->s2));
-                        side.pending = true;
-                    } else {
-                        scan_u32_to_u64(ar.slots.get(), G.get(), nslots, s, nullptr);
-                    }
+                    level_count(b, CountWork{ar.descs.get(), ar.gstart.get(), ar.gchunk.get(), ngroups, gchunks,
+                                             ar.items.get(), ar.tickets.get()}, k);
                 }
                 level_pi(b, ar.descs.get(), ncand, k, ar.stats.get());
             }
@@ -1138,8 +1153,11 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         if (ar.out_bytes) rb.copy(hout.data(), ar.out, ar.out_bytes);
         DevFlags hflags{};
         if (ns) rb.copy(&hflags, b.flags(), sizeof(hflags));
+        COLO_CUDA(cudaEventRecord(ctx->ev_counted, s));
+        // the fill's output offsets: the scan runs behind the copies, while the host reads them
+        if (ncand && !plain) scan_u32_to_u64(ar.chunk_rows.get(), ar.offs.get(), nch_all, ar.words.get(), s);
         kt.mark("refine launches");
-        rb.finish();
+        rb.finish(ctx->ev_counted);
         kt.mark("refine wait");
         if (ncand) {
             std::memcpy(hrows.data(), hout.data(), ncand * 8);
@@ -1309,24 +1327,17 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         tables_cur.reset(new TableBuf());
         tables_cur->alloc(total_rows * k ? total_rows * k : 1, s, host_tables);
         if (tables_cur->on_host()) cnt_host_table_bytes += total_rows * k * 4;
-        // output offsets of every parent row: exclusive scan of the slots (batched: already
-        // launched with the count, on the side stream; the main stream waits for it here)
-        if (side.pending) {
-            COLO_CUDA(cudaStreamWaitEvent(s, ctx->ev_scanned, 0));
-            side.pending = false;
-        }
-        if (!fillq.empty() && plain) {
-            G.alloc(nslots, s);
-            for (uint64_t q : fillq)   // one scan per candidate, as the reference does
-                scan_u32_to_u64(ar.slots.get() + slot_base[q], G.get() + slot_base[q], hd[q].prow, s, nullptr);
-        }
+        if (plain)   // one scan per candidate, as the reference does
+            for (uint64_t q : fillq)
+                scan_u32_to_u64(ar.chunk_rows.get() + first_chunk(q), ar.offs.get() + first_chunk(q),
+                                (hd[q].prow + 31) / 32, s, nullptr);
         std::vector<CandDesc> fd;
         std::vector<uint64_t> fchunk(1, 0);
         uint64_t obase = 0;
         for (uint64_t q : fillq) {
             CandDesc d = hd[q];
             uint64_t rows = gb[q + 1] - gb[q];
-            d.offs = G.get() + slot_base[q];
+            d.offs = ar.offs.get() + first_chunk(q);
             d.out = tables_cur->get() + obase;
             d.out_rows = rows;
             obase += rows * k;
@@ -1505,10 +1516,7 @@ colo_status colo_create(colo_ctx** out, int device) {
     c->device = device;
     if (cudaSetDevice(device) != cudaSuccess) return COLO_ERR_CUDA;
     if (cudaStreamCreateWithFlags(&c->s, cudaStreamNonBlocking) != cudaSuccess) return COLO_ERR_CUDA;
-    if (cudaStreamCreateWithFlags(&c->s2, cudaStreamNonBlocking) != cudaSuccess) return COLO_ERR_CUDA;
-    if (cudaEventCreateWithFlags(&c->ev_counted, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_scanned, cudaEventDisableTiming) != cudaSuccess)
-        return COLO_ERR_CUDA;
+    if (cudaEventCreateWithFlags(&c->ev_counted, cudaEventDisableTiming) != cudaSuccess) return COLO_ERR_CUDA;
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return COLO_ERR_CUDA;

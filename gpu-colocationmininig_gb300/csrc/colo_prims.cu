@@ -351,6 +351,19 @@ __global__ void __launch_bounds__(kSortThreads, SortShape<KT>::min_blocks) k_one
 
 }  // namespace
 
+uint64_t scan_words(uint64_t n) { return (n + kScan1Tile - 1) / kScan1Tile + 1; }
+
+void scan_u32_to_u64(const uint32_t* in, uint64_t* out, uint64_t n, unsigned long long* words, cudaStream_t s) {
+    const uint64_t tiles = (n + kScan1Tile - 1) / kScan1Tile;
+    if (tiles >= (1ull << 31)) throw StatusError{COLO_ERR_CAPACITY, "scan supports < 2^31 tiles"};
+    if (!tiles) return;
+    KScope ks("scan");
+    k_scan_1p<uint32_t, uint64_t><<<(unsigned)tiles, kScanThreads, 0, s>>>(
+        in, out, n, words, reinterpret_cast<uint32_t*>(words + tiles), nullptr);
+    COLO_LAUNCH_CHECK();
+    count_launch();
+}
+
 void scan_u32_to_u64(const uint32_t* in, uint64_t* out, uint64_t n, cudaStream_t s,
                      uint64_t* total_host, uint64_t* total_dev) {
     scan_impl<uint32_t, uint64_t>(in, out, n, s, total_host, total_dev);
