@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import ctypes as C
 from dataclasses import dataclass, field
+from functools import cached_property
 from pathlib import Path
 from typing import List, Optional, Sequence
 
@@ -117,7 +118,7 @@ def load(build: bool = True) -> C.CDLL:
         "colo_result_num_levels": (C.c_uint32, [_P]),
         "colo_result_level_size": (C.c_uint32, [_P, C.c_uint32]),
         "colo_result_level_candidates": (C.c_uint64, [_P, C.c_uint32]),
-        "colo_result_level": (C.c_int, [_P, C.c_uint32, _u32p, _u64p, _u8p, _u64p, _u64p, _f32p, _u8p, _u32p]),
+        "colo_result_level": (C.c_int, [_P, C.c_uint32] + [_P] * 8),
         "colo_result_table": (C.c_uint64, [_P, C.c_uint32, C.c_uint64, _u32p]),
         "colo_result_write_patterns": (C.c_int, [_P, _P, C.c_char_p]),
         "colo_result_times": (C.c_int, [_P, C.POINTER(C.c_double)]),
@@ -260,23 +261,38 @@ class Level:
 
 
 class Result:
-    def __init__(self, lib, handle):
+    """A mine's result; what it holds is read from the library when first asked for.  `params`: the mine's
+    parameters (tables and features that were not asked for are then not looked for)."""
+
+    def __init__(self, lib, handle, params: Optional[Params] = None):
         self._lib = lib
         self.h = handle
-        self._levels = None          # parsed on first access
+        self._levels = None
+        self._has_tables = params is None or params.keep_tables != 0
+        self._has_features = params is None or (params.reserved[0] & 2) != 0
+
+    @cached_property
+    def times(self) -> dict:
         t = (C.c_double * 8)()
-        lib.colo_result_times(handle, t)
-        self.times = dict(zip(["total", "upload", "bucket", "join", "filter", "refine", "fill", "apriori"], list(t)))
+        self._lib.colo_result_times(self.h, t)
+        return dict(zip(["total", "upload", "bucket", "join", "filter", "refine", "fill", "apriori"], list(t)))
+
+    @cached_property
+    def counters(self) -> dict:
         c = np.zeros(len(COUNTERS), np.uint64)
-        lib.colo_result_counters(handle, _ptr(c, _u64p), len(COUNTERS))
-        self.counters = dict(zip(COUNTERS, c.tolist()))
-        self.kernels = {}
-        for i in range(lib.colo_result_num_kernels(handle)):
+        self._lib.colo_result_counters(self.h, _ptr(c, _u64p), len(COUNTERS))
+        return dict(zip(COUNTERS, c.tolist()))
+
+    @cached_property
+    def kernels(self) -> dict:
+        out = {}
+        for i in range(self._lib.colo_result_num_kernels(self.h)):
             name = C.create_string_buffer(64)
             nl = C.c_uint64()
             ms = C.c_double()
-            lib.colo_result_kernel(handle, i, name, 64, C.byref(nl), C.byref(ms))
-            self.kernels[name.value.decode()] = (int(nl.value), float(ms.value))
+            self._lib.colo_result_kernel(self.h, i, name, 64, C.byref(nl), C.byref(ms))
+            out[name.value.decode()] = (int(nl.value), float(ms.value))
+        return out
 
     @property
     def levels(self) -> List[Level]:
@@ -290,20 +306,23 @@ class Result:
         for li in range(lib.colo_result_num_levels(handle)):
             k = lib.colo_result_level_size(handle, li)
             n = lib.colo_result_level_candidates(handle, li)
-            cand = np.zeros((n, k), np.uint32)
-            ub = np.zeros((n, k), np.uint64)
-            pas = np.zeros(n, np.uint8)
-            rows = np.zeros(n, np.uint64)
-            num = np.zeros((n, k), np.uint64)
-            pi = np.zeros(n, np.float32)
-            prev = np.zeros(n, np.uint8)
-            am = np.zeros(n, np.uint32)
-            lib.colo_result_level(handle, li, _ptr(cand, _u32p), _ptr(ub, _u64p), _ptr(pas, _u8p), _ptr(rows, _u64p),
-                                  _ptr(num, _u64p), _ptr(pi, _f32p), _ptr(prev, _u8p), _ptr(am, _u32p))
+            # the library writes every value of these
+            cand = np.empty((n, k), np.uint32)
+            ub = np.empty((n, k), np.uint64)
+            pas = np.empty(n, np.uint8)
+            rows = np.empty(n, np.uint64)
+            num = np.empty((n, k), np.uint64)
+            pi = np.empty(n, np.float32)
+            prev = np.empty(n, np.uint8)
+            am = np.empty(n, np.uint32)
+            lib.colo_result_level(handle, li, cand.ctypes.data, ub.ctypes.data, pas.ctypes.data, rows.ctypes.data,
+                                  num.ctypes.data, pi.ctypes.data, prev.ctypes.data, am.ctypes.data)
             feat = np.zeros((n, MODEL_FEATURES), np.float32)
-            lib.colo_result_features(handle, li, _ptr(feat, _f32p))
+            if self._has_features:
+                lib.colo_result_features(handle, li, _ptr(feat, _f32p))
             lev = Level(k, cand, ub, pas, rows, num, pi, prev, am, feat)
-            for c in range(n):
+            # only prevalent candidates can have a table (a call for each of 21,000 candidates took 10 of a mine's 14 ms)
+            for c in np.flatnonzero(prev).tolist() if self._has_tables else ():
                 r = lib.colo_result_table(handle, li, c, None)
                 if r != 2 ** 64 - 1:
                     t = np.zeros((r, k), np.uint32)
@@ -355,7 +374,7 @@ class Context:
     def mine(self, ds: "Dataset", params: Params) -> Result:
         out = _P()
         self.check(self.lib.colo_mine(self.h, ds.h, C.byref(params), C.byref(out)), "colo_mine")
-        return Result(self.lib, out)
+        return Result(self.lib, out, params)
 
     def mine_batch(self, dss: Sequence["Dataset"], params: Sequence[Params]) -> List[Result]:
         n = len(dss)
@@ -363,7 +382,7 @@ class Context:
         ps = (Params * n)(*params)
         outs = (_P * n)()
         self.check(self.lib.colo_mine_batch(self.h, hs, ps, n, outs), "colo_mine_batch")
-        return [Result(self.lib, outs[i]) for i in range(n)]
+        return [Result(self.lib, outs[i], params[i]) for i in range(n)]
 
     def stage_neighbors(self, ds: "Dataset", R: float):
         tot = C.c_uint64(0)
