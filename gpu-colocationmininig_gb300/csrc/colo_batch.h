@@ -28,7 +28,10 @@ struct alignas(128) BatchCtrl {
     uint32_t M, Rn;              // occupied cells, runs
     uint32_t keys_done;          // blocks of the cell-key pass that have added their histograms
     LineCounter nlistq;          // cells queued for a neighbourhood run list
-    LineCounter entries, anchors, capacity;   // of the lists; capacity of the single-pass layout = pair evaluations
+    // neighbourhood lists: target points, runs, anchors with short and with long lists, and the
+    // pair evaluations (= room that the single-pass join may need)
+    LineCounter targets, list_runs, anchors, long_anchors, pairs;
+    LineCounter nb_used;         // room taken by the single-pass join's tiles
 };
 
 struct Batch {
@@ -44,7 +47,7 @@ struct Batch {
     uint64_t Rn = 0;             // (cell, feature) runs (the same)
     uint64_t key_bits = 1;
     // Sizes that bucketing finds are kept on the device, and arrays over cells, runs, list
-    // entries and neighbours are laid out for an upper bound (capM, capR, nrl_cap, nb_cap), so
+    // entries and neighbours are laid out for an upper bound (capM, capR, targets_cap, nb_cap), so
     // that everything up to the pairs' bounds is queued without a host wait.  Batches whose
     // bounds are too large a reservation wait for the sizes instead (bounded = false).
     bool bounded = true;
@@ -104,21 +107,18 @@ struct Batch {
     Span<uint8_t> qfirst;        // per cell: bit q set when it is the first occupied cell of its quad q
     // runs: run r's points are sorted positions rstart[r] .. rstart[r+1] (rstart has an end entry)
     Span<uint32_t> rfeat, rstart, rcell;
-    // neighbourhood run lists: for each cell with targets, the runs of its
-    // adjacent cells ordered by (feature, cell), entries above the cell's lowest
-    // own feature, each the run's (first sorted position, point count); the
-    // lists are in no particular order
-    Span<uint2> nrl_ent;
-    uint64_t nrl_cap = 0, nrl_total = 0;
-    // per own run of those cells: first entry of its cell's list with a higher
-    // feature (absolute index), the entries from there to the list's end, and
-    // the number of target points in them
+    // neighbourhood lists: for each cell with targets, the points (sorted positions) of its
+    // adjacent cells' runs above the cell's lowest own feature, ordered by (feature, cell, id);
+    // the lists are in no particular order
+    Span<uint32_t> targets;
+    uint64_t targets_cap = 0, nrl_total = 0;   // nrl_total: runs in the lists
+    // scratch of the list kernel, per own run of those cells: first target with a higher
+    // feature (absolute index), and the targets from there to the list's end
     Span<uint64_t> run_sfx;
-    Span<uint32_t> run_qn;
     Span<uint32_t> run_L;
-    // the join's anchors (points of runs with targets), in no particular order:
-    // sorted position, start in the single-pass layout, first entry of the list
-    // slice (40 bits) and its entries (24 bits)
+    // the join's anchors (points of runs with targets), in no particular order: sorted
+    // position, number of targets, first target (low, high word); anchors of at most
+    // kLongList targets from the front, the others from the back
     Span<uint4> act;
     // neighbour lists N+(a) = nb[nb_beg[a] .. nb_beg[a] + nb_cnt[a]), each in
     // (feature, neighbour cell, id) order; nb_beg[a] is set only where nb_cnt[a] > 0
@@ -128,8 +128,9 @@ struct Batch {
     uint64_t nb_cap = 0;         // allocated entries (upper bound in single-pass mode)
     uint64_t join_pairs = 0;     // pair distance evaluations
     uint64_t active_anchors = 0; // anchors whose cell has higher-feature neighbours
+    uint64_t long_anchors = 0;   // of them, with long lists
     bool lists_built = false, join_queued = false;
-    int join_group = 8;          // lanes per anchor in the join (autotuned)
+    int join_group = 1;          // lanes per anchor in the join (autotuned): a warp takes 32 / join_group anchors
     int filter_unit = 32;        // candidates per warp unit in the level filter (autotuned: 8, 16, 32)
     int level_block = 256;       // threads per block of the level kernels (autotuned: 64, 128, 256)
     int level_queue = 0;         // 1: level count/fill kernels as a persistent work queue (autotuned)
@@ -143,6 +144,7 @@ void bucket_points(Batch& b);            // cells, runs, masks, nb9, runs per fe
 void build_neighborhoods(Batch& b);      // neighbourhood lists and anchors (launches)
 // colo_join.cu
 constexpr int kEntrySlots = 64, kEntryStride = 16;   // dE: counters on separate 128-byte lines
+constexpr uint32_t kLongList = 64;                   // targets above which an anchor gets a warp to itself
 constexpr uint64_t kSinglePassCap = 1ull << 30;      // largest single-pass layout (entries)
 void join_queue(Batch& b);               // single-pass join into nb_cap entries, skipped on the device when they
                                          // or the lists did not fit (bounded batches, before settle)

@@ -563,117 +563,124 @@ __device__ __forceinline__ int adjacent_cells(uint64_t c, const uint64_t* ckey, 
     return cnt;
 }
 
-// A cell's list keeps only the adjacent runs with a feature above the cell's
-// lowest own feature: the join reads a list from an own run's suffix on, and
-// the lowest own run's suffix starts past every entry of feature <= its own.
-// Most lists are then empty; the cells whose 3x3 mask allows one were queued
-// by k_quad_masks.
+// A cell's list keeps only the points of adjacent runs with a feature above the
+// cell's lowest own feature: an anchor reads the list from its own run's suffix
+// on, and the lowest own run's suffix starts past every entry of feature <= its
+// own.  Most lists are then empty; the cells whose 3x3 mask allows one were
+// queued by k_quad_masks.
 
-constexpr uint32_t kBigList = 128;       // cells with longer lists are merged by their whole warp
+constexpr uint32_t kBigRuns = 128, kBigPoints = 512;   // cells with longer lists are merged by their whole warp
 constexpr uint32_t kHeavyAnchors = 32;   // cells with more anchors are listed by their whole warp
 
-// The list of cell c by a whole warp.  In the full (feature, slot) order a run
-// of feature f in adjacent slot s is at the sum over slots of (#runs with
-// feature < f) plus the number of earlier slots that also hold f; the kept
-// list (from entry `first` on) drops the entries of feature <= the cell's
-// lowest own feature.  Per own run of the cell: the first entry with a higher
-// feature, the entries from there on, and the number of target points in them
-// (the points of each adjacent cell past its runs of features <= f), from one
+// Sorted positions st .. st + rc - 1 to dst for every lane; runs of more than 32
+// points by the whole warp.
+__device__ __forceinline__ void put_run(uint32_t* __restrict__ targets, uint64_t at, uint32_t st, uint32_t rc, int lane) {
+    if (rc <= 32)
+        for (uint32_t q = 0; q < rc; ++q) targets[at + q] = st + q;
+    for (uint32_t m = __ballot_sync(0xffffffffu, rc > 32); m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        const uint64_t aj = __shfl_sync(0xffffffffu, at, j);
+        const uint32_t sj = __shfl_sync(0xffffffffu, st, j), nj = __shfl_sync(0xffffffffu, rc, j);
+        for (uint32_t q = lane; q < nj; q += 32) targets[aj + q] = sj + q;
+    }
+}
+
+// The list of cell c by a whole warp, from `first` on.  In the full (feature,
+// slot) order the points of a run of feature f in adjacent slot s start at the
+// sum over slots of the points with a feature below f plus those of earlier
+// slots' runs of f; the kept list drops the points of feature <= the cell's
+// lowest own feature.  A slot's points are one range of sorted positions, so the
+// points before a run are a difference of run starts.  Per own run of the cell:
+// the first target with a higher feature and the targets from there on, from one
 // binary search per slot.
-__device__ __forceinline__ void nrl_cell_warp(uint64_t c, int l, uint64_t first, uint32_t kept,
-                                              const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob,
-                                              const JobGrid* __restrict__ grids, const int32_t* __restrict__ nb9,
-                                              const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ crun,
-                                              const uint32_t* __restrict__ rfeat, const uint32_t* __restrict__ rstart,
-                                              uint2* __restrict__ nrl_ent, uint64_t* run_sfx,
-                                              uint32_t* run_qn, uint32_t* run_L) {
+__device__ __forceinline__ void list_cell_warp(uint64_t c, int lane, uint64_t first, const uint64_t* __restrict__ ckey,
+                                               const uint32_t* __restrict__ cjob, const JobGrid* __restrict__ grids,
+                                               const int32_t* __restrict__ nb9, const uint32_t* __restrict__ crun,
+                                               const uint32_t* __restrict__ rfeat, const uint32_t* __restrict__ rstart,
+                                               uint32_t* __restrict__ targets, uint64_t* run_sfx, uint32_t* run_L) {
     int32_t adj[9];
     const int na = adjacent_cells(c, ckey, cjob, grids, nb9, adj);
     const uint32_t fmin = rfeat[crun[c]];
-    uint32_t q0[9], q1[9], pre[10];
-    uint64_t off0 = 0;
+    uint32_t q0[9], q1[9], pre[10];   // kept runs of each slot, and their number before it
+    uint64_t total = 0;
     pre[0] = 0;
 #pragma unroll
     for (int t = 0; t < 9; ++t) {
+        q0[t] = q1[t] = 0;
         if (t < na) {
-            q0[t] = crun[adj[t]];
             q1[t] = crun[adj[t] + 1];
-            off0 += lower_bound_dev(rfeat, (uint64_t)q0[t], (uint64_t)q1[t], fmin + 1) - q0[t];
-        } else {
-            q0[t] = q1[t] = 0;
+            q0[t] = (uint32_t)lower_bound_dev(rfeat, (uint64_t)crun[adj[t]], (uint64_t)q1[t], fmin + 1);
+            total += rstart[q1[t]] - rstart[q0[t]];
         }
         pre[t + 1] = pre[t] + (q1[t] - q0[t]);
     }
-    const uint64_t base = first - off0;   // where entry 0 of the full order would be
-    for (uint32_t e = l; e < pre[9]; e += 32) {
-        int sl = 0;
-        uint32_t r = 0;
+    for (uint32_t e0 = 0; e0 < pre[9]; e0 += 32) {
+        const uint32_t e = e0 + lane;
+        uint64_t at = first;
+        uint32_t st = 0, rc = 0;
+        if (e < pre[9]) {
+            int sl = 0;
+            uint32_t r = 0;
 #pragma unroll
-        for (int t = 0; t < 9; ++t)
-            if (e >= pre[t] && e < pre[t + 1]) {
-                sl = t;
-                r = q0[t] + (e - pre[t]);
-            }
-        const uint32_t f = rfeat[r];
-        if (f <= fmin) continue;
-        uint64_t pos = 0;
+            for (int t = 0; t < 9; ++t)
+                if (e >= pre[t] && e < pre[t + 1]) {
+                    sl = t;
+                    r = q0[t] + (e - pre[t]);
+                }
+            const uint32_t f = rfeat[r];
 #pragma unroll
-        for (int t = 0; t < 9; ++t) {
-            if (t < na) {
-                const uint32_t lb = (uint32_t)lower_bound_dev(rfeat, (uint64_t)q0[t], (uint64_t)q1[t], f);
-                pos += lb - q0[t];
-                if (t < sl && lb < q1[t] && rfeat[lb] == f) pos += 1;
+            for (int t = 0; t < 9; ++t) {
+                if (t < na) {
+                    uint32_t lb = (uint32_t)lower_bound_dev(rfeat, (uint64_t)q0[t], (uint64_t)q1[t], f);
+                    if (t < sl && lb < q1[t] && rfeat[lb] == f) lb += 1;   // earlier slots' runs of f come first
+                    at += rstart[lb] - rstart[q0[t]];
+                }
             }
+            st = rstart[r];
+            rc = rstart[r + 1] - st;
         }
-        nrl_ent[base + pos] = make_uint2(rstart[r], rstart[r + 1] - rstart[r]);
+        put_run(targets, at, st, rc, lane);
     }
-    for (uint32_t r = crun[c] + l; r < crun[c + 1]; r += 32) {
+    for (uint32_t r = crun[c] + lane; r < crun[c + 1]; r += 32) {
         const uint32_t f = rfeat[r];
-        uint64_t sfx = base;
-        uint32_t L = 0;
+        uint64_t before = 0;
 #pragma unroll
         for (int t = 0; t < 9; ++t) {
             if (t < na) {
                 const uint32_t ub = (uint32_t)lower_bound_dev(rfeat, (uint64_t)q0[t], (uint64_t)q1[t], f + 1);
-                sfx += ub - q0[t];
-                if (ub < q1[t]) L += cstart[adj[t] + 1] - rstart[ub];
+                before += rstart[ub] - rstart[q0[t]];
             }
         }
-        run_sfx[r] = sfx;
-        run_qn[r] = (uint32_t)(first + kept - sfx);
-        run_L[r] = L;
+        run_sfx[r] = first + before;
+        run_L[r] = (uint32_t)(total - before);
     }
 }
 
-// Neighbourhood run lists and the join's anchors in one pass over the queued
-// cells.  A thread takes a cell: its list is the 9-way merge, by (feature,
-// slot), of the adjacent cells' runs above the lowest own feature (each slot
-// ascending by feature).  The running point count P gives the suffix counts:
-// the cell's own run of feature f gets sfx = the first position after every
-// entry of feature <= f and L = (points in the list) - P(sfx).  Then every
-// point of an own run with targets (L > 0) is listed as an anchor with its
-// sorted position, its start in the single-pass layout, where it owns L entries
-// (32 bits: a layout of more than 2^30 entries is not used), and its list slice
-// (first entry sfx, entries qn), in one 16-byte word.
+// Neighbourhood lists and the join's anchors in one pass over the queued cells.
+// A thread takes a cell: its list is the 9-way merge, by (feature, slot), of the
+// adjacent cells' runs above the lowest own feature (each slot ascending by
+// feature), written as the runs' points.  The running point count P gives the
+// suffixes: the cell's own run of feature f reads the list from P targets on,
+// P taken after every entry of feature <= f.  Then every point of an own run with
+// targets is listed as an anchor, those with long lists from the array's back.
 //
-// Bound by the merge's chain of dependent loads.  The lists, anchors and
-// capacities are not in cell order: a warp reserves its 32 cells' room with one
-// atomic on each of the three totals (list entries, anchors, capacity), so
-// nothing is counted or scanned over the cells and runs beforehand (the order
-// within a list is all that a result depends on).  This replaces a count
-// kernel, a scan over the cells, the list fill, a second kernel for long lists
-// and a scan over the runs, with a clear of two arrays: 413 us of kernels (64 count, 149 fill, 200
-// scans) became 154 us on the 20M workload; the 200,000-point dense one, whose few long lists
-// share a neighbourhood, 327 became 135 us.  Eight blocks an SM (64 registers) hide more of the
-// chain than the six that the compiler's choice of registers left: 172 us at 20M points.
-// Lists past `cap` entries are not written; the host sees it in the total and runs
+// Bound by the merge's chain of dependent loads.  The lists and anchors are not
+// in cell order: a warp reserves its 32 cells' room with one atomic per total,
+// so nothing is counted or scanned over the cells and runs beforehand (the order
+// within a list is all that a result depends on).  With the two scans, the count
+// and the clears that this replaces, 413 us of kernels became 147 us on the 20M
+// workload; the 200,000-point dense one, whose few long lists share a
+// neighbourhood, 327 became 147 us.
+// Eight blocks an SM (64 registers) hide more of the chain than the six that the
+// compiler's choice of registers left (154 against 172 us at 20M points).
+// Lists past `cap` targets are not written; the host sees it in the total and runs
 // the kernel again with room for all.
 __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
-    const uint32_t* __restrict__ listq, BatchCtrl* __restrict__ ctrl, const uint64_t* __restrict__ ckey,
-    const uint32_t* __restrict__ cjob, const JobGrid* __restrict__ grids, const int32_t* __restrict__ nb9,
-    const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ crun, const uint32_t* __restrict__ rfeat,
-    const uint32_t* __restrict__ rstart, uint64_t cap, uint2* __restrict__ nrl_ent, uint64_t* run_sfx,
-    uint32_t* run_qn, uint32_t* run_L, uint4* __restrict__ act) {
+    uint64_t npoints, const uint32_t* __restrict__ listq, BatchCtrl* __restrict__ ctrl,
+    const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob, const JobGrid* __restrict__ grids,
+    const int32_t* __restrict__ nb9, const uint32_t* __restrict__ crun, const uint32_t* __restrict__ rfeat,
+    const uint32_t* __restrict__ rstart, uint64_t cap, uint32_t* __restrict__ targets, uint64_t* run_sfx,
+    uint32_t* run_L, uint4* __restrict__ act) {
     const uint32_t n = (uint32_t)ctrl->nlistq.v;
     const int lane = threadIdx.x & 31;
     const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5), w = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -686,7 +693,7 @@ __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
     for (uint64_t i0 = deal ? w : w * 32; i0 < (deal ? dealt : n); i0 += nw * 32) {
         const uint64_t i = deal ? i0 + (uint64_t)lane * dealt : i0 + lane;
         const bool in = i < n && (!deal || lane < 16);
-        uint32_t c = 0, r0 = 0, r1 = 0, kept = 0;
+        uint32_t c = 0, r0 = 0, r1 = 0, kept = 0, points = 0;
         // each slot's cursor starts at its first run above the lowest own feature
         uint32_t h[9], e[9], f[9];
         int own = 0;
@@ -707,28 +714,32 @@ __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
                 if (t < na) {
                     e[t] = crun[adj[t] + 1];
                     h[t] = (uint32_t)lower_bound_dev(rfeat, (uint64_t)crun[adj[t]], (uint64_t)e[t], fmin + 1);
-                    f[t] = h[t] < e[t] ? rfeat[h[t]] : 0xffffffffu;
+                    if (h[t] < e[t]) {
+                        f[t] = rfeat[h[t]];
+                        points += rstart[e[t]] - rstart[h[t]];
+                    }
                     kept += e[t] - h[t];
                     if ((uint32_t)adj[t] == c) own = t;
                 }
         }
-        const uint32_t kincl = warp_incl_scan(kept);
-        const uint32_t ktot = __shfl_sync(0xffffffffu, kincl, 31);
-        if (ktot == 0) continue;
-        unsigned long long kb = 0;
-        if (lane == 0) kb = atomicAdd(&ctrl->entries.v, (unsigned long long)ktot);
-        kb = __shfl_sync(0xffffffffu, kb, 0);
-        if (kb + ktot > cap) continue;   // no room: the host runs the kernel again
-        const uint64_t first = kb + (kincl - kept);
-        const bool big = kept > kBigList;
+        const uint64_t pincl = warp_incl_scan((uint64_t)points);
+        const uint64_t ptot = __shfl_sync(0xffffffffu, pincl, 31);
+        if (ptot == 0) continue;
+        const uint32_t runs = __reduce_add_sync(0xffffffffu, kept);
+        unsigned long long pb = 0;
+        if (lane == 0) {
+            pb = atomicAdd(&ctrl->targets.v, (unsigned long long)ptot);
+            atomicAdd(&ctrl->list_runs.v, (unsigned long long)runs);
+        }
+        pb = __shfl_sync(0xffffffffu, pb, 0);
+        if (pb + ptot > cap) continue;   // no room: the host runs the kernel again
+        const uint64_t first = pb + (pincl - points);
+        const bool big = kept > kBigRuns || points > kBigPoints;
         if (kept && !big) {
             // the lowest own run's suffix is the whole list
-            const uint64_t end = first + kept;
             run_sfx[r0] = first;
-            run_qn[r0] = kept;
-            run_L[r0] = 0;
+            run_L[r0] = points;
             for (uint32_t r = r0 + 1; r < r1; ++r) run_L[r] = 0;
-            uint64_t pos = first;
             uint32_t P = 0, pend_r = 0, pend_f = 0;
             bool pend = false;
             for (;;) {
@@ -742,9 +753,8 @@ __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
                     }
                 if (fm == 0xffffffffu) break;
                 if (pend && pend_f < fm) {
-                    run_sfx[pend_r] = pos;
-                    run_qn[pend_r] = (uint32_t)(end - pos);
-                    run_L[pend_r] = P;
+                    run_sfx[pend_r] = first + P;
+                    run_L[pend_r] = points - P;
                     pend = false;
                 }
                 uint32_t r = 0;
@@ -755,7 +765,7 @@ __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
                         f[t] = h[t] < e[t] ? rfeat[h[t]] : 0xffffffffu;
                     }
                 const uint32_t st = rstart[r], rc = rstart[r + 1] - st;
-                nrl_ent[pos++] = make_uint2(st, rc);
+                for (uint32_t q = 0; q < rc; ++q) targets[first + P + q] = st + q;
                 P += rc;
                 if (ts == own) {
                     pend = true;
@@ -763,67 +773,61 @@ __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
                     pend_f = fm;
                 }
             }
-            if (pend) {
-                run_sfx[pend_r] = pos;
-                run_qn[pend_r] = 0;
-                run_L[pend_r] = P;
-            }
-            for (uint32_t r = r0; r < r1; ++r) run_L[r] = P - run_L[r];
         }
         for (uint32_t m = __ballot_sync(0xffffffffu, big); m; m &= m - 1) {   // the merge above is serial in the list
             const int j = __ffs(m) - 1;
-            nrl_cell_warp(__shfl_sync(0xffffffffu, c, j), lane, __shfl_sync(0xffffffffu, first, j),
-                          __shfl_sync(0xffffffffu, kept, j), ckey, cjob, grids, nb9, cstart, crun, rfeat, rstart, nrl_ent,
-                          run_sfx, run_qn, run_L);
+            const uint32_t cj = __shfl_sync(0xffffffffu, c, j);
+            const uint64_t fj = __shfl_sync(0xffffffffu, first, j);
+            list_cell_warp(cj, lane, fj, ckey, cjob, grids, nb9, crun, rfeat, rstart, targets, run_sfx, run_L);
         }
         __syncwarp();
-        // anchors: the points of own runs with targets
-        uint32_t na = 0;
-        uint64_t nu = 0;
+        // anchors: the points of own runs with targets, short lists and long ones
+        uint32_t ns = 0, nl = 0;
+        uint64_t np = 0;
         if (kept)
             for (uint32_t r = r0; r < r1; ++r) {
                 const uint32_t L = run_L[r];
                 if (!L) continue;
                 const uint32_t rc = rstart[r + 1] - rstart[r];
-                na += rc;
-                nu += (uint64_t)rc * L;
+                if (L <= kLongList) ns += rc;
+                else nl += rc;
+                np += (uint64_t)rc * L;
             }
-        const uint32_t aincl = warp_incl_scan(na);
-        const uint64_t uincl = warp_incl_scan(nu);
-        unsigned long long ab = 0, ub = 0;
-        if (lane == 31 && aincl) {
-            ab = atomicAdd(&ctrl->anchors.v, (unsigned long long)aincl);
-            ub = atomicAdd(&ctrl->capacity.v, (unsigned long long)uincl);
+        const uint32_t sincl = warp_incl_scan(ns), lincl = warp_incl_scan(nl);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) np += __shfl_xor_sync(0xffffffffu, np, o);
+        unsigned long long sb = 0, lb = 0;
+        if (lane == 31) {
+            if (sincl) sb = atomicAdd(&ctrl->anchors.v, (unsigned long long)sincl);
+            if (lincl) lb = atomicAdd(&ctrl->long_anchors.v, (unsigned long long)lincl);
+            if (np) atomicAdd(&ctrl->pairs.v, (unsigned long long)np);
         }
-        uint64_t o = __shfl_sync(0xffffffffu, ab, 31) + (aincl - na);
-        uint64_t u = __shfl_sync(0xffffffffu, ub, 31) + (uincl - nu);
-        const bool heavy = na > kHeavyAnchors;
-        if (na && !heavy)
+        uint64_t so = __shfl_sync(0xffffffffu, sb, 31) + (sincl - ns);
+        uint64_t lo = npoints - 1 - (__shfl_sync(0xffffffffu, lb, 31) + (lincl - nl));   // downwards
+        const bool heavy = ns + nl > kHeavyAnchors;
+        if (ns + nl && !heavy)
             for (uint32_t r = r0; r < r1; ++r) {
                 const uint32_t L = run_L[r];
                 if (!L) continue;
                 const uint32_t st = rstart[r], rc = rstart[r + 1] - st;
                 const uint64_t sfx = run_sfx[r];
-                const uint32_t hi = run_qn[r] << 8 | (uint32_t)(sfx >> 32);
-                for (uint32_t q = 0; q < rc; ++q) {
-                    act[o++] = make_uint4(st + q, (uint32_t)u, (uint32_t)sfx, hi);
-                    u += L;
-                }
+                for (uint32_t q = 0; q < rc; ++q)
+                    act[L <= kLongList ? so++ : lo--] = make_uint4(st + q, L, (uint32_t)sfx, (uint32_t)(sfx >> 32));
             }
         for (uint32_t m = __ballot_sync(0xffffffffu, heavy); m; m &= m - 1) {   // the loop above is serial in the points
             const int j = __ffs(m) - 1;
             const uint32_t s0 = __shfl_sync(0xffffffffu, r0, j), s1 = __shfl_sync(0xffffffffu, r1, j);
-            uint64_t oj = __shfl_sync(0xffffffffu, o, j), uj = __shfl_sync(0xffffffffu, u, j);
+            uint64_t sj = __shfl_sync(0xffffffffu, so, j), lj = __shfl_sync(0xffffffffu, lo, j);
             for (uint32_t r = s0; r < s1; ++r) {   // the whole warp reads the run
                 const uint32_t L = run_L[r];
                 if (!L) continue;
                 const uint32_t st = rstart[r], rc = rstart[r + 1] - st;
                 const uint64_t sfx = run_sfx[r];
-                const uint32_t hi = run_qn[r] << 8 | (uint32_t)(sfx >> 32);
+                const bool is_long = L > kLongList;
                 for (uint32_t q = lane; q < rc; q += 32)
-                    act[oj + q] = make_uint4(st + q, (uint32_t)(uj + (uint64_t)q * L), (uint32_t)sfx, hi);
-                oj += rc;
-                uj += (uint64_t)rc * L;
+                    act[is_long ? lj - q : sj + q] = make_uint4(st + q, L, (uint32_t)sfx, (uint32_t)(sfx >> 32));
+                if (is_long) lj -= rc;
+                else sj += rc;
             }
         }
     }
@@ -843,11 +847,10 @@ constexpr uint64_t kBoundBytes = 8ull << 30;
 // Look-back words of all digit passes in one clear, up to this much (above 100 million points
 // one pass's words are cleared before each pass).
 constexpr uint64_t kSortStatusBytes = 256ull << 20;
-// Room for list entries and neighbours before their numbers are known: four entries per run
-// (0.2 on the 20M workload, 3.4 on a batch of many small jobs; nine at most: a run is adjacent
-// to nine cells) and eight neighbours per point (0.14 on the 20M workload, 16 on that batch,
+// Room for the lists' targets and for neighbours before their numbers are known: four targets
+// per point (nine at most: a point is adjacent to nine cells) and eight neighbours per point (0.14 on the 20M workload, 16 on that batch,
 // 30 in dense clusters).  What does not fit is built again with the counted room.
-inline uint64_t list_room(uint64_t runs) { return std::min<uint64_t>(9 * runs, 4 * runs + 65536); }
+inline uint64_t list_room(uint64_t n) { return std::min<uint64_t>(9 * n, 4 * n + 65536); }
 inline uint64_t neighbour_room(uint64_t n) { return std::min<uint64_t>(kSinglePassCap, 8 * n + 65536); }
 
 namespace {
@@ -878,11 +881,10 @@ void lay_cells(Batch& b, Carver& c, uint64_t M, uint64_t R) {
     c.add(b.qfirst, M);
     c.add(b.listq, M);
     c.add(b.run_sfx, R);
-    c.add(b.run_qn, R);
     c.add(b.run_L, R);
     if (b.row_table) c.add(b.rowstart, b.rows + 1);
 }
-void lay_lists(Batch& b, Carver& c) { c.add(b.nrl_ent, b.nrl_cap); }
+void lay_lists(Batch& b, Carver& c) { c.add(b.targets, b.targets_cap); }
 void lay_act(Batch& b, Carver& c) { c.add(b.act, b.N); }
 
 // The row table when it is not much larger than the cell list.
@@ -987,7 +989,7 @@ void bucket_points(Batch& b) {
     // everything up to the pairs' bounds in one block laid out by bounds, when that is small
     // enough to reserve; a device that has no such block left takes the other way
     b.capM = b.capR = n;
-    b.nrl_cap = list_room(n);
+    b.targets_cap = list_room(n);
     b.nb_cap = neighbour_room(n);
     b.row_table = wants_row_table(b, n);
     auto bounds = [&](Carver& c) {
@@ -1075,21 +1077,20 @@ void build_neighborhoods(Batch& b) {
     cudaStream_t s = b.s;
     if (!b.bounded && !b.act.get()) {
         Carver::place(b.mem_act, s, [&](Carver& c) { lay_act(b, c); });
-        b.nrl_cap = list_room(b.Rn);
+        b.targets_cap = std::min<uint64_t>(9 * b.N, b.N / 2 + 65536);   // (large batches: less in reserve)
         Carver::place(b.mem_lists, s, [&](Carver& c) { lay_lists(b, c); });
     }
-    if (b.lists_built) {   // the lists did not fit: room for all of them, and the totals from zero
-        b.nrl_cap = b.nrl_total;
+    if (b.lists_built) {   // the lists did not fit: room for all of them (targets_cap), and the totals from zero
         Carver::place(b.mem_lists, s, [&](Carver& c) { lay_lists(b, c); });
-        COLO_CUDA(cudaMemsetAsync(&b.ctrl.get()->entries, 0, 3 * sizeof(LineCounter), s));
+        COLO_CUDA(cudaMemsetAsync(&b.ctrl.get()->targets, 0, 5 * sizeof(LineCounter), s));
     }
     b.lists_built = true;
     const unsigned qgrid = (unsigned)std::min<uint64_t>(grid_for(b.capM, 128), (uint64_t)b.sms * 16);
     KScope ks("neighbour_lists");
-    k_neighbour_lists<<<qgrid, 128, 0, s>>>(b.listq.get(), b.ctrl.get(), b.ckey.get(), b.cjob.get(), b.grids.get(),
-                                            b.nb9.get(), b.cstart.get(), b.crun.get(), b.rfeat.get(), b.rstart.get(),
-                                            b.nrl_cap, b.nrl_ent.get(), b.run_sfx.get(), b.run_qn.get(),
-                                            b.run_L.get(), b.act.get());
+    k_neighbour_lists<<<qgrid, 128, 0, s>>>(b.N, b.listq.get(), b.ctrl.get(), b.ckey.get(), b.cjob.get(),
+                                            b.grids.get(), b.nb9.get(), b.crun.get(), b.rfeat.get(), b.rstart.get(),
+                                            b.targets_cap, b.targets.get(), b.run_sfx.get(), b.run_L.get(),
+                                            b.act.get());
     COLO_LAUNCH_CHECK();
     count_launch();
 }

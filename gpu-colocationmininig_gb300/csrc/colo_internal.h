@@ -13,12 +13,11 @@
 //               qmask[M*4*W] (masks of the 4 quads containing the cell)
 //   runs        (cell, feature) runs rfeat/rstart/rcnt/rcell[Rn], cell-major;
 //               runs per feature on the host (h_frun_off prefix)
-//   NRL         per cell with targets, the runs of its adjacent cells with a
-//               feature above the cell's lowest own feature, ordered by
-//               (feature, cell): nrl_ent (start, count); per run the start of
-//               its higher-feature suffix run_sfx and its size run_L
-//   anchors     act[A], act_base[A]: the points of runs with targets, with
-//               their list slices and their starts in the single-pass layout
+//   lists       per cell with targets, the points of its adjacent cells' runs with
+//               a feature above the cell's lowest own feature, ordered by
+//               (feature, cell, id): targets (sorted positions)
+//   anchors     act[]: the points of runs with targets, with their slices of the
+//               lists
 //   neighbours  N+(a) = nb[nb_beg[a] .. nb_beg[a] + nb_cnt[a]) by point id
 #pragma once
 #include <cuda_runtime.h>

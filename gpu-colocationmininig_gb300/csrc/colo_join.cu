@@ -4,17 +4,18 @@
 // degree2TableSlotCounter_Kernel / generalInstanceTableSlotCounter_Kernel
 // visit candidates (Codes/DeviceProcess_Kernel.h:12-55, 255-316).
 //
-// Work is organised by run (the points of one feature in one cell): a run's
-// targets are the suffix of its cell's neighbourhood run list with higher
-// features, so runs without targets cost nothing and every anchor of a run
-// walks the same target list (L1/L2 reuse).  A group of T lanes serves one
-// anchor; target points are read straight from the cell-sorted coordinate
-// arrays, and hits are compacted with one group ballot per step.
+// An anchor's targets are one slice of its cell's neighbourhood list (the
+// suffix with higher features), so points without targets cost nothing and the
+// anchors of a cell read the same list.  A warp takes a tile of 32 anchors,
+// flattens their slices with a prefix sum and tests 32 (anchor, target) pairs a
+// step whatever the slices' lengths; an anchor with a long slice gets a warp to
+// itself.
 //
-// Single pass: each anchor owns a region of its run's upper bound L (the
-// number of target points) and writes its hits there, so no counting pass is
-// needed; when the upper bounds would not fit, a count pass + scan + fill
-// pass produces a compact layout instead.
+// Single pass: a tile reserves room for all its pairs with one atomic and
+// writes its hits there end to end, in the order of the flattened pairs, which
+// is the order of each anchor's list; no counting pass is needed.  When that
+// room would be too large, a count pass + scan + fill pass produces a compact
+// layout instead.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -27,129 +28,158 @@ namespace {
 
 enum { J_SINGLE = 0, J_COUNT = 1, J_FILL = 2 };
 
-constexpr uint64_t kJoinWaves = 8;   // waves of resident blocks at most (the groups take anchors grid-stride)
+constexpr int kLongSteps = 4;        // steps of 32 targets an iteration for an anchor with a long slice
+constexpr uint64_t kJoinWaves = 8;   // waves of resident blocks at most (warps take tiles grid-stride)
 
-// One anchor's neighbour list, by its group of T lanes; returns the list length.
-template <int T, int MODE>
-__device__ __forceinline__ uint32_t join_anchor(
-    uint64_t i, const uint4* __restrict__ act, const uint32_t* __restrict__ sid, const uint32_t* __restrict__ sfeat,
-    const float2* __restrict__ sxy, const uint2* __restrict__ nrl_ent, const uint32_t* __restrict__ fjob,
-    const JobGrid* __restrict__ grids, uint64_t* __restrict__ nb_beg, uint32_t* __restrict__ nb_cnt,
-    uint32_t* __restrict__ nb) {
-    const int lane = threadIdx.x & 31;
-    const int gl = lane % T;
-    const int gbase = lane - gl;
-    const uint32_t gmask = (T == 32) ? 0xffffffffu : (((1u << T) - 1u) << gbase);
-    // position, list start and list slice in one load: the slice's first entry waits on this one alone
-    const uint4 an = act[i];
-    const uint32_t p = an.x;
-    const uint32_t a = sid[p];
-    const float2 pa = sxy[p];
-    const float xa = pa.x, ya = pa.y;
-    const JobGrid& g = grids[fjob ? fjob[sfeat[p]] : 0u];   // fjob is null for one-job batches
-    const float R2 = g.R2, hu = g.R2hu;
-    const uint64_t q0 = (uint64_t)(an.w & 0xffu) << 32 | an.z, qend = q0 + (an.w >> 8);
-    uint64_t base = 0;
-    if (MODE == J_SINGLE) base = an.y;
-    if (MODE == J_FILL) base = nb_beg[a];
-    uint32_t k = 0;
-    for (uint64_t q = q0; q < qend; ++q) {
-        const uint2 te = nrl_ent[q];   // the target run's first sorted position and point count
-        const uint32_t ts = te.x, tc = te.y;
-        if constexpr (T == 1) {
-            // one lane per anchor: no group vote
-            for (uint32_t t = 0; t < tc; ++t) {
-                const float2 pb = sxy[ts + t];
-                if (ref_within(xa, ya, pb.x, pb.y, R2, hu)) {
-                    if (MODE != J_COUNT) nb[base + k] = sid[ts + t];
-                    ++k;
-                }
-            }
-        } else {
-            for (uint32_t b0 = 0; b0 < tc; b0 += T) {
-                const uint32_t t = b0 + gl;
-                bool ok = false;
-                if (t < tc) {
-                    const float2 pb = sxy[ts + t];
-                    ok = ref_within(xa, ya, pb.x, pb.y, R2, hu);
-                }
-                const uint32_t bal = (__ballot_sync(gmask, ok) >> gbase) & ((T == 32) ? 0xffffffffu : ((1u << T) - 1u));
-                if (MODE != J_COUNT && ok) nb[base + k + __popc(bal & ((1u << gl) - 1u))] = sid[ts + t];
-                k += __popc(bal);
-            }
-        }
-    }
-    if (gl == 0) {
-        nb_cnt[a] = k;
-        if (MODE == J_SINGLE) nb_beg[a] = base;
-    }
-    return k;
-}
-
-
-// Six blocks per SM (40 registers): the join is latency-bound, and the sixth block
-// measured 0.398 -> 0.377 ms per step on the 20M workload.  The anchors are counted on the
-// device; the groups take them grid-stride.  Lists or a layout that did not fit their room
-// are left to a later launch with room.
-template <int T, int MODE>
+// Bound by instruction issue and the dependent loads target -> coordinates.  Groups of eight lanes
+// per anchor walking the lists run by run left most lanes idle, since runs average two points:
+// 0.33 ms became 0.095 ms on the 20M workload (1.2 M anchors, 2.7 M pairs), 2.2 became 0.83 ms on a
+// batch of 128 jobs (134 M pairs), 0.36 became 0.042 ms on 200,000 dense points (6 M pairs), where
+// the longest slices alone, eight lanes each, took most of it.  Six blocks an SM (40 registers, some
+// spilled) suit many short slices best (batch: 0.93 ms against 1.08 ms at four).
+// `per` anchors a tile (32 / lanes per anchor).  The anchors are counted on the device; tiles are
+// taken grid-stride.  Lists or neighbours that did not fit their room are left to a later launch.
+template <int MODE>
 __global__ void __launch_bounds__(256, 6) k_join(
-    const BatchCtrl* __restrict__ ctrl, uint64_t nrl_cap, uint64_t nb_cap, const uint4* __restrict__ act,
-    const uint32_t* __restrict__ sid, const uint32_t* __restrict__ sfeat, const float2* __restrict__ sxy,
-    const uint2* __restrict__ nrl_ent, const uint32_t* __restrict__ fjob, const JobGrid* __restrict__ grids,
-    uint64_t* __restrict__ nb_beg, uint32_t* __restrict__ nb_cnt, uint32_t* __restrict__ nb,
-    unsigned long long* __restrict__ total) {
-    if (ctrl->entries.v > nrl_cap || (MODE == J_SINGLE && ctrl->capacity.v > nb_cap)) return;
-    const uint64_t A = ctrl->anchors.v;
+    BatchCtrl* __restrict__ ctrl, uint64_t npoints, uint64_t targets_cap, uint64_t nb_cap, int per,
+    const uint4* __restrict__ act, const uint32_t* __restrict__ sid, const uint32_t* __restrict__ sfeat,
+    const float2* __restrict__ sxy, const uint32_t* __restrict__ targets, const uint32_t* __restrict__ fjob,
+    const JobGrid* __restrict__ grids, uint64_t* __restrict__ nb_beg, uint32_t* __restrict__ nb_cnt,
+    uint32_t* __restrict__ nb, unsigned long long* __restrict__ total) {
+    if (ctrl->targets.v > targets_cap || (MODE == J_SINGLE && ctrl->pairs.v > nb_cap)) return;
+    const uint64_t A = ctrl->anchors.v, AL = ctrl->long_anchors.v;
+    const uint64_t tiles = (A + per - 1) / per;
     const int lane = threadIdx.x & 31;
-    const int gl = lane % T;
-    const uint64_t thread = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long v = 0;
-    for (uint64_t i = thread / T; i < A; i += (uint64_t)gridDim.x * blockDim.x / T) {
-        const uint32_t k = join_anchor<T, MODE>(i, act, sid, sfeat, sxy, nrl_ent, fjob, grids, nb_beg, nb_cnt, nb);
-        if (gl == 0) v += k;
-    }
-    if (MODE == J_SINGLE) {
-        // the entries of the warp's anchors (each group's count once), one atomic per warp into
-        // one of kEntrySlots counters on separate lines: the list total without another pass
-        // over the counts, and no block barrier (one made every warp wait for its block's
-        // longest list: the 512-job batch's join ran 10.96 ms against 9.38 ms)
-        __syncwarp();
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    unsigned long long found = 0;
+    // long slices first: they take longest
+    for (uint64_t i = warp; i < AL + tiles; i += warps) {
+        if (i < AL) {
+            const uint4 an = act[npoints - 1 - i];
+            const uint32_t a = sid[an.x], L = an.y;
+            const float2 pa = sxy[an.x];
+            const JobGrid& g = grids[fjob ? fjob[sfeat[an.x]] : 0u];   // fjob is null for one-job batches
+            const float R2 = g.R2, hu = g.R2hu;
+            const uint32_t* list = targets + ((uint64_t)an.w << 32 | an.z);
+            unsigned long long base = 0;
+            if (MODE == J_SINGLE && lane == 0) base = atomicAdd(&ctrl->nb_used.v, (unsigned long long)L);
+            if (MODE == J_SINGLE) base = __shfl_sync(0xffffffffu, base, 0);
+            if (MODE == J_FILL) base = nb_beg[a];
+            uint32_t k = 0;
+            for (uint32_t t0 = 0; t0 < L; t0 += 32 * kLongSteps) {   // several steps' loads in flight
+                uint32_t p[kLongSteps];
+                float2 pb[kLongSteps];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0 && v) atomicAdd(total + ((thread >> 5) % kEntrySlots) * kEntryStride, v);
+                for (int i = 0; i < kLongSteps; ++i) p[i] = t0 + i * 32 + lane < L ? list[t0 + i * 32 + lane] : 0xffffffffu;
+#pragma unroll
+                for (int i = 0; i < kLongSteps; ++i) pb[i] = p[i] != 0xffffffffu ? sxy[p[i]] : make_float2(0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < kLongSteps; ++i) {
+                    const bool ok = p[i] != 0xffffffffu && ref_within(pa.x, pa.y, pb[i].x, pb[i].y, R2, hu);
+                    const uint32_t bal = __ballot_sync(0xffffffffu, ok);
+                    if (MODE != J_COUNT && ok) nb[base + k + __popc(bal & lt)] = sid[p[i]];
+                    k += __popc(bal);
+                }
+            }
+            if (lane == 0) {
+                nb_cnt[a] = k;
+                if (MODE == J_SINGLE) nb_beg[a] = base;
+            }
+            found += k;
+            continue;
+        }
+        const uint64_t at = (i - AL) * per + lane;
+        const bool in = lane < per && at < A;
+        uint32_t a = 0, L = 0;
+        float xa = 0.f, ya = 0.f, R2 = 0.f, hu = 0.f;
+        uint64_t from = 0, beg = 0;
+        if (in) {
+            const uint4 an = act[at];
+            L = an.y;
+            from = (uint64_t)an.w << 32 | an.z;
+            a = sid[an.x];
+            const float2 pa = sxy[an.x];
+            xa = pa.x;
+            ya = pa.y;
+            const JobGrid& g = grids[fjob ? fjob[sfeat[an.x]] : 0u];
+            R2 = g.R2;
+            hu = g.R2hu;
+            if (MODE == J_FILL) beg = nb_beg[a];
+        }
+        const uint32_t incl = warp_incl_scan(L), excl = incl - L;
+        const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
+        from -= excl;   // pair t of the tile is target from_j + t, j its anchor's lane
+        unsigned long long base = 0;
+        if (MODE == J_SINGLE && lane == 0 && tot) base = atomicAdd(&ctrl->nb_used.v, (unsigned long long)tot);
+        if (MODE == J_SINGLE) base = __shfl_sync(0xffffffffu, base, 0);
+        uint32_t hits = 0, before = 0, mine = 0;   // the tile's so far; those before this lane's anchor; this anchor's
+        for (uint32_t t0 = 0; t0 < tot; t0 += 32) {
+            const uint32_t t = t0 + lane;
+            int j = 0;
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1) {
+                const uint32_t ev = __shfl_sync(0xffffffffu, excl, j + step);
+                if (ev <= t) j += step;
+            }
+            const uint64_t from_j = __shfl_sync(0xffffffffu, from, j);
+            const float xj = __shfl_sync(0xffffffffu, xa, j), yj = __shfl_sync(0xffffffffu, ya, j);
+            // one job: one threshold; several: the anchor's own
+            const float R2j = fjob ? __shfl_sync(0xffffffffu, R2, j) : __shfl_sync(0xffffffffu, R2, 0);
+            const float huj = fjob ? __shfl_sync(0xffffffffu, hu, j) : __shfl_sync(0xffffffffu, hu, 0);
+            bool ok = false;
+            uint32_t p = 0;
+            if (t < tot) {
+                p = targets[from_j + t];
+                const float2 pb = sxy[p];
+                ok = ref_within(xj, yj, pb.x, pb.y, R2j, huj);
+            }
+            const uint32_t bal = __ballot_sync(0xffffffffu, ok);
+            // lanes of this step before and in this lane's own slice
+            const uint32_t r0 = excl <= t0 ? 0u : excl - t0 < 32 ? excl - t0 : 32u;
+            const uint32_t r1 = incl <= t0 ? 0u : incl - t0 < 32 ? incl - t0 : 32u;
+            const uint32_t m0 = r0 == 32 ? 0xffffffffu : (1u << r0) - 1u, m1 = r1 == 32 ? 0xffffffffu : (1u << r1) - 1u;
+            if (MODE == J_FILL) {
+                // compact layout: the pair's place in its own anchor's list
+                const uint64_t beg_j = __shfl_sync(0xffffffffu, beg, j);
+                const uint32_t mine_j = __shfl_sync(0xffffffffu, mine, j);
+                const uint32_t own_j = __shfl_sync(0xffffffffu, m1 & ~m0, j);
+                if (ok) nb[beg_j + mine_j + __popc(bal & own_j & lt)] = sid[p];
+            }
+            if (MODE == J_SINGLE && ok) nb[base + hits + __popc(bal & lt)] = sid[p];
+            before += __popc(bal & m0);
+            mine += __popc(bal & m1 & ~m0);
+            hits += __popc(bal);
+        }
+        if (in) {
+            nb_cnt[a] = mine;
+            if (MODE == J_SINGLE) nb_beg[a] = base + before;
+        }
+        found += hits;
     }
+    // the list total, added to one of kEntrySlots counters on separate lines by each warp
+    if (MODE == J_SINGLE && lane == 0 && found) atomicAdd(total + (warp % kEntrySlots) * kEntryStride, found);
 }
 
-// `anchors`: as many as there are, or a bound.
-template <int T>
-void run_join(Batch& b, int mode, uint64_t anchors) {
-    const uint64_t nrl_cap = b.nrl_cap, nb_cap = b.nb_cap;
-    uint64_t grid = (anchors * T + 255) / 256;
-    grid = std::min<uint64_t>(grid, (uint64_t)b.sms * 6 * kJoinWaves);
+// `anchors`: as many as there are (and `longs` of them with long lists), or bounds.
+void run_join(Batch& b, int mode, uint64_t anchors, uint64_t longs) {
+    const int per = 32 / (b.join_group > 0 ? b.join_group : 1);
+    const uint64_t warps = longs + (anchors - longs + per - 1) / per;
+    const unsigned grid = (unsigned)std::min<uint64_t>((warps + 7) / 8, (uint64_t)b.sms * 6 * kJoinWaves);
     if (grid == 0) return;
     KScope ks(mode == J_SINGLE ? "join" : mode == J_COUNT ? "join_count" : "join_fill");
-#define COLO_JOIN(MD)                                                                                        \
-    k_join<T, MD><<<(unsigned)grid, 256, 0, b.s>>>(b.ctrl.get(), nrl_cap, nb_cap, b.act.get(), b.sid.get(), \
-                                         b.sfeat.get(), b.sxy.get(), b.nrl_ent.get(),                           \
-                                         b.J > 1 ? b.fjob.get() : nullptr,                                      \
-                                         b.grids.get(), b.nb_beg.get(), b.nb_cnt.get(), b.nb.get(), b.dE.get())
+#define COLO_JOIN(MD)                                                                                            \
+    k_join<MD><<<grid, 256, 0, b.s>>>(b.ctrl.get(), b.N, b.targets_cap, b.nb_cap, per, b.act.get(), b.sid.get(), \
+                                      b.sfeat.get(), b.sxy.get(), b.targets.get(),                              \
+                                      b.J > 1 ? b.fjob.get() : nullptr, b.grids.get(), b.nb_beg.get(),          \
+                                      b.nb_cnt.get(), b.nb.get(), b.dE.get())
     if (mode == J_SINGLE) COLO_JOIN(J_SINGLE);
     else if (mode == J_COUNT) COLO_JOIN(J_COUNT);
     else COLO_JOIN(J_FILL);
 #undef COLO_JOIN
     COLO_LAUNCH_CHECK();
     count_launch();
-}
-
-void dispatch_join(Batch& b, int mode, uint64_t anchors) {
-    switch (b.join_group) {
-        case 1: run_join<1>(b, mode, anchors); break;
-        case 2: run_join<2>(b, mode, anchors); break;
-        case 4: run_join<4>(b, mode, anchors); break;
-        case 16: run_join<16>(b, mode, anchors); break;
-        case 32: run_join<32>(b, mode, anchors); break;
-        default: run_join<8>(b, mode, anchors); break;
-    }
 }
 
 __global__ void k_sqdist(const float* __restrict__ x1, const float* __restrict__ y1,
@@ -165,7 +195,7 @@ __global__ void k_sqdist(const float* __restrict__ x1, const float* __restrict__
 
 void join_queue(Batch& b) {
     b.join_queued = true;
-    dispatch_join(b, J_SINGLE, b.N);
+    run_join(b, J_SINGLE, b.N, 0);
     b.E = UINT64_MAX;
 }
 
@@ -173,7 +203,7 @@ void join_queue(Batch& b) {
 // start is never read (every reader takes nb_cnt first).
 void join_neighbors(Batch& b) {
     cudaStream_t s = b.s;
-    const uint64_t A = b.active_anchors, U = b.join_pairs;
+    const uint64_t A = b.active_anchors, AL = b.long_anchors, U = b.join_pairs;
     b.join_queued = false;
     // layouts above kSinglePassCap entries are counted first and then compact
     const bool single = U <= kSinglePassCap;
@@ -185,14 +215,15 @@ void join_neighbors(Batch& b) {
         // total entries: summed by the join's warps and read at the mine's next wait
         if (U > b.nb_cap || !b.nb.get()) room(U);
         COLO_CUDA(cudaMemsetAsync(b.dE.get(), 0, kEntrySlots * kEntryStride * 8, s));
-        dispatch_join(b, J_SINGLE, A);
+        COLO_CUDA(cudaMemsetAsync(&b.ctrl.get()->nb_used, 0, sizeof(LineCounter), s));
+        run_join(b, J_SINGLE, A, AL);
         b.E = UINT64_MAX;
     } else {
-        dispatch_join(b, J_COUNT, A);
+        run_join(b, J_COUNT, A, AL);
         uint64_t E = 0;
         scan_u32_to_u64(b.nb_cnt.get(), b.nb_beg.get(), b.N, s, &E);
         room(E);
-        dispatch_join(b, J_FILL, A);
+        run_join(b, J_FILL, A, AL);
         b.E = E;
     }
 }

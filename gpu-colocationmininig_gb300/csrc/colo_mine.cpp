@@ -591,18 +591,19 @@ void settle(colo_ctx* ctx, Batch& b, std::vector<uint32_t>* ub2) {
     b.dlist_have.assign(b.F, 0);
     if (ub2) ub2->assign(counts + 2 * b.F, counts + 2 * b.F + b.h_job_off[b.J]);
     if (!b.lists_built) return;
-    b.nrl_total = h.entries.v;
     bool again = false;
-    while (b.nrl_total > b.nrl_cap) {
+    while (h.targets.v > b.targets_cap) {
         again = true;
+        b.targets_cap = h.targets.v;
         build_neighborhoods(b);
         Readback rb(ctx, b.s, sizeof(h));
         rb.copy(&h, b.ctrl.get(), sizeof(h));
         rb.finish();
-        b.nrl_total = h.entries.v;
     }
-    b.active_anchors = h.anchors.v;
-    b.join_pairs = h.capacity.v;
+    b.nrl_total = h.list_runs.v;
+    b.long_anchors = h.long_anchors.v;
+    b.active_anchors = h.anchors.v + h.long_anchors.v;
+    b.join_pairs = h.pairs.v;
     if (b.join_queued && (again || b.join_pairs > b.nb_cap)) join_neighbors(b);
 }
 
@@ -705,6 +706,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         settled = true;
         if (!b.bounded) join_neighbors(b);
         b.mem_act.release();
+        b.mem_lists.release();
     };
 
     double t_filter = 0, t_refine = 0, t_fill = 0, t_apriori = 0;

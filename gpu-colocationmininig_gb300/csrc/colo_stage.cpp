@@ -95,11 +95,13 @@ colo_status colo_stage_neighbors(colo_ctx* ctx, colo_dataset* ds, float R, uint6
         if ((offs || nbr) && b.N) {
             // compact the per-anchor lists into a CSR
             std::vector<uint64_t> beg(b.N);
-            std::vector<uint32_t> cnt(b.N), all(b.nb_cap);
+            // (a single-pass layout takes no more than the pairs it was built from)
+            const uint64_t used = std::min(b.nb_cap, b.join_pairs);
+            std::vector<uint32_t> cnt(b.N), all(used);
             COLO_CUDA(cudaMemcpyAsync(beg.data(), b.nb_beg.get(), b.N * 8, cudaMemcpyDeviceToHost, s));
             COLO_CUDA(cudaMemcpyAsync(cnt.data(), b.nb_cnt.get(), b.N * 4, cudaMemcpyDeviceToHost, s));
-            if (b.nb_cap)
-                COLO_CUDA(cudaMemcpyAsync(all.data(), b.nb.get(), b.nb_cap * 4, cudaMemcpyDeviceToHost, s));
+            if (used)
+                COLO_CUDA(cudaMemcpyAsync(all.data(), b.nb.get(), used * 4, cudaMemcpyDeviceToHost, s));
             COLO_CUDA(cudaStreamSynchronize(s));
             if (nbr && cap < neighbor_entries(b)) return COLO_ERR_CAPACITY;
             uint64_t o = 0;

@@ -260,14 +260,14 @@ colo_status colo_stage_apriori(colo_ctx* ctx, const uint32_t* prev, uint64_t npr
 colo_status colo_autotune(colo_ctx* ctx, colo_dataset* ds, const colo_params* p, int32_t* join_group,
                           double* ms);
 /* Sets the join's lanes per anchor for later mines on this context without
- * timing (1, 2, 4, 8, 16 or 32; 0 restores the default).  COLO_ERR_ARG for any
+ * timing (1, 2, 4, 8, 16 or 32; 0 restores the default, 1).  COLO_ERR_ARG for any
  * other width. */
 colo_status colo_set_join_group(colo_ctx* ctx, int32_t join_group);
 
 /* Launch shapes tuned per dataset (no counterpart in the reference): lanes
  * per anchor in the cell-pair join (1, 2, 4, 8, 16, 32), candidates per warp
  * unit in the level filter (8, 16, 32), threads per block of the level
- * kernels (64, 128, 256; 0 keeps the defaults 8, 32, 256) and the level
+ * kernels (64, 128, 256; 0 keeps the defaults 1, 32, 256) and the level
  * queue (0: one warp per 32-row chunk; 1: a persistent grid whose warps take
  * chunks by ticket, largest candidates first in COLO_MODE_LEARNED).  Every
  * setting gives the same results. */
