@@ -9,6 +9,10 @@
 
 namespace colo {
 
+// Queues a copy of host bytes through the context's page-locked staging (no wait; colo_mine.cpp).
+void staged_upload(colo_ctx* ctx, cudaStream_t s, void* dst, const void* src, size_t bytes);
+
+
 // Host description of one job inside a batch.
 struct JobHost {
     JobGrid grid;
@@ -35,6 +39,7 @@ struct alignas(128) BatchCtrl {
 };
 
 struct Batch {
+    colo_ctx* ctx = nullptr;
     cudaStream_t s = 0;
     int sms = 148;
     // sizes
@@ -150,6 +155,7 @@ void join_queue(Batch& b);               // single-pass join into nb_cap entries
                                          // or the lists did not fit (bounded batches, before settle)
 void join_neighbors(Batch& b);           // neighbour CSR (after settle)
 uint64_t neighbor_entries(Batch& b);     // E (waits for the device sum once)
+uint64_t sum_entries(const unsigned long long* dE);   // of a copy of dE
 // Level-k candidates of every job from its prevalent (k-1)-patterns (km1
 // features each, lexicographic), with each candidate's prefix pattern index;
 // a null entry is a job with no next level.  colo_apriori.cu.
@@ -167,9 +173,8 @@ void filter_pairs(Batch& b);
 // Level-k upper bounds for host candidates cand[c*k + j] (global features) of
 // jobs job[c]: d_ub[c*k + j] (zeroed by the caller).  d_stats (optional,
 // zeroed, 2 per candidate): full quads and cells of U_c.
-// d_cand (optional): the same candidates already on the device.
 void filter_level(Batch& b, const uint32_t* h_cand, const uint32_t* h_job, uint64_t ncand, uint32_t k,
-                  uint32_t* d_ub, unsigned long long* d_stats, const uint32_t* d_cand = nullptr);
+                  uint32_t* d_ub, unsigned long long* d_stats);
 
 // colo_level.cu --------------------------------------------------------------
 // One member of a candidate: its feature's first point id and instances, and where its
@@ -222,6 +227,9 @@ struct CountWork {
     unsigned long long* items;   // optional: sum of candidate-slice lengths examined
     unsigned long long* ticket;  // chunk tickets of the persistent queue, zeroed
     uint64_t chunk0 = 0;         // gchunk[0]
+    // non-null: candidates c whose bounds ub[c*k + j] do not all reach need[c*k + j] are passed over
+    const uint32_t* ub = nullptr;
+    const uint32_t* need = nullptr;
 };
 
 // count pass: rows per chunk + bitmaps; fill pass: rows; single pass: rows per

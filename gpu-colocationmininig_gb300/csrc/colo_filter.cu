@@ -410,14 +410,15 @@ void driver_lists_fill(Batch& b, const std::vector<uint8_t>& need) {
     }
     const uint64_t total = b.h_doff[b.F];
     b.dlist.alloc(total ? total : 1, s);
-    b.doff.alloc(b.F + 1 + (want.size() + 1) / 2, s);   // offsets, then the want bitset
+    // offsets, the want bitset and the cleared cursors: one upload
+    std::vector<uint64_t> in(b.F + 1 + (want.size() + b.F + 1) / 2, 0);
+    std::copy(b.h_doff.begin(), b.h_doff.end(), in.begin());
+    std::memcpy(in.data() + b.F + 1, want.data(), want.size() * 4);
+    b.doff.alloc(in.size(), s);
     uint32_t* d_want = reinterpret_cast<uint32_t*>(b.doff.get() + b.F + 1);
-    COLO_CUDA(cudaMemcpyAsync(b.doff.get(), b.h_doff.data(), (b.F + 1) * 8, cudaMemcpyHostToDevice, s));
-    COLO_CUDA(cudaMemcpyAsync(d_want, want.data(), want.size() * 4, cudaMemcpyHostToDevice, s));
+    uint32_t* d_cursor = d_want + want.size();
+    staged_upload(b.ctx, s, b.doff.get(), in.data(), in.size() * 8);
     if (total == 0) return;
-    DevBuf<uint32_t> cursor;
-    cursor.alloc(b.F, s);
-    cursor.zero(s);
     // one range of consecutive cells per block (a multiple of 256 cells), one wave of resident blocks;
     // shared memory for the block histogram of the batch's features (none past kDilHist)
     const size_t dsmem = b.F <= kDilHist ? (size_t)b.F * 16 : 0;
@@ -432,7 +433,7 @@ void driver_lists_fill(Batch& b, const std::vector<uint8_t>& need) {
         blocks = (b.M + per - 1) / per;                                                                          \
         k_dil_fill<WW><<<(unsigned)blocks, kDilThreads, dsmem, s>>>(b.M, per, b.J > 1 ? b.cjob.get() : nullptr,  \
                                                                b.grids.get(), b.nbmask.get(), b.F, b.doff.get(), \
-                                                               cursor.get(), b.dlist.get(), d_want);             \
+                                                               d_cursor, b.dlist.get(), d_want);             \
     } while (0)
     COLO_W_SWITCH(b.W, COLO_DF)
 #undef COLO_DF
@@ -468,8 +469,7 @@ void filter_pairs(Batch& b) {
 }
 
 void filter_level(Batch& b, const uint32_t* h_cand, const uint32_t* h_job, uint64_t ncand, uint32_t k,
-                  uint32_t* d_ub, unsigned long long* d_stats, const uint32_t* d_cand_in) {
-    (void)d_cand_in;
+                  uint32_t* d_ub, unsigned long long* d_stats) {
     if (ncand == 0) return;
     if (b.W > kMaxW) throw StatusError{COLO_ERR_CAPACITY, "the filter handles at most 1024 features per job"};
     cudaStream_t s = b.s;
@@ -548,7 +548,7 @@ void filter_level(Batch& b, const uint32_t* h_cand, const uint32_t* h_job, uint6
     std::memcpy(pack.data() + o, uoff.data(), uoff.size() * 8);
     DevBuf<uint32_t> dpack;
     dpack.alloc(pack.size(), s);
-    COLO_CUDA(cudaMemcpyAsync(dpack.get(), pack.data(), pack.size() * 4, cudaMemcpyHostToDevice, s));
+    staged_upload(b.ctx, s, dpack.get(), pack.data(), pack.size() * 4);
     const uint32_t* d_need = dpack.get();
     const uint32_t* d_lmem = d_need + n_need;
     const uint32_t* d_order = d_lmem + n_lmem;

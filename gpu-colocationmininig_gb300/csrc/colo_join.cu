@@ -228,14 +228,18 @@ void join_neighbors(Batch& b) {
     }
 }
 
+uint64_t sum_entries(const unsigned long long* dE) {
+    uint64_t t = 0;
+    for (int i = 0; i < kEntrySlots; ++i) t += dE[(size_t)i * kEntryStride];
+    return t;
+}
+
 uint64_t neighbor_entries(Batch& b) {
     if (b.E == UINT64_MAX) {
         std::vector<unsigned long long> e(kEntrySlots * kEntryStride);
         COLO_CUDA(cudaMemcpyAsync(e.data(), b.dE.get(), e.size() * 8, cudaMemcpyDeviceToHost, b.s));
         stream_wait(b.s);
-        uint64_t t = 0;
-        for (int i = 0; i < kEntrySlots; ++i) t += e[(size_t)i * kEntryStride];
-        b.E = t;
+        b.E = sum_entries(e.data());
     }
     return b.E;
 }

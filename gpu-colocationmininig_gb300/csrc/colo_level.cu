@@ -106,12 +106,14 @@ __device__ __forceinline__ uint64_t chunk_owner(const uint64_t* __restrict__ fir
 // (members kept in global memory, slower; only reached for k > 8).
 constexpr int kCountWarps = 8;
 
-template <int K>
+// VERDICT: the candidates' filter bounds are tested here (ub, need; not for pairs).
+template <int K, bool VERDICT>
 __global__ void __launch_bounds__(32 * kCountWarps, K == 2 ? 8 : 6) k_level_count(
     const CandDesc* __restrict__ cands, const uint32_t* __restrict__ gstart, const uint64_t* __restrict__ gchunk,
     uint64_t ngroups, uint64_t chunk0, uint64_t nchunks, const uint64_t* __restrict__ nb_beg,
     const uint32_t* __restrict__ nb_cnt, const uint32_t* __restrict__ nb, const float2* __restrict__ xy,
-    unsigned long long* __restrict__ items, unsigned long long* __restrict__ ticket, int persistent) {
+    unsigned long long* __restrict__ items, unsigned long long* __restrict__ ticket, int persistent,
+    const uint32_t* __restrict__ ub, const uint32_t* __restrict__ need) {
     constexpr int KR = (K == 0) ? 1 : K;   // register members kept for K > 0
     __shared__ uint32_t s_cnt[kCountWarps][32], s_row[kCountWarps][32];   // hits per extension, extensions hit per row
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -144,6 +146,18 @@ __global__ void __launch_bounds__(32 * kCountWarps, K == 2 ? 8 : 6) k_level_coun
             est = c.last_start;
             eend = c.last_end;
             ebm = c.bm_base + c.last_off;
+        }
+        if (VERDICT) {
+            // the filter's verdict was not waited for: a candidate passes when every member's bound
+            // reaches the least one that its ratio test accepts; the others extend no row
+            bool pass = (uint32_t)lane < n;
+            if (pass)
+                for (uint32_t i = 0; i < k; ++i) pass &= ub[(uint64_t)(q0 + lane) * k + i] >= need[(uint64_t)(q0 + lane) * k + i];
+            if (!pass) eend = 0;
+            if (!__any_sync(0xffffffffu, pass)) {
+                if ((uint32_t)lane < n) cands[q0 + lane].chunk_rows[row >> 5] = 0;
+                continue;
+            }
         }
         const float R2 = d.R2, hu = d.R2hu;
 
@@ -622,20 +636,22 @@ void level_count(Batch& b, const CountWork& w, uint32_t k) {
     unsigned grid = (unsigned)((w.nchunks * 32 + block - 1) / block);
     const int persistent = (b.level_queue && w.ticket) ? 1 : 0;   // as launch_level's
     if (persistent) grid = (unsigned)std::min<uint64_t>(grid, (uint64_t)b.sms * (32u * 32u / block));
-#define COLO_CNT(KK)                                                                                              \
-    k_level_count<KK><<<grid, block, 0, b.s>>>(w.cands, w.gstart, w.gchunk, w.ngroups, w.chunk0, w.nchunks,        \
+#define COLO_CNT(KK, V)                                                                                           \
+    k_level_count<KK, V><<<grid, block, 0, b.s>>>(w.cands, w.gstart, w.gchunk, w.ngroups, w.chunk0, w.nchunks,        \
                                                b.nb_beg.get(), b.nb_cnt.get(), b.nb.get(), b.xy.get(), w.items,   \
-                                               w.ticket, persistent)
+                                               w.ticket, persistent, w.ub, w.need)
+#define COLO_CNT_K(KK) case KK: if (w.ub) COLO_CNT(KK, true); else COLO_CNT(KK, false); break
     switch (k) {
-        case 2: COLO_CNT(2); break;
-        case 3: COLO_CNT(3); break;
-        case 4: COLO_CNT(4); break;
-        case 5: COLO_CNT(5); break;
-        case 6: COLO_CNT(6); break;
-        case 7: COLO_CNT(7); break;
-        case 8: COLO_CNT(8); break;
-        default: COLO_CNT(0); break;
+        case 2: COLO_CNT(2, false); break;
+        COLO_CNT_K(3);
+        COLO_CNT_K(4);
+        COLO_CNT_K(5);
+        COLO_CNT_K(6);
+        COLO_CNT_K(7);
+        COLO_CNT_K(8);
+        default: if (w.ub) COLO_CNT(0, true); else COLO_CNT(0, false); break;
     }
+#undef COLO_CNT_K
 #undef COLO_CNT
     COLO_LAUNCH_CHECK();
     count_launch();

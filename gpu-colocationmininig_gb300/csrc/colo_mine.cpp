@@ -254,6 +254,25 @@ bool filter_pass(const uint64_t* ub, const uint32_t* mem, uint32_t k, const std:
     return pi0 >= thr;
 }
 
+// The least bound of a feature with n instances that filter_pass accepts: the ratio does not
+// fall as the bound grows, so it is looked for around thr * n (UINT32_MAX: none up to n is accepted).
+uint32_t least_bound(uint32_t n, float thr) {
+    auto ok = [&](double u) { return (float)(u / (double)(float)n) >= thr; };
+    if (ok(0.0)) return 0;
+    if (!ok((double)n)) return UINT32_MAX;
+    uint32_t u = (uint32_t)std::min<double>(n, std::max(1.0, std::floor((double)thr * (double)(float)n)));
+    while (!ok((double)u)) ++u;
+    while (ok((double)(u - 1))) --u;
+    return u;
+}
+
+// A level of at least three members is filtered and counted with one wait when no candidate's
+// table can be chosen for the single pass: none was asked for, there is no cost model, or every
+// parent table is this short (2^20 rows from it would need 64 a parent row).  Its candidates'
+// bitmaps and chunks, those of candidates that the filter stops among them, take at most this room.
+constexpr uint64_t kOneWaitRows = 1u << 14;
+constexpr uint64_t kOneWaitWords = 1u << 26, kOneWaitChunks = 1u << 24;
+
 // Readbacks staged in page-locked memory: a device-to-host copy into pageable
 // memory blocks the host until the stream reaches it, one into the context's
 // pinned buffer is only queued, so one wait covers all of a phase's copies and
@@ -328,13 +347,6 @@ void upload_from(cudaStream_t s, void* dst, const unsigned char* staged, size_t 
     if (bytes) COLO_CUDA(cudaMemcpyAsync(dst, staged, bytes, cudaMemcpyHostToDevice, s));
 }
 
-void upload(colo_ctx* ctx, cudaStream_t s, void* dst, const void* src, size_t bytes) {
-    if (!bytes) return;
-    unsigned char* h = upload_area(ctx, s, bytes);
-    std::memcpy(h, src, bytes);
-    upload_from(s, dst, h, bytes);
-}
-
 // A typed view into the level arena's one allocation.
 template <class T>
 struct ArenaSpan {
@@ -365,12 +377,17 @@ struct LevelArena {
     ArenaSpan<uint64_t> stats;
     // the refine's results (rows | items | overflow | stats) and inputs (descs | chunk
     // prefixes | groups | members) are each one contiguous block: one copy back, one copy in
-    size_t out_bytes = 0, in_bytes = 0, chunk_at = 0, gchunk_at = 0, gstart_at = 0, mem_at = 0;
+    // with `bounds`, the filter's results (bounds, cell statistics) follow the refine's, and the
+    // least accepted bounds the inputs
+    size_t out_bytes = 0, in_bytes = 0, chunk_at = 0, gchunk_at = 0, gstart_at = 0, mem_at = 0, need_at = 0;
+    size_t ub_at = 0, fs_at = 0;
+    ArenaSpan<uint32_t> ub, need;
+    ArenaSpan<unsigned long long> fs;
     unsigned char* out = nullptr;
     unsigned char* in = nullptr;
 
     // nchunks: the single pass's; nall: all chunks
-    void init(uint64_t nall, uint64_t nwords, uint64_t ncand, uint64_t nchunks, uint32_t k, bool single,
+    void init(uint64_t nall, uint64_t nwords, uint64_t ncand, uint64_t nchunks, uint32_t k, bool single, bool bounds,
               cudaStream_t s) {
         size_t off = 0;
         auto take = [&](uint64_t bytes) {
@@ -379,7 +396,9 @@ struct LevelArena {
             return o;
         };
         const size_t r_items = ncand * 8, r_ovf = r_items + 8, r_stats = (r_ovf + ncand * 4 + 15) & ~(size_t)15;
-        out_bytes = r_stats + ncand * k * 4 * 8;
+        fs_at = r_stats + ncand * k * 4 * 8;
+        ub_at = fs_at + (bounds ? ncand * 2 * 8 : 0);
+        out_bytes = ub_at + (bounds ? ncand * k * 4 : 0);
         const size_t o_out = take(out_bytes);
         const size_t o_status = single ? take((nchunks + 1) * 8) : 0;
         const size_t o_tickets = take(2 * 8);
@@ -392,7 +411,8 @@ struct LevelArena {
         gchunk_at = chunk_at + (ncand + 2) * 8;
         gstart_at = gchunk_at + (ncand + 1) * 8;
         mem_at = (gstart_at + (ncand + 1) * 4 + 15) & ~(size_t)15;
-        in_bytes = mem_at + ncand * k * sizeof(MemberInfo);
+        need_at = mem_at + ncand * k * sizeof(MemberInfo);
+        in_bytes = need_at + (bounds ? ncand * k * 4 : 0);
         const size_t o_in = take(in_bytes);
         block.alloc(off, s);
         unsigned char* b = block.get();
@@ -413,18 +433,23 @@ struct LevelArena {
         gchunk.p = reinterpret_cast<uint64_t*>(in + gchunk_at);
         gstart.p = reinterpret_cast<uint32_t*>(in + gstart_at);
         mem.p = reinterpret_cast<MemberInfo*>(in + mem_at);
+        need.p = reinterpret_cast<uint32_t*>(in + need_at);
+        fs.p = reinterpret_cast<unsigned long long*>(out + fs_at);
+        ub.p = reinterpret_cast<uint32_t*>(out + ub_at);
         COLO_CUDA(cudaMemsetAsync(b, 0, zeroed, s));
     }
     // descs, chunk prefixes, groups and members (written by `put_members` in the staging) in one upload
     template <class Fn>
     void put_inputs(colo_ctx* ctx, cudaStream_t s, const std::vector<CandDesc>& hd, const std::vector<uint64_t>& ch,
-                    const std::vector<uint64_t>& gc, const std::vector<uint32_t>& gs, Fn&& put_members) {
+                    const std::vector<uint64_t>& gc, const std::vector<uint32_t>& gs, Fn&& put_members,
+                    const std::vector<uint32_t>& least) {
         unsigned char* h = upload_area(ctx, s, in_bytes);
         std::memcpy(h, hd.data(), hd.size() * sizeof(CandDesc));
         std::memcpy(h + chunk_at, ch.data(), std::min<size_t>(ch.size() * 8, gchunk_at - chunk_at));
         std::memcpy(h + gchunk_at, gc.data(), gc.size() * 8);
         std::memcpy(h + gstart_at, gs.data(), gs.size() * 4);
         put_members(reinterpret_cast<MemberInfo*>(h + mem_at));
+        std::memcpy(h + need_at, least.data(), least.size() * 4);
         upload_from(s, in, h, in_bytes);
     }
 };
@@ -442,12 +467,20 @@ uint64_t presize_rows(float pred) {
 
 }  // namespace
 
+void staged_upload(colo_ctx* ctx, cudaStream_t s, void* dst, const void* src, size_t bytes) {
+    if (!bytes) return;
+    unsigned char* h = upload_area(ctx, s, bytes);
+    std::memcpy(h, src, bytes);
+    upload_from(s, dst, h, bytes);
+}
+
 // ---------------------------------------------------------------------------
 // The mining driver for a batch of jobs.
 // ---------------------------------------------------------------------------
 void setup_batch(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params* pv, uint32_t J, Batch& b,
                  std::vector<DevBuf<float>>& ownf, double* t_upload) {
     cudaStream_t s = ctx->s;
+    b.ctx = ctx;
     b.s = s;
     b.sms = ctx->sms;
     b.J = J;
@@ -730,6 +763,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
     bool host_tables = false;
     for (uint32_t j = 0; j < J; ++j) host_tables |= (pv[j].reserved[0] & 8) != 0;
     uint64_t cnt_host_table_bytes = 0;
+    std::vector<uint32_t> h_least;   // per feature, least_bound (once asked for)
     for (uint32_t k = 2;; ++k) {
         bool any = false;
         for (auto& st : js) any |= (st.active && !st.cands.empty());
@@ -762,6 +796,8 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         const bool learned_mode = mode == COLO_MODE_LEARNED && !ctx->model.empty();
         bool force_single_any = false;
         for (uint32_t j = 0; j < J; ++j) force_single_any |= (pv[j].reserved[0] & 16) != 0;
+        bool one_wait = false;   // the filter's results come back with the counts'
+        std::vector<uint32_t> hc, hjob;
         if (k == 2) {
             // the mine's first wait: sizes, counts and the pairs' bounds
             std::vector<uint32_t> h;
@@ -781,8 +817,8 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
                 }
             }
         } else {
-            std::vector<uint32_t> hc, hjob;
             std::vector<std::pair<uint32_t, size_t>> owner;
+            uint64_t longest = 0, chunks = 0, words = 0;
             for (uint32_t j = 0; j < J; ++j) {
                 if (!tr[j]) continue;
                 const LevelTrace& L = *tr[j];
@@ -790,11 +826,21 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
                     hc.insert(hc.end(), L.cand.begin() + c * k, L.cand.begin() + (c + 1) * k);
                     hjob.push_back(j);
                     owner.push_back({j, c});
+                    const uint64_t prow = js[j].prev_tables[js[j].parent[c]].rows;
+                    longest = std::max(longest, prow);
+                    chunks += (prow + 31) / 32;
+                    for (uint32_t t = 0; t < k; ++t) words += (b.h_fcount[L.cand[c * k + t]] + 31) / 32;
                 }
             }
             uint64_t ncand = owner.size();
             bool rec_all = false;
             for (uint32_t j = 0; j < J; ++j) rec_all |= tr[j] && (pv[j].reserved[0] & 2) != 0;
+            one_wait = !plain && !rec_all && !force_single_any && (!learned_mode || longest <= kOneWaitRows) &&
+                       chunks <= kOneWaitChunks && words <= kOneWaitWords;
+            if (one_wait)
+                for (uint32_t j = 0; j < J; ++j)
+                    if (tr[j]) tr[j]->pass.assign(tr[j]->pass.size(), 1);   // until the bounds are back
+            if (!one_wait) {
             const bool infer = learned_mode && ncand > 0;
             const bool want_x = (rec_all || infer) && ncand;
             // the level's filter buffers from one allocation: the results (bounds, cell
@@ -833,7 +879,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
                 if (infer) std::memcpy(hin + (o_par - o_cand), ctx->model.data(), kMlpParams * 4);
                 upload_from(s, d_cand, hin, in_end - o_cand);
             }
-            filter_level(b, hc.data(), hjob.data(), ncand, k, d_ub, d_fs, d_cand);
+            filter_level(b, hc.data(), hjob.data(), ncand, k, d_ub, d_fs);
             const auto tl0 = Clock::now();
             // cost-model features and predictions on the device, read back with the bounds
             Readback rb(ctx, s, (rec_all ? ncand * kMlpIn * 4 : 0) + out_bytes);
@@ -885,6 +931,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
                 size_t c = owner[q].second;
                 for (uint32_t t = 0; t < k; ++t) L.ub[c * k + t] = hub[q * k + t];
                 L.pass[c] = filter_pass(&L.ub[c * k], &L.cand[c * k], k, b.h_fcount, js[owner[q].first].thr);
+            }
             }
         }
         // pairs: cost-model features on the host (every candidate when the caller
@@ -945,14 +992,12 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         t0 = Clock::now();
         std::vector<CandDesc> hd;
         std::vector<std::pair<uint32_t, size_t>> owner;
-        std::vector<uint64_t> chunk_off(1, 0);
         {
             size_t most = 0;   // every candidate of the level passes at most
             for (uint32_t j = 0; j < J; ++j)
                 if (tr[j]) most += tr[j]->cand.size() / k;
             hd.reserve(most);
             owner.reserve(most);
-            chunk_off.reserve(most + 1);
         }
         uint64_t nwords = 0;
         for (uint32_t j = 0; j < J; ++j) {
@@ -987,15 +1032,14 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
                 }
                 d.bm_base = nwords;
                 nwords += w;
-                chunk_off.push_back(chunk_off.back() + (d.prow + 31) / 32);
                 hd.push_back(d);
                 owner.push_back({j, c});
             }
         }
-        const uint64_t ncand = hd.size();
+        uint64_t ncand = hd.size();
         kt.mark("refine descriptors");
         // LEARNED: predicted rows presize one-pass tables; the queue runs largest first
-        bool learned = mode == COLO_MODE_LEARNED && !ctx->model.empty() && ncand > 0;
+        bool learned = mode == COLO_MODE_LEARNED && !ctx->model.empty() && ncand > 0 && !one_wait;
         std::vector<uint64_t> cap, pc;
         if (learned) {
             std::vector<float> y(ncand);
@@ -1037,12 +1081,10 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
             std::vector<CandDesc> hd2(ncand);
             std::vector<std::pair<uint32_t, size_t>> own2(ncand);
             cap.resize(ncand);
-            chunk_off.assign(1, 0);
             for (uint64_t i = 0; i < ncand; ++i) {
                 hd2[i] = hd[perm[i]];
                 own2[i] = owner[perm[i]];
                 cap[i] = pc[perm[i]];
-                chunk_off.push_back(chunk_off.back() + (hd2[i].prow + 31) / 32);
             }
             hd.swap(hd2);
             owner.swap(own2);
@@ -1083,8 +1125,22 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         LevelArena ar;
         const uint64_t nch_all = nch_single + nch_count;
         // candidate q's first chunk among all (the single pass's chunks come first)
-        auto first_chunk = [&](uint64_t q) { return q < ns ? chunk_all[q] : nch_single + chunk_all[q + 1]; };
-        ar.init(nch_all, nwords, ncand, nch_single, k, ns > 0, s);
+        std::vector<uint64_t> first_chunk(ncand);
+        for (uint64_t q = 0; q < ncand; ++q) first_chunk[q] = q < ns ? chunk_all[q] : nch_single + chunk_all[q + 1];
+        ar.init(nch_all, nwords, ncand, nch_single, k, ns > 0, one_wait, s);
+        const auto tl0 = Clock::now();
+        std::vector<uint32_t> least;   // per member, the least bound that passes
+        if (one_wait && ncand) {
+            filter_level(b, hc.data(), hjob.data(), ncand, k, ar.ub.get(), ar.fs.get());
+            least.resize(ncand * k);
+            if (h_least.empty()) h_least.assign(b.F, UINT32_MAX - 1);   // not looked for yet
+            for (uint64_t q = 0; q < ncand; ++q)
+                for (uint32_t t = 0; t < k; ++t) {
+                    uint32_t& u = h_least[hc[q * k + t]];
+                    if (u == UINT32_MAX - 1) u = least_bound(b.h_fcount[hc[q * k + t]], js[hjob[q]].thr);
+                    least[q * k + t] = u;
+                }
+        }
         std::unique_ptr<TableBuf> single_cur;
         uint64_t single_words = 0;
         if (ns) {
@@ -1094,7 +1150,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
             if (single_cur->on_host()) cnt_host_table_bytes += single_words * 4;
         }
         for (uint64_t q = 0, o = 0; q < ncand; ++q) {
-            hd[q].chunk_rows = ar.chunk_rows.get() + first_chunk(q);
+            hd[q].chunk_rows = ar.chunk_rows.get() + first_chunk[q];
             hd[q].bitmap = ar.bitmap.get();
             hd[q].mem = ar.mem.get() + q * k;
             hd[q].rows = ar.rows.get() + q;
@@ -1107,10 +1163,8 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         }
         kt.mark("refine arena");
         std::vector<uint64_t> hstats(ncand * k * 4);
-        Readback rb(ctx, s, ar.out_bytes + sizeof(DevFlags));
-        cnt_refined += ncand;
-        cnt_bmw += nwords;
-        for (uint64_t q = 0; q < ncand; ++q) cnt_parent += (uint64_t)(k - 1) * hd[q].prow;
+        std::vector<unsigned long long> he(k == 2 ? kEntrySlots * kEntryStride : 0);
+        Readback rb(ctx, s, ar.out_bytes + sizeof(DevFlags) + he.size() * 8);
         if (ncand) {
             ar.put_inputs(ctx, s, hd, chunk_all, gchunk, gstart, [&](MemberInfo* out) {
                 for (uint64_t q = 0; q < ncand; ++q) {
@@ -1122,7 +1176,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
                         off += (n + 31) / 32;
                     }
                 }
-            });
+            }, least);
             if (plain) {
                 // per candidate, as the reference refines (one candidate at a time)
                 for (uint64_t q = 0; q < ncand; ++q) {
@@ -1141,8 +1195,13 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
                     level_single(b, w, k, ar.overflow.get());
                 }
                 if (ns < ncand) {
-                    level_count(b, CountWork{ar.descs.get(), ar.gstart.get(), ar.gchunk.get(), ngroups, gchunks,
-                                             ar.items.get(), ar.tickets.get()}, k);
+                    CountWork w{ar.descs.get(), ar.gstart.get(), ar.gchunk.get(), ngroups, gchunks, ar.items.get(),
+                                ar.tickets.get()};
+                    if (one_wait) {
+                        w.ub = ar.ub.get();
+                        w.need = ar.need.get();
+                    }
+                    level_count(b, w, k);
                 }
                 level_pi(b, ar.descs.get(), ncand, k, ar.stats.get());
             }
@@ -1155,6 +1214,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         if (ar.out_bytes) rb.copy(hout.data(), ar.out, ar.out_bytes);
         DevFlags hflags{};
         if (ns) rb.copy(&hflags, b.flags(), sizeof(hflags));
+        if (k == 2 && b.E == UINT64_MAX) rb.copy(he.data(), b.dE.get(), he.size() * 8);   // the join has run by now
         COLO_CUDA(cudaEventRecord(ctx->ev_counted, s));
         // the fill's output offsets: the scan runs behind the copies, while the host reads them
         if (ncand && !plain) scan_u32_to_u64(ar.chunk_rows.get(), ar.offs.get(), nch_all, ar.words.get(), s);
@@ -1168,6 +1228,40 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
             if (!plain)
                 std::memcpy(hstats.data(), hout.data() + (reinterpret_cast<unsigned char*>(ar.stats.get()) - ar.out),
                             hstats.size() * 8);
+        }
+        if (k == 2 && b.E == UINT64_MAX) b.E = sum_entries(he.data());
+        if (one_wait) {
+            // the filter's results, and the refined candidates among all
+            us_level_wait += (uint64_t)(ms_since(tl0) * 1000.0);
+            const uint32_t* hub = reinterpret_cast<const uint32_t*>(hout.data() + ar.ub_at);
+            const unsigned char* hfs = hout.data() + ar.fs_at;
+            uint64_t kept = 0;
+            for (uint64_t q = 0; q < ncand; ++q) {
+                LevelTrace& L = *tr[owner[q].first];
+                const size_t c = owner[q].second;
+                uint64_t fs[2];
+                std::memcpy(fs, hfs + q * 16, 16);
+                L.fquads[c] = fs[0];
+                L.fcells[c] = fs[1];
+                cnt_fcm += fs[1] * std::min<uint32_t>(k, kMaxMembersFiltered);
+                cnt_fquads += fs[0];
+                cnt_fcells += fs[1];
+                for (uint32_t t = 0; t < k; ++t) L.ub[c * k + t] = hub[q * k + t];
+                L.pass[c] = filter_pass(&L.ub[c * k], &L.cand[c * k], k, b.h_fcount, js[owner[q].first].thr);
+                if (!L.pass[c]) continue;
+                hd[kept] = hd[q];
+                owner[kept] = owner[q];
+                hrows[kept] = hrows[q];
+                first_chunk[kept] = first_chunk[q];
+                std::copy(hstats.begin() + q * k * 4, hstats.begin() + (q + 1) * k * 4, hstats.begin() + kept * k * 4);
+                ++kept;
+            }
+            ncand = kept;
+        }
+        cnt_refined += ncand;
+        for (uint64_t q = 0; q < ncand; ++q) {
+            cnt_parent += (uint64_t)(k - 1) * hd[q].prow;
+            cnt_bmw += hd[q].last_off + (hd[q].last_end - hd[q].last_start + 31) / 32;
         }
         if (hflags.timeout)
             throw StatusError{COLO_ERR_TIMEOUT, "single-pass tables: a chunk waited too long for its predecessors"};
@@ -1204,7 +1298,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         cnt_single += ns;
         for (uint64_t q = 0; q < ns; ++q) cnt_single_ovf += hovf[q] ? 1 : 0;
         cnt_items += h_items;
-        cnt_d2h += ncand * 8 + hstats.size() * 8;
+        cnt_d2h += ncand * 8 + ncand * k * 4 * 8;
         std::vector<uint64_t> gb(ncand + 1, 0);
         for (uint64_t q = 0; q < ncand; ++q) gb[q + 1] = gb[q] + hrows[q];
         for (uint64_t q = 0; q < ncand; ++q) tr[owner[q].first]->rows[owner[q].second] = gb[q + 1] - gb[q];
@@ -1331,7 +1425,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         if (tables_cur->on_host()) cnt_host_table_bytes += total_rows * k * 4;
         if (plain)   // one scan per candidate, as the reference does
             for (uint64_t q : fillq)
-                scan_u32_to_u64(ar.chunk_rows.get() + first_chunk(q), ar.offs.get() + first_chunk(q),
+                scan_u32_to_u64(ar.chunk_rows.get() + first_chunk[q], ar.offs.get() + first_chunk[q],
                                 (hd[q].prow + 31) / 32, s, nullptr);
         std::vector<CandDesc> fd;
         std::vector<uint64_t> fchunk(1, 0);
@@ -1339,7 +1433,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         for (uint64_t q : fillq) {
             CandDesc d = hd[q];
             uint64_t rows = gb[q + 1] - gb[q];
-            d.offs = ar.offs.get() + first_chunk(q);
+            d.offs = ar.offs.get() + first_chunk[q];
             d.out = tables_cur->get() + obase;
             d.out_rows = rows;
             obase += rows * k;
