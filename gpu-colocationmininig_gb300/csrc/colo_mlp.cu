@@ -15,6 +15,8 @@
 //   W1[32][64] (rows 24..31 zero), b1[64], W2[64][64], b2[64], W3[64], b3
 #include <cuda_bf16.h>
 
+#include <cstddef>
+
 #include "colo_internal.h"
 #include "colo_mlp.h"
 
@@ -40,11 +42,12 @@ __device__ __forceinline__ void mma16816(float* d, const uint32_t* a, uint32_t b
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// Shared weights: BF16, both orientations for the hidden layer.
+// Shared weights: BF16, both orientations for the hidden layer.  Rows are padded by 16 bytes: the
+// eight rows that a B fragment is read from then lie in different banks.
 struct SmemW {
-    __nv_bfloat16 w1t[H][INP];   // [out][in]  (B operand of X.W1)
-    __nv_bfloat16 w2t[H][H];     // [out][in]  (B operand of H1.W2)
-    __nv_bfloat16 w2[H][H];      // [in][out]  (B operand of dZ2.W2^T)
+    __nv_bfloat16 w1t[H][INP + 8];   // [out][in]  (B operand of X.W1)
+    __nv_bfloat16 w2t[H][H + 8];     // [out][in]  (B operand of H1.W2)
+    __nv_bfloat16 w2[H][H + 8];      // [in][out]  (B operand of dZ2.W2^T)
     float b1[H], b2[H], w3[H];
     float b3;
 };
@@ -69,8 +72,8 @@ __device__ void load_weights(SmemW& s, const float* __restrict__ P) {
 }
 
 // B fragment of a [N][K] row-major BF16 matrix for n-tile nt, k-tile kt.
-template <int K>
-__device__ __forceinline__ void bfrag(const __nv_bfloat16 (*m)[K], int nt, int kt, int gid, int tig, uint32_t& b0,
+template <int LD>
+__device__ __forceinline__ void bfrag(const __nv_bfloat16 (*m)[LD], int nt, int kt, int gid, int tig, uint32_t& b0,
                                       uint32_t& b1) {
     const __nv_bfloat16* r = m[nt * 8 + gid] + kt * 16 + tig * 2;
     b0 = *reinterpret_cast<const uint32_t*>(r);
@@ -107,7 +110,7 @@ __device__ __forceinline__ void forward16(const SmemW& s, const float* __restric
         z1[nt][3] = bb1;
         for (int kt = 0; kt < 2; ++kt) {
             uint32_t b0, b1;
-            bfrag<INP>(s.w1t, nt, kt, gid, tig, b0, b1);
+            bfrag(s.w1t, nt, kt, gid, tig, b0, b1);
             mma16816(z1[nt], xa[kt], b0, b1);
         }
     }
@@ -129,7 +132,7 @@ __device__ __forceinline__ void forward16(const SmemW& s, const float* __restric
         z2[nt][3] = bb1;
         for (int kt = 0; kt < 4; ++kt) {
             uint32_t b0, b1;
-            bfrag<H>(s.w2t, nt, kt, gid, tig, b0, b1);
+            bfrag(s.w2t, nt, kt, gid, tig, b0, b1);
             mma16816(z2[nt], ha[kt], b0, b1);
         }
     }
@@ -167,12 +170,42 @@ __global__ void __launch_bounds__(256) k_mlp_forward(const float* __restrict__ P
     }
 }
 
-// Shared memory of the gradient kernel (dynamic: about 100 KB).
+// Shared memory of the gradient kernel (dynamic): the weights and, for the tile's 128 rows, the
+// BF16 operands of the weight gradients.  Rows are padded by 16 bytes: the eight rows of an
+// ldmatrix then lie in different banks.
 struct GradSmem {
     SmemW w;
-    float gw1[INP * H], gw2[H * H], gb1[H], gb2[H], gw3[H], gb3, lsum;
-    __nv_bfloat16 h1s[kWarps][16][H], dz2s[kWarps][16][H], dz1s[kWarps][16][H], xs[kWarps][16][INP];
+    alignas(16) __nv_bfloat16 h1[kRowsPerBlock][H + 8];
+    alignas(16) __nv_bfloat16 dz2[kRowsPerBlock][H + 8];
+    alignas(16) __nv_bfloat16 dz1[kRowsPerBlock][H + 8];
+    alignas(16) __nv_bfloat16 x[kRowsPerBlock][INP + 8];
+    float col[3][H], gb3, lsum;   // the block's sums at the end: b1, b2, W3
 };
+// ldmatrix reads 16-byte rows at 16-byte addresses
+static_assert(offsetof(GradSmem, h1) % 16 == 0 && offsetof(GradSmem, dz2) % 16 == 0 && offsetof(GradSmem, dz1) % 16 == 0 &&
+                  offsetof(GradSmem, x) % 16 == 0 && sizeof(__nv_bfloat16) * (H + 8) % 16 == 0 &&
+                  sizeof(__nv_bfloat16) * (INP + 8) % 16 == 0 && alignof(GradSmem) == 16,
+              "alignment");
+
+// A fragment (16 x 16) of S^T, S[k][m] in shared memory: rows m0.., columns (S's rows) k0...
+template <int LD>
+__device__ __forceinline__ void frag_a_t(const __nv_bfloat16 (*S)[LD], int k0, int m0, int lane, uint32_t (&a)[4]) {
+    const int t = lane >> 3;   // 8x8 tile: m half t & 1, k half t >> 1
+    const __nv_bfloat16* p = &S[k0 + (t >> 1) * 8 + (lane & 7)][m0 + (t & 1) * 8];
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+
+// B fragments (16 x 8) of two neighbouring column tiles of S[k][n]: columns n0.. and n0 + 8...
+template <int LD>
+__device__ __forceinline__ void frag_b2(const __nv_bfloat16 (*S)[LD], int k0, int n0, int lane, uint32_t (&b)[4]) {
+    const int t = lane >> 3;   // k half t & 1, column tile t >> 1
+    const __nv_bfloat16* p = &S[k0 + (t & 1) * 8 + (lane & 7)][n0 + (t >> 1) * 8];
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
 
 __device__ __forceinline__ float quad_sum(float v) {   // sum over the 8 lanes sharing tig
     for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -182,159 +215,153 @@ __device__ __forceinline__ float quad_sum(float v) {   // sum over the 8 lanes s
 // Forward + backward of a mini-batch; gradients of the mean of 0.5*(y-t)^2
 // over `n` rows (rows idx[r], or r when idx is null) accumulate (FP32
 // atomics) into G (kMlpParams floats).
-__global__ void __launch_bounds__(256) k_mlp_grad(const float* __restrict__ P, const float* __restrict__ X,
-                                                  const float* __restrict__ T, const uint32_t* __restrict__ idx,
-                                                  uint64_t n, float inv_n, float* __restrict__ G,
-                                                  float* __restrict__ loss) {
+//
+// A block takes 128 rows at a time.  Each warp runs 16 of them forward and back
+// and leaves the operands of the weight gradients in shared memory; the warps
+// then split dW2 (64 x 64) and dW1 (32 x 64) between them, 128 rows deep, and
+// keep their parts, and the bias and W3 sums of their rows, in registers over
+// all of the block's rows: one round of atomics per block at the end.  (Summing
+// each 16-row product into shared memory, 6,144 FP32 atomics a warp and tile,
+// took 387 us for 205,545 rows; this takes 55 us.)  The call is then bound by the host
+// link: 20 MB of rows, 115 us.
+__global__ void __launch_bounds__(256, 1) k_mlp_grad(const float* __restrict__ P, const float* __restrict__ X,
+                                                     const float* __restrict__ T, const uint32_t* __restrict__ idx,
+                                                     uint64_t n, float inv_n, float* __restrict__ G,
+                                                     float* __restrict__ loss) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     GradSmem& S = *reinterpret_cast<GradSmem*>(smem_raw);
     const SmemW& s = S.w;
     load_weights(S.w, P);
-    for (int i = threadIdx.x; i < INP * H; i += blockDim.x) S.gw1[i] = 0.f;
-    for (int i = threadIdx.x; i < H * H; i += blockDim.x) S.gw2[i] = 0.f;
-    for (int i = threadIdx.x; i < H; i += blockDim.x) S.gb1[i] = S.gb2[i] = S.gw3[i] = 0.f;
+    for (int i = threadIdx.x; i < H; i += blockDim.x) S.col[0][i] = S.col[1][i] = S.col[2][i] = 0.f;
     if (threadIdx.x == 0) S.gb3 = S.lsum = 0.f;
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
-    for (uint64_t row0 = ((uint64_t)blockIdx.x * kWarps + w) * kRowsPerWarp; row0 < n;
-         row0 += (uint64_t)gridDim.x * kRowsPerBlock) {
+    // this warp's parts: dW2 rows (in) 16 (w / 2).., columns 32 (w % 2)..; dW1 rows 16 (w % 2).., columns 16 (w / 2)..
+    const int m2 = (w >> 1) * 16, n2 = (w & 1) * 32, m1 = (w & 1) * 16, n1 = (w >> 1) * 16;
+    float gw2[4][4], gw1[2][4], gb1[16], gb2[16], gw3[16], gb3 = 0.f, lsum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        gw2[i >> 2][i & 3] = gb1[i] = gb2[i] = gw3[i] = 0.f;
+        if (i < 8) gw1[i >> 2][i & 3] = 0.f;
+    }
+    for (uint64_t tile0 = (uint64_t)blockIdx.x * kRowsPerBlock; tile0 < n; tile0 += (uint64_t)gridDim.x * kRowsPerBlock) {
+        const uint64_t row0 = tile0 + (uint64_t)w * kRowsPerWarp;
+        const int r_lo = w * kRowsPerWarp + gid, r_hi = r_lo + 8;
         float z1[8][4], z2[8][4], ylo, yhi;
         uint32_t xa[2][4];
-        forward16(s, X, idx, row0, n, gid, tig, z1, z2, ylo, yhi, xa);
+        forward16(s, X, idx, row0, n, gid, tig, z1, z2, ylo, yhi, xa);   // rows past n read as zeros
         const bool vlo = row0 + gid < n, vhi = row0 + gid + 8 < n;
         const float tlo = vlo ? T[idx ? idx[row0 + gid] : row0 + gid] : 0.f;
         const float thi = vhi ? T[idx ? idx[row0 + gid + 8] : row0 + gid + 8] : 0.f;
         const float dlo = vlo ? (ylo - tlo) * inv_n : 0.f;
         const float dhi = vhi ? (yhi - thi) * inv_n : 0.f;
-        {
-            // loss and db3 over the 16 rows: lanes with tig == 0 hold one row pair each
-            float l = tig == 0 ? ((vlo ? 0.5f * (ylo - tlo) * (ylo - tlo) : 0.f) +
-                                  (vhi ? 0.5f * (yhi - thi) * (yhi - thi) : 0.f)) * inv_n
-                               : 0.f;
-            float g = tig == 0 ? dlo + dhi : 0.f;
-            for (int o = 1; o < 32; o <<= 1) {
-                l += __shfl_xor_sync(0xffffffffu, l, o);
-                g += __shfl_xor_sync(0xffffffffu, g, o);
-            }
-            if (lane == 0) {
-                atomicAdd(&S.lsum, l);
-                atomicAdd(&S.gb3, g);
-            }
+        if (tig == 0) {   // one lane per row pair
+            lsum += ((vlo ? 0.5f * (ylo - tlo) * (ylo - tlo) : 0.f) + (vhi ? 0.5f * (yhi - thi) * (yhi - thi) : 0.f)) * inv_n;
+            gb3 += dlo + dhi;
         }
-        // layer 3: dW3 = H2b^T dy; dZ2 = dy * w3 * (z2 > 0)
-        float dz2[8][4];
-        for (int nt = 0; nt < 8; ++nt)
+        __syncthreads();   // the last tile's operands have been read
+        // layer 3: dW3 = H2b^T dy; dZ2 = dy * w3 * (z2 > 0), summed for db2 and left in BF16
+        uint32_t da[4][4], on1 = 0;   // dZ2b as the A operand; bit 4 nt + i: z1[nt][i] > 0
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+            float lo[2], hi[2];
+#pragma unroll
             for (int e = 0; e < 2; ++e) {
-                int col = nt * 8 + tig * 2 + e;
-                float h_lo = bf16r(fmaxf(z2[nt][e], 0.f)), h_hi = bf16r(fmaxf(z2[nt][2 + e], 0.f));
-                float g = quad_sum(h_lo * dlo + h_hi * dhi);
-                if (gid == 0) atomicAdd(&S.gw3[col], g);
-                dz2[nt][e] = z2[nt][e] > 0.f ? dlo * s.w3[col] : 0.f;
-                dz2[nt][2 + e] = z2[nt][2 + e] > 0.f ? dhi * s.w3[col] : 0.f;
+                const int col = nt * 8 + tig * 2 + e;
+                gw3[nt * 2 + e] += bf16r(fmaxf(z2[nt][e], 0.f)) * dlo + bf16r(fmaxf(z2[nt][2 + e], 0.f)) * dhi;
+                lo[e] = z2[nt][e] > 0.f ? dlo * s.w3[col] : 0.f;
+                hi[e] = z2[nt][2 + e] > 0.f ? dhi * s.w3[col] : 0.f;
+                gb2[nt * 2 + e] += lo[e] + hi[e];
+                on1 |= (z1[nt][e] > 0.f ? 1u : 0u) << (nt * 4 + e) | (z1[nt][2 + e] > 0.f ? 1u : 0u) << (nt * 4 + 2 + e);
             }
-        // stash H1b, dZ2b, X (BF16) for the transposed weight-gradient products
-        for (int nt = 0; nt < 8; ++nt)
-            for (int e = 0; e < 2; ++e) {
-                int col = nt * 8 + tig * 2 + e;
-                S.h1s[w][gid][col] = __float2bfloat16_rn(fmaxf(z1[nt][e], 0.f));
-                S.h1s[w][gid + 8][col] = __float2bfloat16_rn(fmaxf(z1[nt][2 + e], 0.f));
-                S.dz2s[w][gid][col] = __float2bfloat16_rn(dz2[nt][e]);
-                S.dz2s[w][gid + 8][col] = __float2bfloat16_rn(dz2[nt][2 + e]);
-            }
+            const int c = nt * 8 + tig * 2;
+            const uint32_t plo = pack_bf16(lo[0], lo[1]), phi = pack_bf16(hi[0], hi[1]);
+            da[nt >> 1][(nt & 1) * 2] = plo;
+            da[nt >> 1][(nt & 1) * 2 + 1] = phi;
+            *reinterpret_cast<uint32_t*>(&S.dz2[r_lo][c]) = plo;
+            *reinterpret_cast<uint32_t*>(&S.dz2[r_hi][c]) = phi;
+            *reinterpret_cast<uint32_t*>(&S.h1[r_lo][c]) = pack_bf16(fmaxf(z1[nt][0], 0.f), fmaxf(z1[nt][1], 0.f));
+            *reinterpret_cast<uint32_t*>(&S.h1[r_hi][c]) = pack_bf16(fmaxf(z1[nt][2], 0.f), fmaxf(z1[nt][3], 0.f));
+        }
+#pragma unroll
         for (int kt = 0; kt < 2; ++kt) {
-            *reinterpret_cast<uint32_t*>(&S.xs[w][gid][kt * 16 + tig * 2]) = xa[kt][0];
-            *reinterpret_cast<uint32_t*>(&S.xs[w][gid + 8][kt * 16 + tig * 2]) = xa[kt][1];
-            *reinterpret_cast<uint32_t*>(&S.xs[w][gid][kt * 16 + 8 + tig * 2]) = xa[kt][2];
-            *reinterpret_cast<uint32_t*>(&S.xs[w][gid + 8][kt * 16 + 8 + tig * 2]) = xa[kt][3];
+            *reinterpret_cast<uint32_t*>(&S.x[r_lo][kt * 16 + tig * 2]) = xa[kt][0];
+            *reinterpret_cast<uint32_t*>(&S.x[r_hi][kt * 16 + tig * 2]) = xa[kt][1];
+            *reinterpret_cast<uint32_t*>(&S.x[r_lo][kt * 16 + 8 + tig * 2]) = xa[kt][2];
+            *reinterpret_cast<uint32_t*>(&S.x[r_hi][kt * 16 + 8 + tig * 2]) = xa[kt][3];
         }
-        // db2 = sum over rows of dZ2
-        for (int nt = 0; nt < 8; ++nt)
-            for (int e = 0; e < 2; ++e) {
-                float g = quad_sum(dz2[nt][e] + dz2[nt][2 + e]);
-                if (gid == 0) atomicAdd(&S.gb2[nt * 8 + tig * 2 + e], g);
-            }
-        __syncwarp();
-        // dH1 = dZ2b . W2^T  (A = dZ2b from the accumulator layout)
-        uint32_t da[4][4];
-        for (int kt = 0; kt < 4; ++kt) {
-            const float* c0 = dz2[2 * kt];
-            const float* c1 = dz2[2 * kt + 1];
-            da[kt][0] = pack_bf16(c0[0], c0[1]);
-            da[kt][1] = pack_bf16(c0[2], c0[3]);
-            da[kt][2] = pack_bf16(c1[0], c1[1]);
-            da[kt][3] = pack_bf16(c1[2], c1[3]);
-        }
+        // dH1 = dZ2b . W2^T; dZ1 = dH1 * (z1 > 0), summed for db1 and left in BF16
+#pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
             float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
             for (int kt = 0; kt < 4; ++kt) {
                 uint32_t b0, b1;
-                bfrag<H>(s.w2, nt, kt, gid, tig, b0, b1);
+                bfrag(s.w2, nt, kt, gid, tig, b0, b1);
                 mma16816(acc, da[kt], b0, b1);
             }
-            // dZ1 = dH1 * (z1 > 0); db1; stash BF16
-            for (int e = 0; e < 2; ++e) {
-                int col = nt * 8 + tig * 2 + e;
-                float lo = z1[nt][e] > 0.f ? acc[e] : 0.f;
-                float hi = z1[nt][2 + e] > 0.f ? acc[2 + e] : 0.f;
-                S.dz1s[w][gid][col] = __float2bfloat16_rn(lo);
-                S.dz1s[w][gid + 8][col] = __float2bfloat16_rn(hi);
-                float g = quad_sum(lo + hi);
-                if (gid == 0) atomicAdd(&S.gb1[col], g);
-            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[i] = on1 >> (nt * 4 + i) & 1u ? acc[i] : 0.f;
+            gb1[nt * 2] += acc[0] + acc[2];
+            gb1[nt * 2 + 1] += acc[1] + acc[3];
+            const int c = nt * 8 + tig * 2;
+            *reinterpret_cast<uint32_t*>(&S.dz1[r_lo][c]) = pack_bf16(acc[0], acc[1]);
+            *reinterpret_cast<uint32_t*>(&S.dz1[r_hi][c]) = pack_bf16(acc[2], acc[3]);
         }
-        __syncwarp();
-        // dW2[in][out] = sum_r H1b[r][in] * dZ2b[r][out]: M = in (4 tiles), N = out (8 tiles), K = 16 rows
-        const int k0 = tig * 2;
-        for (int mt = 0; mt < 4; ++mt) {
-            const int m0 = mt * 16 + gid, m1 = m0 + 8;
-            uint32_t a[4];
-            a[0] = pack_bf16(__bfloat162float(S.h1s[w][k0][m0]), __bfloat162float(S.h1s[w][k0 + 1][m0]));
-            a[1] = pack_bf16(__bfloat162float(S.h1s[w][k0][m1]), __bfloat162float(S.h1s[w][k0 + 1][m1]));
-            a[2] = pack_bf16(__bfloat162float(S.h1s[w][k0 + 8][m0]), __bfloat162float(S.h1s[w][k0 + 9][m0]));
-            a[3] = pack_bf16(__bfloat162float(S.h1s[w][k0 + 8][m1]), __bfloat162float(S.h1s[w][k0 + 9][m1]));
-            for (int nt = 0; nt < 8; ++nt) {
-                const int nn = nt * 8 + gid;
-                uint32_t b0 = pack_bf16(__bfloat162float(S.dz2s[w][k0][nn]), __bfloat162float(S.dz2s[w][k0 + 1][nn]));
-                uint32_t b1 = pack_bf16(__bfloat162float(S.dz2s[w][k0 + 8][nn]), __bfloat162float(S.dz2s[w][k0 + 9][nn]));
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
-                mma16816(acc, a, b0, b1);
-                const int col = nt * 8 + tig * 2;
-                atomicAdd(&S.gw2[m0 * H + col], acc[0]);
-                atomicAdd(&S.gw2[m0 * H + col + 1], acc[1]);
-                atomicAdd(&S.gw2[m1 * H + col], acc[2]);
-                atomicAdd(&S.gw2[m1 * H + col + 1], acc[3]);
+        __syncthreads();
+        // dW2[in][out] += sum_r H1b[r][in] dZ2b[r][out]; dW1[in][out] += sum_r Xb[r][in] dZ1b[r][out]
+#pragma unroll
+        for (int k0 = 0; k0 < kRowsPerBlock; k0 += 16) {
+            uint32_t a[4], b[4];
+            frag_a_t(S.h1, k0, m2, lane, a);
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                frag_b2(S.dz2, k0, n2 + t * 16, lane, b);
+                mma16816(gw2[t * 2], a, b[0], b[1]);
+                mma16816(gw2[t * 2 + 1], a, b[2], b[3]);
             }
+            frag_a_t(S.x, k0, m1, lane, a);
+            frag_b2(S.dz1, k0, n1, lane, b);
+            mma16816(gw1[0], a, b[0], b[1]);
+            mma16816(gw1[1], a, b[2], b[3]);
         }
-        // dW1[in][out] = sum_r Xb[r][in] * dZ1b[r][out]: M = in (2 tiles), N = out (8 tiles)
-        for (int mt = 0; mt < 2; ++mt) {
-            const int m0 = mt * 16 + gid, m1 = m0 + 8;
-            uint32_t a[4];
-            a[0] = pack_bf16(__bfloat162float(S.xs[w][k0][m0]), __bfloat162float(S.xs[w][k0 + 1][m0]));
-            a[1] = pack_bf16(__bfloat162float(S.xs[w][k0][m1]), __bfloat162float(S.xs[w][k0 + 1][m1]));
-            a[2] = pack_bf16(__bfloat162float(S.xs[w][k0 + 8][m0]), __bfloat162float(S.xs[w][k0 + 9][m0]));
-            a[3] = pack_bf16(__bfloat162float(S.xs[w][k0 + 8][m1]), __bfloat162float(S.xs[w][k0 + 9][m1]));
-            for (int nt = 0; nt < 8; ++nt) {
-                const int nn = nt * 8 + gid;
-                uint32_t b0 = pack_bf16(__bfloat162float(S.dz1s[w][k0][nn]), __bfloat162float(S.dz1s[w][k0 + 1][nn]));
-                uint32_t b1 = pack_bf16(__bfloat162float(S.dz1s[w][k0 + 8][nn]), __bfloat162float(S.dz1s[w][k0 + 9][nn]));
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
-                mma16816(acc, a, b0, b1);
-                const int col = nt * 8 + tig * 2;
-                atomicAdd(&S.gw1[m0 * H + col], acc[0]);
-                atomicAdd(&S.gw1[m0 * H + col + 1], acc[1]);
-                atomicAdd(&S.gw1[m1 * H + col], acc[2]);
-                atomicAdd(&S.gw1[m1 * H + col + 1], acc[3]);
-            }
+    }
+    // the block's sums, one atomic per parameter
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            atomicAdd(&G[OFF_W2 + (m2 + gid + (i >> 1) * 8) * H + n2 + t * 8 + tig * 2 + (i & 1)], gw2[t][i]);
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int in = m1 + gid + (i >> 1) * 8;
+            if (in < IN) atomicAdd(&G[OFF_W1 + in * H + n1 + t * 8 + tig * 2 + (i & 1)], gw1[t][i]);   // rows >= 24 stay 0
         }
-        __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const int col = (i >> 1) * 8 + tig * 2 + (i & 1);
+        const float v1 = quad_sum(gb1[i]), v2 = quad_sum(gb2[i]), v3 = quad_sum(gw3[i]);
+        if (gid == 0) {
+            atomicAdd(&S.col[0][col], v1);
+            atomicAdd(&S.col[1][col], v2);
+            atomicAdd(&S.col[2][col], v3);
+        }
+    }
+    for (int o = 1; o < 32; o <<= 1) {
+        lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+        gb3 += __shfl_xor_sync(0xffffffffu, gb3, o);
+    }
+    if (lane == 0) {
+        atomicAdd(&S.lsum, lsum);
+        atomicAdd(&S.gb3, gb3);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < IN * H; i += blockDim.x) atomicAdd(&G[OFF_W1 + i], S.gw1[i]);   // rows >= 24 stay 0
-    for (int i = threadIdx.x; i < H * H; i += blockDim.x) atomicAdd(&G[OFF_W2 + i], S.gw2[i]);
     for (int i = threadIdx.x; i < H; i += blockDim.x) {
-        atomicAdd(&G[OFF_B1 + i], S.gb1[i]);
-        atomicAdd(&G[OFF_B2 + i], S.gb2[i]);
-        atomicAdd(&G[OFF_W3 + i], S.gw3[i]);
+        atomicAdd(&G[OFF_B1 + i], S.col[0][i]);
+        atomicAdd(&G[OFF_B2 + i], S.col[1][i]);
+        atomicAdd(&G[OFF_W3 + i], S.col[2][i]);
     }
     if (threadIdx.x == 0) {
         atomicAdd(&G[OFF_B3], S.gb3);
@@ -425,7 +452,9 @@ void mlp_grad(const float* d_params, const float* d_x, const float* d_t, const u
         attr_dev = dev;
     }
     uint64_t blocks = (n + kRowsPerBlock - 1) / kRowsPerBlock;
-    if (blocks > 1024) blocks = 1024;
+    int sms = 0;
+    COLO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (blocks > (uint64_t)sms) blocks = (uint64_t)sms;   // one resident block an SM (255 registers)
     KScope ks("mlp_grad");
     k_mlp_grad<<<(unsigned)blocks, 256, sizeof(GradSmem), s>>>(d_params, d_x, d_t, d_idx, n, 1.0f / (float)n, d_grad,
                                                                 d_loss);
