@@ -80,9 +80,7 @@ struct Batch {
     uint32_t* frun() const { return dcnt() + F; }
     uint32_t* ub2() const { return frun() + F; }
     DevFlags* flags() const { return &ctrl.get()->flags; }
-    // points (by id)
-    const float* x = nullptr;    // borrowed (dataset device copy)
-    const float* y = nullptr;
+    // points (by id; the jobs' own coordinates are in their grids)
     DevBuf<unsigned char> mem_points, mem_heads, mem_cells, mem_lists, mem_act, mem_nb;
     Span<float2> xy;             // coordinates by id, packed (built by the cell-key pass)
     // bucketed (sorted by cell key, then id)

@@ -21,10 +21,9 @@ namespace {
 // scans them in place), so the sort does not read the keys again to count
 // them.  When the sort runs a pass its first pass makes the ids itself.
 template <class KT>
-__global__ void __launch_bounds__(256) k_cell_keys(
-    uint64_t n, const float* __restrict__ x, const float* __restrict__ y, uint32_t F,
-    const uint32_t* __restrict__ fstart, const uint32_t* __restrict__ fjob, const JobGrid* __restrict__ grids,
-    KT* __restrict__ keys, uint32_t* __restrict__ vals, float2* __restrict__ xy, uint32_t* __restrict__ nb_cnt,
+__global__ void __launch_bounds__(256, 4) k_cell_keys(
+    uint64_t n, uint32_t F, const uint32_t* __restrict__ fstart, const uint32_t* __restrict__ fjob,
+    const JobGrid* __restrict__ grids, KT* __restrict__ keys, uint32_t* __restrict__ vals, float2* __restrict__ xy, uint32_t* __restrict__ nb_cnt,
     BatchCtrl* __restrict__ ctrl, RadixPlan plan, unsigned long long* __restrict__ hist) {
     static_assert(kRadixDigits == 256, "one digit a thread in the scan");
     __shared__ uint32_t h[kRadixMaxPasses * kRadixDigits];
@@ -36,15 +35,16 @@ __global__ void __launch_bounds__(256) k_cell_keys(
     // one point usually covers the next)
     const uint64_t per = ((n + gridDim.x - 1) / gridDim.x + blockDim.x - 1) / blockDim.x * blockDim.x;
     const uint64_t i0 = (uint64_t)blockIdx.x * per, i1 = i0 + per < n ? i0 + per : n;
-    uint32_t f = 0, flo = 1, fhi = 0;   // cached feature and its point range [flo, fhi)
-    for (uint64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-        if (!(i >= flo && i < fhi)) {
-            f = feature_of((uint32_t)i, F, fstart);
-            flo = fstart[f];
-            fhi = f + 1 < F ? fstart[f + 1] : (uint32_t)n;
-        }
-        const JobGrid g = grids[fjob[f]];
-        const float xi = x[i], yi = y[i];
+    uint32_t f = 0, flo = 1, fhi = 0;   // cached feature, its point range [flo, fhi) and its job
+    JobGrid g{};
+    auto seek = [&](uint64_t i) {
+        if (i >= flo && i < fhi) return;
+        f = feature_of((uint32_t)i, F, fstart);
+        flo = fstart[f];
+        fhi = f + 1 < F ? fstart[f + 1] : (uint32_t)n;
+        g = grids[fjob[f]];
+    };
+    auto put = [&](uint64_t i, float xi, float yi) {
         xy[i] = make_float2(xi, yi);
         nb_cnt[i] = 0;
         uint64_t c = ref_cell(g, xi, yi);
@@ -57,6 +57,28 @@ __global__ void __launch_bounds__(256) k_cell_keys(
         if (vals) vals[i] = (uint32_t)i;
         for (int p = 0; p < plan.n; ++p)
             atomicAdd(&h[p * kRadixDigits + ((uint32_t)(key >> plan.shift[p]) & ((1u << plan.width[p]) - 1u))], 1u);
+    };
+    // several points' coordinates in flight (the loads come from memory or over the host link)
+    constexpr int kUnroll = 4;
+    for (uint64_t i = i0 + threadIdx.x; i < i1; i += (uint64_t)kUnroll * blockDim.x) {
+        seek(i);
+        const uint64_t last = i + (uint64_t)(kUnroll - 1) * blockDim.x;
+        if (last < i1 && last < fhi) {   // one feature
+            float xs[kUnroll], ys[kUnroll];
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                const uint64_t q = i - g.p0 + (uint64_t)u * blockDim.x;
+                xs[u] = __ldg(g.x + q);
+                ys[u] = __ldg(g.y + q);
+            }
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) put(i + (uint64_t)u * blockDim.x, xs[u], ys[u]);
+        } else {
+            for (uint64_t q = i; q <= last && q < i1; q += blockDim.x) {
+                seek(q);
+                put(q, __ldg(g.x + (q - g.p0)), __ldg(g.y + (q - g.p0)));
+            }
+        }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < plan.n * kRadixDigits; i += blockDim.x) {
@@ -936,7 +958,7 @@ void sort_and_compact(Batch& b) {
         const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, (uint64_t)b.sms * 8);
         // the ids are written here only when the sort runs no pass (its first pass makes them)
         k_cell_keys<KT><<<(unsigned)(blocks ? blocks : 1), 256, 0, s>>>(
-            n, b.x, b.y, b.F, b.fstart.get(), b.fjob.get(), b.grids.get(), ka.get(), sorts ? nullptr : b.sid.get(),
+            n, b.F, b.fstart.get(), b.fjob.get(), b.grids.get(), ka.get(), sorts ? nullptr : b.sid.get(),
             b.xy.get(), b.nb_cnt.get(), b.ctrl.get(), b.plan, b.hist.get());
         COLO_LAUNCH_CHECK();
         count_launch();

@@ -44,6 +44,8 @@ struct JobGrid {
     uint64_t row_base;           // first grid row of this job in the batch's row table
     int32_t compat32;            // 32-bit reference cell arithmetic is exact
     uint32_t f0, nf;             // global feature range of the job
+    const float *x, *y;          // the job's coordinates, from its first point (batch id p0) on: device
+    uint64_t p0;                 // memory, or host memory that the device reads over the link
 };
 
 // Error carrier for kernels: bounded waits and range checks record here.

@@ -499,38 +499,54 @@ void setup_batch(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params* pv,
     if (N >= (1ull << 32) - 1) throw StatusError{COLO_ERR_CAPACITY, "at most 2^32-2 points per batch"};
     b.N = N;
     b.F = job_f0[J];
-    if (J == 1) {
-        colo_dataset* ds = dsv[0];
-        if (!ds->resident) pin_dataset(ds);
-        if (!ds->resident && ds->mx && ds->my) {
-            // streamed: the cell-key pass reads the page-locked host arrays over
-            // the host link (the only pass that reads them: it writes the packed
-            // device copy every later pass uses), so no separate upload runs
-            b.x = ds->mx;
-            b.y = ds->my;
-            b.h2d_points = 8 * N;
+    // where each job's coordinates are read from: only the cell-key pass reads them (it writes the
+    // packed device copy every later pass uses), so host arrays need no upload of their own when
+    // the device can read them over the link
+    std::vector<const float*> px(J), py(J);
+    bool copies = false;
+    for (uint32_t j = 0; j < J; ++j) {
+        colo_dataset* ds = dsv[j];
+        const uint64_t n = ds->hp.x.size();
+        if (!ds->resident && J == 1) pin_dataset(ds);   // (the link is read fastest from page-locked memory)
+        if (ds->resident) {
+            px[j] = ds->dx.get();
+            py[j] = ds->dy.get();
+        } else if (ds->mx && ds->my) {
+            px[j] = ds->mx;
+            py[j] = ds->my;
+            b.h2d_points += 8 * n;
+        } else if (J > 1 && ctx->host_reads) {
+            px[j] = ds->hp.x.data();
+            py[j] = ds->hp.y.data();
+            b.h2d_points += 8 * n;
+        } else if (J == 1) {
+            b.h2d_points += upload_dataset(ds, s);
+            px[j] = ds->dx.get();
+            py[j] = ds->dy.get();
         } else {
-            b.h2d_points = upload_dataset(ds, s);
-            b.x = ds->dx.get();
-            b.y = ds->dy.get();
+            copies = true;
         }
-    } else {
+    }
+    if (copies) {   // the jobs that the device cannot read where they are
+        uint64_t need = 0;
+        for (uint32_t j = 0; j < J; ++j)
+            if (!px[j]) need += dsv[j]->hp.x.size();
         ownf.resize(2);
-        ownf[0].alloc(N, s);
-        ownf[1].alloc(N, s);
+        ownf[0].alloc(need, s);
+        ownf[1].alloc(need, s);
         uint64_t off = 0;
         for (uint32_t j = 0; j < J; ++j) {
             colo_dataset* ds = dsv[j];
-            uint64_t n = ds->hp.x.size();
-            if (!n) continue;
+            const uint64_t n = ds->hp.x.size();
+            if (px[j] || !n) continue;
+            px[j] = ownf[0].get() + off;
+            py[j] = ownf[1].get() + off;
             COLO_CUDA(cudaMemcpyAsync(ownf[0].get() + off, ds->hp.x.data(), n * 4, cudaMemcpyHostToDevice, s));
             COLO_CUDA(cudaMemcpyAsync(ownf[1].get() + off, ds->hp.y.data(), n * 4, cudaMemcpyHostToDevice, s));
             off += n;
+            b.h2d_points += 8 * n;
         }
         stream_wait(s);
-        b.h2d_points = 8 * N;
-        b.x = ownf[0].get();
-        b.y = ownf[1].get();
     }
     if (t_upload) *t_upload = ms_since(t0);
     b.h_fstart.resize(b.F);
@@ -551,6 +567,9 @@ void setup_batch(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params* pv,
         g.row_base = row_base;
         g.f0 = job_f0[j];
         g.nf = (uint32_t)ds->names.size();
+        g.x = px[j];
+        g.y = py[j];
+        g.p0 = p0;
         key_base += g.total;
         row_base += g.gy;
         b.jobs[j].grid = g;
@@ -1617,6 +1636,9 @@ colo_status colo_create(colo_ctx** out, int device) {
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return COLO_ERR_CUDA;
     c->device_bytes = total_b;
+    int pageable = 0;
+    if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device) != cudaSuccess) cudaGetLastError();
+    c->host_reads = pageable != 0;
     // keep freed blocks in the stream-ordered pool between calls
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
