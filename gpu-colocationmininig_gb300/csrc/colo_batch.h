@@ -228,7 +228,10 @@ struct CountWork {
     // non-null: candidates c whose bounds ub[c*k + j] do not all reach need[c*k + j] are passed over
     const uint32_t* ub = nullptr;
     const uint32_t* need = nullptr;
+    // 1 << split_log warps share a chunk (count_split of nchunks; the chunk_rows are then cleared first)
+    uint32_t split_log = 0;
 };
+uint32_t count_split(const Batch& b, uint64_t nchunks);
 
 // count pass: rows per chunk + bitmaps; fill pass: rows; single pass: rows per
 // chunk + bitmaps + rows at their count-and-fill positions (overflow recorded per

@@ -1216,6 +1216,8 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
                 if (ns < ncand) {
                     CountWork w{ar.descs.get(), ar.gstart.get(), ar.gchunk.get(), ngroups, gchunks, ar.items.get(),
                                 ar.tickets.get()};
+                    w.split_log = count_split(b, gchunks);
+                    if (w.split_log) COLO_CUDA(cudaMemsetAsync(ar.chunk_rows.get() + nch_single, 0, nch_count * 4, s));
                     if (one_wait) {
                         w.ub = ar.ub.get();
                         w.need = ar.need.get();
