@@ -260,8 +260,13 @@ __global__ void __launch_bounds__(kDilThreads) k_dil_fill(uint64_t M, uint64_t p
 // candidates; a (cell Z, candidate c) pair is tested exactly as in a scan
 // of every cell with the driver in its 3x3 block: Z is in U_c when one of
 // its four quads covers c's members, each cell of U_c is met once, and a
-// full quad is counted at its first occupied cell (qfirst).  Sums go to a
-// block-private accumulator when the level's counters fit (acc_n).
+// full quad is counted at its first occupied cell (qfirst).  Lane t loads the
+// unit's candidate t up front (a candidate then comes by shuffles, not by
+// dependent loads), and a candidate's counts are summed over the warp's cells
+// before one atomic per sum, into a block-private accumulator when the level's
+// counters fit (acc_n).  One atomic per cell and sum cost a batch of 128 jobs,
+// whose counters do not fit, 1.25 ms against 0.65 ms; single mines take the same
+// time either way.
 template <int WT>
 __global__ void __launch_bounds__(256, (WT <= 4 ? 5 : (WT <= 6 ? 4 : (WT <= 8 ? 2 : 1)))) k_filter_drv(
     uint64_t nunits, uint32_t ngroups, const uint64_t* __restrict__ uoff, const uint32_t* __restrict__ gfeat,
@@ -273,6 +278,9 @@ __global__ void __launch_bounds__(256, (WT <= 4 ? 5 : (WT <= 6 ? 4 : (WT <= 8 ? 
     uint32_t acc_n, uint32_t cu) {
     constexpr uint32_t W = WT;
     constexpr bool kCacheQuads = WT <= 8;
+    // need masks by shuffle (else loaded per candidate: at 2 to 4 words the shuffles' registers
+    // spill, 0.45 against 0.43 ms on the 20M workload; at 1 and 7 words shuffles are faster)
+    constexpr bool kShuffleNeed = WT == 1 || (WT > 4 && WT <= 8);
     extern __shared__ uint32_t acc[];
     const uint32_t m = k < kMaxMembersFiltered ? k : kMaxMembersFiltered;
     const uint32_t stride = m + 2;
@@ -298,12 +306,18 @@ __global__ void __launch_bounds__(256, (WT <= 4 ? 5 : (WT <= 6 ? 4 : (WT <= 8 ? 
         const uint64_t Z = valid ? __ldg(dlist + l0 + zi) : 0u;
         const uint32_t* q4 = qmask + Z * 4 * W;
         uint32_t qr[kCacheQuads ? 4 : 1][kCacheQuads ? WT : 1];
-        // the cell's own mask and first run, issued with its quads (most list cells are
-        // in U_c of some candidate, and these loads would otherwise wait for the first)
+        // the cell's own mask, first run and first quads, issued with its quads (most list cells
+        // are in U_c of some candidate, and these loads would otherwise wait for the first)
         uint32_t cm[WT];
-        uint32_t q0 = 0;
+        uint32_t q0 = 0, qf = 0;
 #pragma unroll
         for (int w = 0; w < WT; ++w) cm[w] = 0;
+        if constexpr (kCacheQuads) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int w = 0; w < WT; ++w) qr[q][w] = 0;
+        }
         if (valid) {
             if constexpr (kCacheQuads) {
 #pragma unroll
@@ -311,53 +325,76 @@ __global__ void __launch_bounds__(256, (WT <= 4 ? 5 : (WT <= 6 ? 4 : (WT <= 8 ? 
             }
             load_row<WT>(cmask + Z * W, cm);
             q0 = crun[Z];
+            qf = qfirst[Z];
         }
-        const uint32_t t1 = gc * cu + cu < G ? gc * cu + cu : G;
-        for (uint32_t t = gc * cu; t < t1; ++t) {
-            const uint32_t c = __ldg(order + gs + t);
+        // lane t: the unit's candidate t
+        const uint32_t t0 = gc * cu, cnt = t0 + cu < G ? cu : G - t0;
+        uint32_t c_l = 0, lm_l[4] = {0, 0, 0, 0}, need_l[kShuffleNeed ? WT : 1];
+        if ((uint32_t)lane < cnt) {
+            c_l = __ldg(order + gs + t0 + lane);
+            load_row<4>(lmem + (uint64_t)c_l * 4, lm_l);
+            if constexpr (kShuffleNeed) load_row<WT>(need_all + (uint64_t)c_l * W, need_l);
+        }
+        for (uint32_t t = 0; t < cnt; ++t) {
+            const uint32_t c = __shfl_sync(0xffffffffu, c_l, t);
             uint32_t need[WT];
-            load_row<WT>(need_all + (uint64_t)c * W, need);
-            if (!valid) continue;
+            if constexpr (kShuffleNeed) {
+#pragma unroll
+                for (int w = 0; w < WT; ++w) need[w] = __shfl_sync(0xffffffffu, need_l[w], t);
+            } else {
+                load_row<WT>(need_all + (uint64_t)c * W, need);
+            }
             uint32_t full = 0;
+            if (valid) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                bool ok;
-                if constexpr (kCacheQuads) {
-                    ok = covers<WT>(qr[q], need);
-                } else {
-                    uint32_t qm[WT];
-                    load_row<WT>(q4 + q * W, qm);
-                    ok = covers<WT>(qm, need);
-                }
-                if (ok) full |= 1u << q;
-            }
-            if (!full) continue;
-            uint32_t lm[4];
-            load_row<4>(lmem + (uint64_t)c * 4, lm);
-#pragma unroll
-            for (int jj = 0; jj < kMaxMembersFiltered; ++jj) {
-                if ((uint32_t)jj >= m) break;
-                const uint32_t lf = (lm[jj >> 1] >> ((jj & 1) * 16)) & 0xFFFFu, wq = lf >> 5;
-                uint32_t rk = 0, word = 0;
-#pragma unroll
-                for (int w = 0; w < WT; ++w) {
-                    if ((uint32_t)w < wq) rk += __popc(cm[w]);
-                    if ((uint32_t)w == wq) word = cm[w];
-                }
-                if (word >> (lf & 31) & 1u) {
-                    const uint32_t ri = q0 + rk + __popc(word & ((1u << (lf & 31)) - 1u));
-                    const uint32_t v = rstart[ri + 1] - rstart[ri];
-                    if (acc_n) atomicAdd(&acc[c * stride + jj], v);
-                    else atomicAdd(&ub[(uint64_t)c * k + jj], v);
+                for (int q = 0; q < 4; ++q) {
+                    bool ok;
+                    if constexpr (kCacheQuads) {
+                        ok = covers<WT>(qr[q], need);
+                    } else {
+                        uint32_t qm[WT];
+                        load_row<WT>(q4 + q * W, qm);
+                        ok = covers<WT>(qm, need);
+                    }
+                    if (ok) full |= 1u << q;
                 }
             }
-            const uint32_t nq = __popc(full & qfirst[Z]);
-            if (acc_n) {
-                if (nq) atomicAdd(&acc[c * stride + m], nq);
-                atomicAdd(&acc[c * stride + m + 1], 1u);
-            } else if (stats) {
-                if (nq) atomicAdd(&stats[(uint64_t)c * 2], (unsigned long long)nq);
-                atomicAdd(&stats[(uint64_t)c * 2 + 1], 1ull);
+            const uint32_t cells = __ballot_sync(0xffffffffu, full != 0);
+            if (!cells) continue;
+            // the warp's sums, lane r holding sum r: members' counts, full quads, cells
+            uint32_t sum = (uint32_t)lane == m + 1 ? (uint32_t)__popc(cells) : 0u;
+#pragma unroll
+            for (int jp = 0; jp < kMaxMembersFiltered / 2; ++jp) {
+                if ((uint32_t)jp * 2 >= m) break;
+                const uint32_t lm = __shfl_sync(0xffffffffu, lm_l[jp], t);   // members 2 jp and 2 jp + 1
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t jj = jp * 2 + h;
+                    if (jj >= m) break;
+                    const uint32_t lf = (lm >> (h * 16)) & 0xFFFFu, wq = lf >> 5;
+                    uint32_t v = 0;
+                    if (full) {
+                        uint32_t rk = 0, word = 0;
+#pragma unroll
+                        for (int w = 0; w < WT; ++w) {
+                            if ((uint32_t)w < wq) rk += __popc(cm[w]);
+                            if ((uint32_t)w == wq) word = cm[w];
+                        }
+                        if (word >> (lf & 31) & 1u) {
+                            const uint32_t ri = q0 + rk + __popc(word & ((1u << (lf & 31)) - 1u));
+                            v = rstart[ri + 1] - rstart[ri];
+                        }
+                    }
+                    v = __reduce_add_sync(0xffffffffu, v);
+                    if ((uint32_t)lane == jj) sum = v;
+                }
+            }
+            const uint32_t nq = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(full & qf));
+            if ((uint32_t)lane == m) sum = nq;
+            if ((uint32_t)lane < stride && sum) {
+                if (acc_n) atomicAdd(&acc[c * stride + lane], sum);
+                else if ((uint32_t)lane < m) atomicAdd(&ub[(uint64_t)c * k + lane], sum);
+                else if (stats) atomicAdd(&stats[(uint64_t)c * 2 + (lane - m)], (unsigned long long)sum);
             }
         }
     }
