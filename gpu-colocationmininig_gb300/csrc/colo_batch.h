@@ -243,6 +243,13 @@ void level_single(Batch& b, const LevelWork& w, uint32_t k, uint32_t* d_overflow
 // (A = set bits in [0, n-2]), added into d_stats, which must be zero.
 void level_pi(Batch& b, const CandDesc* d_cands, uint64_t ncand, uint32_t k, uint64_t* d_stats);
 
+// Rows row0 .. row0 + rows of a column-major table, row-major at word `at` of `out`.
+struct TablePiece {
+    const uint32_t* cols;
+    uint64_t stride, row0, rows, at;
+};
+void table_rows(cudaStream_t s, const TablePiece* d_pieces, uint32_t n, uint32_t k, uint64_t most_words, uint32_t* out);
+
 // Squared-distance evaluation of the reference expression for n pairs; with
 // `within`, also the kernels' decision ref_within(...) for threshold R2.
 void eval_sqdist(const float* x1, const float* y1, const float* x2, const float* y2, uint64_t n,

@@ -101,6 +101,8 @@ struct colo_ctx {
     void* ustage = nullptr;     // page-locked staging for the level loop's uploads
     size_t ustage_bytes = 0;
     size_t ustage_off = 0;      // bytes in use since the stream last drained
+    void* tstage = nullptr;     // page-locked staging for the tables kept in results (at most 64 MiB)
+    size_t tstage_bytes = 0;
     uint64_t pool_peak = 0;     // most device-pool memory in use by one earlier mine (bytes)
 };
 

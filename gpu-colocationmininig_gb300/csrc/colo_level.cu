@@ -547,6 +547,18 @@ __global__ void __launch_bounds__(256, (MODE == MODE_FILL && K == 2) ? 6 : (MODE
     }   // chunks of this warp
 }
 
+// Kept tables, row-major: one y block row per piece.  Bound by the copy that follows over the host
+// link; turning the columns into rows on the host, table by table, took 20 us a table.
+__global__ void __launch_bounds__(256) k_table_rows(const TablePiece* __restrict__ pieces, uint32_t k,
+                                                    uint32_t* __restrict__ out) {
+    const TablePiece p = pieces[blockIdx.y];
+    const uint64_t words = p.rows * k;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t row = i / k;
+        out[p.at + i] = p.cols[(i - row * k) * p.stride + p.row0 + row];
+    }
+}
+
 // Participation statistics: per (candidate, member) [A, last, first, full]
 // where A counts set bits in [0, n-2] (the window getParticipationIndex sums,
 // Codes/DeviceProcess.cu:108-132).  A block takes one (candidate, member)
@@ -684,6 +696,15 @@ void level_count(Batch& b, const CountWork& w, uint32_t k) {
 void level_fill(Batch& b, const LevelWork& w, uint32_t k) { launch_level<MODE_FILL>(b, w, k, nullptr); }
 void level_single(Batch& b, const LevelWork& w, uint32_t k, uint32_t* d_overflow) {
     launch_level<MODE_SINGLE>(b, w, k, d_overflow);
+}
+
+void table_rows(cudaStream_t s, const TablePiece* d_pieces, uint32_t n, uint32_t k, uint64_t most_words, uint32_t* out) {
+    if (n == 0 || most_words == 0) return;
+    KScope ks("table_rows");
+    const unsigned gx = (unsigned)std::min<uint64_t>((most_words + 255) / 256, 1024);
+    k_table_rows<<<dim3(gx, n), 256, 0, s>>>(d_pieces, k, out);
+    COLO_LAUNCH_CHECK();
+    count_launch();
 }
 
 void level_pi(Batch& b, const CandDesc* d_cands, uint64_t ncand, uint32_t k, uint64_t* d_stats) {

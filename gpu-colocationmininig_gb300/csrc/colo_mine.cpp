@@ -108,6 +108,7 @@ void ctx_release(colo_ctx* ctx) {
     if (ctx->ev_counted) cudaEventDestroy(ctx->ev_counted);
     if (ctx->stage) cudaFreeHost(ctx->stage);
     if (ctx->ustage) cudaFreeHost(ctx->ustage);
+    if (ctx->tstage) cudaFreeHost(ctx->tstage);
     delete ctx;
 }
 
@@ -467,6 +468,82 @@ uint64_t presize_rows(float pred) {
 
 }  // namespace
 
+namespace {
+
+// Instance tables kept in results: turned into rows on the device and copied through page-locked
+// staging behind the level's fill, without a wait of their own; finish() (after a wait, or once the
+// staging is full) moves them to their vectors, whose storage does not move with the level's trace.
+// The staging grows to kTableStage bytes at most.
+constexpr size_t kTableStage = (size_t)64 << 20;
+
+struct TableReads {
+    colo_ctx* ctx;
+    cudaStream_t s;
+    struct Item {
+        uint32_t* dst;
+        size_t off, bytes;
+    };
+    std::vector<Item> items;
+    size_t used = 0;
+
+    void finish() {
+        for (const Item& it : items) std::memcpy(it.dst, static_cast<char*>(ctx->tstage) + it.off, it.bytes);
+        items.clear();
+        used = 0;
+    }
+    // room for `bytes` more; what is pending is finished first when there is none
+    void room(size_t bytes) {
+        if (used + bytes <= ctx->tstage_bytes) return;
+        stream_wait(s);
+        finish();
+        if (bytes <= ctx->tstage_bytes) return;
+        if (ctx->tstage) cudaFreeHost(ctx->tstage);
+        ctx->tstage = nullptr;
+        ctx->tstage_bytes = 0;
+        const size_t nb = std::min(kTableStage, std::max<size_t>(bytes * 2, (size_t)1 << 20));
+        COLO_CUDA(cudaHostAlloc(&ctx->tstage, nb, cudaHostAllocDefault));
+        ctx->tstage_bytes = nb;
+    }
+    // the level's tables (cols, rows, stride) to dst[i], sized rows * k
+    void read(const std::vector<TableRef>& tables, const std::vector<uint32_t*>& dst, uint32_t k) {
+        const uint64_t most = kTableStage / (4 * (uint64_t)k);   // rows of one batch
+        std::vector<TablePiece> pieces;
+        std::vector<uint32_t*> to;
+        uint64_t rows = 0, longest = 0;
+        auto flush = [&]() {
+            if (pieces.empty()) return;
+            const size_t bytes = (size_t)rows * k * 4;
+            room(bytes);
+            DevBuf<uint32_t> out;
+            DevBuf<TablePiece> dp;
+            out.alloc(rows * k, s);
+            dp.alloc(pieces.size(), s);
+            staged_upload(ctx, s, dp.get(), pieces.data(), pieces.size() * sizeof(TablePiece));
+            table_rows(s, dp.get(), (uint32_t)pieces.size(), k, longest * k, out.get());
+            COLO_CUDA(cudaMemcpyAsync(static_cast<char*>(ctx->tstage) + used, out.get(), bytes, cudaMemcpyDeviceToHost, s));
+            for (size_t i = 0; i < pieces.size(); ++i)
+                items.push_back({to[i], used + (size_t)pieces[i].at * 4, (size_t)pieces[i].rows * k * 4});
+            used += bytes;
+            pieces.clear();
+            to.clear();
+            rows = longest = 0;
+        };
+        for (size_t i = 0; i < tables.size(); ++i)
+            for (uint64_t r = 0; r < tables[i].rows;) {
+                const uint64_t n = std::min(tables[i].rows - r, most - rows);
+                pieces.push_back({tables[i].cols, tables[i].stride, r, n, rows * k});
+                to.push_back(dst[i] + r * k);
+                longest = std::max(longest, n);
+                rows += n;
+                r += n;
+                if (rows == most || pieces.size() == 65535) flush();
+            }
+        flush();
+    }
+};
+
+}  // namespace
+
 void staged_upload(colo_ctx* ctx, cudaStream_t s, void* dst, const void* src, size_t bytes) {
     if (!bytes) return;
     unsigned char* h = upload_area(ctx, s, bytes);
@@ -783,6 +860,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
     for (uint32_t j = 0; j < J; ++j) host_tables |= (pv[j].reserved[0] & 8) != 0;
     uint64_t cnt_host_table_bytes = 0;
     std::vector<uint32_t> h_least;   // per feature, least_bound (once asked for)
+    TableReads table_reads{ctx, s};
     for (uint32_t k = 2;; ++k) {
         bool any = false;
         for (auto& st : js) any |= (st.active && !st.cands.empty());
@@ -1503,11 +1581,6 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
             if (!needed[owner[q].first][owner[q].second]) continue;
             tr[owner[q].first]->has_table[owner[q].second] = 1;
         }
-        // the tables are read back only when kept in the result (a copy on another stream); else
-        // the next level's launches queue behind the fill on this stream without a wait
-        bool keep_any = false;
-        for (uint32_t j = 0; j < J; ++j) keep_any |= pv[j].keep_tables != 0;
-        if (keep_any) stream_wait(s);
         // register the new tables (prefixes of the next level)
         for (uint32_t j = 0; j < J; ++j) {
             js[j].prev_tables.clear();
@@ -1522,6 +1595,8 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
             made.push_back({q, TableRef{hd[q].out, gb[q + 1] - gb[q], cap[q]}});
             tr[owner[q].first]->has_table[owner[q].second] = 1;
         }
+        std::vector<TableRef> kept;
+        std::vector<uint32_t*> kept_to;
         for (const auto& mt : made) {
             const uint64_t q = mt.first;
             const TableRef& t = mt.second;
@@ -1529,18 +1604,13 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
             size_t c = owner[q].second;
             js[owner[q].first].prev_tables[c] = t;
             if (pv[owner[q].first].keep_tables) {
-                uint64_t rows = t.rows;
-                std::vector<uint32_t> colm(rows * k);
-                if (rows)
-                    COLO_CUDA(cudaMemcpy2D(colm.data(), rows * 4, t.cols, t.stride * 4, rows * 4, k,
-                                           cudaMemcpyDefault));   // the tables may be in host memory
                 if (L.tables.size() < L.cand.size() / k) L.tables.resize(L.cand.size() / k);
-                std::vector<uint32_t>& rm = L.tables[c];
-                rm.resize(rows * k);
-                for (uint64_t r = 0; r < rows; ++r)
-                    for (uint32_t t = 0; t < k; ++t) rm[r * k + t] = colm[(uint64_t)t * rows + r];
+                L.tables[c].resize(t.rows * k);
+                kept.push_back(t);
+                kept_to.push_back(L.tables[c].data());
             }
         }
+        table_reads.read(kept, kept_to, k);   // (the next level's launches queue behind it without a wait)
         t_fill += ms_since(t0);
         kt.mark("fill launches");
         tables_prev = std::move(tables_cur);
@@ -1549,6 +1619,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
             if (st.cands.empty()) st.active = false;
     }
     stream_wait(s);
+    table_reads.finish();
     kt.resolve();
     for (uint32_t j = 0; j < J; ++j) {
         MineResult* r = outs[j];
