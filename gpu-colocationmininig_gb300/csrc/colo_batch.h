@@ -84,9 +84,10 @@ struct Batch {
     DevBuf<unsigned char> mem_points, mem_heads, mem_cells, mem_lists, mem_act, mem_nb;
     Span<float2> xy;             // coordinates by id, packed (built by the cell-key pass)
     // bucketed (sorted by cell key, then id)
-    Span<uint32_t> sid, sfeat, scell;     // scell (cell of each sorted point) only when keep_scell
+    Span<uint32_t> sid, sfeat, scell;     // sfeat for several jobs, scell (cell of each sorted point) only when keep_scell
+    Span<float2> sxy;                     // coordinates in cell-sorted order, where gathered
+    bool gathered = false;                // lists and anchors name points by sorted position, else by id
     bool keep_scell = false;              // colo_stage_cells reports each point's cell
-    Span<float2> sxy;            // coordinates in cell-sorted order
     // cells
     Span<uint64_t> ckey;
     Span<uint32_t> cstart, crun, cjob;    // cstart, crun with an end entry
@@ -110,8 +111,8 @@ struct Batch {
     Span<uint8_t> qfirst;        // per cell: bit q set when it is the first occupied cell of its quad q
     // runs: run r's points are sorted positions rstart[r] .. rstart[r+1] (rstart has an end entry)
     Span<uint32_t> rfeat, rstart, rcell;
-    // neighbourhood lists: for each cell with targets, the points (sorted positions) of its
-    // adjacent cells' runs above the cell's lowest own feature, ordered by (feature, cell, id);
+    // neighbourhood lists: for each cell with targets, the points of its adjacent
+    // cells' runs above the cell's lowest own feature, ordered by (feature, cell, id);
     // the lists are in no particular order
     Span<uint32_t> targets;
     uint64_t targets_cap = 0, nrl_total = 0;   // nrl_total: runs in the lists
@@ -119,8 +120,8 @@ struct Batch {
     // feature (absolute index), and the targets from there to the list's end
     Span<uint64_t> run_sfx;
     Span<uint32_t> run_L;
-    // the join's anchors (points of runs with targets), in no particular order: sorted
-    // position, number of targets, first target (low, high word); anchors of at most
+    // the join's anchors (points of runs with targets), in no particular order: point, number
+    // of targets, first target (low, high word); anchors of at most
     // kLongList targets from the front, the others from the back
     Span<uint4> act;
     // neighbour lists N+(a) = nb[nb_beg[a] .. nb_beg[a] + nb_cnt[a]), each in

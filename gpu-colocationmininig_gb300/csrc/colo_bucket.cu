@@ -99,30 +99,34 @@ __global__ void __launch_bounds__(256, 4) k_cell_keys(
     }
 }
 
-// Sorted copies, cells and runs in one pass over the sorted keys.  A block
-// takes a 2048-point tile (eight warp segments of 256 points, 32 consecutive
-// points at a time): per point its coordinates (one 8-byte gather) and its
-// feature (from the feature start table, points being grouped by feature; it
-// stays in L1); a cell starts where the key changes, a run where the key or
-// the feature does (a point's predecessor comes from the lane before it, lane 0
-// reads it).  The tile's head counts go through a decoupled look-back (warp 0
+// Cells and runs in one pass over the sorted keys.  A block takes a 2048-point
+// tile (eight warp segments of 256 points, 32 consecutive points at a time): per
+// point its feature (from the feature start table, points being grouped by
+// feature; it stays in L1); a cell starts where the key changes, a run where the
+// key or the feature does (a point's predecessor comes from the lane before it,
+// lane 0 reads it).  The tile's head counts go through a decoupled look-back (warp 0
 // for cells, warp 1 for runs), and the heads are written at the offsets found,
 // as far as the arrays reach (capM, capR: a launch with no room counts them).
 // The last tile records the totals and the end entries.
 //
-// Bound by the gather (an 8-byte load by a sorted id moves a whole DRAM
-// sector).  One kernel instead of four (gather and count, scan of the tile
-// counts, compaction, run lengths): the tile's keys and features are read once,
-// and no host wait is needed for the totals (20M points: 0.50 ms against 0.32 + 0.21; a few
-// thousand points: 14 us against 64 us with the wait).
+// GATHER also writes the points' coordinates in cell order (and, for several jobs,
+// their features), which makes the lists' and the join's reads of them nearly
+// sequential.  The 8-byte reads by id move a DRAM sector each once the
+// coordinates outgrow L2, for every point, and the join looks at a tenth of them:
+// from kGatherPoints on they stay in id order and the lists hold ids (20M points:
+// this kernel 495 -> 299 us, a mine 3.99 -> 3.83 ms; 1M to 4M: within 1% either
+// way; 128 jobs of 30,000: 2% slower ungathered, so several jobs always gather).
+//
+// Bound by the gather, else by the features' searches and the look-back.
 //
 // After a sort that timed out the keys are not a sorted permutation: nothing
 // is written, the totals stay zero and every later kernel finds no cells.  A
 // look-back that waits too long counts the heads before its tile itself.
+constexpr uint64_t kGatherPoints = 1ull << 23;   // 64 MiB of coordinates, half of L2
 constexpr int kHeadThreads = 256, kHeadRounds = 8, kHeadTile = kHeadThreads * kHeadRounds;
 constexpr int kHeadWarps = kHeadThreads / 32;
 
-template <class KT>
+template <class KT, bool GATHER>
 __global__ void __launch_bounds__(kHeadThreads, 6) k_heads(
     uint64_t n, uint32_t F, const KT* __restrict__ keys, const uint32_t* __restrict__ sid,
     const float2* __restrict__ xy, const uint32_t* __restrict__ fstart, const uint32_t* __restrict__ fjob,
@@ -150,9 +154,9 @@ __global__ void __launch_bounds__(kHeadThreads, 6) k_heads(
         f[r] = 0;
         if (in) {
             const uint32_t id = sid[p];
-            sxy[p] = xy[id];
+            if (GATHER) sxy[p] = xy[id];
             f[r] = feature_of(id, F, fstart);
-            sfeat[p] = f[r];
+            if (GATHER && sfeat) sfeat[p] = f[r];   // null for one-job batches
             key[r] = keys[p];
         }
         KT pkey = __shfl_up_sync(0xffffffffu, key[r], 1);
@@ -594,16 +598,21 @@ __device__ __forceinline__ int adjacent_cells(uint64_t c, const uint64_t* ckey, 
 constexpr uint32_t kBigRuns = 128, kBigPoints = 512;   // cells with longer lists are merged by their whole warp
 constexpr uint32_t kHeavyAnchors = 32;   // cells with more anchors are listed by their whole warp
 
-// Sorted positions st .. st + rc - 1 to dst for every lane; runs of more than 32
-// points by the whole warp.
-__device__ __forceinline__ void put_run(uint32_t* __restrict__ targets, uint64_t at, uint32_t st, uint32_t rc, int lane) {
+// The point at sorted position p as lists and anchors name it: by that position
+// where the coordinates were gathered (ids is null), else by its id.
+__device__ __forceinline__ uint32_t list_point(const uint32_t* __restrict__ ids, uint32_t p) { return ids ? ids[p] : p; }
+
+// The points at sorted positions st .. st + rc - 1 for every lane; runs of more
+// than 32 points by the whole warp.
+__device__ __forceinline__ void put_run(uint32_t* __restrict__ targets, uint64_t at, const uint32_t* __restrict__ ids,
+                                        uint32_t st, uint32_t rc, int lane) {
     if (rc <= 32)
-        for (uint32_t q = 0; q < rc; ++q) targets[at + q] = st + q;
+        for (uint32_t q = 0; q < rc; ++q) targets[at + q] = list_point(ids, st + q);
     for (uint32_t m = __ballot_sync(0xffffffffu, rc > 32); m; m &= m - 1) {
         const int j = __ffs(m) - 1;
         const uint64_t aj = __shfl_sync(0xffffffffu, at, j);
         const uint32_t sj = __shfl_sync(0xffffffffu, st, j), nj = __shfl_sync(0xffffffffu, rc, j);
-        for (uint32_t q = lane; q < nj; q += 32) targets[aj + q] = sj + q;
+        for (uint32_t q = lane; q < nj; q += 32) targets[aj + q] = list_point(ids, sj + q);
     }
 }
 
@@ -619,7 +628,8 @@ __device__ __forceinline__ void list_cell_warp(uint64_t c, int lane, uint64_t fi
                                                const uint32_t* __restrict__ cjob, const JobGrid* __restrict__ grids,
                                                const int32_t* __restrict__ nb9, const uint32_t* __restrict__ crun,
                                                const uint32_t* __restrict__ rfeat, const uint32_t* __restrict__ rstart,
-                                               uint32_t* __restrict__ targets, uint64_t* run_sfx, uint32_t* run_L) {
+                                               const uint32_t* __restrict__ ids, uint32_t* __restrict__ targets,
+                                               uint64_t* run_sfx, uint32_t* run_L) {
     int32_t adj[9];
     const int na = adjacent_cells(c, ckey, cjob, grids, nb9, adj);
     const uint32_t fmin = rfeat[crun[c]];
@@ -661,7 +671,7 @@ __device__ __forceinline__ void list_cell_warp(uint64_t c, int lane, uint64_t fi
             st = rstart[r];
             rc = rstart[r + 1] - st;
         }
-        put_run(targets, at, st, rc, lane);
+        put_run(targets, at, ids, st, rc, lane);
     }
     for (uint32_t r = crun[c] + lane; r < crun[c + 1]; r += 32) {
         const uint32_t f = rfeat[r];
@@ -701,8 +711,8 @@ __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
     uint64_t npoints, const uint32_t* __restrict__ listq, BatchCtrl* __restrict__ ctrl,
     const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob, const JobGrid* __restrict__ grids,
     const int32_t* __restrict__ nb9, const uint32_t* __restrict__ crun, const uint32_t* __restrict__ rfeat,
-    const uint32_t* __restrict__ rstart, uint64_t cap, uint32_t* __restrict__ targets, uint64_t* run_sfx,
-    uint32_t* run_L, uint4* __restrict__ act) {
+    const uint32_t* __restrict__ rstart, const uint32_t* __restrict__ ids, uint64_t cap,
+    uint32_t* __restrict__ targets, uint64_t* run_sfx, uint32_t* run_L, uint4* __restrict__ act) {
     const uint32_t n = (uint32_t)ctrl->nlistq.v;
     const int lane = threadIdx.x & 31;
     const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5), w = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -787,7 +797,7 @@ __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
                         f[t] = h[t] < e[t] ? rfeat[h[t]] : 0xffffffffu;
                     }
                 const uint32_t st = rstart[r], rc = rstart[r + 1] - st;
-                for (uint32_t q = 0; q < rc; ++q) targets[first + P + q] = st + q;
+                for (uint32_t q = 0; q < rc; ++q) targets[first + P + q] = list_point(ids, st + q);
                 P += rc;
                 if (ts == own) {
                     pend = true;
@@ -800,7 +810,7 @@ __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
             const int j = __ffs(m) - 1;
             const uint32_t cj = __shfl_sync(0xffffffffu, c, j);
             const uint64_t fj = __shfl_sync(0xffffffffu, first, j);
-            list_cell_warp(cj, lane, fj, ckey, cjob, grids, nb9, crun, rfeat, rstart, targets, run_sfx, run_L);
+            list_cell_warp(cj, lane, fj, ckey, cjob, grids, nb9, crun, rfeat, rstart, ids, targets, run_sfx, run_L);
         }
         __syncwarp();
         // anchors: the points of own runs with targets, short lists and long ones
@@ -834,7 +844,7 @@ __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
                 const uint32_t st = rstart[r], rc = rstart[r + 1] - st;
                 const uint64_t sfx = run_sfx[r];
                 for (uint32_t q = 0; q < rc; ++q)
-                    act[L <= kLongList ? so++ : lo--] = make_uint4(st + q, L, (uint32_t)sfx, (uint32_t)(sfx >> 32));
+                    act[L <= kLongList ? so++ : lo--] = make_uint4(list_point(ids, st + q), L, (uint32_t)sfx, (uint32_t)(sfx >> 32));
             }
         for (uint32_t m = __ballot_sync(0xffffffffu, heavy); m; m &= m - 1) {   // the loop above is serial in the points
             const int j = __ffs(m) - 1;
@@ -847,7 +857,7 @@ __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
                 const uint64_t sfx = run_sfx[r];
                 const bool is_long = L > kLongList;
                 for (uint32_t q = lane; q < rc; q += 32)
-                    act[is_long ? lj - q : sj + q] = make_uint4(st + q, L, (uint32_t)sfx, (uint32_t)(sfx >> 32));
+                    act[is_long ? lj - q : sj + q] = make_uint4(list_point(ids, st + q), L, (uint32_t)sfx, (uint32_t)(sfx >> 32));
                 if (is_long) lj -= rc;
                 else sj += rc;
             }
@@ -879,8 +889,6 @@ namespace {
 
 void lay_points(Batch& b, Carver& c) {
     c.add(b.xy, b.N);
-    c.add(b.sxy, b.N);
-    c.add(b.sfeat, b.N);
     c.add(b.sid, b.N);
     c.add(b.nb_beg, b.N);
     c.add(b.nb_cnt, b.N);
@@ -893,6 +901,8 @@ void lay_heads(Batch& b, Carver& c, uint64_t M, uint64_t R) {
     c.add(b.rfeat, R);
     c.add(b.rstart, R + 1);
     c.add(b.rcell, R);
+    if (b.gathered) c.add(b.sxy, b.N);
+    if (b.gathered && b.J > 1) c.add(b.sfeat, b.N);
     if (b.keep_scell) c.add(b.scell, b.N);
 }
 void lay_cells(Batch& b, Carver& c, uint64_t M, uint64_t R) {
@@ -917,8 +927,9 @@ bool wants_row_table(const Batch& b, uint64_t cells) {
 template <class KT>
 void launch_heads(Batch& b, const KT* keys, uint64_t capM, uint64_t capR) {
     const uint64_t tiles = (b.N + kHeadTile - 1) / kHeadTile;
-    KScope ks("gather_sorted");
-    k_heads<KT><<<(unsigned)tiles, kHeadThreads, 0, b.s>>>(
+    KScope ks("cell_heads");
+    auto* const kernel = b.gathered ? k_heads<KT, true> : k_heads<KT, false>;
+    kernel<<<(unsigned)tiles, kHeadThreads, 0, b.s>>>(
         b.N, b.F, keys, b.sid.get(), b.xy.get(), b.fstart.get(), b.fjob.get(), b.sxy.get(), b.sfeat.get(),
         b.ckey.get(), b.cstart.get(), b.crun.get(), b.cjob.get(), b.rfeat.get(), b.rstart.get(), b.rcell.get(),
         capM ? b.scell.get() : nullptr, capM, capR, b.head_status.get(), b.tickets.get() + b.plan.n, b.ctrl.get());
@@ -1014,6 +1025,7 @@ void bucket_points(Batch& b) {
     b.targets_cap = list_room(n);
     b.nb_cap = neighbour_room(n);
     b.row_table = wants_row_table(b, n);
+    b.gathered = b.J > 1 || n <= kGatherPoints;
     auto bounds = [&](Carver& c) {
         lay_points(b, c);
         lay_heads(b, c, n, n);
@@ -1111,7 +1123,7 @@ void build_neighborhoods(Batch& b) {
     KScope ks("neighbour_lists");
     k_neighbour_lists<<<qgrid, 128, 0, s>>>(b.N, b.listq.get(), b.ctrl.get(), b.ckey.get(), b.cjob.get(),
                                             b.grids.get(), b.nb9.get(), b.crun.get(), b.rfeat.get(), b.rstart.get(),
-                                            b.targets_cap, b.targets.get(), b.run_sfx.get(), b.run_L.get(),
+                                            b.gathered ? nullptr : b.sid.get(), b.targets_cap, b.targets.get(), b.run_sfx.get(), b.run_L.get(),
                                             b.act.get());
     COLO_LAUNCH_CHECK();
     count_launch();

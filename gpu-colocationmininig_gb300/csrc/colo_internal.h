@@ -6,7 +6,8 @@
 //               packed coordinates by id
 //   features    fstart[F], fcount[F], fjob[F]
 //   jobs        JobGrid[J] (the reference grid of each job, R^2, threshold)
-//   bucketed    points sorted by (job cell key, point id): sid/sxy/sfeat/scell
+//   bucketed    points sorted by (job cell key, point id): sid, and
+//               with gathered coordinates sxy (sfeat for several jobs)
 //   cells       occupied cells ckey[M], cstart[M+1] (sorted positions),
 //               crun[M+1] (run ranges), nb9[M*9] (geometric 3x3 neighbours),
 //               cmask[M*W] (feature bit masks, local feature index),
@@ -15,7 +16,8 @@
 //               runs per feature on the host (h_frun_off prefix)
 //   lists       per cell with targets, the points of its adjacent cells' runs with
 //               a feature above the cell's lowest own feature, ordered by
-//               (feature, cell, id): targets (sorted positions)
+//               (feature, cell, id): targets (sorted positions, or
+//               ids where the coordinates were not gathered)
 //   anchors     act[]: the points of runs with targets, with their slices of the
 //               lists
 //   neighbours  N+(a) = nb[nb_beg[a] .. nb_beg[a] + nb_cnt[a]) by point id

@@ -42,8 +42,8 @@ constexpr uint64_t kJoinWaves = 8;   // waves of resident blocks at most (warps 
 template <int MODE>
 __global__ void __launch_bounds__(256, 6) k_join(
     BatchCtrl* __restrict__ ctrl, uint64_t npoints, uint64_t targets_cap, uint64_t nb_cap, int per,
-    const uint4* __restrict__ act, const uint32_t* __restrict__ sid, const uint32_t* __restrict__ sfeat,
-    const float2* __restrict__ sxy, const uint32_t* __restrict__ targets, const uint32_t* __restrict__ fjob,
+    const uint4* __restrict__ act, const uint32_t* __restrict__ ids, const uint32_t* __restrict__ sfeat,
+    const float2* __restrict__ coords, const uint32_t* __restrict__ targets, const uint32_t* __restrict__ fjob,
     const JobGrid* __restrict__ grids, uint64_t* __restrict__ nb_beg, uint32_t* __restrict__ nb_cnt,
     uint32_t* __restrict__ nb, unsigned long long* __restrict__ total) {
     if (ctrl->targets.v > targets_cap || (MODE == J_SINGLE && ctrl->pairs.v > nb_cap)) return;
@@ -58,8 +58,8 @@ __global__ void __launch_bounds__(256, 6) k_join(
     for (uint64_t i = warp; i < AL + tiles; i += warps) {
         if (i < AL) {
             const uint4 an = act[npoints - 1 - i];
-            const uint32_t a = sid[an.x], L = an.y;
-            const float2 pa = sxy[an.x];
+            const uint32_t a = ids ? ids[an.x] : an.x, L = an.y;
+            const float2 pa = coords[an.x];
             const JobGrid& g = grids[fjob ? fjob[sfeat[an.x]] : 0u];   // fjob is null for one-job batches
             const float R2 = g.R2, hu = g.R2hu;
             const uint32_t* list = targets + ((uint64_t)an.w << 32 | an.z);
@@ -74,12 +74,12 @@ __global__ void __launch_bounds__(256, 6) k_join(
 #pragma unroll
                 for (int i = 0; i < kLongSteps; ++i) p[i] = t0 + i * 32 + lane < L ? list[t0 + i * 32 + lane] : 0xffffffffu;
 #pragma unroll
-                for (int i = 0; i < kLongSteps; ++i) pb[i] = p[i] != 0xffffffffu ? sxy[p[i]] : make_float2(0.f, 0.f);
+                for (int i = 0; i < kLongSteps; ++i) pb[i] = p[i] != 0xffffffffu ? coords[p[i]] : make_float2(0.f, 0.f);
 #pragma unroll
                 for (int i = 0; i < kLongSteps; ++i) {
                     const bool ok = p[i] != 0xffffffffu && ref_within(pa.x, pa.y, pb[i].x, pb[i].y, R2, hu);
                     const uint32_t bal = __ballot_sync(0xffffffffu, ok);
-                    if (MODE != J_COUNT && ok) nb[base + k + __popc(bal & lt)] = sid[p[i]];
+                    if (MODE != J_COUNT && ok) nb[base + k + __popc(bal & lt)] = ids ? ids[p[i]] : p[i];
                     k += __popc(bal);
                 }
             }
@@ -99,8 +99,8 @@ __global__ void __launch_bounds__(256, 6) k_join(
             const uint4 an = act[at];
             L = an.y;
             from = (uint64_t)an.w << 32 | an.z;
-            a = sid[an.x];
-            const float2 pa = sxy[an.x];
+            a = ids ? ids[an.x] : an.x;
+            const float2 pa = coords[an.x];
             xa = pa.x;
             ya = pa.y;
             const JobGrid& g = grids[fjob ? fjob[sfeat[an.x]] : 0u];
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(256, 6) k_join(
             uint32_t p = 0;
             if (t < tot) {
                 p = targets[from_j + t];
-                const float2 pb = sxy[p];
+                const float2 pb = coords[p];
                 ok = ref_within(xj, yj, pb.x, pb.y, R2j, huj);
             }
             const uint32_t bal = __ballot_sync(0xffffffffu, ok);
@@ -145,9 +145,9 @@ __global__ void __launch_bounds__(256, 6) k_join(
                 const uint64_t beg_j = __shfl_sync(0xffffffffu, beg, j);
                 const uint32_t mine_j = __shfl_sync(0xffffffffu, mine, j);
                 const uint32_t own_j = __shfl_sync(0xffffffffu, m1 & ~m0, j);
-                if (ok) nb[beg_j + mine_j + __popc(bal & own_j & lt)] = sid[p];
+                if (ok) nb[beg_j + mine_j + __popc(bal & own_j & lt)] = ids ? ids[p] : p;
             }
-            if (MODE == J_SINGLE && ok) nb[base + hits + __popc(bal & lt)] = sid[p];
+            if (MODE == J_SINGLE && ok) nb[base + hits + __popc(bal & lt)] = ids ? ids[p] : p;
             before += __popc(bal & m0);
             mine += __popc(bal & m1 & ~m0);
             hits += __popc(bal);
@@ -170,8 +170,9 @@ void run_join(Batch& b, int mode, uint64_t anchors, uint64_t longs) {
     if (grid == 0) return;
     KScope ks(mode == J_SINGLE ? "join" : mode == J_COUNT ? "join_count" : "join_fill");
 #define COLO_JOIN(MD)                                                                                            \
-    k_join<MD><<<grid, 256, 0, b.s>>>(b.ctrl.get(), b.N, b.targets_cap, b.nb_cap, per, b.act.get(), b.sid.get(), \
-                                      b.sfeat.get(), b.sxy.get(), b.targets.get(),                              \
+    k_join<MD><<<grid, 256, 0, b.s>>>(b.ctrl.get(), b.N, b.targets_cap, b.nb_cap, per, b.act.get(),              \
+                                      b.gathered ? b.sid.get() : nullptr, b.sfeat.get(),                        \
+                                      b.gathered ? b.sxy.get() : b.xy.get(), b.targets.get(),                   \
                                       b.J > 1 ? b.fjob.get() : nullptr, b.grids.get(), b.nb_beg.get(),          \
                                       b.nb_cnt.get(), b.nb.get(), b.dE.get())
     if (mode == J_SINGLE) COLO_JOIN(J_SINGLE);
