@@ -104,9 +104,13 @@ __global__ void __launch_bounds__(256, 4) k_cell_keys(
 // point its feature (from the feature start table, points being grouped by
 // feature; it stays in L1); a cell starts where the key changes, a run where the
 // key or the feature does (a point's predecessor comes from the lane before it,
-// lane 0 reads it).  The tile's head counts go through a decoupled look-back (warp 0
-// for cells, warp 1 for runs), and the heads are written at the offsets found,
-// as far as the arrays reach (capM, capR: a launch with no room counts them).
+// lane 0's from the last lane of the round before).  The features of four rounds
+// are searched side by side, which hides most of the chain of dependent loads
+// (20M points, nothing gathered: 297 -> 200 us; one search at a time without lane
+// 0's second search 273, eight at a time 198, the starts in shared memory 207).
+// The tile's head counts go through a decoupled look-back (warp 0 for cells, warp
+// 1 for runs), and the heads are written at the offsets found, as far as the
+// arrays reach (capM, capR: a launch with no room counts them).
 // The last tile records the totals and the end entries.
 //
 // GATHER also writes the points' coordinates in cell order (and, for several jobs,
@@ -114,10 +118,10 @@ __global__ void __launch_bounds__(256, 4) k_cell_keys(
 // sequential.  The 8-byte reads by id move a DRAM sector each once the
 // coordinates outgrow L2, for every point, and the join looks at a tenth of them:
 // from kGatherPoints on they stay in id order and the lists hold ids (20M points:
-// this kernel 495 -> 299 us, a mine 3.99 -> 3.83 ms; 1M to 4M: within 1% either
+// this kernel 495 -> 298 us, a mine 3.99 -> 3.83 ms; 1M to 4M: within 1% either
 // way; 128 jobs of 30,000: 2% slower ungathered, so several jobs always gather).
 //
-// Bound by the gather, else by the features' searches and the look-back.
+// Bound by the gather, else by instruction issue and the wait for the look-back.
 //
 // After a sort that timed out the keys are not a sorted permutation: nothing
 // is written, the totals stay zero and every later kernel finds no cells.  A
@@ -146,22 +150,53 @@ __global__ void __launch_bounds__(kHeadThreads, 6) k_heads(
     KT key[kHeadRounds];
     uint32_t f[kHeadRounds], chm = 0, rhm = 0;   // the lane's own head bits, one a round
     uint32_t cc = 0, rc = 0;
+    uint32_t top = 1;
+    while (top < F && top < 1u << 31) top <<= 1;
+#pragma unroll
+    for (int r0 = 0; r0 < kHeadRounds; r0 += 4) {   // four searches at a time
+        uint32_t id[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint64_t p = seg + (uint64_t)(r0 + i) * 32 + lane;
+            id[i] = p < n ? sid[p] : 0u;
+            key[r0 + i] = p < n ? keys[p] : KT(0);
+            f[r0 + i] = 0;
+        }
+        if (GATHER) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint64_t p = seg + (uint64_t)(r0 + i) * 32 + lane;
+                if (p < n) sxy[p] = xy[id[i]];
+            }
+        }
+        for (uint32_t step = top >> 1; step > 0; step >>= 1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t mid = f[r0 + i] + step;
+                if (mid < F && fstart[mid] <= id[i]) f[r0 + i] = mid;
+            }
+        if (GATHER && sfeat) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint64_t p = seg + (uint64_t)(r0 + i) * 32 + lane;
+                if (p < n) sfeat[p] = f[r0 + i];
+            }
+        }
+    }
 #pragma unroll
     for (int r = 0; r < kHeadRounds; ++r) {
         const uint64_t p = seg + (uint64_t)r * 32 + lane;
         const bool in = p < n;
-        key[r] = 0;
-        f[r] = 0;
-        if (in) {
-            const uint32_t id = sid[p];
-            if (GATHER) sxy[p] = xy[id];
-            f[r] = feature_of(id, F, fstart);
-            if (GATHER && sfeat) sfeat[p] = f[r];   // null for one-job batches
-            key[r] = keys[p];
-        }
         KT pkey = __shfl_up_sync(0xffffffffu, key[r], 1);
         uint32_t pf = __shfl_up_sync(0xffffffffu, f[r], 1);
-        if (lane == 0 && in && p > 0) {
+        if (r > 0) {   // lane 0's predecessor: the last lane's point of the round before
+            const KT k31 = __shfl_sync(0xffffffffu, key[r > 0 ? r - 1 : 0], 31);
+            const uint32_t f31 = __shfl_sync(0xffffffffu, f[r > 0 ? r - 1 : 0], 31);
+            if (lane == 0) {
+                pkey = k31;
+                pf = f31;
+            }
+        } else if (lane == 0 && in && p > 0) {
             pkey = keys[p - 1];
             pf = feature_of(sid[p - 1], F, fstart);
         }
