@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(256, 4) k_cell_keys(
     uint64_t n, uint32_t F, const uint32_t* __restrict__ fstart, const uint32_t* __restrict__ fjob,
     const JobGrid* __restrict__ grids, KT* __restrict__ keys, uint32_t* __restrict__ vals, float2* __restrict__ xy, uint32_t* __restrict__ nb_cnt,
     BatchCtrl* __restrict__ ctrl, RadixPlan plan, unsigned long long* __restrict__ hist) {
-    static_assert(kRadixDigits == 256, "one digit a thread in the scan");
+    static_assert(kRadixDigits == 512, "two digits a thread in the scan");
     __shared__ uint32_t h[kRadixMaxPasses * kRadixDigits];
     __shared__ bool s_last;
     for (int i = threadIdx.x; i < plan.n * kRadixDigits; i += blockDim.x) h[i] = 0;
@@ -92,10 +92,12 @@ __global__ void __launch_bounds__(256, 4) k_cell_keys(
     if (!s_last) return;
     __threadfence();
     for (int p = 0; p < plan.n; ++p) {
-        unsigned long long* hp = hist + p * kRadixDigits + threadIdx.x;
+        unsigned long long* hp = hist + p * kRadixDigits + 2 * threadIdx.x;
         unsigned long long tot;
-        const unsigned long long v = __ldcg(hp);
-        *hp = block_excl_scan<unsigned long long>(v, &tot);
+        const unsigned long long v = __ldcg(hp), v1 = __ldcg(hp + 1);
+        const unsigned long long at = block_excl_scan<unsigned long long>(v + v1, &tot);
+        hp[0] = at;
+        hp[1] = at + v;
     }
 }
 
@@ -997,7 +999,7 @@ void sort_and_compact(Batch& b) {
         c.add(ka, n);
         c.add(kb, n);
         c.add(other, n);
-        if (b.sort_shared) c.add(b.sort_status, radix_status_words(n));
+        if (b.sort_shared) c.add(b.sort_status, radix_status_words(n, b.plan));
     });
     {
         KScope ks("cell_keys");
@@ -1043,7 +1045,7 @@ void sort_and_compact(Batch& b) {
 }  // namespace
 
 void bucket_layout(Batch& b, Carver& c) {
-    const uint64_t tiles = (b.N + kHeadTile - 1) / kHeadTile, sw = b.N ? radix_status_words(b.N) : 0;
+    const uint64_t tiles = (b.N + kHeadTile - 1) / kHeadTile, sw = b.N ? radix_status_words(b.N, b.plan) : 0;
     b.sort_shared = sw * 8 * (uint64_t)b.plan.n > kSortStatusBytes;
     c.add(b.hist, (uint64_t)std::max(b.plan.n, 1) * kRadixDigits);
     c.add(b.tickets, (uint64_t)b.plan.n + 1);

@@ -363,8 +363,8 @@ void scan_u64_to_u64(const uint64_t* in, uint64_t* out, uint64_t n, cudaStream_t
 // The same with the caller's cleared look-back words (scan_words(n)); no total, launch only.
 uint64_t scan_words(uint64_t n);
 void scan_u32_to_u64(const uint32_t* in, uint64_t* out, uint64_t n, unsigned long long* words, cudaStream_t s);
-// Digit split of a radix sort: pass p sorts width[p] (<= 8) bits from shift[p].
-constexpr int kRadixDigits = 256;
+// Digit split of a radix sort: pass p sorts width[p] (<= kRadixBits) bits from shift[p].
+constexpr int kRadixBits = 9, kRadixDigits = 1 << kRadixBits;
 constexpr int kRadixMaxPasses = 8;
 struct RadixPlan {
     int n;
@@ -377,7 +377,7 @@ RadixPlan radix_plan(int bits);
 // pass writes the other pair of buffers, and ka / va name the sorted ones on
 // return.  Launches only.
 //   hist      every pass's digit starts (hist[p * kRadixDigits + d])
-//   status    look-back words, radix_status_words(n) per pass, all cleared when
+//   status    look-back words, radix_status_words(n, plan) per pass, all cleared when
 //             `shared` is false; with `shared` one pass's words, cleared here
 //   tickets   one cleared word per pass
 //   err       receives a look-back wait that ran out (the failed pass + 1): the
@@ -390,7 +390,7 @@ struct RadixBufs {
     KT *ka, *kb;
     uint32_t *va, *vb;
 };
-uint64_t radix_status_words(uint64_t n);
+uint64_t radix_status_words(uint64_t n, const RadixPlan& plan);
 void radix_sort(RadixBufs<uint32_t>& bufs, uint64_t n, const RadixPlan& plan, cudaStream_t s,
                 const unsigned long long* hist, unsigned long long* status, bool shared, uint32_t* tickets,
                 uint32_t* err, uint32_t test_spin);

@@ -96,36 +96,26 @@ void scan_impl(const Tin* in, Tout* out, uint64_t n, cudaStream_t s, Tout* total
 // Radix sort
 // ---------------------------------------------------------------------------
 
-constexpr int kMaxRadixBits = 8;                        // digits of at most 8 bits
-static_assert((1 << kMaxRadixBits) == kRadixDigits, "digit count");
-constexpr int kMaxRadix = kRadixDigits;
-constexpr int kMaxPasses = kRadixMaxPasses;
 // Tile shape: 512 threads of 8 items (4096-key tiles) and four resident blocks
-// per SM (32 registers for 32-bit keys, a few spilled; 4 x 51 KB of shared
-// memory).  A pass is bound by its look-back: each tile walks back over its
-// predecessors' published counts (about 30 tiles on the 20M workload) one
-// dependent load at a time, so fewer, larger tiles at the same occupancy finish
-// sooner: 0.704 ms per sort against 0.763 ms for 2048-key tiles of 256 threads
-// (eight blocks per SM) and 0.753 ms for 8192-key tiles of 1024 threads (two);
-// 4096-key tiles of 256 threads x 16 items (three blocks per SM, 80 registers)
-// were slower than either.
-template <class KT>
-struct SortShape {
-    static constexpr int threads = 512, rounds = 8, min_blocks = 4;
-};
+// per SM (32 registers, a few spilled; 4 x 43 KB of shared memory), three with
+// digits of nine bits (55 KB; four measured the same and spill).  Ranking takes most
+// of a pass: without any look-back a sort of random keys is a quarter faster, no more.
+// 2048-key tiles of 256 threads (eight blocks an SM) and 8192-key tiles of 1024
+// (two) take 8% longer, 256 threads of 16 items more than either.
+constexpr int kSortThreads = 512, kSortRounds = 8, kSortTile = kSortThreads * kSortRounds;
+constexpr int sort_blocks(int RB) { return RB == 8 ? 4 : 3; }
 
 // Shared memory of one sort block (dynamic): the tile's keys and ids (bulk-copy
 // targets, 16-byte aligned), each digit's global base, the per-warp digit
 // counts and each digit's tile-local start.
 template <class KT, int RB>
 struct SortSmem {
-    static constexpr int T = SortShape<KT>::threads, W = T / 32, R = 1 << RB;
-    static constexpr int tile = T * SortShape<KT>::rounds;
+    static constexpr int W = kSortThreads / 32, R = 1 << RB, tile = kSortTile;
     static constexpr size_t key_at = 0;
     static constexpr size_t val_at = key_at + (size_t)tile * sizeof(KT);
     static constexpr size_t base_at = val_at + (size_t)tile * sizeof(uint32_t);
     static constexpr size_t wh_at = base_at + (size_t)R * sizeof(unsigned long long);
-    static constexpr size_t off_at = wh_at + (size_t)W * R * sizeof(uint32_t);
+    static constexpr size_t off_at = wh_at + (size_t)W * R * sizeof(uint16_t);
     static constexpr size_t bytes = off_at + (size_t)R * sizeof(uint32_t);
     static_assert(val_at % 16 == 0 && base_at % 8 == 0, "alignment");
 };
@@ -141,9 +131,14 @@ struct SortSmem {
 // a block only waits on tiles of blocks already running.  Every wait is
 // bounded: past the limit the block sets *err, uses what it has and finishes
 // (the host reports COLO_ERR_TIMEOUT).  The key's bits are split evenly over
-// the fewest passes of at most 8 bits (25 bits: 7 + 6 + 6 + 6): narrower
-// digits leave more keys per digit in a tile, so the scatter writes longer
-// runs.
+// the fewest passes of at most 8 bits (narrower digits leave more keys per digit in
+// a tile, so the scatter writes longer runs), or of at most 9 where that saves a
+// pass: 25 bits in 4 passes of 7 or less take 80 us for 1M points, in 3 of 9 or less
+// 68; 33 bits of 2M 155 us in 5, 139 in 4; where both take as many (20M points,
+// 28 bits) the wide digits gain nothing.
+//
+// A key's peers in its warp (the lanes with its digit) come from one ballot per bit:
+// match_any over the digit took 8% longer (20M points: 688 -> 636 us a sort).
 // ---------------------------------------------------------------------------
 
 constexpr unsigned long long kFlagA = 1ull << 62;   // tile count published
@@ -190,26 +185,24 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
 // ranking reads them from there, and the same buffers then stage the tile
 // in digit order.  vin == nullptr: the ids are the input positions (the first
 // pass over keys in id order), generated rather than read.
-template <class KT, int RB, int kSortThreads = SortShape<KT>::threads, int kSortRounds = SortShape<KT>::rounds>
-__global__ void __launch_bounds__(kSortThreads, SortShape<KT>::min_blocks) k_onesweep(
+template <class KT, int RB>
+__global__ void __launch_bounds__(kSortThreads, sort_blocks(RB)) k_onesweep(
     const KT* __restrict__ kin, const uint32_t* __restrict__ vin, KT* __restrict__ kout, uint32_t* __restrict__ vout,
     uint64_t n, int shift, uint32_t dmask, const unsigned long long* __restrict__ gofs,
     unsigned long long* __restrict__ status, uint32_t* __restrict__ ticket, uint32_t* __restrict__ err, int bulk,
     uint32_t spin_limit, int withhold, int pass) {
     constexpr int R = 1 << RB;
     constexpr int kSortWarps = kSortThreads / 32;
-    constexpr int kSortTile = kSortThreads * kSortRounds;
     // digits per thread in the look-back (1 or 2); with more threads than digits the
     // first R threads take one each
     constexpr int D = R >= kSortThreads ? R / kSortThreads : 1;
     static_assert(R < kSortThreads || D * kSortThreads == R, "digit count");
     using SM = SortSmem<KT, RB>;
-    static_assert(SM::T == kSortThreads && SM::tile == kSortTile, "shape");
     extern __shared__ __align__(16) unsigned char s_dyn[];
     KT* s_key = reinterpret_cast<KT*>(s_dyn + SM::key_at);
     uint32_t* s_val = reinterpret_cast<uint32_t*>(s_dyn + SM::val_at);
     unsigned long long* s_base = reinterpret_cast<unsigned long long*>(s_dyn + SM::base_at);  // digit's global base
-    uint32_t (*wh)[R] = reinterpret_cast<uint32_t (*)[R]>(s_dyn + SM::wh_at);                 // per-warp digit counts
+    uint16_t (*wh)[R] = reinterpret_cast<uint16_t (*)[R]>(s_dyn + SM::wh_at);                 // per-warp digit counts
     uint32_t* s_off = reinterpret_cast<uint32_t*>(s_dyn + SM::off_at);                       // digit's tile-local start
     const bool owner = (int)threadIdx.x * D < R;   // this thread owns digits in the look-back
     __shared__ alignas(8) uint64_t s_bar;
@@ -225,7 +218,7 @@ __global__ void __launch_bounds__(kSortThreads, SortShape<KT>::min_blocks) k_one
         s_tile = atomicAdd(ticket, 1u);
         if (bulk && !s_skip) mbar_init(&s_bar, 1);
     }
-    for (int i = threadIdx.x; i < kSortWarps * R; i += blockDim.x) (&wh[0][0])[i] = 0;
+    for (int i = threadIdx.x; i < kSortWarps * R / 2; i += blockDim.x) reinterpret_cast<uint32_t*>(wh)[i] = 0;
     __syncthreads();
     if (s_skip) return;
     const uint32_t tile = s_tile;
@@ -260,12 +253,17 @@ __global__ void __launch_bounds__(kSortThreads, SortShape<KT>::min_blocks) k_one
         key[r] = ok ? (staged ? s_key[li] : kin[i]) : 0;
         val[r] = !ok ? 0u : !vin ? (uint32_t)i : staged ? s_val[li] : vin[i];
         const uint32_t d = ok ? ((uint32_t)(key[r] >> shift) & dmask) : 0xFFFFu;
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        uint32_t peers = __ballot_sync(0xffffffffu, ok);
+        if (!ok) peers = ~peers;
+        for (uint32_t bit = 1; bit <= dmask; bit <<= 1) {
+            const uint32_t v = __ballot_sync(0xffffffffu, d & bit);
+            peers &= d & bit ? v : ~v;
+        }
         const int leader = __ffs(peers) - 1;
         uint32_t old = 0;
         if (ok && lane == leader) {
             old = wh[w][d];
-            wh[w][d] = old + __popc(peers);
+            wh[w][d] = (uint16_t)(old + __popc(peers));
         }
         old = __shfl_sync(0xffffffffu, old, leader);
         rank[r] = ok ? old + __popc(peers & lt) : 0xFFFFFFFFu;
@@ -282,7 +280,7 @@ __global__ void __launch_bounds__(kSortThreads, SortShape<KT>::min_blocks) k_one
             if (owner)
                 for (int ww = 0; ww < kSortWarps; ++ww) {
                     const uint32_t t = wh[ww][d];
-                    wh[ww][d] = c;
+                    wh[ww][d] = (uint16_t)c;
                     c += t;
                 }
             cnt[i] = c;
@@ -291,7 +289,7 @@ __global__ void __launch_bounds__(kSortThreads, SortShape<KT>::min_blocks) k_one
         uint32_t tot;
         uint32_t ex = block_excl_scan<uint32_t>(sum, &tot);
         // status words and look-back for the dmask + 1 digits in use only (a tile's words
-        // are kMaxRadix apart: packing them closer measured slower)
+        // are R apart: packing them closer measured slower)
         const uint32_t nd = dmask + 1;
 #pragma unroll
         for (int i = 0; i < D; ++i) {
@@ -376,32 +374,35 @@ void scan_u64_to_u64(const uint64_t* in, uint64_t* out, uint64_t n, cudaStream_t
 
 namespace {
 
-template <class KT>
+// Digit width the passes are compiled for (the first pass is the widest).
+int plan_bits(const RadixPlan& plan) { return plan.n && plan.width[0] > 8 ? 9 : 8; }
+
+template <class KT, int RB>
 void radix_sort_impl(RadixBufs<KT>& bufs, uint64_t n, const RadixPlan& plan, cudaStream_t s,
                      const unsigned long long* hist, unsigned long long* status, bool shared, uint32_t* tickets,
                      uint32_t* err, uint32_t test_spin) {
     if (n >= (1ull << 32)) throw StatusError{COLO_ERR_CAPACITY, "radix sort supports < 2^32 items"};
-    using SM = SortSmem<KT, kMaxRadixBits>;
-    const uint32_t ntiles = (uint32_t)((n + SM::tile - 1) / SM::tile);
+    using SM = SortSmem<KT, RB>;
+    constexpr int R = 1 << RB;
+    const uint32_t ntiles = (uint32_t)((n + kSortTile - 1) / kSortTile);
     // several blocks per SM: ask for the largest shared-memory carveout
-    COLO_CUDA(cudaFuncSetAttribute((const void*)k_onesweep<KT, kMaxRadixBits>,
+    COLO_CUDA(cudaFuncSetAttribute((const void*)k_onesweep<KT, RB>,
                                    cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    COLO_CUDA(cudaFuncSetAttribute((const void*)k_onesweep<KT, kMaxRadixBits>,
+    COLO_CUDA(cudaFuncSetAttribute((const void*)k_onesweep<KT, RB>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM::bytes));
     for (int p = 0; p < plan.n; ++p) {
         KScope ks("radix_sort");   // one timed launch per digit pass
         const uint32_t dm = (1u << plan.width[p]) - 1u;
         // shared words: those of the digits in use are cleared for every pass (a pitched clear:
-        // a tile's words stay kMaxRadix apart, which spreads the polled lines over L2)
-        unsigned long long* st = status + (shared ? 0 : (uint64_t)p * ntiles * kMaxRadix);
+        // a tile's words stay R apart, which spreads the polled lines over L2)
+        unsigned long long* st = status + (shared ? 0 : (uint64_t)p * ntiles * R);
         if (shared)
-            COLO_CUDA(cudaMemset2DAsync(st, kMaxRadix * 8, 0, ((size_t)1 << plan.width[p]) * 8, ntiles, s));
+            COLO_CUDA(cudaMemset2DAsync(st, R * 8, 0, ((size_t)1 << plan.width[p]) * 8, ntiles, s));
         const int bulk = ((uintptr_t)bufs.ka % 16 == 0 && (uintptr_t)bufs.va % 16 == 0) ? 1 : 0;
         const uint32_t* vin = p == 0 ? nullptr : bufs.va;   // the first pass makes the ids (no read)
-        k_onesweep<KT, kMaxRadixBits><<<ntiles, SM::T, SM::bytes, s>>>(bufs.ka, vin, bufs.kb, bufs.vb, n, plan.shift[p], dm,
-                                                                     hist + p * kMaxRadix, st, tickets + p, err, bulk,
-                                                                     test_spin ? test_spin : kSpinLimit,
-                                                                     test_spin && p == 0 ? 1 : 0, p);
+        k_onesweep<KT, RB><<<ntiles, kSortThreads, SM::bytes, s>>>(
+            bufs.ka, vin, bufs.kb, bufs.vb, n, plan.shift[p], dm, hist + p * kRadixDigits, st, tickets + p, err, bulk,
+            test_spin ? test_spin : kSpinLimit, test_spin && p == 0 ? 1 : 0, p);
         COLO_LAUNCH_CHECK();
         count_launch();
         std::swap(bufs.ka, bufs.kb);
@@ -411,17 +412,15 @@ void radix_sort_impl(RadixBufs<KT>& bufs, uint64_t n, const RadixPlan& plan, cud
 
 }  // namespace
 
-uint64_t radix_status_words(uint64_t n) {
-    static_assert(SortSmem<uint32_t, kMaxRadixBits>::tile == SortSmem<uint64_t, kMaxRadixBits>::tile, "one tile size");
-    const uint64_t tile = SortSmem<uint32_t, kMaxRadixBits>::tile;
-    return (n + tile - 1) / tile * kMaxRadix;
+uint64_t radix_status_words(uint64_t n, const RadixPlan& plan) {
+    return (n + kSortTile - 1) / kSortTile << plan_bits(plan);
 }
 
 RadixPlan radix_plan(int bits) {
-    // fewest passes of at most 8 bits, widths as even as possible (25 bits: 7 + 6 + 6 + 6)
+    // fewest passes of at most 9 bits, widths as even as possible (25 bits: 9 + 8 + 8)
     RadixPlan plan{};
     if (bits <= 0) return plan;
-    plan.n = (bits + kMaxRadixBits - 1) / kMaxRadixBits;
+    plan.n = (bits + kRadixBits - 1) / kRadixBits;
     for (int p = 0, sh = 0; p < plan.n; ++p) {
         plan.width[p] = bits / plan.n + (p < bits % plan.n ? 1 : 0);
         plan.shift[p] = sh;
@@ -433,13 +432,15 @@ RadixPlan radix_plan(int bits) {
 void radix_sort(RadixBufs<uint32_t>& bufs, uint64_t n, const RadixPlan& plan, cudaStream_t s,
                 const unsigned long long* hist, unsigned long long* status, bool shared, uint32_t* tickets,
                 uint32_t* err, uint32_t test_spin) {
-    radix_sort_impl<uint32_t>(bufs, n, plan, s, hist, status, shared, tickets, err, test_spin);
+    (plan_bits(plan) == 9 ? radix_sort_impl<uint32_t, 9> : radix_sort_impl<uint32_t, 8>)(
+        bufs, n, plan, s, hist, status, shared, tickets, err, test_spin);
 }
 
 void radix_sort(RadixBufs<uint64_t>& bufs, uint64_t n, const RadixPlan& plan, cudaStream_t s,
                 const unsigned long long* hist, unsigned long long* status, bool shared, uint32_t* tickets,
                 uint32_t* err, uint32_t test_spin) {
-    radix_sort_impl<uint64_t>(bufs, n, plan, s, hist, status, shared, tickets, err, test_spin);
+    (plan_bits(plan) == 9 ? radix_sort_impl<uint64_t, 9> : radix_sort_impl<uint64_t, 8>)(
+        bufs, n, plan, s, hist, status, shared, tickets, err, test_spin);
 }
 
 }  // namespace colo
