@@ -9,7 +9,9 @@
 //
 // Exactness: a coordinate is converted on the device only when the decimal
 // has at most 19 significant digits and the value is m * 10^e with
-// m < 2^53 and |e| <= 22.  Then m and 10^|e| are exact doubles and one IEEE
+// m < 2^53 and |e| <= 22.  With -11 <= e <= 0, as coordinates are written, the
+// correctly rounded float comes from one integer quotient and its remainder
+// (FP64 divisions are slow here).  Else m and 10^|e| are exact doubles and one IEEE
 // multiply or divide gives the correctly rounded double of the decimal
 // (Clinger's fast path, "How to read floating point numbers accurately",
 // PLDI 1990).  Rounding that double to float is the correctly rounded float
@@ -44,42 +46,66 @@ namespace {
 
 enum : uint8_t { L_OK = 0, L_EMPTY = 1, L_HOST = 2, L_BAD = 3, L_MINUS1 = 4 };
 
-constexpr uint32_t kNlBytes = 64;   // bytes per thread when finding line ends
+constexpr int kNlThreads = 256, kNlSteps = 4;
+constexpr uint32_t kNlBytes = 16 * kNlSteps, kNlTile = kNlThreads * kNlBytes;   // a thread's bytes, a block's
+constexpr uint32_t kMinLine = 6;   // "0,0,0" and its newline: the shortest point line
 
-__device__ __forceinline__ uint32_t count_nl_word(uint32_t w) {
-    // bytes equal to '\n' (0x0A) in a 32-bit word
+// One bit per byte of a 32-bit word that equals '\n' (0x0A), lowest byte first.
+__device__ __forceinline__ uint32_t nl_bits(uint32_t w) {
     const uint32_t x = w ^ 0x0A0A0A0Au;
-    const uint32_t t = ((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x;   // high bit set in bytes that are non-zero
-    return __popc(~t & 0x80808080u);
+    const uint32_t t = ~(((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) & 0x80808080u;   // high bit of every matching byte
+    return (t >> 7) * 0x10204080u >> 28;   // bits 0, 8, 16, 24 to 28 .. 31
 }
 
-__global__ void k_count_lines(const uint8_t* __restrict__ buf, uint64_t n, uint32_t* __restrict__ cnt) {
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t b = t * kNlBytes;
-    if (b >= n) return;
-    uint32_t c = 0;
-    if (b + kNlBytes <= n) {
-        const uint4* p = reinterpret_cast<const uint4*>(buf + b);
+// Positions of the line ends in one pass: a block marks the newlines of a 16 KB tile
+// (a bit a byte, from coalesced 16-byte loads), counts them, takes its place from a
+// decoupled look-back and writes as many as nl holds (cap; the total is the last
+// tile's status word).  buf is 16-byte aligned and readable up to a multiple of 16.
+// Bound by the look-back and the launch at this size: a count, a scan and a
+// second read byte by byte took 90 us for 24 MB (1M lines), this 25.
+__global__ void __launch_bounds__(kNlThreads) k_line_ends(const uint8_t* __restrict__ buf, uint64_t n,
+                                                          unsigned long long* __restrict__ status,
+                                                          uint32_t* __restrict__ ticket, uint64_t* __restrict__ nl,
+                                                          uint64_t cap) {
+    __shared__ uint32_t s_tile;
+    __shared__ unsigned long long s_prefix;
+    __shared__ __align__(8) uint16_t s_bits[kNlThreads * kNlSteps];
+    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    const uint64_t t0 = (uint64_t)tile * kNlTile;
 #pragma unroll
-        for (int i = 0; i < (int)(kNlBytes / 16); ++i) {
-            const uint4 v = p[i];
-            c += count_nl_word(v.x) + count_nl_word(v.y) + count_nl_word(v.z) + count_nl_word(v.w);
+    for (int i = 0; i < kNlSteps; ++i) {
+        const uint32_t at = (uint32_t)i * kNlThreads + threadIdx.x;
+        const uint64_t b = t0 + (uint64_t)at * 16;
+        uint32_t m = 0;
+        if (b < n) {
+            const uint4 v = *reinterpret_cast<const uint4*>(buf + b);
+            m = nl_bits(v.x) | nl_bits(v.y) << 4 | nl_bits(v.z) << 8 | nl_bits(v.w) << 12;
+            if (n - b < 16) m &= (1u << (uint32_t)(n - b)) - 1u;
         }
-    } else {
-        for (uint64_t i = b; i < n; ++i) c += buf[i] == '\n';
+        s_bits[at] = (uint16_t)m;
     }
-    cnt[t] = c;
-}
-
-__global__ void k_line_ends(const uint8_t* __restrict__ buf, uint64_t n, const uint64_t* __restrict__ off,
-                            uint64_t* __restrict__ nl) {
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t b = t * kNlBytes;
-    if (b >= n) return;
-    uint64_t o = off[t];
-    const uint64_t e = b + kNlBytes < n ? b + kNlBytes : n;
-    for (uint64_t i = b; i < e; ++i)
-        if (buf[i] == '\n') nl[o++] = i;
+    __syncthreads();
+    uint64_t mine = reinterpret_cast<const uint64_t*>(s_bits)[threadIdx.x];
+    uint32_t tot;
+    const uint32_t ex = block_excl_scan<uint32_t>((uint32_t)__popcll(mine), &tot);
+    if (threadIdx.x < 32) {
+        unsigned long long prefix;
+        if (!warp_lookback(status, tile, tot, prefix)) {   // the text before this tile, counted here
+            unsigned long long add = 0;
+            for (uint64_t b = threadIdx.x; b < t0; b += 32) add += buf[b] == '\n';
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+            prefix = add;
+            lookback_publish(status, tile, prefix + tot);
+        }
+        if (threadIdx.x == 0) s_prefix = prefix;
+    }
+    __syncthreads();
+    uint64_t o = s_prefix + ex;
+    const uint64_t b = t0 + (uint64_t)threadIdx.x * kNlBytes;
+    for (; mine && o < cap; mine &= mine - 1) nl[o++] = b + (uint64_t)(__ffsll((long long)mine) - 1);
 }
 
 __device__ __forceinline__ bool is_space(uint8_t c) {
@@ -101,6 +127,53 @@ __device__ int parse_int_dev(const uint8_t* b, const uint8_t* e, int32_t* v) {
     if (r < INT32_MIN || r > INT32_MAX) return 1;
     *v = (int32_t)r;
     return 0;
+}
+
+// 10^k, its reciprocal floor(2^(63 + L) / 10^k) with 2^(L-1) < 10^k <= 2^L, and L - 1.
+constexpr int kIntDigits = 11;
+struct Tenth {
+    uint64_t d, inv;
+    int shift;
+};
+constexpr Tenth tenth(int k) {
+    uint64_t d = 1;
+    for (int i = 0; i < k; ++i) d *= 10;
+    int L = 0;
+    while ((1ull << L) < d) ++L;
+    uint64_t q = 0, r = 1;   // long division of 2^(63 + L), a bit at a time
+    for (int i = 0; i < 63 + L; ++i) {
+        r <<= 1;
+        q <<= 1;
+        if (r >= d) {
+            r -= d;
+            q |= 1;
+        }
+    }
+    return {d, q, L - 1};
+}
+__constant__ Tenth c_tenth[kIntDigits + 1] = {{1, 0, 0}, tenth(1), tenth(2), tenth(3), tenth(4), tenth(5),
+                                              tenth(6),  tenth(7), tenth(8), tenth(9), tenth(10), tenth(11)};
+__constant__ double c_p10[23] = {1e0,  1e1,  1e2,  1e3,  1e4,  1e5,  1e6,  1e7,  1e8,  1e9,  1e10, 1e11,
+                                 1e12, 1e13, 1e14, 1e15, 1e16, 1e17, 1e18, 1e19, 1e20, 1e21, 1e22};
+
+// The float nearest to m / 10^k (ties to even), m in 1 .. 2^53 - 1, 1 <= k <= kIntDigits, in integers.
+// m is shifted to 64 bits, so the quotient has at least 27; the product with the reciprocal,
+// which is below 2^(63 + L) / 10^k by less than one, gives it or one less.
+__device__ __forceinline__ float decimal_to_float(uint64_t m, int k) {
+    const Tenth t = c_tenth[k];
+    const int z = __clzll((long long)m);
+    const uint64_t num = m << z;
+    uint64_t q = __umul64hi(num, t.inv) >> t.shift;
+    uint64_t r = num - q * t.d;
+    if (r >= t.d) {
+        r -= t.d;
+        ++q;
+    }
+    const int drop = 40 - __clzll((long long)q);   // bits of q below the 24 kept
+    const uint64_t half = 1ull << (drop - 1), low = q & (2 * half - 1);
+    uint32_t mant = (uint32_t)(q >> drop);
+    if (low > half || (low == half && (r || (mant & 1u)))) ++mant;
+    return ldexpf((float)mant, drop - z);   // exact: 24 bits (2^24 on a carry) in the normal range
 }
 
 // std::stof on [b, e) as the host reader does it: 0 converted exactly here,
@@ -167,10 +240,13 @@ __device__ int parse_float_dev(const uint8_t* b, const uint8_t* e, float* v) {
     }
     const int e10 = ex - frac;
     if (m >= (1ull << 53) || e10 < -22 || e10 > 22) return 1;
-    const double p10[23] = {1e0,  1e1,  1e2,  1e3,  1e4,  1e5,  1e6,  1e7,  1e8,  1e9,  1e10, 1e11,
-                            1e12, 1e13, 1e14, 1e15, 1e16, 1e17, 1e18, 1e19, 1e20, 1e21, 1e22};
+    if (e10 <= 0 && e10 >= -kIntDigits) {
+        const float f = e10 == 0 ? __ull2float_rn(m) : decimal_to_float(m, -e10);
+        *v = neg ? -f : f;
+        return 0;
+    }
     const double dm = (double)m;   // exact: m < 2^53
-    const double d = e10 >= 0 ? __dmul_rn(dm, p10[e10]) : __ddiv_rn(dm, p10[-e10]);
+    const double d = e10 >= 0 ? __dmul_rn(dm, c_p10[e10]) : __ddiv_rn(dm, c_p10[-e10]);
     // float normal range only (no subnormal or overflow handling here)
     if (!(d >= 1.1754943508222875e-38) || d > 3.4028234663852886e38) return 1;
     // a float rounding midpoint: the 29 low mantissa bits are exactly 1000...0
@@ -194,26 +270,42 @@ __device__ __forceinline__ void failed(uint64_t i, uint8_t code, uint8_t* st, un
 }
 
 // One thread per line of the body: lines 0 .. L-1 end at nl[i]; line L (if
-// the text does not end with a newline) ends at n.
-__global__ void k_parse_lines(const uint8_t* __restrict__ buf, uint64_t n, const uint64_t* __restrict__ nl,
-                              uint64_t L, uint64_t lines, float* __restrict__ x, float* __restrict__ y,
-                              int32_t* __restrict__ raw, uint8_t* __restrict__ st,
-                              unsigned long long* __restrict__ marks, uint64_t* __restrict__ host_list,
-                              uint64_t host_cap) {
+// the text does not end with a newline) ends at n.  A block's 256 lines are one
+// range of the text, brought into shared memory by coalesced loads unless it is
+// longer than kParseText.  Bound by instruction issue in the walks over a line's
+// bytes: 24 MB (1M lines) take 123 us (from global memory 169, staged 159, and 123
+// with the coordinates converted in integers); the host's arrays, made meanwhile,
+// take as long.
+constexpr uint32_t kParseText = 16384;
+__global__ void __launch_bounds__(256) k_parse_lines(
+    const uint8_t* __restrict__ buf, uint64_t n, const uint64_t* __restrict__ nl, uint64_t L, uint64_t lines,
+    float* __restrict__ x, float* __restrict__ y, int32_t* __restrict__ raw, uint8_t* __restrict__ st,
+    unsigned long long* __restrict__ marks, uint64_t* __restrict__ host_list, uint64_t host_cap) {
+    __shared__ uint4 s_text[kParseText / 16];
     // marks[0]: first empty line, marks[1]: first malformed / id -1 line,
     // marks[2]: lines left to the host (their indices in host_list, unordered)
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x, i = i0 + threadIdx.x;
+    const uint64_t i1 = i0 + blockDim.x < lines ? i0 + blockDim.x : lines;
+    const uint64_t first = (i0 == 0 ? 0 : nl[i0 - 1] + 1) & ~15ull;   // 16-byte aligned
+    const uint64_t last = i1 - 1 < L ? nl[i1 - 1] : n;
+    const bool staged = last - first <= kParseText;
+    if (staged) {
+        const uint32_t words = (uint32_t)((last - first + 15) / 16);
+        for (uint32_t q = threadIdx.x; q < words; q += blockDim.x)
+            s_text[q] = reinterpret_cast<const uint4*>(buf + first)[q];
+        __syncthreads();
+    }
     if (i >= lines) return;
     const uint64_t b = i == 0 ? 0 : nl[i - 1] + 1;
     uint64_t e = i < L ? nl[i] : n;
-    if (e > b && buf[e - 1] == '\r') --e;
+    const uint8_t* p = staged ? reinterpret_cast<const uint8_t*>(s_text) + (b - first) : buf + b;
+    if (e > b && p[e - b - 1] == '\r') --e;
     if (e == b) {
         st[i] = L_EMPTY;
         atomicMin(&marks[0], (unsigned long long)i);
         return;
     }
-    const uint8_t* p = buf + b;
-    const uint8_t* pe = buf + e;
+    const uint8_t* pe = p + (e - b);
     const uint8_t *c1 = nullptr, *c2 = nullptr, *c3 = nullptr;
     for (const uint8_t* q = p; q < pe; ++q) {
         const uint8_t ch = *q;
@@ -253,14 +345,22 @@ __global__ void k_parse_lines(const uint8_t* __restrict__ buf, uint64_t n, const
     st[i] = L_OK;
 }
 
-// Group starts (the first point of every run of equal ids) with the byte
-// range of their id field, for the feature names.
-__global__ void k_group_starts(const int32_t* __restrict__ raw, uint64_t np, const uint64_t* __restrict__ nl,
-                               unsigned long long* __restrict__ cnt, uint64_t* __restrict__ out) {
+// Group starts (the first point of every run of equal ids before the first empty
+// line) with the byte range of their id field, for the feature names: out[2 q],
+// out[2 q + 1], q < marks[3].  The bounds line (the one after the empty line)
+// is marks[4] .. marks[5].
+__global__ void k_group_starts(const int32_t* __restrict__ raw, uint64_t lines, const uint64_t* __restrict__ nl,
+                               uint64_t L, uint64_t n, unsigned long long* __restrict__ marks,
+                               uint64_t* __restrict__ out) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= np) return;
+    const uint64_t empty = marks[0];
+    if (i == 0 && empty < lines && empty + 1 < lines) {
+        marks[4] = nl[empty] + 1;
+        marks[5] = empty + 1 < L ? nl[empty + 1] : n;
+    }
+    if (i >= lines || i >= empty) return;
     if (i > 0 && raw[i] == raw[i - 1]) return;
-    const unsigned long long k = atomicAdd(cnt, 1ull);
+    const unsigned long long k = atomicAdd(&marks[3], 1ull);
     out[2 * k] = i;
     out[2 * k + 1] = i == 0 ? 0 : nl[i - 1] + 1;
 }
@@ -338,68 +438,82 @@ colo_status parse_points_csv_device(cudaStream_t s, const char* path, HostPoints
     const char* body = nl0 ? nl0 + 1 : end;
     const uint64_t nb = (uint64_t)(end - body);
     hp.clear();
-    // the text on the device, and its line ends
+    // the text on the device, and its line ends: into room for lines of points, and once more
+    // when there are more (the kernel counts them all)
     DevBuf<uint8_t> dbuf;
-    dbuf.alloc(nb ? nb : 16, s);
+    dbuf.alloc((nb + 15) / 16 * 16 + 16, s);
     if (nb) COLO_CUDA(cudaMemcpyAsync(dbuf.get(), body, nb, cudaMemcpyHostToDevice, s));
-    const uint64_t nthreads = (nb + kNlBytes - 1) / kNlBytes;
-    DevBuf<uint32_t> cnt;
-    DevBuf<uint64_t> off;
-    uint64_t L = 0;
-    if (nthreads) {
-        cnt.alloc(nthreads, s);
-        off.alloc(nthreads, s);
-        {
-            KScope ks("csv_lines");
-            k_count_lines<<<(unsigned)((nthreads + 255) / 256), 256, 0, s>>>(dbuf.get(), nb, cnt.get());
-            COLO_LAUNCH_CHECK();
-            count_launch();
-        }
-        scan_u32_to_u64(cnt.get(), off.get(), nthreads, s, &L);
-    }
+    const uint64_t tiles = (nb + kNlTile - 1) / kNlTile;
+    DevBuf<unsigned long long> words;
     DevBuf<uint64_t> dnl;
-    dnl.alloc(L ? L : 1, s);
-    uint64_t last_nl = 0;
-    if (L) {
+    uint64_t L = 0, cap = nb / kMinLine + 64;
+    // the host's arrays are made while the device works (at most a line of the text per point)
+    const uint64_t room = std::min<uint64_t>(N > 0 ? (uint64_t)N : 0u, nb / kMinLine + 1);
+    for (bool again = tiles > 0; again;) {
+        dnl.alloc(cap, s);
+        words.alloc(tiles + 1, s);
+        words.zero(s);
         {
             KScope ks("csv_lines");
-            k_line_ends<<<(unsigned)((nthreads + 255) / 256), 256, 0, s>>>(dbuf.get(), nb, off.get(), dnl.get());
+            k_line_ends<<<(unsigned)tiles, kNlThreads, 0, s>>>(
+                dbuf.get(), nb, words.get(), reinterpret_cast<uint32_t*>(words.get() + tiles), dnl.get(), cap);
             COLO_LAUNCH_CHECK();
             count_launch();
         }
-        COLO_CUDA(cudaMemcpyAsync(&last_nl, dnl.get() + L - 1, 8, cudaMemcpyDeviceToHost, s));
-        COLO_CUDA(cudaStreamSynchronize(s));
+        hp.x.resize(room);
+        COLO_CUDA(cudaMemcpyAsync(&L, words.get() + tiles - 1, 8, cudaMemcpyDeviceToHost, s));
+        stream_wait(s);
+        L &= kScanVal;
+        again = L > cap;
+        cap = L;
     }
     // a last line without its newline counts too (std::getline)
-    const uint64_t lines = L + ((L == 0 ? nb > 0 : last_nl + 1 < nb) ? 1 : 0);
-    // every line parsed on the device
+    const uint64_t lines = L + (nb > 0 && end[-1] != '\n' ? 1 : 0);
+    // every line parsed on the device, then the groups of the lines before the first empty one
     DevBuf<float> px, py;
     DevBuf<int32_t> praw;
     DevBuf<uint8_t> pst;
-    DevBuf<unsigned long long> marks;
     DevBuf<uint64_t> hlist;
+    constexpr uint64_t kMarks = 6, kFirstGroups = 256;
     const uint64_t host_cap = std::max<uint64_t>(1024, lines / 64);
-    marks.alloc(3, s);
+    DevBuf<unsigned long long> marks;   // the marks, then the groups
+    marks.alloc(kMarks + 2 * std::max(lines, kFirstGroups), s);
     hlist.alloc(host_cap, s);
     {
-        const unsigned long long init[3] = {~0ull, ~0ull, 0ull};
+        const unsigned long long init[kMarks] = {~0ull, ~0ull, 0ull, 0ull, 0ull, 0ull};
         COLO_CUDA(cudaMemcpyAsync(marks.get(), init, sizeof(init), cudaMemcpyHostToDevice, s));
     }
+    uint64_t* const groups = reinterpret_cast<uint64_t*>(marks.get() + kMarks);
     px.alloc(lines ? lines : 1, s);
     py.alloc(lines ? lines : 1, s);
     praw.alloc(lines ? lines : 1, s);
     pst.alloc(lines ? lines : 1, s);
-    if (lines) {
-        KScope ks("csv_parse");
-        k_parse_lines<<<(unsigned)((lines + 255) / 256), 256, 0, s>>>(dbuf.get(), nb, dnl.get(), L, lines, px.get(),
-                                                                     py.get(), praw.get(), pst.get(), marks.get(),
-                                                                     hlist.get(), host_cap);
+    auto list_groups = [&] {
+        KScope ks("csv_groups");
+        k_group_starts<<<(unsigned)((lines + 255) / 256), 256, 0, s>>>(praw.get(), lines, dnl.get(), L, nb,
+                                                                      marks.get(), groups);
         COLO_LAUNCH_CHECK();
         count_launch();
+    };
+    if (lines) {
+        {
+            KScope ks("csv_parse");
+            k_parse_lines<<<(unsigned)((lines + 255) / 256), 256, 0, s>>>(dbuf.get(), nb, dnl.get(), L, lines,
+                                                                         px.get(), py.get(), praw.get(), pst.get(),
+                                                                         marks.get(), hlist.get(), host_cap);
+            COLO_LAUNCH_CHECK();
+            count_launch();
+        }
+        list_groups();
     }
-    unsigned long long hm[3] = {~0ull, ~0ull, 0ull};
-    COLO_CUDA(cudaMemcpyAsync(hm, marks.get(), sizeof(hm), cudaMemcpyDeviceToHost, s));
-    COLO_CUDA(cudaStreamSynchronize(s));
+    hp.y.resize(room);
+    hp.raw.resize(room);
+    std::vector<unsigned long long> hm(kMarks + 2 * kFirstGroups);
+    auto read_marks = [&] {
+        COLO_CUDA(cudaMemcpyAsync(hm.data(), marks.get(), hm.size() * 8, cudaMemcpyDeviceToHost, s));
+        stream_wait(s);
+    };
+    read_marks();
     const unsigned long long first_empty = hm[0];
     const uint64_t np = first_empty < lines ? first_empty : lines;   // point lines before the empty line
     // the first failing device line before the empty line, and its kind
@@ -421,7 +535,6 @@ colo_status parse_points_csv_device(cudaStream_t s, const char* path, HostPoints
         std::sort(want.begin(), want.end());
     }
     const bool has_bounds = first_empty < lines && first_empty + 1 < lines;
-    if (has_bounds) want.push_back(first_empty + 1);
     std::vector<uint64_t> rng(2 * want.size());
     if (!want.empty()) {
         DevBuf<uint64_t> didx, drng;
@@ -441,7 +554,7 @@ colo_status parse_points_csv_device(cudaStream_t s, const char* path, HostPoints
         if (*lend > *lb && (*lend)[-1] == '\r') --*lend;
     };
     // host lines in order: the first failing line, device or host, is the one the serial reader names
-    const size_t nhost = has_bounds ? want.size() - 1 : want.size();
+    const size_t nhost = want.size();
     std::vector<std::pair<uint64_t, std::string>> host_tokens;
     std::vector<uint64_t> hidx;
     std::vector<float> hxv, hyv;
@@ -481,8 +594,8 @@ colo_status parse_points_csv_device(cudaStream_t s, const char* path, HostPoints
         return COLO_ERR_PARSE;
     }
     {
-        const char *lb, *lend;
-        line_at(want.size() - 1, &lb, &lend);
+        const char *lb = body + hm[4], *lend = body + hm[5];
+        if (lend > lb && lend[-1] == '\r') --lend;
         if (!csv_parse_bounds(lb, lend, hp.bounds)) {
             err = "dataset: bounds line must be minX,minY,maxX,maxY";
             return COLO_ERR_PARSE;
@@ -506,22 +619,11 @@ colo_status parse_points_csv_device(cudaStream_t s, const char* path, HostPoints
                                                                     px.get(), py.get(), praw.get());
         COLO_LAUNCH_CHECK();
         count_launch();
-        COLO_CUDA(cudaStreamSynchronize(s));   // the host vectors above are about to go
+        COLO_CUDA(cudaMemsetAsync(marks.get() + 3, 0, 8, s));
+        list_groups();
+        read_marks();   // the host vectors above are about to go
     }
-    // group starts and the line start of each (feature names)
-    DevBuf<unsigned long long> gcnt;
-    DevBuf<uint64_t> gout;
-    gcnt.alloc(1, s);
-    gcnt.zero(s);
-    gout.alloc(2 * (np ? np : 1), s);
-    if (np) {
-        KScope ks("csv_groups");
-        k_group_starts<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(praw.get(), np, dnl.get(), gcnt.get(), gout.get());
-        COLO_LAUNCH_CHECK();
-        count_launch();
-    }
-    unsigned long long G = 0;
-    COLO_CUDA(cudaMemcpyAsync(&G, gcnt.get(), 8, cudaMemcpyDeviceToHost, s));
+    const uint64_t G = hm[3];
     hp.x.resize(np);
     hp.y.resize(np);
     hp.raw.resize(np);
@@ -530,12 +632,10 @@ colo_status parse_points_csv_device(cudaStream_t s, const char* path, HostPoints
         COLO_CUDA(cudaMemcpyAsync(hp.y.data(), py.get(), np * 4, cudaMemcpyDeviceToHost, s));
         COLO_CUDA(cudaMemcpyAsync(hp.raw.data(), praw.get(), np * 4, cudaMemcpyDeviceToHost, s));
     }
+    hm.resize(kMarks + 2 * std::max(G, kFirstGroups));
+    if (G > kFirstGroups) COLO_CUDA(cudaMemcpyAsync(hm.data() + kMarks, groups, 2 * G * 8, cudaMemcpyDeviceToHost, s));
     COLO_CUDA(cudaStreamSynchronize(s));
-    std::vector<uint64_t> g(2 * G);
-    if (G) {
-        COLO_CUDA(cudaMemcpyAsync(g.data(), gout.get(), 2 * G * 8, cudaMemcpyDeviceToHost, s));
-        COLO_CUDA(cudaStreamSynchronize(s));
-    }
+    const unsigned long long* g = hm.data() + kMarks;
     std::vector<std::pair<uint64_t, uint64_t>> starts(G);
     for (uint64_t q = 0; q < G; ++q) starts[q] = {g[2 * q], g[2 * q + 1]};
     std::sort(starts.begin(), starts.end());
