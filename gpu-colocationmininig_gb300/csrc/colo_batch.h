@@ -32,6 +32,7 @@ struct alignas(128) BatchCtrl {
     uint32_t M, Rn;              // occupied cells, runs
     uint32_t keys_done;          // blocks of the cell-key pass that have added their histograms
     LineCounter nlistq;          // cells queued for a neighbourhood run list
+    LineCounter nquadq;          // cells with a quad of quad_min features or more
     // neighbourhood lists: target points, runs, anchors with short and with long lists, and the
     // pair evaluations (= room that the single-pass join may need)
     LineCounter targets, list_runs, anchors, long_anchors, pairs;
@@ -99,8 +100,14 @@ struct Batch {
     Span<uint32_t> cmask;
     Span<uint32_t> nbmask;       // per cell: feature mask of its geometric 3x3 block
     Span<uint32_t> listq;        // cells whose 3x3 block has a feature above their lowest own one
-    Span<uint32_t> qmask;        // per cell: masks of the 4 quads containing it ([M][4][W])
-    // driver lists: for global feature f, the cells whose 3x3 block holds f
+    // per cell of quadq: masks of the 4 quads containing it ([M][4][W], other cells' rows unwritten)
+    Span<uint32_t> qmask;
+    // the cells with a quad of at least quad_min features: no other cell is in a candidate's U_c
+    // (a candidate of three or more members needs a quad that covers three)
+    Span<uint32_t> quadq;
+    uint32_t quad_min = 3;
+    uint64_t quad_cells = 0;     // their number (known after settle)
+    // driver lists: for global feature f, the cells of quadq whose 3x3 block holds f
     // (nbmask bit), dlist[doff[f] .. doff[f+1]), in no particular order; the
     // level filters test exactly these cells for the candidates f drives
     DevBuf<uint32_t> dlist;

@@ -456,9 +456,13 @@ constexpr int kQuadThreads = 128;
 // (larger batches count with global atomics).
 constexpr uint32_t kQuadHist = 1024;
 
-// Per cell: the four quad masks and the 3x3 mask (nbmask), the queue of cells
-// that need a neighbourhood run list, and the driver-list sizes: dcnt[f] =
-// cells whose 3x3 mask holds f.  A block walks spans of consecutive cells (so that
+// Per cell: the 3x3 mask (nbmask), the queue of cells that need a neighbourhood
+// run list, the queue of cells with a quad of quad_min features or more, their four
+// quad masks, and the driver-list sizes: dcnt[f] = cells of that queue whose 3x3
+// mask holds f.  Most cells have no such quad (94% at 1M and at 20M points), and
+// no pattern of three is bounded by them: without their 64 bytes of quad masks and
+// their entries in the driver lists this kernel takes 201 us instead of 262 at 20M
+// points, the lists 27 instead of 157 and the level filters 334 instead of 430.  A block walks spans of consecutive cells (so that
 // queued cells stay near each other: the list kernel reads their neighbourhoods)
 // and keeps one histogram for all of them (one global atomic per
 // feature per block at the end); a warp's 32 cells are counted by a bit
@@ -472,18 +476,38 @@ template <int WT>
 __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
     BatchCtrl* __restrict__ ctrl, const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob,
     const JobGrid* __restrict__ grids, const int32_t* __restrict__ nb9, const uint32_t* __restrict__ cmask,
-    uint32_t* __restrict__ qmask, uint32_t* __restrict__ nbmask, uint32_t* __restrict__ listq, uint32_t F,
-    uint32_t* __restrict__ dcnt) {
+    uint32_t* __restrict__ qmask, uint32_t* __restrict__ nbmask, uint32_t* __restrict__ listq,
+    uint32_t* __restrict__ quadq, uint32_t quad_min, bool several, uint32_t F, uint32_t* __restrict__ dcnt) {
     const uint64_t M = ctrl->M;
     __shared__ uint32_t s_hist[kQuadHist];
-    __shared__ uint32_t s_queue[kQuadThreads / 32][64];
+    __shared__ uint32_t s_queue[kQuadThreads / 32][2][64];
     const bool local_hist = F <= kQuadHist;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (local_hist)
         for (uint32_t i = threadIdx.x; i < F; i += blockDim.x) s_hist[i] = 0;
     __syncthreads();
-    uint32_t* queue = s_queue[wid];
-    uint32_t queued = 0;   // cells in the warp's buffer (below 32 between rounds)
+    uint32_t listed = 0, quads = 0;   // cells in the warp's two buffers (below 32 between rounds)
+    auto put = [&](uint32_t* queue, uint32_t& queued, bool mine, uint32_t c, LineCounter& total, uint32_t* out) {
+        const uint32_t has = __ballot_sync(0xffffffffu, mine);
+        if (mine) queue[queued + __popc(has & ((1u << lane) - 1u))] = c;
+        queued += __popc(has);
+        if (queued >= 32) {
+            __syncwarp();
+            unsigned long long at = 0;
+            if (lane == 0) at = atomicAdd(&total.v, 32ull);
+            out[__shfl_sync(0xffffffffu, at, 0) + lane] = queue[lane];
+            queued -= 32;
+            const uint32_t rest = (uint32_t)lane < queued ? queue[32 + lane] : 0u;
+            __syncwarp();
+            if ((uint32_t)lane < queued) queue[lane] = rest;
+        }
+    };
+    auto flush = [&](const uint32_t* queue, uint32_t queued, LineCounter& total, uint32_t* out) {
+        unsigned long long at = 0;
+        if (lane == 0 && queued) at = atomicAdd(&total.v, (unsigned long long)queued);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if ((uint32_t)lane < queued) out[at + lane] = queue[lane];
+    };
     // A warp takes 128 consecutive cells, 32 at a time, next to the block's other warps (32 when
     // there are too few for every block): its queued cells stay together, and blocks that run at
     // the same time read neighbouring rows (one far-apart range per block: 297 us, 20M points).
@@ -492,7 +516,7 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
     for (uint64_t q0 = (uint64_t)blockIdx.x * span; q0 < M; q0 += (uint64_t)gridDim.x * span)
     for (uint32_t round = 0; round < rounds; ++round) {
         const uint64_t c = q0 + ((uint64_t)wid * rounds + round) * 32 + lane;
-        bool above = false;
+        bool above = false, useful = false;
         uint32_t all[WT];
 #pragma unroll
         for (int w = 0; w < WT; ++w) all[w] = 0;
@@ -535,18 +559,33 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
                     above |= (all[w] & ~((low << 1) - 1u)) != 0;
                 }
             }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
+            // the masks of quad q (empty where the quad leaves the grid)
+            auto quad = [&](int q, uint32_t (&qm)[WT]) {
                 const int qx = (q & 1) - 1, qy = (q >> 1) - 1;
                 const int64_t bx = cx + qx, by = cy + qy;
                 const bool valid = bx >= 0 && by >= 0 && bx + 2 <= (int64_t)g.gx && by + 2 <= (int64_t)g.gy;
-                uint32_t qm[WT];
+                uint32_t n = 0;
 #pragma unroll
-                for (int w = 0; w < WT; ++w)
+                for (int w = 0; w < WT; ++w) {
                     qm[w] = valid ? (m[(qy + 1) * 3 + qx + 1][w] | m[(qy + 1) * 3 + qx + 2][w] |
                                      m[(qy + 2) * 3 + qx + 1][w] | m[(qy + 2) * 3 + qx + 2][w])
                                   : 0u;
-                st_row<WT>(qmask + (c * 4 + q) * WT, qm);
+                    n += __popc(qm[w]);
+                }
+                return n;
+            };
+            uint32_t qm[WT];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) useful |= quad(q, qm) >= quad_min;
+            if (useful) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    quad(q, qm);
+                    st_row<WT>(qmask + (c * 4 + q) * WT, qm);
+                }
+            } else {
+#pragma unroll
+                for (int w = 0; w < WT; ++w) all[w] = 0;   // in no driver list
             }
         }
         // driver-list sizes (lanes of another job than lane 0's, at job boundaries of a
@@ -571,27 +610,17 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
                         atomicAdd(&dcnt[f0 + (uint32_t)w * 32 + (uint32_t)(__ffs(bits) - 1)], 1u);
             }
         }
-        const uint32_t has = __ballot_sync(0xffffffffu, above);
-        if (above) queue[queued + __popc(has & ((1u << lane) - 1u))] = (uint32_t)c;
-        queued += __popc(has);
-        if (queued >= 32) {
+        put(s_queue[wid][0], listed, above, (uint32_t)c, ctrl->nlistq, listq);
+        put(s_queue[wid][1], quads, useful, (uint32_t)c, ctrl->nquadq, quadq);
+        if (several && round + 1 == rounds) {   // the warp's next cells may be another job's
             __syncwarp();
-            unsigned long long at = 0;
-            if (lane == 0) at = atomicAdd(&ctrl->nlistq.v, 32ull);
-            listq[__shfl_sync(0xffffffffu, at, 0) + lane] = queue[lane];
-            queued -= 32;
-            const uint32_t rest = (uint32_t)lane < queued ? queue[32 + lane] : 0u;
-            __syncwarp();
-            if ((uint32_t)lane < queued) queue[lane] = rest;
+            flush(s_queue[wid][1], quads, ctrl->nquadq, quadq);
+            quads = 0;
         }
         __syncwarp();
     }
-    if (queued) {
-        unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(&ctrl->nlistq.v, (unsigned long long)queued);
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if ((uint32_t)lane < queued) listq[at + lane] = queue[lane];
-    }
+    flush(s_queue[wid][0], listed, ctrl->nlistq, listq);
+    flush(s_queue[wid][1], quads, ctrl->nquadq, quadq);
     if (local_hist) {
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < F; i += blockDim.x)
@@ -949,6 +978,7 @@ void lay_cells(Batch& b, Carver& c, uint64_t M, uint64_t R) {
     c.add(b.nb9, M * 9);
     c.add(b.qfirst, M);
     c.add(b.listq, M);
+    c.add(b.quadq, M);
     c.add(b.run_sfx, R);
     c.add(b.run_L, R);
     if (b.row_table) c.add(b.rowstart, b.rows + 1);
@@ -1121,7 +1151,8 @@ void bucket_points(Batch& b) {
             1, std::min<uint64_t>(grid_for(capM, kQuadThreads), (uint64_t)b.sms * (uint64_t)std::max(per_sm, 1))); \
         k_quad_masks<WW><<<qblocks, kQuadThreads, 0, s>>>(                                                   \
             b.ctrl.get(), b.ckey.get(), b.cjob.get(), b.grids.get(), b.nb9.get(), b.cmask.get(),             \
-            b.qmask.get(), b.nbmask.get(), b.listq.get(), b.F, b.dcnt());                          \
+            b.qmask.get(), b.nbmask.get(), b.listq.get(), b.quadq.get(), b.quad_min, b.J > 1, \
+            b.F, b.dcnt());                                                                                  \
     } while (0)
         switch (b.W) {
             case 1: COLO_QM(1); break;

@@ -17,9 +17,9 @@
 //
 // Level k >= 3: a cell is in U_c when one of its four quads is full; the
 // cells tested for c are those with c's driver member (the one with the
-// fewest cells) in their 3x3 block, which holds every cell of U_c.  Those
-// cells are listed once per mine, per feature (driver lists), so a level
-// touches only the lists of its drivers.
+// fewest cells) in their 3x3 block, which holds every cell of U_c, and a quad of
+// three features.  Those cells are listed once per mine, per feature (driver
+// lists), so a level touches only the lists of its drivers.
 #include <algorithm>
 #include <cstring>
 
@@ -143,10 +143,10 @@ __device__ __forceinline__ void load_row(const uint32_t* __restrict__ p, uint32_
 }
 
 // ---- driver lists -----------------------------------------------------------
-// The list of feature f holds the cells whose 3x3 block holds f (bit f of
-// nbmask); the lists of the wanted features (the level drivers) are filled
+// The list of feature f holds the queued cells (quadq) whose 3x3 block holds f (bit
+// f of nbmask); the lists of the wanted features (the level drivers) are filled
 // here, their sizes come from the quad masks' kernel.  A block owns a range of
-// consecutive cells and walks it twice, 256 cells (one per thread) at a time.
+// the queue and walks it twice, 256 cells (one per thread) at a time.
 // A warp's 32 cells are a bit matrix (cell x feature) per mask word;
 // transposed, lane b holds feature b's column.  Pass 0 adds the columns'
 // popcounts to a block histogram; one global atomic per (block, feature) then
@@ -167,7 +167,9 @@ __device__ __forceinline__ uint32_t dil_wanted(const uint32_t* __restrict__ want
 }
 
 template <int WT>
-__global__ void __launch_bounds__(kDilThreads) k_dil_fill(uint64_t M, uint64_t per, const uint32_t* __restrict__ cjob,
+__global__ void __launch_bounds__(kDilThreads) k_dil_fill(uint64_t n, uint64_t per,
+                                                          const uint32_t* __restrict__ quadq,
+                                                          const uint32_t* __restrict__ cjob,
                                                           const JobGrid* __restrict__ grids,
                                                           const uint32_t* __restrict__ nbmask, uint32_t F,
                                                           const uint64_t* __restrict__ doff,
@@ -177,20 +179,22 @@ __global__ void __launch_bounds__(kDilThreads) k_dil_fill(uint64_t M, uint64_t p
     extern __shared__ unsigned long long s_base[];
     uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_base + (F <= kDilHist ? F : 0));
     uint32_t* s_touch = s_cnt + (F <= kDilHist ? F : 0);
-    __shared__ uint32_t s_nt;
+    __shared__ uint32_t s_nt, s_cell[kDilThreads];
     const bool local = F <= kDilHist;
     const uint32_t lane = threadIdx.x & 31;
-    const uint64_t z0 = (uint64_t)blockIdx.x * per, z1 = z0 + per < M ? z0 + per : M;
+    const uint64_t z0 = (uint64_t)blockIdx.x * per, z1 = z0 + per < n ? z0 + per : n;
     if (local)
         for (uint32_t i = threadIdx.x; i < F; i += blockDim.x) s_cnt[i] = 0;
     if (threadIdx.x == 0) s_nt = 0;
     __syncthreads();
     for (int pass = local ? 0 : 1; pass < 2; ++pass) {
         for (uint64_t t0 = z0; t0 < z1; t0 += kDilThreads) {
-            // cell positions in 32 bits (M < 2^32) inside: the loops below are issue-bound
             const bool in = t0 + threadIdx.x < z1;
-            const uint32_t z = (uint32_t)(t0 + threadIdx.x);
-            const uint32_t zw = (uint32_t)(t0 + (threadIdx.x & ~31u));   // the warp's first cell
+            const uint32_t z = in ? quadq[t0 + threadIdx.x] : 0u;
+            const uint32_t* zw = s_cell + (threadIdx.x & ~31u);   // the warp's cells
+            __syncwarp();
+            s_cell[threadIdx.x] = z;
+            __syncwarp();
             uint32_t row[WT];
             uint32_t f0 = 0;
             if (in) {
@@ -203,40 +207,34 @@ __global__ void __launch_bounds__(kDilThreads) k_dil_fill(uint64_t M, uint64_t p
 #pragma unroll
                 for (int w = 0; w < WT; ++w) row[w] = 0;
             }
-            const uint32_t fl = __shfl_sync(0xffffffffu, f0, 0);
-            if (!__all_sync(0xffffffffu, !in || f0 == fl)) {
-                // the warp straddles a job boundary (batches of several jobs): in pass 1 every
-                // lane writes its own entries, one global atomic each
+            // one job's cells at a time (a warp holds cells of several only at the jobs' borders in
+            // the queue)
+            for (uint32_t todo = __ballot_sync(0xffffffffu, in); todo;) {
+                const uint32_t fl = __shfl_sync(0xffffffffu, f0, __ffs(todo) - 1);
+                const bool mine = in && f0 == fl;
+                todo &= ~__ballot_sync(0xffffffffu, mine);
 #pragma unroll
                 for (int w = 0; w < WT; ++w) {
-                    if (pass == 1)
-                        for (uint32_t bits = row[w]; bits; bits &= bits - 1) {
-                            const uint32_t f = f0 + (uint32_t)w * 32 + (uint32_t)(__ffs(bits) - 1);
-                            dlist[doff[f] + atomicAdd(&cursor[f], 1u)] = z;
+                    const uint32_t bits_w = mine ? row[w] : 0u;
+                    if (!__any_sync(0xffffffffu, bits_w)) continue;
+                    const uint32_t col = warp_transpose32(bits_w);
+                    const uint32_t cells = __popc(col);
+                    if (!cells) continue;
+                    const uint32_t f = fl + (uint32_t)w * 32 + lane;
+                    uint64_t o;
+                    if (local) {
+                        const uint32_t old = atomicAdd(&s_cnt[f], cells);
+                        if (pass == 0) {
+                            if (old == 0) s_touch[atomicAdd(&s_nt, 1u)] = f;
+                            continue;
                         }
-                    row[w] = 0;
-                }
-            }
-#pragma unroll
-            for (int w = 0; w < WT; ++w) {
-                if (!__any_sync(0xffffffffu, row[w])) continue;
-                const uint32_t col = warp_transpose32(row[w]);
-                const uint32_t n = __popc(col);
-                if (!n) continue;
-                const uint32_t f = fl + (uint32_t)w * 32 + lane;
-                uint64_t o;
-                if (local) {
-                    const uint32_t old = atomicAdd(&s_cnt[f], n);
-                    if (pass == 0) {
-                        if (old == 0) s_touch[atomicAdd(&s_nt, 1u)] = f;
-                        continue;
+                        o = s_base[f] + old;
+                    } else {
+                        o = doff[f] + atomicAdd(&cursor[f], cells);
                     }
-                    o = s_base[f] + old;
-                } else {
-                    o = doff[f] + atomicAdd(&cursor[f], n);
+                    uint32_t* dst = dlist + o;
+                    for (uint32_t bits = col; bits; bits &= bits - 1) *dst++ = zw[__ffs(bits) - 1];
                 }
-                uint32_t* dst = dlist + o;
-                for (uint32_t bits = col; bits; bits &= bits - 1) *dst++ = zw + (uint32_t)(__ffs(bits) - 1);
             }
         }
         if (pass == 0) {   // reserve the block's ranges; pass 1 counts again from zero
@@ -464,11 +462,12 @@ void driver_lists_fill(Batch& b, const std::vector<uint8_t>& need) {
     do {                                                                                                         \
         int per_sm = 1;                                                                                          \
         COLO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dil_fill<WW>, kDilThreads, dsmem));   \
-        uint64_t blocks = std::min<uint64_t>((b.M + kDilThreads - 1) / kDilThreads,                              \
+        uint64_t blocks = std::min<uint64_t>((b.quad_cells + kDilThreads - 1) / kDilThreads,                              \
                                              (uint64_t)b.sms * (uint64_t)std::max(per_sm, 1));                   \
-        const uint64_t per = ((b.M + blocks - 1) / blocks + kDilThreads - 1) / kDilThreads * kDilThreads;        \
-        blocks = (b.M + per - 1) / per;                                                                          \
-        k_dil_fill<WW><<<(unsigned)blocks, kDilThreads, dsmem, s>>>(b.M, per, b.J > 1 ? b.cjob.get() : nullptr,  \
+        const uint64_t per = ((b.quad_cells + blocks - 1) / blocks + kDilThreads - 1) / kDilThreads * kDilThreads;        \
+        blocks = (b.quad_cells + per - 1) / per;                                                                          \
+        k_dil_fill<WW><<<(unsigned)blocks, kDilThreads, dsmem, s>>>(b.quad_cells, per, b.quadq.get(),            \
+                                                               b.J > 1 ? b.cjob.get() : nullptr,                 \
                                                                b.grids.get(), b.nbmask.get(), b.F, b.doff.get(), \
                                                                d_cursor, b.dlist.get(), d_want);             \
     } while (0)

@@ -712,6 +712,7 @@ void settle(colo_ctx* ctx, Batch& b, std::vector<uint32_t>* ub2) {
                                               " point(s) fall outside the grid derived from the bounds line"};
     b.M = h.M;
     b.Rn = h.Rn;
+    b.quad_cells = h.nquadq.v;
     const uint32_t* counts = reinterpret_cast<const uint32_t*>(back.data() + sizeof(BatchCtrl));
     b.h_dcnt.assign(counts, counts + b.F);
     b.h_frun_off.assign(b.F + 1, 0);

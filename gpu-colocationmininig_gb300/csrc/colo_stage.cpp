@@ -3,6 +3,7 @@
 // (Codes/DeviceProcess.h:4-36).  They run one stage on a dataset and copy
 // its result to host arrays, so each kernel can be checked in isolation.
 #include <algorithm>
+#include <set>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -127,6 +128,12 @@ colo_status colo_stage_filter(colo_ctx* ctx, colo_dataset* ds, float R, float th
         colo_dataset* dsv[1] = {ds};
         setup_batch(ctx, dsv, &p, 1, b, of, nullptr);
         std::vector<uint32_t> h;
+        // a pattern that names a feature more than once needs a quad of fewer
+        for (uint64_t c = 0; c < ncand; ++c) {
+            const uint32_t* mem = cand + c * k;
+            std::set<uint32_t> own(mem, mem + std::min<uint32_t>(k, kMaxMembersFiltered));
+            b.quad_min = std::min(b.quad_min, (uint32_t)own.size());
+        }
         if (b.N) {
             bucket_points(b);
             if (k == 2 && ncand) filter_pairs(b);
