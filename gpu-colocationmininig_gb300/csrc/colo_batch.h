@@ -96,7 +96,7 @@ struct Batch {
     uint64_t rows = 0;           // grid rows of all jobs (row table size - 1)
     bool row_table = false;
     Span<uint32_t> rowstart;     // per grid row: first occupied cell at or after the row (unless too large)
-    Span<int32_t> nb9;
+    Span<uint4> nbrs;            // per cell: its occupied neighbours, stencil columns and quads (k_neighbours)
     Span<uint32_t> cmask;
     Span<uint32_t> nbmask;       // per cell: feature mask of its geometric 3x3 block
     Span<uint32_t> listq;        // cells whose 3x3 block has a feature above their lowest own one
@@ -115,7 +115,6 @@ struct Batch {
     std::vector<uint64_t> h_dcnt;    // cells per feature's list (every feature)
     std::vector<uint64_t> h_doff;    // offsets of the lists filled (features in dlist_have; others empty)
     std::vector<uint8_t> dlist_have; // features whose lists are filled (by the level filters, on demand)
-    Span<uint8_t> qfirst;        // per cell: bit q set when it is the first occupied cell of its quad q
     // runs: run r's points are sorted positions rstart[r] .. rstart[r+1] (rstart has an end entry)
     Span<uint32_t> rfeat, rstart, rcell;
     // neighbourhood lists: for each cell with targets, the points of its adjacent
@@ -151,7 +150,7 @@ struct Batch {
 
 // colo_bucket.cu
 void bucket_layout(Batch& b, Carver& c); // the cleared words of mem0 that bucketing uses, after the upload
-void bucket_points(Batch& b);            // cells, runs, masks, nb9, runs per feature (launches; see bounded)
+void bucket_points(Batch& b);            // cells, runs, masks, neighbours, runs per feature (launches; see bounded)
 void build_neighborhoods(Batch& b);      // neighbourhood lists and anchors (launches)
 // colo_join.cu
 constexpr int kEntrySlots = 64, kEntryStride = 16;   // dE: counters on separate 128-byte lines

@@ -333,44 +333,48 @@ __global__ void k_cell_masks(const BatchCtrl* __restrict__ ctrl, const uint64_t*
     }
 }
 
-// nb9[c*9 + (dy+1)*3 + (dx+1)] = occupied index of the geometric neighbour
-// (cx+dx, cy+dy) inside the job's grid, or -1.  Keys ascend along a grid row,
-// so the row of the cell itself is read from the adjacent entries and each
-// other row needs one lower_bound (above: after c, below: before c).
-//
-// qfirst[c] bit q: c is the first occupied cell of its quad q in (ey, ex)
-// order (the level filter counts each full quad once, at that cell).  Quad q
-// has lower-left cell (cx+qx, cy+qy), qx = (q & 1) - 1, qy = (q >> 1) - 1, and
+// A cell's occupied neighbours (nbrs[c]).  Keys ascend along a grid row, so the up
+// to three neighbours of a row are consecutive cells: x and y are the positions of
+// the first one in the row below (dy = -1) and above, the cell's own row surrounds c.
+//   z bits 0-8    occupied, bit (dy+1)*3 + (dx+1)
+//     bits 9-11   the reference's stencil takes column dx (bit 9 + dx+1)
+//     bits 12-15  c is the first occupied cell of its quad q in (ey, ex) order (the
+//                 level filter counts each full quad once, at that cell)
+//     bits 16-19  quad q lies in the grid
+//   w             the job's first feature
+// Quad q has lower-left cell (cx+qx, cy+qy), qx = (q & 1) - 1, qy = (q >> 1) - 1, and
 // holds c at corner (ex, ey) = (-qx, -qy); quads outside 0 <= bx <= gx-2,
-// 0 <= by <= gy-2 are never full and get no bit.
+// 0 <= by <= gy-2 are never full and are first nowhere.
+//
 // rowstart (optional, rows + 1 entries) bounds the search of a row to the
-// cells of that row.
-__global__ void __launch_bounds__(128, 16) k_nb9(const BatchCtrl* __restrict__ ctrl,
-                      const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob,
-                      const JobGrid* __restrict__ grids, const uint32_t* __restrict__ rowstart,
-                      int32_t* __restrict__ nb9, uint8_t* __restrict__ qfirst) {
+// cells of that row.  Bound by the searches' dependent loads (most of the
+// instructions).  Nine positions and a byte a cell, 37 bytes in strided stores, made
+// this 185 us, the quad masks 201 and the neighbourhood lists 192 at 20M points (8.3M
+// cells); with these 16 bytes they take 167, 162 and 170.
+__global__ void __launch_bounds__(128, 16) k_neighbours(const BatchCtrl* __restrict__ ctrl,
+                                                        const uint64_t* __restrict__ ckey,
+                                                        const uint32_t* __restrict__ cjob,
+                                                        const JobGrid* __restrict__ grids,
+                                                        const uint32_t* __restrict__ rowstart,
+                                                        uint4* __restrict__ nbrs) {
     const uint64_t M = ctrl->M;
     for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < M; c += (uint64_t)gridDim.x * blockDim.x) {
-    const JobGrid g = grids[cjob[c]];
-    const uint64_t key = ckey[c];
-    uint64_t ucx, ucy;
-    cell_col_row(key - g.key_base, g.gx, ucx, ucy);
-    const int64_t cx = (int64_t)ucx, cy = (int64_t)ucy;
-    const int64_t x0 = cx > 0 ? cx - 1 : 0, x1 = cx + 1 < (int64_t)g.gx ? cx + 1 : cx;
-    int32_t* out = nb9 + c * 9;
-    uint32_t occ = 0;   // bit (dy+1)*3 + (dx+1): that neighbour is occupied
-    for (int dy = -1; dy <= 1; ++dy) {
-        int32_t v0 = -1, v1 = -1, v2 = -1;
-        const int64_t ny = cy + dy;
-        if (dy == 0) {
-            v1 = (int32_t)c;
-            if (cx > 0 && c > 0 && ckey[c - 1] == key - 1) v0 = (int32_t)(c - 1);
-            if (cx + 1 < (int64_t)g.gx && c + 1 < M && ckey[c + 1] == key + 1) v2 = (int32_t)(c + 1);
-        } else if (ny >= 0 && ny < (int64_t)g.gy) {
-            const uint64_t k0 = g.key_base + (uint64_t)ny * g.gx + (uint64_t)x0;
-            const uint64_t k1 = g.key_base + (uint64_t)ny * g.gx + (uint64_t)x1;
+        const JobGrid g = grids[cjob[c]];
+        const uint64_t key = ckey[c];
+        uint64_t ucx, ucy;
+        cell_col_row(key - g.key_base, g.gx, ucx, ucy);
+        const int64_t cx = (int64_t)ucx, cy = (int64_t)ucy;
+        const int64_t x0 = cx > 0 ? cx - 1 : 0, x1 = cx + 1 < (int64_t)g.gx ? cx + 1 : cx;
+        uint32_t first[2] = {0, 0}, occ = 1u << 4;
+        if (cx > 0 && c > 0 && ckey[c - 1] == key - 1) occ |= 1u << 3;
+        if (cx + 1 < (int64_t)g.gx && c + 1 < M && ckey[c + 1] == key + 1) occ |= 1u << 5;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int64_t ny = cy + 2 * r - 1;
+            if (ny < 0 || ny >= (int64_t)g.gy) continue;
+            const uint64_t row = g.key_base + (uint64_t)ny * g.gx, k0 = row + (uint64_t)x0, k1 = row + (uint64_t)x1;
             // 32-bit positions (M < 2^32): the search is most of this kernel's instructions
-            uint32_t lo = dy < 0 ? 0u : (uint32_t)c + 1u, hi = dy < 0 ? (uint32_t)c : (uint32_t)M;
+            uint32_t lo = r == 0 ? 0u : (uint32_t)c + 1u, hi = r == 0 ? (uint32_t)c : (uint32_t)M;
             if (rowstart) {
                 const uint64_t Y = g.row_base + (uint64_t)ny;
                 lo = rowstart[Y];
@@ -381,36 +385,43 @@ __global__ void __launch_bounds__(128, 16) k_nb9(const BatchCtrl* __restrict__ c
                 if (ckey[mid] < k0) lo = mid + 1;
                 else hi = mid;
             }
-            for (uint32_t pos = lo; pos < (uint32_t)M && ckey[pos] <= k1; ++pos) {
-                const int64_t dx = (int64_t)(ckey[pos] - g.key_base - (uint64_t)ny * g.gx) - cx;
-                if (dx < 0) v0 = (int32_t)pos;
-                else if (dx == 0) v1 = (int32_t)pos;
-                else v2 = (int32_t)pos;
+            first[r] = lo;
+            for (uint32_t pos = lo; pos < (uint32_t)M; ++pos) {
+                const uint64_t k = ckey[pos];
+                if (k > k1) break;
+                occ |= 1u << (r * 6 + 1 + (int)((int64_t)(k - row) - cx));
             }
         }
-        out[(dy + 1) * 3 + 0] = v0;
-        out[(dy + 1) * 3 + 1] = v1;
-        out[(dy + 1) * 3 + 2] = v2;
-        occ |= ((v0 >= 0 ? 1u : 0u) | (v1 >= 0 ? 2u : 0u) | (v2 >= 0 ? 4u : 0u)) << ((dy + 1) * 3);
-    }
-    uint32_t qf = 0;
+        uint32_t bits = occ;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int qx = (q & 1) - 1, qy = (q >> 1) - 1;
-        const int64_t bx = cx + qx, by = cy + qy;
-        if (!(bx >= 0 && by >= 0 && bx + 2 <= (int64_t)g.gx && by + 2 <= (int64_t)g.gy)) continue;
-        const int ex = -qx, ey = -qy;
-        bool first = true;
+        for (int dx = -1; dx <= 1; ++dx)
+            if (ref_adjacent_col((uint32_t)cx, (uint32_t)(cx + dx), g.gx)) bits |= 1u << (10 + dx);
 #pragma unroll
-        for (int e = 0; e < 3; ++e) {
-            if (e >= ey * 2 + ex) break;
-            const int ox = (e & 1) - ex, oy = (e >> 1) - ey;
-            if (occ >> ((oy + 1) * 3 + (ox + 1)) & 1u) first = false;
+        for (int q = 0; q < 4; ++q) {
+            const int qx = (q & 1) - 1, qy = (q >> 1) - 1;
+            const int64_t bx = cx + qx, by = cy + qy;
+            if (!(bx >= 0 && by >= 0 && bx + 2 <= (int64_t)g.gx && by + 2 <= (int64_t)g.gy)) continue;
+            bits |= 1u << (16 + q);
+            const int ex = -qx, ey = -qy;
+            bool is_first = true;
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                if (e >= ey * 2 + ex) break;
+                const int ox = (e & 1) - ex, oy = (e >> 1) - ey;
+                if (occ >> ((oy + 1) * 3 + (ox + 1)) & 1u) is_first = false;
+            }
+            if (is_first) bits |= 1u << (12 + q);
         }
-        if (first) qf |= 1u << q;
+        nbrs[c] = make_uint4(first[0], first[1], bits, g.f0);
     }
-    qfirst[c] = (uint8_t)qf;
-    }   // cells
+}
+
+// Neighbour q = (dy+1)*3 + (dx+1) of cell c, or -1 (there are fewer than 2^31 cells).
+__device__ __forceinline__ int32_t neighbour(const uint4& v, uint32_t c, int q) {
+    if (!(v.z >> q & 1u)) return -1;
+    const uint32_t before = __popc(v.z & (((1u << (q % 3)) - 1u) << (q / 3 * 3)));
+    const uint32_t at = q < 3 ? v.x : q < 6 ? c - (v.z >> 3 & 1u) : v.y;
+    return (int32_t)(at + before);
 }
 
 // Per cell: the feature masks of the four quads (2x2 cell blocks) containing
@@ -461,7 +472,7 @@ constexpr uint32_t kQuadHist = 1024;
 // quad masks, and the driver-list sizes: dcnt[f] = cells of that queue whose 3x3
 // mask holds f.  Most cells have no such quad (94% at 1M and at 20M points), and
 // no pattern of three is bounded by them: without their 64 bytes of quad masks and
-// their entries in the driver lists this kernel takes 201 us instead of 262 at 20M
+// their entries in the driver lists this kernel took 201 us instead of 262 at 20M
 // points, the lists 27 instead of 157 and the level filters 334 instead of 430.  A block walks spans of consecutive cells (so that
 // queued cells stay near each other: the list kernel reads their neighbourhoods)
 // and keeps one histogram for all of them (one global atomic per
@@ -474,8 +485,7 @@ constexpr uint32_t kQuadHist = 1024;
 // 20M points).
 template <int WT>
 __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
-    BatchCtrl* __restrict__ ctrl, const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob,
-    const JobGrid* __restrict__ grids, const int32_t* __restrict__ nb9, const uint32_t* __restrict__ cmask,
+    BatchCtrl* __restrict__ ctrl, const uint4* __restrict__ nbrs, const uint32_t* __restrict__ cmask,
     uint32_t* __restrict__ qmask, uint32_t* __restrict__ nbmask, uint32_t* __restrict__ listq,
     uint32_t* __restrict__ quadq, uint32_t quad_min, bool several, uint32_t F, uint32_t* __restrict__ dcnt) {
     const uint64_t M = ctrl->M;
@@ -522,14 +532,11 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
         for (int w = 0; w < WT; ++w) all[w] = 0;
         uint32_t f0 = 0;
         if (c < M) {
-            const JobGrid g = grids[cjob[c]];
-            f0 = g.f0;
-            uint64_t ucx, ucy;
-            cell_col_row(ckey[c] - g.key_base, g.gx, ucx, ucy);
-            const int64_t cx = (int64_t)ucx, cy = (int64_t)ucy;
+            const uint4 around = nbrs[c];
+            f0 = around.w;
             int32_t nb[9];
 #pragma unroll
-            for (int q = 0; q < 9; ++q) nb[q] = nb9[c * 9 + q];
+            for (int q = 0; q < 9; ++q) nb[q] = neighbour(around, (uint32_t)c, q);
             uint32_t m[9][WT];
 #pragma unroll
             for (int q = 0; q < 9; ++q) {
@@ -562,8 +569,7 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
             // the masks of quad q (empty where the quad leaves the grid)
             auto quad = [&](int q, uint32_t (&qm)[WT]) {
                 const int qx = (q & 1) - 1, qy = (q >> 1) - 1;
-                const int64_t bx = cx + qx, by = cy + qy;
-                const bool valid = bx >= 0 && by >= 0 && bx + 2 <= (int64_t)g.gx && by + 2 <= (int64_t)g.gy;
+                const bool valid = around.z >> (16 + q) & 1u;
                 uint32_t n = 0;
 #pragma unroll
                 for (int w = 0; w < WT; ++w) {
@@ -636,22 +642,14 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
 // higher features holds exactly the join targets of the run's points.
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ int adjacent_cells(uint64_t c, const uint64_t* ckey, const uint32_t* cjob,
-                                              const JobGrid* grids, const int32_t* nb9,
-                                              int32_t* out) {
-    const JobGrid g = grids[cjob[c]];
-    uint64_t ucx, ucy;
-    cell_col_row(ckey[c] - g.key_base, g.gx, ucx, ucy);
-    const uint32_t cx = (uint32_t)ucx;
+__device__ __forceinline__ int adjacent_cells(uint32_t c, const uint4* __restrict__ nbrs, int32_t* out) {
+    const uint4 around = nbrs[c];
     int cnt = 0;
-    for (int dy = -1; dy <= 1; ++dy)
-        for (int dx = -1; dx <= 1; ++dx) {
-            int32_t v = nb9[c * 9 + (dy + 1) * 3 + (dx + 1)];
-            if (v < 0) continue;
-            uint32_t nx = (uint32_t)((int64_t)cx + dx);
-            if (!ref_adjacent_col(cx, nx, g.gx)) continue;
-            out[cnt++] = v;
-        }
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+        const int32_t v = neighbour(around, c, q);
+        if (v >= 0 && (around.z >> (9 + q % 3) & 1u)) out[cnt++] = v;
+    }
     return cnt;
 }
 
@@ -690,14 +688,13 @@ __device__ __forceinline__ void put_run(uint32_t* __restrict__ targets, uint64_t
 // points before a run are a difference of run starts.  Per own run of the cell:
 // the first target with a higher feature and the targets from there on, from one
 // binary search per slot.
-__device__ __forceinline__ void list_cell_warp(uint64_t c, int lane, uint64_t first, const uint64_t* __restrict__ ckey,
-                                               const uint32_t* __restrict__ cjob, const JobGrid* __restrict__ grids,
-                                               const int32_t* __restrict__ nb9, const uint32_t* __restrict__ crun,
+__device__ __forceinline__ void list_cell_warp(uint32_t c, int lane, uint64_t first,
+                                               const uint4* __restrict__ nbrs, const uint32_t* __restrict__ crun,
                                                const uint32_t* __restrict__ rfeat, const uint32_t* __restrict__ rstart,
                                                const uint32_t* __restrict__ ids, uint32_t* __restrict__ targets,
                                                uint64_t* run_sfx, uint32_t* run_L) {
     int32_t adj[9];
-    const int na = adjacent_cells(c, ckey, cjob, grids, nb9, adj);
+    const int na = adjacent_cells(c, nbrs, adj);
     const uint32_t fmin = rfeat[crun[c]];
     uint32_t q0[9], q1[9], pre[10];   // kept runs of each slot, and their number before it
     uint64_t total = 0;
@@ -775,8 +772,7 @@ __device__ __forceinline__ void list_cell_warp(uint64_t c, int lane, uint64_t fi
 // the kernel again with room for all.
 __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
     uint64_t npoints, const uint32_t* __restrict__ listq, BatchCtrl* __restrict__ ctrl,
-    const uint64_t* __restrict__ ckey, const uint32_t* __restrict__ cjob, const JobGrid* __restrict__ grids,
-    const int32_t* __restrict__ nb9, const uint32_t* __restrict__ crun, const uint32_t* __restrict__ rfeat,
+    const uint4* __restrict__ nbrs, const uint32_t* __restrict__ crun, const uint32_t* __restrict__ rfeat,
     const uint32_t* __restrict__ rstart, const uint32_t* __restrict__ ids, uint64_t cap,
     uint32_t* __restrict__ targets, uint64_t* run_sfx, uint32_t* run_L, uint4* __restrict__ act) {
     const uint32_t n = (uint32_t)ctrl->nlistq.v;
@@ -806,7 +802,7 @@ __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
             r1 = crun[c + 1];
             const uint32_t fmin = rfeat[r0];
             int32_t adj[9];
-            const int na = adjacent_cells(c, ckey, cjob, grids, nb9, adj);
+            const int na = adjacent_cells(c, nbrs, adj);
 #pragma unroll
             for (int t = 0; t < 9; ++t)
                 if (t < na) {
@@ -876,7 +872,7 @@ __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
             const int j = __ffs(m) - 1;
             const uint32_t cj = __shfl_sync(0xffffffffu, c, j);
             const uint64_t fj = __shfl_sync(0xffffffffu, first, j);
-            list_cell_warp(cj, lane, fj, ckey, cjob, grids, nb9, crun, rfeat, rstart, ids, targets, run_sfx, run_L);
+            list_cell_warp(cj, lane, fj, nbrs, crun, rfeat, rstart, ids, targets, run_sfx, run_L);
         }
         __syncwarp();
         // anchors: the points of own runs with targets, short lists and long ones
@@ -975,8 +971,7 @@ void lay_cells(Batch& b, Carver& c, uint64_t M, uint64_t R) {
     c.add(b.cmask, M * b.W);
     c.add(b.nbmask, M * b.W);
     c.add(b.qmask, M * 4 * b.W);
-    c.add(b.nb9, M * 9);
-    c.add(b.qfirst, M);
+    c.add(b.nbrs, M);
     c.add(b.listq, M);
     c.add(b.quadq, M);
     c.add(b.run_sfx, R);
@@ -1135,8 +1130,8 @@ void bucket_points(Batch& b) {
     {
         KScope ks("cell_neighbours");
         const unsigned grid = (unsigned)std::min<uint64_t>(grid_for(capM, 128), (uint64_t)b.sms * 64);
-        k_nb9<<<grid, 128, 0, s>>>(b.ctrl.get(), b.ckey.get(), b.cjob.get(), b.grids.get(),
-                                   b.row_table ? b.rowstart.get() : nullptr, b.nb9.get(), b.qfirst.get());
+        k_neighbours<<<grid, 128, 0, s>>>(b.ctrl.get(), b.ckey.get(), b.cjob.get(), b.grids.get(),
+                                          b.row_table ? b.rowstart.get() : nullptr, b.nbrs.get());
         COLO_LAUNCH_CHECK();
         count_launch();
     }
@@ -1150,9 +1145,8 @@ void bucket_points(Batch& b) {
         const unsigned qblocks = (unsigned)std::max<uint64_t>(                                               \
             1, std::min<uint64_t>(grid_for(capM, kQuadThreads), (uint64_t)b.sms * (uint64_t)std::max(per_sm, 1))); \
         k_quad_masks<WW><<<qblocks, kQuadThreads, 0, s>>>(                                                   \
-            b.ctrl.get(), b.ckey.get(), b.cjob.get(), b.grids.get(), b.nb9.get(), b.cmask.get(),             \
-            b.qmask.get(), b.nbmask.get(), b.listq.get(), b.quadq.get(), b.quad_min, b.J > 1, \
-            b.F, b.dcnt());                                                                                  \
+            b.ctrl.get(), b.nbrs.get(), b.cmask.get(), b.qmask.get(), b.nbmask.get(), b.listq.get(),         \
+            b.quadq.get(), b.quad_min, b.J > 1, b.F, b.dcnt());                                              \
     } while (0)
         switch (b.W) {
             case 1: COLO_QM(1); break;
@@ -1189,8 +1183,8 @@ void build_neighborhoods(Batch& b) {
     b.lists_built = true;
     const unsigned qgrid = (unsigned)std::min<uint64_t>(grid_for(b.capM, 128), (uint64_t)b.sms * 16);
     KScope ks("neighbour_lists");
-    k_neighbour_lists<<<qgrid, 128, 0, s>>>(b.N, b.listq.get(), b.ctrl.get(), b.ckey.get(), b.cjob.get(),
-                                            b.grids.get(), b.nb9.get(), b.crun.get(), b.rfeat.get(), b.rstart.get(),
+    k_neighbour_lists<<<qgrid, 128, 0, s>>>(b.N, b.listq.get(), b.ctrl.get(), b.nbrs.get(), b.crun.get(),
+                                            b.rfeat.get(), b.rstart.get(),
                                             b.gathered ? nullptr : b.sid.get(), b.targets_cap, b.targets.get(), b.run_sfx.get(), b.run_L.get(),
                                             b.act.get());
     COLO_LAUNCH_CHECK();

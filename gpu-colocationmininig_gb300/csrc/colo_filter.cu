@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kDilThreads) k_dil_fill(uint64_t n, uint64_t p
 // candidates; a (cell Z, candidate c) pair is tested exactly as in a scan
 // of every cell with the driver in its 3x3 block: Z is in U_c when one of
 // its four quads covers c's members, each cell of U_c is met once, and a
-// full quad is counted at its first occupied cell (qfirst).  Lane t loads the
+// full quad is counted at its first occupied cell (nbrs).  Lane t loads the
 // unit's candidate t up front (a candidate then comes by shuffles, not by
 // dependent loads), and a candidate's counts are summed over the warp's cells
 // before one atomic per sum, into a block-private accumulator when the level's
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(256, (WT <= 4 ? 5 : (WT <= 6 ? 4 : (WT <= 8 ? 
     const uint32_t* __restrict__ gstart, const uint32_t* __restrict__ gcount, const uint64_t* __restrict__ doff,
     const uint32_t* __restrict__ dlist, const uint32_t* __restrict__ order, const uint32_t* __restrict__ need_all,
     const uint32_t* __restrict__ lmem, uint32_t k, const uint32_t* __restrict__ qmask,
-    const uint32_t* __restrict__ cmask, const uint32_t* __restrict__ crun, const uint8_t* __restrict__ qfirst,
+    const uint32_t* __restrict__ cmask, const uint32_t* __restrict__ crun, const uint4* __restrict__ nbrs,
     const uint32_t* __restrict__ rstart, uint32_t* __restrict__ ub, unsigned long long* __restrict__ stats,
     uint32_t acc_n, uint32_t cu) {
     constexpr uint32_t W = WT;
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(256, (WT <= 4 ? 5 : (WT <= 6 ? 4 : (WT <= 8 ? 
             }
             load_row<WT>(cmask + Z * W, cm);
             q0 = crun[Z];
-            qf = qfirst[Z];
+            qf = nbrs[Z].z >> 12 & 15u;
         }
         // lane t: the unit's candidate t
         const uint32_t t0 = gc * cu, cnt = t0 + cu < G ? cu : G - t0;
@@ -610,7 +610,7 @@ void filter_level(Batch& b, const uint32_t* h_cand, const uint32_t* h_job, uint6
 #define COLO_FL(WW)                                                                                             \
     k_filter_drv<WW><<<grid((const void*)k_filter_drv<WW>), 256, smem, s>>>(                                    \
         nunits, ngroups, d_uoff, d_gfeat, d_gstart, d_gcount, b.doff.get(), b.dlist.get(), d_order, d_need,       \
-        d_lmem, k, b.qmask.get(), b.cmask.get(), b.crun.get(), b.qfirst.get(), b.rstart.get(), d_ub, d_stats, acc_n, cu)
+        d_lmem, k, b.qmask.get(), b.cmask.get(), b.crun.get(), b.nbrs.get(), b.rstart.get(), d_ub, d_stats, acc_n, cu)
     COLO_W_SWITCH(b.W, COLO_FL)
 #undef COLO_FL
     COLO_LAUNCH_CHECK();

@@ -9,7 +9,7 @@
 //   bucketed    points sorted by (job cell key, point id): sid, and
 //               with gathered coordinates sxy (sfeat for several jobs)
 //   cells       occupied cells ckey[M], cstart[M+1] (sorted positions),
-//               crun[M+1] (run ranges), nb9[M*9] (geometric 3x3 neighbours),
+//               crun[M+1] (run ranges), nbrs[M] (geometric 3x3 neighbours),
 //               cmask[M*W] (feature bit masks, local feature index),
 //               qmask[M*4*W] (masks of the 4 quads containing the cell)
 //   runs        (cell, feature) runs rfeat/rstart/rcnt/rcell[Rn], cell-major;
