@@ -33,6 +33,7 @@ struct alignas(128) BatchCtrl {
     uint32_t keys_done;          // blocks of the cell-key pass that have added their histograms
     LineCounter nlistq;          // cells queued for a neighbourhood run list
     LineCounter nquadq;          // cells with a quad of quad_min features or more
+    LineCounter npairq;          // with pairq: cells with two features or more in their 3x3 block
     // neighbourhood lists: target points, runs, anchors with short and with long lists, and the
     // pair evaluations (= room that the single-pass join may need)
     LineCounter targets, list_runs, anchors, long_anchors, pairs;
@@ -98,7 +99,11 @@ struct Batch {
     Span<uint32_t> rowstart;     // per grid row: first occupied cell at or after the row (unless too large)
     Span<uint4> nbrs;            // per cell: its occupied neighbours, stencil columns and quads (k_neighbours)
     Span<uint32_t> cmask;
-    Span<uint32_t> nbmask;       // per cell: feature mask of its geometric 3x3 block
+    // feature mask of a cell's geometric 3x3 block (with pairq: of its cells and of quadq's only)
+    Span<uint32_t> nbmask;
+    // the cells with two features or more there: one job of kPairQueuePoints points or more
+    bool pair_queue = false;
+    Span<uint32_t> pairq;
     Span<uint32_t> listq;        // cells whose 3x3 block has a feature above their lowest own one
     // per cell of quadq: masks of the 4 quads containing it ([M][4][W], other cells' rows unwritten)
     Span<uint32_t> qmask;

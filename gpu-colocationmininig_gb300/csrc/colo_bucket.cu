@@ -128,6 +128,9 @@ __global__ void __launch_bounds__(256, 4) k_cell_keys(
 // After a sort that timed out the keys are not a sorted permutation: nothing
 // is written, the totals stay zero and every later kernel finds no cells.  A
 // look-back that waits too long counts the heads before its tile itself.
+// A queue of cells for the pairs' bounds costs the quad masks up to 4 us and pays from here on: 2M
+// points 41 -> 35 us for the two kernels, 4M 84 -> 65, 20M 319 -> 232; 1M 29 -> 33.
+constexpr uint64_t kPairQueuePoints = 1ull << 21;
 constexpr uint64_t kGatherPoints = 1ull << 23;   // 64 MiB of coordinates, half of L2
 constexpr int kHeadThreads = 256, kHeadRounds = 8, kHeadTile = kHeadThreads * kHeadRounds;
 constexpr int kHeadWarps = kHeadThreads / 32;
@@ -487,16 +490,16 @@ template <int WT>
 __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
     BatchCtrl* __restrict__ ctrl, const uint4* __restrict__ nbrs, const uint32_t* __restrict__ cmask,
     uint32_t* __restrict__ qmask, uint32_t* __restrict__ nbmask, uint32_t* __restrict__ listq,
-    uint32_t* __restrict__ quadq, uint32_t quad_min, bool several, uint32_t F, uint32_t* __restrict__ dcnt) {
+    uint32_t* __restrict__ quadq, uint32_t* __restrict__ pairq, uint32_t quad_min, bool several, uint32_t F, uint32_t* __restrict__ dcnt) {
     const uint64_t M = ctrl->M;
     __shared__ uint32_t s_hist[kQuadHist];
-    __shared__ uint32_t s_queue[kQuadThreads / 32][2][64];
+    __shared__ uint32_t s_queue[kQuadThreads / 32][3][64];
     const bool local_hist = F <= kQuadHist;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (local_hist)
         for (uint32_t i = threadIdx.x; i < F; i += blockDim.x) s_hist[i] = 0;
     __syncthreads();
-    uint32_t listed = 0, quads = 0;   // cells in the warp's two buffers (below 32 between rounds)
+    uint32_t listed = 0, quads = 0, pairs = 0;   // cells in the warp's buffers (below 32 between rounds)
     auto put = [&](uint32_t* queue, uint32_t& queued, bool mine, uint32_t c, LineCounter& total, uint32_t* out) {
         const uint32_t has = __ballot_sync(0xffffffffu, mine);
         if (mine) queue[queued + __popc(has & ((1u << lane) - 1u))] = c;
@@ -526,7 +529,7 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
     for (uint64_t q0 = (uint64_t)blockIdx.x * span; q0 < M; q0 += (uint64_t)gridDim.x * span)
     for (uint32_t round = 0; round < rounds; ++round) {
         const uint64_t c = q0 + ((uint64_t)wid * rounds + round) * 32 + lane;
-        bool above = false, useful = false;
+        bool above = false, useful = false, paired = false;
         uint32_t all[WT];
 #pragma unroll
         for (int w = 0; w < WT; ++w) all[w] = 0;
@@ -549,7 +552,10 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
 #pragma unroll
                 for (int w = 0; w < WT; ++w) all[w] |= m[q][w];
             }
-            st_row<WT>(nbmask + c * WT, all);
+            uint32_t feats = 0;
+#pragma unroll
+            for (int w = 0; w < WT; ++w) feats += __popc(all[w]);
+            paired = feats >= 2;
             // the cell needs a neighbourhood run list when its 3x3 block holds a
             // feature above its own lowest one (m[4] is the cell's own mask; the block
             // is the union over all nine slots, a superset of the adjacent cells):
@@ -583,6 +589,8 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
             uint32_t qm[WT];
 #pragma unroll
             for (int q = 0; q < 4; ++q) useful |= quad(q, qm) >= quad_min;
+            // the readers: the driver lists (queued quads) and the pairs (queued pairs, or every run)
+            if (!pairq || paired || useful) st_row<WT>(nbmask + c * WT, all);
             if (useful) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
@@ -618,6 +626,7 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
         }
         put(s_queue[wid][0], listed, above, (uint32_t)c, ctrl->nlistq, listq);
         put(s_queue[wid][1], quads, useful, (uint32_t)c, ctrl->nquadq, quadq);
+        if (pairq) put(s_queue[wid][2], pairs, paired, (uint32_t)c, ctrl->npairq, pairq);
         if (several && round + 1 == rounds) {   // the warp's next cells may be another job's
             __syncwarp();
             flush(s_queue[wid][1], quads, ctrl->nquadq, quadq);
@@ -627,6 +636,7 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
     }
     flush(s_queue[wid][0], listed, ctrl->nlistq, listq);
     flush(s_queue[wid][1], quads, ctrl->nquadq, quadq);
+    if (pairq) flush(s_queue[wid][2], pairs, ctrl->npairq, pairq);
     if (local_hist) {
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < F; i += blockDim.x)
@@ -974,6 +984,7 @@ void lay_cells(Batch& b, Carver& c, uint64_t M, uint64_t R) {
     c.add(b.nbrs, M);
     c.add(b.listq, M);
     c.add(b.quadq, M);
+    if (b.pair_queue) c.add(b.pairq, M);
     c.add(b.run_sfx, R);
     c.add(b.run_L, R);
     if (b.row_table) c.add(b.rowstart, b.rows + 1);
@@ -1088,6 +1099,7 @@ void bucket_points(Batch& b) {
     b.nb_cap = neighbour_room(n);
     b.row_table = wants_row_table(b, n);
     b.gathered = b.J > 1 || n <= kGatherPoints;
+    b.pair_queue = b.J == 1 && n >= kPairQueuePoints;
     auto bounds = [&](Carver& c) {
         lay_points(b, c);
         lay_heads(b, c, n, n);
@@ -1146,7 +1158,7 @@ void bucket_points(Batch& b) {
             1, std::min<uint64_t>(grid_for(capM, kQuadThreads), (uint64_t)b.sms * (uint64_t)std::max(per_sm, 1))); \
         k_quad_masks<WW><<<qblocks, kQuadThreads, 0, s>>>(                                                   \
             b.ctrl.get(), b.nbrs.get(), b.cmask.get(), b.qmask.get(), b.nbmask.get(), b.listq.get(),         \
-            b.quadq.get(), b.quad_min, b.J > 1, b.F, b.dcnt());                                              \
+            b.quadq.get(), b.pair_queue ? b.pairq.get() : nullptr, b.quad_min, b.J > 1, b.F, b.dcnt());                               \
     } while (0)
         switch (b.W) {
             case 1: COLO_QM(1); break;

@@ -100,6 +100,60 @@ __global__ void __launch_bounds__(kFilterThreads) k_filter_pairs(
     }
 }
 
+// The same for one job of many points: over the runs of the queued cells (two features or more in
+// their 3x3 block; the others are in no pair's bound).  A warp takes 32 cells of
+// the queue and their runs one after another, a run a lane, so a cell of many runs costs as
+// much a run as one of few.  Bound by the masks' loads and the shared atomics; a thread for
+// each of all runs took 157 us at 20M points (8.9M runs, one cell in nine queued), this 67.
+__global__ void __launch_bounds__(kFilterThreads) k_filter_pairs_queue(
+    const BatchCtrl* __restrict__ ctrl, const uint32_t* __restrict__ pairq, const uint32_t* __restrict__ crun,
+    const JobGrid* __restrict__ grids, const uint32_t* __restrict__ nbmask, uint32_t W,
+    const uint32_t* __restrict__ rfeat, const uint32_t* __restrict__ rstart, uint32_t* __restrict__ ub2,
+    uint32_t acc_dim) {
+    extern __shared__ uint32_t acc[];   // acc_dim x acc_dim, acc_dim the job's features or 0 (no privatisation)
+    const JobGrid& g = grids[0];
+    if (g.gx < 2 || g.gy < 2) return;
+    const uint32_t nf = g.nf, accn = acc_dim * acc_dim;
+    for (uint32_t i = threadIdx.x; i < accn; i += blockDim.x) acc[i] = 0;
+    __syncthreads();
+    const uint64_t n = ctrl->npairq.v;
+    const int lane = threadIdx.x & 31;
+    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    for (uint64_t i0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; i0 < n; i0 += warps * 32) {
+        uint32_t c = 0, r0 = 0, runs = 0;
+        if (i0 + lane < n) {
+            c = pairq[i0 + lane];
+            r0 = crun[c];
+            runs = crun[c + 1] - r0;
+        }
+        const uint32_t incl = warp_incl_scan(runs), excl = incl - runs;
+        const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
+        for (uint32_t t0 = 0; t0 < tot; t0 += 32) {
+            const uint32_t t = t0 + lane;
+            int j = 0;
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1) {
+                const uint32_t ev = __shfl_sync(0xffffffffu, excl, j + step);
+                if (ev <= t) j += step;
+            }
+            const uint32_t cj = __shfl_sync(0xffffffffu, c, j);
+            const uint32_t r = __shfl_sync(0xffffffffu, r0 - excl, j) + t;
+            if (t >= tot) continue;
+            const uint32_t lf = rfeat[r], cnt = rstart[r + 1] - rstart[r];
+            for (uint32_t w = 0; w < W; ++w)
+                for (uint32_t bits = nbmask[(uint64_t)cj * W + w]; bits; bits &= bits - 1) {
+                    const uint32_t lg = w * 32 + (uint32_t)(__ffs(bits) - 1);
+                    if (lg == lf) continue;
+                    if (acc_dim) atomicAdd(&acc[lf * acc_dim + lg], cnt);
+                    else atomicAdd(&ub2[(uint64_t)lf * nf + lg], cnt);
+                }
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < accn; i += blockDim.x)
+        if (acc[i]) atomicAdd(&ub2[i], acc[i]);
+}
+
 template <int WT>
 __device__ __forceinline__ bool covers(const uint32_t* __restrict__ qm, const uint32_t (&need)[WT]) {
     bool ok = true;
@@ -489,7 +543,8 @@ void filter_pairs(Batch& b) {
         smem = 0;
     }
     if (smem > 48 * 1024)
-        COLO_CUDA(cudaFuncSetAttribute(k_filter_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        COLO_CUDA(cudaFuncSetAttribute(b.pair_queue ? (const void*)k_filter_pairs_queue : (const void*)k_filter_pairs,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // as many resident blocks per SM as the accumulator allows (at most 8), each with its share of the runs
     uint64_t per_sm = smem ? (200 * 1024) / smem : 8;
     if (per_sm < 1) per_sm = 1;
@@ -497,6 +552,14 @@ void filter_pairs(Batch& b) {
     const uint64_t blocks = std::min<uint64_t>((uint64_t)b.sms * per_sm, (b.capR + kFilterThreads - 1) / kFilterThreads);
     if (!blocks) return;
     KScope ks("filter_pairs");
+    if (b.pair_queue) {
+        k_filter_pairs_queue<<<(unsigned)blocks, kFilterThreads, smem, s>>>(
+            b.ctrl.get(), b.pairq.get(), b.crun.get(), b.grids.get(), b.nbmask.get(), b.W, b.rfeat.get(),
+            b.rstart.get(), b.ub2(), acc_dim);
+        COLO_LAUNCH_CHECK();
+        count_launch();
+        return;
+    }
     k_filter_pairs<<<(unsigned)blocks, kFilterThreads, smem, s>>>(
         b.ctrl.get(), b.rcell.get(), b.J > 1 ? b.cjob.get() : nullptr, b.grids.get(), b.nbmask.get(), b.W,
         b.rfeat.get(), b.rstart.get(), b.job_off.get(), b.ub2(), acc_dim);

@@ -70,3 +70,23 @@ def test_jobs_that_share_warps(ctx, jobs):
     got = ctx.mine_batch(dss, [colo.default_params(w.R, w.thr, max_size=w.max_size) for w in wls])
     for w, r in zip(wls, got):
         assert_same_trace(r, oracle_for(ctx, w))
+
+
+@pytest.mark.parametrize("n", [(1 << 21) - 1, 1 << 21])
+@pytest.mark.parametrize("features", [6, 300])
+def test_pairs_on_both_sides_of_the_queue(ctx, n, features):
+    """From 2^21 points on a single job's pairs are bounded over a queue of cells, else over every run (as beside a
+    second job): the same bounds, with block-private sums and without, and a spot of cells with many runs."""
+    rng = np.random.default_rng(n + features)
+    x, y = (rng.random(n, np.float32) * 2000 for _ in range(2))
+    fid = np.sort(rng.integers(0, features, n, np.int32))
+    spot = rng.choice(n, 4000, replace=False)
+    x[spot], y[spot] = (rng.normal(700, 1.5, 4000).astype(np.float32) for _ in range(2))
+    box = np.array([0, 0, 2000, 2000], np.float32)
+    ds = colo.Dataset.from_arrays(ctx, x, y, fid, box)
+    few = colo.Dataset.from_arrays(ctx, x[:50], y[:50], np.zeros(50, np.int32), box)
+    p = colo.default_params(0.5, 0.9, max_size=2)
+    alone, beside = ctx.mine(ds, p), ctx.mine_batch([ds, few], [p, p])[0]
+    assert len(alone.levels) == 1 and alone.levels[0].ub.any()
+    for f in ("cand", "ub", "passed", "rows", "num", "pi"):
+        assert np.array_equal(getattr(alone.levels[0], f), getattr(beside.levels[0], f)), f
