@@ -193,20 +193,18 @@ def algorithmic_bytes(name: str, c: dict, launches: float, words: int) -> float:
     kb = 4.0 if c.get("key_bits", 64) <= 32 else 8.0   # cell keys are 32-bit when every key fits
     if name == "radix_sort":       # per digit pass over the points: read and write the key and the 4 B id
         return 2.0 * (kb + 4.0) * N * launches
-    if name == "radix_hist":       # one read of the keys for every pass's digit histogram
-        return kb * N
-    if name == "run_sort":         # per digit pass over the runs
-        return 24.0 * Rn * launches
     if name == "cell_keys":        # read x, y, feature; write key, id
         return 24.0 * N
-    if name == "gather_sorted":    # read the sorted ids and keys, gather x, y, write x, y, feature in cell order
-        return (28.0 + kb) * N
-    if name == "cell_neighbours":  # read the key, write 9 neighbour indices
-        return 44.0 * M
-    if name == "quad_masks":       # read 9 indices + masks, write 4 quad masks + the 3x3 union
-        return 36.0 * M + 4.0 * words * M * 6
-    if name == "nrl_fill":         # write the run per list entry + per-run suffix and count
-        return 4.0 * c["nrl_entries"] + 12.0 * Rn
+    if name == "cell_heads":       # read the sorted ids and keys (up to 2^23 points also gather x, y), write cells and runs
+        return (4.0 + kb + (16.0 if N <= 1 << 23 else 0.0)) * N + 24.0 * M + 12.0 * Rn
+    if name == "cell_masks":       # read the runs' features, write the cells' masks
+        return 4.0 * Rn + 4.0 * words * M
+    if name == "cell_neighbours":  # read the key and the job, write the neighbour word
+        return 28.0 * M
+    if name == "quad_masks":       # read the neighbour word and the masks (few cells write theirs)
+        return 16.0 * M + 4.0 * words * M
+    if name == "neighbour_lists":  # write a point or more per run listed, the runs' suffixes, the anchors
+        return 4.0 * c["nrl_entries"] + 12.0 * Rn + 16.0 * c["active_anchors"]
     if name == "join":             # B_b = 12 N + 4 E + 8 (N + 1): points once, lists and offsets written
         return 12.0 * N + 4.0 * E + 8.0 * (N + 1)
     if name in ("join_count", "join_fill"):   # the same split over the two-pass layout

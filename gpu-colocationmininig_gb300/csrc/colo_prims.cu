@@ -133,9 +133,9 @@ struct SortSmem {
 // (the host reports COLO_ERR_TIMEOUT).  The key's bits are split evenly over
 // the fewest passes of at most 8 bits (narrower digits leave more keys per digit in
 // a tile, so the scatter writes longer runs), or of at most 9 where that saves a
-// pass: 25 bits in 4 passes of 7 or less take 80 us for 1M points, in 3 of 9 or less
-// 68; 33 bits of 2M 155 us in 5, 139 in 4; where both take as many (20M points,
-// 28 bits) the wide digits gain nothing.
+// pass: 25 to 27 bits take 80 us in 4 passes for 1M points, 68 in 3; 33 to 36 bits of 2M
+// points 155 us in 5, 139 in 4; where both take as many (20M points, 32 bits) wide digits
+// gain nothing.
 //
 // A key's peers in its warp (the lanes with its digit) come from one ballot per bit:
 // match_any over the digit took 8% longer (20M points: 688 -> 636 us a sort).

@@ -132,7 +132,8 @@ colo_status colo_csv_to_binary(const char* csv_path, const char* bin_path, uint3
  * (initializeDeviceMemory, colocationFinder.cpp:443-464).  Otherwise a mine of
  * one dataset page-locks and maps the host arrays and its cell-key pass reads
  * them over the host link (no device copy is kept); a batch of several
- * datasets copies them. */
+ * datasets reads them there too where the device can read pageable host
+ * memory, and copies them elsewhere. */
 colo_status colo_dataset_upload(colo_dataset* ds);
 /* Drop the device copy (the next mine reads the host arrays again). */
 colo_status colo_dataset_evict(colo_dataset* ds);
