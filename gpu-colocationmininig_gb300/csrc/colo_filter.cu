@@ -29,7 +29,7 @@
 namespace colo {
 namespace {
 
-constexpr int kFilterThreads = 256;
+constexpr int kFilterThreads = 256, kPairThreads = 1024;   // a pair block: 256 to 1024 threads
 constexpr int kMaxW = 32;  // mask words per cell (1024 features per job); rows of 9+ words are padded
                            // to 12, 16, 24 or 32 words when the batch is set up
 constexpr uint64_t kAccMax = 16384;   // block-private level sums (64 KB of shared memory)
@@ -38,7 +38,7 @@ constexpr uint64_t kAccMax = 16384;   // block-private level sums (64 KB of shar
 // job changes rarely and the F x F accumulator lives in shared memory.  cjob is
 // null for a one-job batch (job 0 everywhere): the mask load then waits on one
 // dependent load (the run's cell) instead of three.
-__global__ void __launch_bounds__(kFilterThreads) k_filter_pairs(
+__global__ void __launch_bounds__(kPairThreads) k_filter_pairs(
     const BatchCtrl* __restrict__ ctrl, const uint32_t* __restrict__ rcell, const uint32_t* __restrict__ cjob,
     const JobGrid* __restrict__ grids, const uint32_t* __restrict__ nbmask,
     uint32_t W, const uint32_t* __restrict__ rfeat, const uint32_t* __restrict__ rstart,
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kFilterThreads) k_filter_pairs(
 // the queue and their runs one after another, a run a lane, so a cell of many runs costs as
 // much a run as one of few.  Bound by the masks' loads and the shared atomics; a thread for
 // each of all runs took 157 us at 20M points (8.9M runs, one cell in nine queued), this 67.
-__global__ void __launch_bounds__(kFilterThreads) k_filter_pairs_queue(
+__global__ void __launch_bounds__(kPairThreads) k_filter_pairs_queue(
     const BatchCtrl* __restrict__ ctrl, const uint32_t* __restrict__ pairq, const uint32_t* __restrict__ crun,
     const JobGrid* __restrict__ grids, const uint32_t* __restrict__ nbmask, uint32_t W,
     const uint32_t* __restrict__ rfeat, const uint32_t* __restrict__ rstart, uint32_t* __restrict__ ub2,
@@ -545,22 +545,27 @@ void filter_pairs(Batch& b) {
     if (smem > 48 * 1024)
         COLO_CUDA(cudaFuncSetAttribute(b.pair_queue ? (const void*)k_filter_pairs_queue : (const void*)k_filter_pairs,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // as many resident blocks per SM as the accumulator allows (at most 8), each with its share of the runs
-    uint64_t per_sm = smem ? (200 * 1024) / smem : 8;
-    if (per_sm < 1) per_sm = 1;
-    if (per_sm > 8) per_sm = 8;
-    const uint64_t blocks = std::min<uint64_t>((uint64_t)b.sms * per_sm, (b.capR + kFilterThreads - 1) / kFilterThreads);
+    // as many resident threads per SM as the accumulators leave: blocks of 256 threads where eight
+    // fit (each with its share of the runs), larger ones where the accumulator is large
+    // (200 features, 160 KB, one block an SM: 72 -> 31 us; 100 features, 40 KB, 20M points: 66 -> 48)
+    const uint64_t fit = smem ? std::max<uint64_t>(1, (200 * 1024) / smem) : 8;
+    unsigned threads = kFilterThreads;
+    auto resident = [&](unsigned t) { return std::min<uint64_t>(fit, 2048 / t) * t; };
+    for (unsigned t = 2 * kFilterThreads; t <= (unsigned)kPairThreads; t *= 2)
+        if (resident(t) > resident(threads)) threads = t;
+    const uint64_t per_sm = std::min<uint64_t>(fit, 2048 / threads);
+    const uint64_t blocks = std::min<uint64_t>((uint64_t)b.sms * per_sm, (b.capR + threads - 1) / threads);
     if (!blocks) return;
     KScope ks("filter_pairs");
     if (b.pair_queue) {
-        k_filter_pairs_queue<<<(unsigned)blocks, kFilterThreads, smem, s>>>(
+        k_filter_pairs_queue<<<(unsigned)blocks, threads, smem, s>>>(
             b.ctrl.get(), b.pairq.get(), b.crun.get(), b.grids.get(), b.nbmask.get(), b.W, b.rfeat.get(),
             b.rstart.get(), b.ub2(), acc_dim);
         COLO_LAUNCH_CHECK();
         count_launch();
         return;
     }
-    k_filter_pairs<<<(unsigned)blocks, kFilterThreads, smem, s>>>(
+    k_filter_pairs<<<(unsigned)blocks, threads, smem, s>>>(
         b.ctrl.get(), b.rcell.get(), b.J > 1 ? b.cjob.get() : nullptr, b.grids.get(), b.nbmask.get(), b.W,
         b.rfeat.get(), b.rstart.get(), b.job_off.get(), b.ub2(), acc_dim);
     COLO_LAUNCH_CHECK();

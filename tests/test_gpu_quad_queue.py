@@ -90,3 +90,17 @@ def test_pairs_on_both_sides_of_the_queue(ctx, n, features):
     assert len(alone.levels) == 1 and alone.levels[0].ub.any()
     for f in ("cand", "ub", "passed", "rows", "num", "pi"):
         assert np.array_equal(getattr(alone.levels[0], f), getattr(beside.levels[0], f)), f
+
+
+@pytest.mark.parametrize("features", [79, 80, 81, 113, 114, 160, 161, 226, 227])
+def test_pair_block_sizes(ctx, features):
+    """Feature counts on both sides of every block size that the accumulator allows, and past it."""
+    rng = np.random.default_rng(features)
+    n = 6000
+    x, y = (rng.uniform(0, 40, n).astype(np.float32) for _ in range(2))
+    fid = np.sort(np.r_[np.arange(features), rng.integers(0, features, n - features)]).astype(np.int32)
+    ds = colo.Dataset.from_arrays(ctx, x, y, fid, np.array([0, 0, 40, 40], np.float32))
+    cand = rng.choice(features, (40, 2), replace=True)
+    cand = np.sort(cand[cand[:, 0] != cand[:, 1]], axis=1)
+    ub, _ = ctx.stage_filter(ds, 1.0, 0.1, cand.astype(np.uint32))
+    assert np.array_equal(ub.astype(np.int64), _bounds(x, y, fid, 40, 41, cand))
