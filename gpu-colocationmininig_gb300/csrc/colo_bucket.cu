@@ -988,6 +988,9 @@ namespace {
 
 void lay_points(Batch& b, Carver& c) {
     c.add(b.xy, b.N);
+    // written by every launch of the heads, one that only counts them too
+    if (b.gathered) c.add(b.sxy, b.N);
+    if (b.gathered && b.J > 1) c.add(b.sfeat, b.N);
     c.add(b.sid, b.N);
     c.add(b.nb_beg, b.N);
     c.add(b.nb_cnt, b.N);
@@ -1000,8 +1003,6 @@ void lay_heads(Batch& b, Carver& c, uint64_t M, uint64_t R) {
     c.add(b.rfeat, R);
     c.add(b.rstart, R + 1);
     c.add(b.rcell, R);
-    if (b.gathered) c.add(b.sxy, b.N);
-    if (b.gathered && b.J > 1) c.add(b.sfeat, b.N);
     if (b.keep_scell) c.add(b.scell, b.N);
 }
 void lay_cells(Batch& b, Carver& c, uint64_t M, uint64_t R) {
