@@ -31,7 +31,7 @@ struct alignas(128) BatchCtrl {
     DevFlags flags;
     uint32_t M, Rn;              // occupied cells, runs
     uint32_t keys_done;          // blocks of the cell-key pass that have added their histograms
-    LineCounter nlistq;          // cells queued for a neighbourhood run list
+    LineCounter nlistq;          // cells queued for a neighbourhood list
     LineCounter nquadq;          // cells with a quad of quad_min features or more
     LineCounter npairq;          // with pairq: cells with two features or more in their 3x3 block
     // neighbourhood lists: target points, runs, anchors with short and with long lists, and the

@@ -1,7 +1,7 @@
 // colo_bucket.cu -- grid bucketing: a stable radix sort of points by cell key
 // into a cell CSR with (cell, feature) runs, per-cell feature masks and the
 // geometric 3x3 occupied-neighbour table; then the per-cell neighbourhood
-// run lists that the join walks.
+// lists that the join walks.
 //
 // Replaces CountCellFeatures (Codes/DeviceProcess.cu:312-369) and
 // kernel_CountCellFeatures (Codes/DeviceProcess_Kernel.h:629-647): instead of
@@ -471,7 +471,7 @@ constexpr int kQuadThreads = 128;
 constexpr uint32_t kQuadHist = 1024;
 
 // Per cell: the 3x3 mask (nbmask), the queue of cells that need a neighbourhood
-// run list, the queue of cells with a quad of quad_min features or more, their four
+// list, the queue of cells with a quad of quad_min features or more, their four
 // quad masks, and the driver-list sizes: dcnt[f] = cells of that queue whose 3x3
 // mask holds f.  Most cells have no such quad (94% at 1M and at 20M points), and
 // no pattern of three is bounded by them: without their 64 bytes of quad masks and
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
 #pragma unroll
             for (int w = 0; w < WT; ++w) feats += __popc(all[w]);
             paired = feats >= 2;
-            // the cell needs a neighbourhood run list when its 3x3 block holds a
+            // the cell needs a neighbourhood list when its 3x3 block holds a
             // feature above its own lowest one (m[4] is the cell's own mask; the block
             // is the union over all nine slots, a superset of the adjacent cells):
             // such cells are queued for the list kernels
@@ -645,7 +645,7 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad_masks(
 }
 
 // ---------------------------------------------------------------------------
-// Neighbourhood run lists.  For cell c the adjacent cells A(c) (the
+// Neighbourhood lists.  For cell c the adjacent cells A(c) (the
 // reference's stencil, ascending cell ids) contribute their runs; NRL(c)
 // orders them by (feature, cell), which is the order the reference's kernels
 // visit candidates of one feature.  For each run of c the list suffix with

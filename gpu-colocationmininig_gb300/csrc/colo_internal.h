@@ -12,7 +12,7 @@
 //               crun[M+1] (run ranges), nbrs[M] (geometric 3x3 neighbours),
 //               cmask[M*W] (feature bit masks, local feature index),
 //               qmask[M*4*W] (masks of the 4 quads containing the cell)
-//   runs        (cell, feature) runs rfeat/rstart/rcnt/rcell[Rn], cell-major;
+//   runs        (cell, feature) runs rfeat/rstart/rcell[Rn], cell-major;
 //               runs per feature on the host (h_frun_off prefix)
 //   lists       per cell with targets, the points of its adjacent cells' runs with
 //               a feature above the cell's lowest own feature, ordered by
