@@ -87,7 +87,7 @@ struct colo_ctx {
     cudaStream_t s = nullptr;
     int sms = 0;
     uint64_t device_bytes = 0;  // the device's memory
-    bool host_reads = false;    // kernels may read any host memory over the link (no copy, no page-locking)
+    bool host_reads = false;    // kernels may read any host memory over the link (only the library's own arrays are read so)
     std::string err;
     int refs = 1;          // the owner plus one per live dataset (freed at zero)
     std::vector<float> model;   // cost-model parameters for LEARNED mines (empty: none)

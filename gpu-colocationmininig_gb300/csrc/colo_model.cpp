@@ -84,18 +84,13 @@ colo_status colo_model_grad(colo_ctx* ctx, const float* params, const float* x, 
         dl.zero(s);
         COLO_CUDA(cudaMemcpyAsync(dp.get(), params, kMlpParams * 4, cudaMemcpyHostToDevice, s));
         if (n) {
-            // the rows are read once: by the kernel itself over the host link, when the device can
-            // (copied first, the link and the kernel take turns)
-            const float *px = x, *pt = t;
-            if (!ctx->host_reads) {
-                dx.alloc(n * kMlpIn, s);
-                dt.alloc(n, s);
-                COLO_CUDA(cudaMemcpyAsync(dx.get(), x, n * kMlpIn * 4, cudaMemcpyHostToDevice, s));
-                COLO_CUDA(cudaMemcpyAsync(dt.get(), t, n * 4, cudaMemcpyHostToDevice, s));
-                px = dx.get();
-                pt = dt.get();
-            }
-            mlp_grad(dp.get(), px, pt, nullptr, n, dg.get(), dl.get(), s);
+            // copied, though the kernel could read them in place over the host link: the arrays are the
+            // caller's, and a mapped file cut short meanwhile would be a fault of the GPU
+            dx.alloc(n * kMlpIn, s);
+            dt.alloc(n, s);
+            COLO_CUDA(cudaMemcpyAsync(dx.get(), x, n * kMlpIn * 4, cudaMemcpyHostToDevice, s));
+            COLO_CUDA(cudaMemcpyAsync(dt.get(), t, n * 4, cudaMemcpyHostToDevice, s));
+            mlp_grad(dp.get(), dx.get(), dt.get(), nullptr, n, dg.get(), dl.get(), s);
         }
         COLO_CUDA(cudaMemcpyAsync(grad, dg.get(), kMlpParams * 4, cudaMemcpyDeviceToHost, s));
         float l = 0.f;
