@@ -382,7 +382,7 @@ class Context:
         ps = (Params * n)(*params)
         outs = (_P * n)()
         self.check(self.lib.colo_mine_batch(self.h, hs, ps, n, outs), "colo_mine_batch")
-        return [Result(self.lib, outs[i], params[i]) for i in range(n)]
+        return [Result(self.lib, outs[i], ps[i]) for i in range(n)]
 
     def stage_neighbors(self, ds: "Dataset", R: float):
         tot = C.c_uint64(0)
