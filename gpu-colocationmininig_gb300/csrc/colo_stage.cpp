@@ -267,7 +267,7 @@ colo_status colo_autotune(colo_ctx* ctx, colo_dataset* ds, const colo_params* p,
         std::vector<DevBuf<float>> of;
         colo_dataset* dsv[1] = {ds};
         setup_batch(ctx, dsv, p, 1, b, of, nullptr);
-        int best = 8;
+        int best = 1;   // the default (nothing to time without points)
         double best_ms = 1e300, t[kJoinWidths] = {0, 0, 0, 0, 0, 0};
         if (b.N) {
             bucket_points(b);
@@ -311,9 +311,10 @@ namespace {
 
 // ---- tuning cache ----------------------------------------------------------
 // One text line per tuned dataset shape:
-//   colo-tune 2 n=<points> f=<features> m=<occupied cells> r=<R float bits, hex> sms=<SMs> join=<lanes>
-//   funit=<candidates per filter unit> lblock=<level threads per block> lqueue=<0|1>
-// Lines that do not parse are skipped; a shape tuned twice keeps its first line.
+//   colo-tune 2 n=<points> f=<features> m=<occupied cells> r=<R float bits, hex> sms=<SMs> lanes=<lanes per
+//   anchor in a join tile> funit=<candidates per filter unit> lblock=<level threads per block> lqueue=<0|1>
+// Lines that do not parse are skipped (older ones among them, whose join=<lanes> was timed on a join that
+// gave each anchor a group of lanes); a shape tuned twice keeps its first line.
 struct TuneKey {
     uint64_t n = 0, f = 0, m = 0;
     uint32_t rbits = 0;
@@ -332,7 +333,7 @@ bool cache_lookup(const char* path, const TuneKey& key, colo_tuning* t) {
         unsigned long long n, f, m;
         unsigned rb;
         int sms, j, u, lb, lq, ver;
-        if (std::sscanf(line, "colo-tune %d n=%llu f=%llu m=%llu r=%x sms=%d join=%d funit=%d lblock=%d lqueue=%d",
+        if (std::sscanf(line, "colo-tune %d n=%llu f=%llu m=%llu r=%x sms=%d lanes=%d funit=%d lblock=%d lqueue=%d",
                         &ver, &n, &f, &m, &rb, &sms, &j, &u, &lb, &lq) != 10 || ver != 2)
             continue;
         TuneKey k;
@@ -355,7 +356,7 @@ bool cache_lookup(const char* path, const TuneKey& key, colo_tuning* t) {
 bool cache_store(const char* path, const TuneKey& key, const colo_tuning& t) {
     FILE* fp = std::fopen(path, "a");
     if (!fp) return false;
-    std::fprintf(fp, "colo-tune 2 n=%llu f=%llu m=%llu r=%08x sms=%d join=%d funit=%d lblock=%d lqueue=%d\n",
+    std::fprintf(fp, "colo-tune 2 n=%llu f=%llu m=%llu r=%08x sms=%d lanes=%d funit=%d lblock=%d lqueue=%d\n",
                  (unsigned long long)key.n, (unsigned long long)key.f, (unsigned long long)key.m, key.rbits, key.sms,
                  t.join_group, t.filter_unit, t.level_block, t.level_queue);
     return std::fclose(fp) == 0;
@@ -429,7 +430,7 @@ colo_status colo_autotune_all(colo_ctx* ctx, colo_dataset* ds, const colo_params
         return COLO_OK;
     }
     // lanes per anchor in the join
-    int32_t jg = 8;
+    int32_t jg = 1;
     st = colo_autotune(ctx, ds, p, &jg, nullptr);
     if (st != COLO_OK) return st;
     t.join_group = jg;
