@@ -40,6 +40,9 @@ struct alignas(128) BatchCtrl {
     LineCounter nb_used;         // room taken by the single-pass join's tiles
 };
 
+// Largest single-pass neighbour layout (entries): 4 GiB, and a 64th of the device.
+constexpr uint64_t kSinglePassCap = 1ull << 30;
+
 struct Batch {
     colo_ctx* ctx = nullptr;
     cudaStream_t s = 0;
@@ -59,7 +62,9 @@ struct Batch {
     // bounds are too large a reservation wait for the sizes instead (bounded = false).
     bool bounded = true;
     uint64_t capM = 0, capR = 0;
-    uint64_t device_bytes = 0;   // the device's memory
+    uint64_t device_bytes = 0;   // the device's memory, as the layouts' rules see it
+    // the largest single-pass neighbour layout (entries)
+    uint64_t single_cap() const { return device_bytes / 256 < kSinglePassCap ? device_bytes / 256 : kSinglePassCap; }
     // host copies of small arrays
     std::vector<JobHost> jobs;
     std::vector<uint32_t> h_fstart, h_fcount, h_fjob;
@@ -160,7 +165,6 @@ void build_neighborhoods(Batch& b);      // neighbourhood lists and anchors (lau
 // colo_join.cu
 constexpr int kEntrySlots = 64, kEntryStride = 16;   // dE: counters on separate 128-byte lines
 constexpr uint32_t kLongList = 64;                   // targets above which an anchor gets a warp to itself
-constexpr uint64_t kSinglePassCap = 1ull << 30;      // largest single-pass layout (entries)
 void join_queue(Batch& b);               // single-pass join into nb_cap entries, skipped on the device when they
                                          // or the lists did not fit (bounded batches, before settle)
 void join_neighbors(Batch& b);           // neighbour CSR (after settle)

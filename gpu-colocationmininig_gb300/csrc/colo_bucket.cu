@@ -975,14 +975,14 @@ inline unsigned grid_for(uint64_t n, int threads) {
 // a sixteenth of the device); the 20M-point workload takes 5 GB.  Larger ones wait for the
 // number of cells and runs before their per-cell arrays are laid out.
 constexpr uint64_t kBoundBytes = 8ull << 30;
-// Look-back words of all digit passes in one clear, up to this much (above 100 million points
-// one pass's words are cleared before each pass).
+// Look-back words of all digit passes in one clear, up to this much and a 1024th of the device (above
+// 67 to 179 million points, by key width, one pass's words are cleared before each pass).
 constexpr uint64_t kSortStatusBytes = 256ull << 20;
 // Room for the lists' targets and for neighbours before their numbers are known: four targets
 // per point (nine at most: a point is adjacent to nine cells) and eight neighbours per point (0.14 on the 20M workload, 16 on that batch,
 // 30 in dense clusters).  What does not fit is built again with the counted room.
 inline uint64_t list_room(uint64_t n) { return std::min<uint64_t>(9 * n, 4 * n + 65536); }
-inline uint64_t neighbour_room(uint64_t n) { return std::min<uint64_t>(kSinglePassCap, 8 * n + 65536); }
+inline uint64_t neighbour_room(const Batch& b) { return std::min<uint64_t>(b.single_cap(), 8 * b.N + 65536); }
 
 namespace {
 
@@ -1110,7 +1110,7 @@ void sort_and_compact(Batch& b) {
 
 void bucket_layout(Batch& b, Carver& c) {
     const uint64_t tiles = (b.N + kHeadTile - 1) / kHeadTile, sw = b.N ? radix_status_words(b.N, b.plan) : 0;
-    b.sort_shared = sw * 8 * (uint64_t)b.plan.n > kSortStatusBytes;
+    b.sort_shared = sw * 8 * (uint64_t)b.plan.n > std::min<uint64_t>(kSortStatusBytes, b.device_bytes / 1024);
     c.add(b.hist, (uint64_t)std::max(b.plan.n, 1) * kRadixDigits);
     c.add(b.tickets, (uint64_t)b.plan.n + 1);
     c.add(b.head_status, 2 * tiles);
@@ -1124,7 +1124,7 @@ void bucket_points(Batch& b) {
     // enough to reserve; a device that has no such block left takes the other way
     b.capM = b.capR = n;
     b.targets_cap = list_room(n);
-    b.nb_cap = neighbour_room(n);
+    b.nb_cap = neighbour_room(b);
     b.row_table = wants_row_table(b, n);
     b.gathered = b.J > 1 || n <= kGatherPoints;
     b.pair_queue = b.J == 1 && n >= kPairQueuePoints;

@@ -206,8 +206,8 @@ void join_neighbors(Batch& b) {
     cudaStream_t s = b.s;
     const uint64_t A = b.active_anchors, AL = b.long_anchors, U = b.join_pairs;
     b.join_queued = false;
-    // layouts above kSinglePassCap entries are counted first and then compact
-    const bool single = U <= kSinglePassCap;
+    // larger layouts are counted first and then compact
+    const bool single = U <= b.single_cap();
     auto room = [&](uint64_t n) {
         b.nb_cap = n;
         Carver::place(b.mem_nb, s, [&](Carver& c) { c.add(b.nb, std::max<uint64_t>(n, 1)); });

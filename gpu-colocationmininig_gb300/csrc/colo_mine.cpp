@@ -662,7 +662,7 @@ void setup_batch(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params* pv,
     b.key_bits = 1;
     while (b.key_bits < 64 && (1ull << b.key_bits) < key_base) b.key_bits++;
     b.rows = row_base;
-    b.device_bytes = ctx->device_bytes;
+    b.device_bytes = pv[0].reserved[2] > 0 ? (uint64_t)pv[0].reserved[2] << 10 : ctx->device_bytes;
     b.plan = radix_plan(b.key_bits <= 32 ? (int)b.key_bits : (int)std::min<uint64_t>(b.key_bits, 64));
     b.h_job_off.assign(J + 1, 0);
     for (uint32_t j = 0; j < J; ++j)

@@ -69,7 +69,10 @@ typedef struct {
                                 bucketing sort's look-back gives up after that many
                                 polls and its first tile withholds its counts, so the
                                 mine fails with COLO_ERR_TIMEOUT (no wait is unbounded;
-                                the context stays usable) */
+                                the context stays usable);
+                                reserved[2] > 0, tests of the layouts only: the device's
+                                memory in KiB, as the rules see it that choose between
+                                layouts by size */
 } colo_params;
 
 const char* colo_status_string(colo_status s);
