@@ -11,7 +11,8 @@ namespace colo {
 
 // Queues a copy of host bytes through the context's page-locked staging (no wait; colo_mine.cpp).
 void staged_upload(colo_ctx* ctx, cudaStream_t s, void* dst, const void* src, size_t bytes);
-
+// Device memory that buffers may take now: free, or idle in the pool (colo_mine.cpp).
+uint64_t device_room(const colo_ctx* ctx);
 
 // Host description of one job inside a batch.
 struct JobHost {
@@ -59,8 +60,11 @@ struct Batch {
     // Sizes that bucketing finds are kept on the device, and arrays over cells, runs, list
     // entries and neighbours are laid out for an upper bound (capM, capR, targets_cap, nb_cap), so
     // that everything up to the pairs' bounds is queued without a host wait.  Batches whose
-    // bounds are too large a reservation wait for the sizes instead (bounded = false).
-    bool bounded = true;
+    // bounds are too large a reservation wait for the sizes instead (bounded = false).  `exact`
+    // asks for that, and for heads that are counted first: the second attempt of a call whose
+    // arrays did not all fit the device (fit_device).
+    bool bounded = true, exact = false;
+    uint64_t reserved_bytes = 0;   // of the arrays laid out for more than the batch turns out to need
     uint64_t capM = 0, capR = 0;
     uint64_t device_bytes = 0;   // the device's memory, as the layouts' rules see it
     // the largest single-pass neighbour layout (entries)

@@ -972,9 +972,10 @@ inline unsigned grid_for(uint64_t n, int threads) {
 }  // namespace
 
 // Bounded batches reserve at most this much for arrays laid out by bounds (and no more than
-// a sixteenth of the device); the 20M-point workload takes 5 GB.  Larger ones wait for the
-// number of cells and runs before their per-cell arrays are laid out.
-constexpr uint64_t kBoundBytes = 8ull << 30;
+// a sixteenth of the device, and blocks of 256 MiB and more no more than half of what is
+// free); the 20M-point workload takes 5 GB.  Larger ones wait for the number of cells and
+// runs before their per-cell arrays are laid out.
+constexpr uint64_t kBoundBytes = 8ull << 30, kSmallBounds = 256ull << 20;
 // Look-back words of all digit passes in one clear, up to this much and a 1024th of the device (above
 // 67 to 179 million points, by key width, one pass's words are cleared before each pass).
 constexpr uint64_t kSortStatusBytes = 256ull << 20;
@@ -1089,8 +1090,9 @@ void sort_and_compact(Batch& b) {
     }
     // heads laid out for every point when that is small against the device, else counted first
     const size_t all = Carver::bytes([&](Carver& c) { lay_heads(b, c, n, n); });
-    if (all <= b.device_bytes / 16) {
+    if (!b.exact && all <= b.device_bytes / 16) {
         Carver::place(b.mem_heads, s, [&](Carver& c) { lay_heads(b, c, n, n); });
+        b.reserved_bytes = all;
         launch_heads<KT>(b, keys, n, n);
         read_sizes(b);
     } else {
@@ -1136,10 +1138,13 @@ void bucket_points(Batch& b) {
         lay_act(b, c);
         c.add(b.nb, b.nb_cap);
     };
-    b.bounded = Carver::bytes(bounds) <= std::min<uint64_t>(kBoundBytes, b.device_bytes / 16);
+    const uint64_t need = Carver::bytes(bounds);
+    b.bounded = !b.exact && need <= std::min<uint64_t>(kBoundBytes, b.device_bytes / 16) &&
+                (need <= kSmallBounds || need <= device_room(b.ctx) / 2);
     if (b.bounded) {
         try {
             Carver::place(b.mem_points, s, bounds);
+            b.reserved_bytes = need;
         } catch (const StatusError& e) {
             if (e.st != COLO_ERR_NOMEM) throw;
             b.bounded = false;

@@ -129,6 +129,9 @@ void candidate_features(uint32_t k, const uint32_t* mem, const uint32_t* fcount,
 colo_status set_err(colo_ctx* ctx, colo_status st, const std::string& msg);
 void ctx_release(colo_ctx* ctx);
 colo_status run_guarded(colo_ctx* ctx, const std::function<colo_status()>& fn);
+// Calls fn(false), and fn(true), which lays out exact sizes (Batch::exact), when the device had no
+// room for the first attempt.
+colo_status fit_device(colo_ctx* ctx, const std::function<colo_status(bool exact)>& fn);
 uint64_t upload_dataset(colo_dataset* ds, cudaStream_t s);   // bytes copied (0 when resident)
 // Points, features, job grids and the bucketed/joined device state of a batch.
 // `own` keeps the concatenated device copies of multi-job batches alive.

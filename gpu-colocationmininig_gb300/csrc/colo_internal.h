@@ -88,6 +88,13 @@ struct StatusError {
     std::string msg;
 };
 
+// Device memory of this thread's buffers, and how much of it they may take (0: what there is; a
+// limit is set by tests of a full device only, for one mine's buffers).
+struct DevBudget {
+    uint64_t used = 0, limit = 0;
+};
+extern thread_local DevBudget g_budget;
+
 // Stream-ordered device buffer (cudaMallocAsync / cudaFreeAsync).
 template <class T>
 struct DevBuf {
@@ -106,19 +113,24 @@ struct DevBuf {
         s = st;
         n = count;
         if (count == 0) return;
-        cudaError_t e = cudaMallocAsync((void**)&p, count * sizeof(T), st);
-        if (e != cudaSuccess) {
+        const uint64_t bytes = count * sizeof(T);
+        const bool fits = !g_budget.limit || g_budget.used + bytes <= g_budget.limit;
+        if (!fits || cudaMallocAsync((void**)&p, bytes, st) != cudaSuccess) {
             p = nullptr;
             n = 0;
             cudaGetLastError();
-            throw StatusError{COLO_ERR_NOMEM, "device allocation of " + std::to_string(count * sizeof(T)) + " bytes failed"};
+            throw StatusError{COLO_ERR_NOMEM, "device allocation of " + std::to_string(bytes) + " bytes failed"};
         }
+        g_budget.used += bytes;
     }
     void zero(cudaStream_t st) {
         if (n) COLO_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), st));
     }
     void release() {
-        if (p) cudaFreeAsync(p, s);
+        if (p) {
+            cudaFreeAsync(p, s);
+            g_budget.used -= n * sizeof(T);
+        }
         p = nullptr;
         n = 0;
     }
@@ -164,7 +176,7 @@ struct Carver {
 
 // Instance-table storage: device memory, or pinned host memory mapped into
 // the device's address space when asked for or when the device allocation
-// fails (on Grace the kernels then read and write them over NVLink-C2C).
+// is refused (mine_jobs; on Grace the kernels then read and write them over NVLink-C2C).
 struct TableBuf {
     DevBuf<uint32_t> dev;
     void* host = nullptr;
@@ -179,13 +191,9 @@ struct TableBuf {
         s = st;
         n = count;
         if (!on_host) {
-            try {
-                dev.alloc(count, st);
-                p = dev.get();
-                return;
-            } catch (const StatusError& e) {
-                if (e.st != COLO_ERR_NOMEM) throw;
-            }
+            dev.alloc(count, st);
+            p = dev.get();
+            return;
         }
         if (cudaHostAlloc(&host, (count ? count : 1) * sizeof(uint32_t), cudaHostAllocMapped) != cudaSuccess) {
             host = nullptr;

@@ -747,13 +747,38 @@ void settle(colo_ctx* ctx, Batch& b, std::vector<uint32_t>* ub2) {
 // mines carve their blocks out of it.  The growth lands in the mine that set
 // the peak (a warm-up mine, typically), not in the next one.  The pool's
 // high-water mark is reset as a mine starts, so it measures that mine alone.
-static cudaMemPool_t device_pool(colo_ctx* ctx) {
+static cudaMemPool_t device_pool(const colo_ctx* ctx) {
     cudaMemPool_t pool = nullptr;
     if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
     return pool;
+}
+
+uint64_t device_room(const colo_ctx* ctx) {
+    if (g_budget.limit) return g_budget.limit - std::min(g_budget.limit, g_budget.used);
+    cudaMemPool_t pool = device_pool(ctx);
+    uint64_t used = 0, reserved = 0;
+    if (pool && (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess ||
+                 cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess))
+        cudaGetLastError();
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) cudaGetLastError();
+    return free_b + (reserved - std::min(reserved, used));
+}
+
+// The pool's free memory goes back to the device in between: blocks of other sizes may then fit.
+colo_status fit_device(colo_ctx* ctx, const std::function<colo_status(bool exact)>& fn) {
+    try {
+        return fn(false);
+    } catch (const StatusError& e) {
+        if (e.st != COLO_ERR_NOMEM) throw;
+    }
+    COLO_CUDA(cudaStreamSynchronize(ctx->s));
+    cudaMemPool_t pool = device_pool(ctx);
+    if (pool && cudaMemPoolTrimTo(pool, 0) != cudaSuccess) cudaGetLastError();
+    return fn(true);
 }
 
 static void pool_reset_mark(colo_ctx* ctx) {
@@ -787,7 +812,7 @@ static void pool_headroom(colo_ctx* ctx) {
 }
 
 static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params* pv, uint32_t J,
-                      MineResult** outs) {
+                      MineResult** outs, bool exact) {
     cudaStream_t s = ctx->s;
     const auto t_all = Clock::now();
     g_launches = 0;
@@ -795,13 +820,18 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
     kt.s = s;
     kt.on = (pv[0].reserved[0] & 1) != 0;
     g_ktimer = &kt;
+    g_budget = DevBudget{0, pv[0].reserved[3] > 0 ? (uint64_t)pv[0].reserved[3] << 10 : 0};
     struct Unset {
-        ~Unset() { g_ktimer = nullptr; }
+        ~Unset() {
+            g_ktimer = nullptr;
+            g_budget.limit = 0;
+        }
     } unset;
     uint64_t cnt_items = 0, cnt_parent = 0, cnt_fillw = 0, cnt_bmw = 0, cnt_d2h = 0, cnt_refined = 0, cnt_fcm = 0;
     uint64_t cnt_single = 0, cnt_single_ovf = 0, cnt_fquads = 0, cnt_fcells = 0;
     uint64_t us_pairs_model = 0, us_level_wait = 0;
     Batch b;
+    b.exact = exact || pv[0].reserved[2] < 0;
     const int mode = pv[0].mode;
     const bool plain = (mode == COLO_MODE_PLAIN);
     std::vector<DevBuf<float>> ownf;
@@ -860,6 +890,18 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
     bool host_tables = false;
     for (uint32_t j = 0; j < J; ++j) host_tables |= (pv[j].reserved[0] & 8) != 0;
     uint64_t cnt_host_table_bytes = 0;
+    auto alloc_tables = [&](TableBuf& t, uint64_t words) {
+        try {
+            t.alloc(words ? words : 1, s, host_tables);
+        } catch (const StatusError& e) {
+            // (where arrays laid out too large may be what is in the way, the mine lays them out exactly first)
+            if (e.st != COLO_ERR_NOMEM || host_tables ||
+                (b.reserved_bytes && words * 4 <= device_room(ctx) + b.reserved_bytes))
+                throw;
+            t.alloc(words ? words : 1, s, true);
+        }
+        if (t.on_host()) cnt_host_table_bytes += words * 4;
+    };
     std::vector<uint32_t> h_least;   // per feature, least_bound (once asked for)
     TableReads table_reads{ctx, s};
     for (uint32_t k = 2;; ++k) {
@@ -1244,8 +1286,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         if (ns) {
             for (uint64_t q = 0; q < ns; ++q) single_words += cap[q] * k;
             single_cur.reset(new TableBuf());
-            single_cur->alloc(single_words ? single_words : 1, s, host_tables);
-            if (single_cur->on_host()) cnt_host_table_bytes += single_words * 4;
+            alloc_tables(*single_cur, single_words);
         }
         for (uint64_t q = 0, o = 0; q < ncand; ++q) {
             hd[q].chunk_rows = ar.chunk_rows.get() + first_chunk[q];
@@ -1521,8 +1562,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
                     cnt_fillw += (gb[q + 1] - gb[q]) * k;
                 }
         tables_cur.reset(new TableBuf());
-        tables_cur->alloc(total_rows * k ? total_rows * k : 1, s, host_tables);
-        if (tables_cur->on_host()) cnt_host_table_bytes += total_rows * k * 4;
+        alloc_tables(*tables_cur, total_rows * k);
         if (plain)   // one scan per candidate, as the reference does
             for (uint64_t q : fillq)
                 scan_u32_to_u64(ar.chunk_rows.get() + first_chunk[q], ar.offs.get() + first_chunk[q],
@@ -1914,11 +1954,13 @@ colo_status colo_mine_batch(colo_ctx* ctx, colo_dataset* const* ds, const colo_p
     }
     colo_status st = guarded(ctx, [&]() {
         pool_reset_mark(ctx);   // from here the pool's high-water mark is this call's
-        if (p[0].mode == COLO_MODE_PLAIN && njobs > 1) {
-            for (uint32_t j = 0; j < njobs; ++j) mine_jobs(ctx, &ds[j], &p[j], 1, &mr[j]);
-        } else {
-            mine_jobs(ctx, ds, p, njobs, mr.data());
-        }
+        const uint32_t at_once = p[0].mode == COLO_MODE_PLAIN ? 1 : njobs;
+        for (uint32_t j = 0; j < njobs; j += at_once)
+            fit_device(ctx, [&](bool exact) {
+                for (uint32_t i = j; i < j + at_once; ++i) mr[i]->levels.clear();
+                mine_jobs(ctx, ds + j, p + j, at_once, &mr[j], exact);
+                return COLO_OK;
+            });
         pool_headroom(ctx);   // the mine's buffers are back in the pool
         return COLO_OK;
     });

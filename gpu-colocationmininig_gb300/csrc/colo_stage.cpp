@@ -24,6 +24,18 @@ colo_params params_for(float R, float thr) {
     return p;
 }
 
+// fn on an empty batch, and once more with exact sizes when the device had no room (fit_device).
+template <class Fn>
+colo_status with_batch(colo_ctx* ctx, Fn&& fn) {
+    return run_guarded(ctx, [&]() -> colo_status {
+        return fit_device(ctx, [&](bool exact) -> colo_status {
+            Batch b;
+            b.exact = exact;
+            return fn(b);
+        });
+    });
+}
+
 }  // namespace
 
 extern "C" {
@@ -31,9 +43,8 @@ extern "C" {
 colo_status colo_stage_cells(colo_ctx* ctx, colo_dataset* ds, float R, uint64_t* cell_of, uint64_t* run_cell,
                              uint32_t* run_feat, uint32_t* run_count, uint64_t* nruns) {
     if (!ctx || !ds || !nruns) return COLO_ERR_ARG;
-    return run_guarded(ctx, [&]() -> colo_status {
+    return with_batch(ctx, [&](Batch& b) -> colo_status {
         colo_params p = params_for(R, 0.f);
-        Batch b;
         std::vector<DevBuf<float>> of;
         colo_dataset* dsv[1] = {ds};
         setup_batch(ctx, dsv, &p, 1, b, of, nullptr);
@@ -77,9 +88,8 @@ colo_status colo_stage_cells(colo_ctx* ctx, colo_dataset* ds, float R, uint64_t*
 colo_status colo_stage_neighbors(colo_ctx* ctx, colo_dataset* ds, float R, uint64_t* offs, uint32_t* nbr,
                                  uint64_t* total) {
     if (!ctx || !ds || !total) return COLO_ERR_ARG;
-    return run_guarded(ctx, [&]() -> colo_status {
+    return with_batch(ctx, [&](Batch& b) -> colo_status {
         colo_params p = params_for(R, 0.f);
-        Batch b;
         std::vector<DevBuf<float>> of;
         colo_dataset* dsv[1] = {ds};
         setup_batch(ctx, dsv, &p, 1, b, of, nullptr);
@@ -121,9 +131,8 @@ colo_status colo_stage_filter(colo_ctx* ctx, colo_dataset* ds, float R, float th
                               uint64_t ncand, uint32_t k, uint64_t* ub, uint8_t* pass) {
     if (!ctx || !ds || (ncand && (!cand || !ub))) return COLO_ERR_ARG;
     if (k < 2 || k > kMaxK) return COLO_ERR_ARG;
-    return run_guarded(ctx, [&]() -> colo_status {
+    return with_batch(ctx, [&](Batch& b) -> colo_status {
         colo_params p = params_for(R, thr);
-        Batch b;
         std::vector<DevBuf<float>> of;
         colo_dataset* dsv[1] = {ds};
         setup_batch(ctx, dsv, &p, 1, b, of, nullptr);
@@ -261,9 +270,8 @@ static constexpr int kJoinWidths = COLO_JOIN_WIDTHS;
 colo_status colo_autotune(colo_ctx* ctx, colo_dataset* ds, const colo_params* p, int32_t* join_group,
                           double* ms) {
     if (!ctx || !ds || !p) return COLO_ERR_ARG;
-    return run_guarded(ctx, [&]() -> colo_status {
+    return with_batch(ctx, [&](Batch& b) -> colo_status {
         static const int widths[kJoinWidths] = {1, 2, 4, 8, 16, 32};
-        Batch b;
         std::vector<DevBuf<float>> of;
         colo_dataset* dsv[1] = {ds};
         setup_batch(ctx, dsv, p, 1, b, of, nullptr);
@@ -406,8 +414,7 @@ colo_status colo_autotune_all(colo_ctx* ctx, colo_dataset* ds, const colo_params
     std::memcpy(&key.rbits, &p->distance, 4);
     key.sms = ctx->sms;
     // the occupied cells of the dataset at this R (one bucketing pass)
-    colo_status st = run_guarded(ctx, [&]() -> colo_status {
-        Batch b;
+    colo_status st = with_batch(ctx, [&](Batch& b) -> colo_status {
         std::vector<DevBuf<float>> of;
         colo_dataset* dsv[1] = {ds};
         setup_batch(ctx, dsv, p, 1, b, of, nullptr);

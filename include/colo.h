@@ -72,7 +72,11 @@ typedef struct {
                                 the context stays usable);
                                 reserved[2] > 0, tests of the layouts only: the device's
                                 memory in KiB, as the rules see it that choose between
-                                layouts by size */
+                                layouts by size; -1: every array over cells and runs
+                                is laid out for the counted size;
+                                reserved[3] > 0, tests of a full device only: the device
+                                memory in KiB that the mine may take; an allocation past
+                                it is refused as on a full device */
 } colo_params;
 
 const char* colo_status_string(colo_status s);
