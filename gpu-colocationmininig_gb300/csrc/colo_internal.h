@@ -93,7 +93,7 @@ struct StatusError {
 struct DevBudget {
     uint64_t used = 0, limit = 0;
 };
-extern thread_local DevBudget g_budget;
+inline thread_local DevBudget g_budget;
 
 // Stream-ordered device buffer (cudaMallocAsync / cudaFreeAsync).
 template <class T>

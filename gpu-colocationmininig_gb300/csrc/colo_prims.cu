@@ -7,7 +7,6 @@
 namespace colo {
 
 thread_local uint64_t g_launches = 0;
-thread_local DevBudget g_budget;
 thread_local KTimer* g_ktimer = nullptr;
 
 namespace {
