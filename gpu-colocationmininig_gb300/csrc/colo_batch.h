@@ -13,6 +13,8 @@ namespace colo {
 void staged_upload(colo_ctx* ctx, cudaStream_t s, void* dst, const void* src, size_t bytes);
 // Device memory that buffers may take now: free, or idle in the pool (colo_mine.cpp).
 uint64_t device_room(const colo_ctx* ctx);
+// A buffer of this size takes no more than half of that, or none that the pool does not hold already.
+bool leaves_half(const colo_ctx* ctx, uint64_t bytes);
 
 // Host description of one job inside a batch.
 struct JobHost {

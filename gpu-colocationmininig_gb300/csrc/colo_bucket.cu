@@ -1140,7 +1140,7 @@ void bucket_points(Batch& b) {
     };
     const uint64_t need = Carver::bytes(bounds);
     b.bounded = !b.exact && need <= std::min<uint64_t>(kBoundBytes, b.device_bytes / 16) &&
-                (need <= kSmallBounds || need <= device_room(b.ctx) / 2);
+                (need <= kSmallBounds || leaves_half(b.ctx, need));
     if (b.bounded) {
         try {
             Carver::place(b.mem_points, s, bounds);

@@ -756,16 +756,27 @@ static cudaMemPool_t device_pool(const colo_ctx* ctx) {
     return pool;
 }
 
-uint64_t device_room(const colo_ctx* ctx) {
-    if (g_budget.limit) return g_budget.limit - std::min(g_budget.limit, g_budget.used);
+static uint64_t pool_idle(const colo_ctx* ctx) {
     cudaMemPool_t pool = device_pool(ctx);
     uint64_t used = 0, reserved = 0;
-    if (pool && (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess ||
-                 cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess))
+    if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess) {
         cudaGetLastError();
+        return 0;
+    }
+    return reserved - std::min(reserved, used);
+}
+
+uint64_t device_room(const colo_ctx* ctx) {
+    if (g_budget.limit) return g_budget.limit - std::min(g_budget.limit, g_budget.used);
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) cudaGetLastError();
-    return free_b + (reserved - std::min(reserved, used));
+    return free_b + pool_idle(ctx);
+}
+
+// (the pool is asked first: cudaMemGetInfo takes 30 us)
+bool leaves_half(const colo_ctx* ctx, uint64_t bytes) {
+    return (!g_budget.limit && bytes <= pool_idle(ctx)) || bytes <= device_room(ctx) / 2;
 }
 
 // The pool's free memory goes back to the device in between: blocks of other sizes may then fit.
