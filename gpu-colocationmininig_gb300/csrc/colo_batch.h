@@ -15,6 +15,8 @@ void staged_upload(colo_ctx* ctx, cudaStream_t s, void* dst, const void* src, si
 uint64_t device_room(const colo_ctx* ctx);
 // A buffer of this size takes no more than half of that, or none that the pool does not hold already.
 bool leaves_half(const colo_ctx* ctx, uint64_t bytes);
+// Notes a block that the mine holds from start to end (the pool's headroom leaves it out).
+void note_block(colo_ctx* ctx, uint64_t bytes);
 
 // Host description of one job inside a batch.
 struct JobHost {

@@ -1145,6 +1145,7 @@ void bucket_points(Batch& b) {
         try {
             Carver::place(b.mem_points, s, bounds);
             b.reserved_bytes = need;
+            note_block(b.ctx, need);
         } catch (const StatusError& e) {
             if (e.st != COLO_ERR_NOMEM) throw;
             b.bounded = false;

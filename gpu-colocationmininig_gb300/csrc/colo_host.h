@@ -104,6 +104,7 @@ struct colo_ctx {
     void* tstage = nullptr;     // page-locked staging for the tables kept in results (at most 64 MiB)
     size_t tstage_bytes = 0;
     uint64_t pool_peak = 0;     // most device-pool memory in use by one earlier mine (bytes)
+    uint64_t pool_block = 0;    // largest block laid out by bounds in the current mine
 };
 
 struct colo_dataset {

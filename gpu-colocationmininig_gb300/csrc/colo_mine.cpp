@@ -742,9 +742,10 @@ void settle(colo_ctx* ctx, Batch& b, std::vector<uint32_t>* ub2) {
 // the last one's may find no free block large enough and map more memory in
 // the middle of a step (about a millisecond per growth on the 20M-point
 // workload).  So after a mine that used more of the pool than any before it,
-// the pool gets one free block of twice that peak, if the device has that
-// much to spare (growing the pool by 10 GB took 4.4 ms on a GB300); later
-// mines carve their blocks out of it.  The growth lands in the mine that set
+// the pool gets one free block of twice that peak, the arrays laid out by bounds
+// (one block, held from the mine's start to its end) counted once, if the device has that
+// much to spare; later mines carve their blocks out of it.  (20 million points hold 5.9 GB;
+// with those arrays counted twice it was 10.8.)  The growth lands in the mine that set
 // the peak (a warm-up mine, typically), not in the next one.  The pool's
 // high-water mark is reset as a mine starts, so it measures that mine alone.
 static cudaMemPool_t device_pool(const colo_ctx* ctx) {
@@ -792,7 +793,10 @@ colo_status fit_device(colo_ctx* ctx, const std::function<colo_status(bool exact
     return fn(true);
 }
 
+void note_block(colo_ctx* ctx, uint64_t bytes) { ctx->pool_block = std::max(ctx->pool_block, bytes); }
+
 static void pool_reset_mark(colo_ctx* ctx) {
+    ctx->pool_block = 0;
     cudaMemPool_t pool = device_pool(ctx);
     uint64_t zero = 0;
     if (pool && cudaMemPoolSetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &zero) != cudaSuccess) cudaGetLastError();
@@ -810,12 +814,13 @@ static void pool_headroom(colo_ctx* ctx) {
     if (high <= ctx->pool_peak) return;   // no new peak (one attempt per peak, whatever its outcome)
     ctx->pool_peak = high;
     size_t free_b = 0, total_b = 0;
-    if (reserved >= 2 * high || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    const uint64_t want = 2 * high - std::min(high, ctx->pool_block);
+    if (reserved >= want || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
         cudaGetLastError();
         return;
     }
     void* p = nullptr;
-    if (2 * high <= free_b / 2 && cudaMallocAsync(&p, 2 * high, ctx->s) == cudaSuccess) {   // most stays free
+    if (want <= free_b / 2 && cudaMallocAsync(&p, want, ctx->s) == cudaSuccess) {   // most stays free
         cudaFreeAsync(p, ctx->s);
         cudaStreamSynchronize(ctx->s);
     }
