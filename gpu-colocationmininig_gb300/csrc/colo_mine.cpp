@@ -473,7 +473,8 @@ namespace {
 // Instance tables kept in results: turned into rows on the device and copied through page-locked
 // staging behind the level's fill, without a wait of their own; finish() (after a wait, or once the
 // staging is full) moves them to their vectors, whose storage does not move with the level's trace.
-// The staging grows to kTableStage bytes at most.
+// The staging grows to kTableStage bytes at most.  Where the device has no room for the rows, or the
+// host none for the staging, the columns are copied one piece at a time and turned into rows here.
 constexpr size_t kTableStage = (size_t)64 << 20;
 
 struct TableReads {
@@ -492,17 +493,51 @@ struct TableReads {
         used = 0;
     }
     // room for `bytes` more; what is pending is finished first when there is none
-    void room(size_t bytes) {
-        if (used + bytes <= ctx->tstage_bytes) return;
+    bool room(size_t bytes) {
+        if (used + bytes <= ctx->tstage_bytes) return true;
         stream_wait(s);
         finish();
-        if (bytes <= ctx->tstage_bytes) return;
+        if (bytes <= ctx->tstage_bytes) return true;
         if (ctx->tstage) cudaFreeHost(ctx->tstage);
         ctx->tstage = nullptr;
         ctx->tstage_bytes = 0;
         const size_t nb = std::min(kTableStage, std::max<size_t>(bytes * 2, (size_t)1 << 20));
-        COLO_CUDA(cudaHostAlloc(&ctx->tstage, nb, cudaHostAllocDefault));
+        if (cudaHostAlloc(&ctx->tstage, nb, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->tstage = nullptr;
+            return false;
+        }
         ctx->tstage_bytes = nb;
+        return true;
+    }
+    // the pieces (of `rows` rows in all, the longest of `longest`) queued by way of the staging
+    bool staged(const std::vector<TablePiece>& pieces, const std::vector<uint32_t*>& to, uint64_t rows,
+                uint64_t longest, uint32_t k) {
+        const size_t bytes = (size_t)rows * k * 4;
+        if (!room(bytes)) return false;
+        DevBuf<uint32_t> out;
+        DevBuf<TablePiece> dp;
+        try {
+            out.alloc(rows * k, s);
+            dp.alloc(pieces.size(), s);
+        } catch (const StatusError& e) {
+            if (e.st != COLO_ERR_NOMEM) throw;
+            return false;
+        }
+        staged_upload(ctx, s, dp.get(), pieces.data(), pieces.size() * sizeof(TablePiece));
+        table_rows(s, dp.get(), (uint32_t)pieces.size(), k, longest * k, out.get());
+        COLO_CUDA(cudaMemcpyAsync(static_cast<char*>(ctx->tstage) + used, out.get(), bytes, cudaMemcpyDeviceToHost, s));
+        for (size_t i = 0; i < pieces.size(); ++i)
+            items.push_back({to[i], used + (size_t)pieces[i].at * 4, (size_t)pieces[i].rows * k * 4});
+        used += bytes;
+        return true;
+    }
+    void direct(const TablePiece& p, uint32_t* to, uint32_t k) {
+        std::vector<uint32_t> cols(p.rows * k);
+        stream_wait(s);
+        COLO_CUDA(cudaMemcpy2D(cols.data(), p.rows * 4, p.cols + p.row0, p.stride * 4, p.rows * 4, k, cudaMemcpyDefault));
+        for (uint64_t r = 0; r < p.rows; ++r)
+            for (uint32_t t = 0; t < k; ++t) to[r * k + t] = cols[t * p.rows + r];
     }
     // the level's tables (cols, rows, stride) to dst[i], sized rows * k
     void read(const std::vector<TableRef>& tables, const std::vector<uint32_t*>& dst, uint32_t k) {
@@ -512,18 +547,8 @@ struct TableReads {
         uint64_t rows = 0, longest = 0;
         auto flush = [&]() {
             if (pieces.empty()) return;
-            const size_t bytes = (size_t)rows * k * 4;
-            room(bytes);
-            DevBuf<uint32_t> out;
-            DevBuf<TablePiece> dp;
-            out.alloc(rows * k, s);
-            dp.alloc(pieces.size(), s);
-            staged_upload(ctx, s, dp.get(), pieces.data(), pieces.size() * sizeof(TablePiece));
-            table_rows(s, dp.get(), (uint32_t)pieces.size(), k, longest * k, out.get());
-            COLO_CUDA(cudaMemcpyAsync(static_cast<char*>(ctx->tstage) + used, out.get(), bytes, cudaMemcpyDeviceToHost, s));
-            for (size_t i = 0; i < pieces.size(); ++i)
-                items.push_back({to[i], used + (size_t)pieces[i].at * 4, (size_t)pieces[i].rows * k * 4});
-            used += bytes;
+            if (!staged(pieces, to, rows, longest, k))
+                for (size_t i = 0; i < pieces.size(); ++i) direct(pieces[i], to[i], k);
             pieces.clear();
             to.clear();
             rows = longest = 0;
