@@ -269,10 +269,17 @@ uint32_t least_bound(uint32_t n, float thr) {
 
 // A level of at least three members is filtered and counted with one wait when no candidate's
 // table can be chosen for the single pass: none was asked for, there is no cost model, or every
-// parent table is this short (2^20 rows from it would need 64 a parent row).  Its candidates'
-// bitmaps and chunks, those of candidates that the filter stops among them, take at most this room.
+// parent table is this short (2^20 rows from it would need 64 a parent row).  The wait saved is
+// worth 12 to 25 us a level; candidates that the filter stops are then described, their chunks
+// launched and their bitmaps cleared and summed for nothing (46 ns a candidate, 55 us a million chunks).
+// Where every one of 220 triples was stopped, one wait cost 17 us up to 2^17 chunks and 2^21 words, but
+// 54 at 660,000 chunks, 169 at 2.2 million; 4,060 triples cost 224.  So level 3, of whose filter nothing is
+// known yet, takes one wait within these bounds, and a later level where the filter stopped at most one
+// in eight of the last level's candidates (past level 3 it stopped none in any workload timed), in at
+// most kOneWaitWords and kOneWaitChunks.
 constexpr uint64_t kOneWaitRows = 1u << 14;
 constexpr uint64_t kOneWaitWords = 1u << 26, kOneWaitChunks = 1u << 24;
+constexpr uint64_t kOneWaitCands3 = 256, kOneWaitWords3 = 1u << 21, kOneWaitChunks3 = 1u << 17;
 
 // Readbacks staged in page-locked memory: a device-to-host copy into pageable
 // memory blocks the host until the stream reaches it, one into the context's
@@ -943,6 +950,7 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
         }
         if (t.on_host()) cnt_host_table_bytes += words * 4;
     };
+    uint64_t last_cands = 0, last_passed = 0;   // the last level's candidates, and those that passed its filter
     std::vector<uint32_t> h_least;   // per feature, least_bound (once asked for)
     TableReads table_reads{ctx, s};
     for (uint32_t k = 2;; ++k) {
@@ -1017,7 +1025,8 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
             bool rec_all = false;
             for (uint32_t j = 0; j < J; ++j) rec_all |= tr[j] && (pv[j].reserved[0] & 2) != 0;
             one_wait = !plain && !rec_all && !force_single_any && (!learned_mode || longest <= kOneWaitRows) &&
-                       chunks <= kOneWaitChunks && words <= kOneWaitWords;
+                       (k == 3 ? ncand <= kOneWaitCands3 && chunks <= kOneWaitChunks3 && words <= kOneWaitWords3
+                               : last_passed * 8 >= last_cands * 7 && chunks <= kOneWaitChunks && words <= kOneWaitWords);
             if (one_wait)
                 for (uint32_t j = 0; j < J; ++j)
                     if (tr[j]) tr[j]->pass.assign(tr[j]->pass.size(), 1);   // until the bounds are back
@@ -1441,6 +1450,10 @@ static void mine_jobs(colo_ctx* ctx, colo_dataset* const* dsv, const colo_params
             ncand = kept;
         }
         cnt_refined += ncand;
+        last_passed = ncand;
+        last_cands = 0;
+        for (uint32_t j = 0; j < J; ++j)
+            if (tr[j]) last_cands += tr[j]->cand.size() / k;
         for (uint64_t q = 0; q < ncand; ++q) {
             cnt_parent += (uint64_t)(k - 1) * hd[q].prow;
             cnt_bmw += hd[q].last_off + (hd[q].last_end - hd[q].last_start + 31) / 32;
