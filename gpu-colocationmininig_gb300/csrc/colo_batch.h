@@ -105,7 +105,7 @@ struct Batch {
     bool keep_scell = false;              // colo_stage_cells reports each point's cell
     // cells
     Span<uint64_t> ckey;
-    Span<uint32_t> cstart, crun, cjob;    // cstart, crun with an end entry
+    Span<uint32_t> crun, cjob;            // crun with an end entry
     uint64_t h2d_points = 0;     // bytes of point data copied to the device for this batch
     uint64_t rows = 0;           // grid rows of all jobs (row table size - 1)
     bool row_table = false;

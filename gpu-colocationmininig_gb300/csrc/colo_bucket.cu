@@ -128,9 +128,6 @@ __global__ void __launch_bounds__(256, 4) k_cell_keys(
 // After a sort that timed out the keys are not a sorted permutation: nothing
 // is written, the totals stay zero and every later kernel finds no cells.  A
 // look-back that waits too long counts the heads before its tile itself.
-// A queue of cells for the pairs' bounds costs the quad masks up to 4 us and pays from here on: 2M
-// points 41 -> 35 us for the two kernels, 4M 84 -> 65, 20M 319 -> 232; 1M 29 -> 33.
-constexpr uint64_t kPairQueuePoints = 1ull << 21;
 constexpr uint64_t kGatherPoints = 1ull << 23;   // 64 MiB of coordinates, half of L2
 constexpr int kHeadThreads = 256, kHeadRounds = 8, kHeadTile = kHeadThreads * kHeadRounds;
 constexpr int kHeadWarps = kHeadThreads / 32;
@@ -139,7 +136,7 @@ template <class KT, bool GATHER>
 __global__ void __launch_bounds__(kHeadThreads, 6) k_heads(
     uint64_t n, uint32_t F, const KT* __restrict__ keys, const uint32_t* __restrict__ sid,
     const float2* __restrict__ xy, const uint32_t* __restrict__ fstart, const uint32_t* __restrict__ fjob,
-    float2* __restrict__ sxy, uint32_t* __restrict__ sfeat, uint64_t* __restrict__ ckey, uint32_t* __restrict__ cstart,
+    float2* __restrict__ sxy, uint32_t* __restrict__ sfeat, uint64_t* __restrict__ ckey,
     uint32_t* __restrict__ crun, uint32_t* __restrict__ cjob, uint32_t* __restrict__ rfeat,
     uint32_t* __restrict__ rstart, uint32_t* __restrict__ rcell, uint32_t* __restrict__ scell, uint64_t capM,
     uint64_t capR, unsigned long long* __restrict__ status, uint32_t* __restrict__ ticket,
@@ -252,7 +249,6 @@ __global__ void __launch_bounds__(kHeadThreads, 6) k_heads(
         if (scell && p < n) scell[p] = c;
         if (ch && c < capM) {
             ckey[c] = key[r];
-            cstart[c] = (uint32_t)p;
             crun[c] = ri;
             cjob[c] = fjob[f[r]];
         }
@@ -269,7 +265,6 @@ __global__ void __launch_bounds__(kHeadThreads, 6) k_heads(
         ctrl->M = cb;
         ctrl->Rn = rb;
         if (cb <= capM && rb <= capR) {
-            cstart[cb] = (uint32_t)n;
             crun[cb] = rb;
             rstart[rb] = (uint32_t)n;
         }
@@ -971,6 +966,10 @@ inline unsigned grid_for(uint64_t n, int threads) {
 
 }  // namespace
 
+// A queue of cells for the pairs' bounds costs the quad masks up to 4 us and pays from here on: 2M
+// points 41 -> 35 us for the two kernels, 4M 84 -> 65, 20M 319 -> 232; 1M 29 -> 33.
+constexpr uint64_t kPairQueuePoints = 1ull << 21;
+
 // Bounded batches reserve at most this much for arrays laid out by bounds (and no more than
 // a sixteenth of the device, and blocks of 256 MiB and more no more than half of what is
 // free); the 20M-point workload takes 5 GB.  Larger ones wait for the number of cells and
@@ -998,7 +997,6 @@ void lay_points(Batch& b, Carver& c) {
 }
 void lay_heads(Batch& b, Carver& c, uint64_t M, uint64_t R) {
     c.add(b.ckey, M);
-    c.add(b.cstart, M + 1);
     c.add(b.crun, M + 1);
     c.add(b.cjob, M);
     c.add(b.rfeat, R);
@@ -1033,7 +1031,7 @@ void launch_heads(Batch& b, const KT* keys, uint64_t capM, uint64_t capR) {
     auto* const kernel = b.gathered ? k_heads<KT, true> : k_heads<KT, false>;
     kernel<<<(unsigned)tiles, kHeadThreads, 0, b.s>>>(
         b.N, b.F, keys, b.sid.get(), b.xy.get(), b.fstart.get(), b.fjob.get(), b.sxy.get(), b.sfeat.get(),
-        b.ckey.get(), b.cstart.get(), b.crun.get(), b.cjob.get(), b.rfeat.get(), b.rstart.get(), b.rcell.get(),
+        b.ckey.get(), b.crun.get(), b.cjob.get(), b.rfeat.get(), b.rstart.get(), b.rcell.get(),
         capM ? b.scell.get() : nullptr, capM, capR, b.head_status.get(), b.tickets.get() + b.plan.n, b.ctrl.get());
     COLO_LAUNCH_CHECK();
     count_launch();

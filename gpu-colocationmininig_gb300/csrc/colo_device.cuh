@@ -80,16 +80,6 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* __restrict__
     return lo;
 }
 
-// Number of set bits of the W-word mask m below bit b.  A cell's runs ascend
-// by feature and its mask has one bit per feature present, so for local
-// feature b the run index in the cell is crun + mask_rank(mask, b).
-__device__ __forceinline__ uint32_t mask_rank(const uint32_t* __restrict__ m, uint32_t b) {
-    const uint32_t wq = b >> 5;
-    uint32_t r = 0;
-    for (uint32_t w = 0; w < wq; ++w) r += __popc(m[w]);
-    return r + __popc(m[wq] & ((1u << (b & 31)) - 1u));
-}
-
 // Column and row of a cell from its id within its grid (id = row * gx + col):
 // a 32-bit division when the id fits, which every grid of fewer than 2^32
 // cells does, else the 64-bit one.

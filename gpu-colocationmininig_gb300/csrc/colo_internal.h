@@ -8,8 +8,7 @@
 //   jobs        JobGrid[J] (the reference grid of each job, R^2, threshold)
 //   bucketed    points sorted by (job cell key, point id): sid, and
 //               with gathered coordinates sxy (sfeat for several jobs)
-//   cells       occupied cells ckey[M], cstart[M+1] (sorted positions),
-//               crun[M+1] (run ranges), nbrs[M] (geometric 3x3 neighbours),
+//   cells       occupied cells ckey[M], crun[M+1] (run ranges), nbrs[M] (geometric 3x3 neighbours),
 //               cmask[M*W] (feature bit masks, local feature index),
 //               qmask[M*4*W] (masks of the 4 quads containing the cell)
 //   runs        (cell, feature) runs rfeat/rstart/rcell[Rn], cell-major;
