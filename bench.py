@@ -196,7 +196,7 @@ def algorithmic_bytes(name: str, c: dict, launches: float, words: int) -> float:
     if name == "cell_keys":        # read x, y, feature; write key, id
         return 24.0 * N
     if name == "cell_heads":       # read the sorted ids and keys (up to 2^23 points also gather x, y), write cells and runs
-        return (4.0 + kb + (16.0 if N <= 1 << 23 else 0.0)) * N + 24.0 * M + 12.0 * Rn
+        return (4.0 + kb + (16.0 if N <= 1 << 23 else 0.0)) * N + 16.0 * M + 12.0 * Rn
     if name == "cell_masks":       # read the runs' features, write the cells' masks
         return 4.0 * Rn + 4.0 * words * M
     if name == "cell_neighbours":  # read the key and the job, write the neighbour word

@@ -664,6 +664,9 @@ __device__ __forceinline__ int adjacent_cells(uint32_t c, const uint4* __restric
 // own.  Most lists are then empty; the cells whose 3x3 mask allows one were
 // queued by k_quad_masks.
 
+// The bounds lie where the kernel's time is flat on 14 workloads (within 5%) with half and twice of each, but
+// for these: 64 runs 117 -> 147 us and 16 anchors 117 -> 143 (400,000 clustered points; 64 anchors 100 there,
+// the same elsewhere), 256 points 411 -> 556 (a batch of 128 jobs).
 constexpr uint32_t kBigRuns = 128, kBigPoints = 512;   // cells with longer lists are merged by their whole warp
 constexpr uint32_t kHeavyAnchors = 32;   // cells with more anchors are listed by their whole warp
 
@@ -794,10 +797,11 @@ __device__ __forceinline__ void list_cell_warp(uint32_t c, int lane, uint64_t fi
 // so nothing is counted or scanned over the cells and runs beforehand (the order
 // within a list is all that a result depends on).  With the two scans, the count
 // and the clears that this replaces, 413 us of kernels became 147 us on the 20M
-// workload; the 200,000-point dense one, whose few long lists share a
-// neighbourhood, 327 became 147 us.
+// workload when the lists still held runs (175 us now that they hold points, which
+// takes the join from 325 to 78); the 200,000-point dense one, whose few long lists
+// share a neighbourhood, 327 became 147, and 75 with ranks from the masks.
 // Eight blocks an SM (64 registers) hide more of the chain than the six that the
-// compiler's choice of registers left (154 against 172 us at 20M points).
+// compiler's choice of registers left (154 against 172 us at 20M points, lists of runs).
 // Lists past `cap` targets are not written; the host sees it in the total and runs
 // the kernel again with room for all.
 __global__ void __launch_bounds__(128, 8) k_neighbour_lists(
@@ -975,8 +979,9 @@ constexpr uint64_t kPairQueuePoints = 1ull << 21;
 // free); the 20M-point workload takes 5 GB.  Larger ones wait for the number of cells and
 // runs before their per-cell arrays are laid out.
 constexpr uint64_t kBoundBytes = 8ull << 30, kSmallBounds = 256ull << 20;
-// Look-back words of all digit passes in one clear, up to this much and a 1024th of the device (above
-// 67 to 179 million points, by key width, one pass's words are cleared before each pass).
+// Look-back words of all digit passes in one clear, up to this much and a 1024th of the device; above (67
+// million points with eight passes, 89 with three of nine bits, 134 with four of eight) one pass's words
+// are cleared before each pass.
 constexpr uint64_t kSortStatusBytes = 256ull << 20;
 // Room for the lists' targets and for neighbours before their numbers are known: four targets
 // per point (nine at most: a point is adjacent to nine cells) and eight neighbours per point (0.14 on the 20M workload, 16 on that batch,

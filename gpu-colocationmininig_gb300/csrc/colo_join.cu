@@ -33,7 +33,8 @@ constexpr uint64_t kJoinWaves = 8;   // waves of resident blocks at most (warps 
 
 // Bound by instruction issue and the dependent loads target -> coordinates.  Groups of eight lanes
 // per anchor walking the lists run by run left most lanes idle, since runs average two points:
-// 0.33 ms became 0.095 ms on the 20M workload (1.2 M anchors, 2.7 M pairs), 2.2 became 0.83 ms on a
+// 0.33 ms became 0.095 ms on 20 million points (1.2 M anchors, 2.7 M pairs; 0.11 ms on the 1.5 M and 3.7 M of
+// another seed), 2.2 became 0.83 ms on a
 // batch of 128 jobs (134 M pairs), 0.36 became 0.042 ms on 200,000 dense points (6 M pairs), where
 // the longest slices alone, eight lanes each, took most of it.  Six blocks an SM (40 registers, some
 // spilled) suit many short slices best (batch: 0.93 ms against 1.08 ms at four).

@@ -648,8 +648,10 @@ void launch_level(Batch& b, const LevelWork& w, uint32_t k, uint32_t* ovf) {
 uint32_t count_split(const Batch& b, uint64_t nchunks) {
     // Where lists are long (four or more pairs tested a point) and the chunks do not fill the GPU,
     // up to 32 warps share a chunk: a chunk of long lists is hundreds of steps for one warp, and the
-    // first levels of dense data are a thousand such chunks (200,000 dense points: counts 1.01 -> 0.93 ms,
-    // a level of 1,100 chunks 82 us before).  Short lists have no steps to share.
+    // first levels of dense data are a thousand such chunks.  Counts with 14 to 30 pairs a point: 198 -> 158 us
+    // (100,000 points), 970 -> 878 (200,000), 280 -> 134 (one hotspot of 4,000 points), and within 1% where
+    // the chunks are many.  Short lists have no steps to share: at 3.2 pairs a point 42 -> 49.  512 warps an
+    // SM are slower (1,094 on the 200,000 points); 64 are on the hotspot (184), but not on the 100,000 (130).
     const uint64_t warps = (uint64_t)b.sms * 192;
     uint32_t log = 0;
     while (b.join_pairs >= 4 * b.N && log < 5 && (nchunks << (log + 1)) <= warps) ++log;

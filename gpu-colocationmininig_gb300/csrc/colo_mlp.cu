@@ -222,8 +222,8 @@ __device__ __forceinline__ float quad_sum(float v) {   // sum over the 8 lanes s
 // keep their parts, and the bias and W3 sums of their rows, in registers over
 // all of the block's rows: one round of atomics per block at the end.  (Summing
 // each 16-row product into shared memory, 6,144 FP32 atomics a warp and tile,
-// took 387 us for 205,545 rows; this takes 55 us.)  The call is then bound by the host
-// link: 20 MB of rows, 115 us.
+// took 387 us for 205,545 rows; this takes 55 us.)  A call on host arrays is then bound by
+// their copy over the link: 20 MB of rows, 115 us of its 238.
 __global__ void __launch_bounds__(256, 1) k_mlp_grad(const float* __restrict__ P, const float* __restrict__ X,
                                                      const float* __restrict__ T, const uint32_t* __restrict__ idx,
                                                      uint64_t n, float inv_n, float* __restrict__ G,

@@ -97,7 +97,8 @@ void scan_impl(const Tin* in, Tout* out, uint64_t n, cudaStream_t s, Tout* total
 // ---------------------------------------------------------------------------
 
 // Tile shape: 512 threads of 8 items (4096-key tiles) and four resident blocks
-// per SM (32 registers, a few spilled; 4 x 43 KB of shared memory), three with
+// per SM (32-bit keys: 32 registers, a few spilled; 4 x 43 KB of shared memory, of
+// which 64-bit keys, 59 KB a block, leave three), three with
 // digits of nine bits (55 KB; four measured the same and spill).  Ranking takes most
 // of a pass: without any look-back a sort of random keys is a quarter faster, no more.
 // 2048-key tiles of 256 threads (eight blocks an SM) and 8192-key tiles of 1024

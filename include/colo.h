@@ -330,8 +330,9 @@ colo_status colo_ctx_set_model(colo_ctx* ctx, const float* params);
  * Quad statistics are 0 for pairs.  Recorded for every candidate when the
  * mine's colo_params.reserved[0] has bit 1 set (training data); zeros
  * otherwise.  (A COLO_MODE_LEARNED mine computes them for its predictions
- * without keeping them: on the device right after the level filter for
- * k >= 3, on the host for pairs.) */
+ * without keeping them: on the device right after the level filter, for the
+ * levels k >= 3 that wait for the filter before they count; on the host for
+ * pairs, when every refined candidate's table is written while counted.) */
 colo_status colo_result_features(const colo_result* r, uint32_t li, float* x);
 
 /* ---- allocation-free entry point -------------------------------------- */
