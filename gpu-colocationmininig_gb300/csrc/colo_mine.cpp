@@ -769,17 +769,6 @@ void settle(colo_ctx* ctx, Batch& b, std::vector<uint32_t>* ub2) {
     if (b.join_queued && (again || b.join_pairs > b.nb_cap)) join_neighbors(b);
 }
 
-// The stream-ordered pool keeps what it has mapped (its release threshold is
-// "everything"), but a mine whose blocks come and go in a different order than
-// the last one's may find no free block large enough and map more memory in
-// the middle of a step (about a millisecond per growth on the 20M-point
-// workload).  So after a mine that used more of the pool than any before it,
-// the pool gets one free block of twice that peak, the arrays laid out by bounds
-// (one block, held from the mine's start to its end) counted once, if the device has that
-// much to spare; later mines carve their blocks out of it.  (20 million points hold 5.9 GB;
-// with those arrays counted twice it was 10.8.)  The growth lands in the mine that set
-// the peak (a warm-up mine, typically), not in the next one.  The pool's
-// high-water mark is reset as a mine starts, so it measures that mine alone.
 static cudaMemPool_t device_pool(const colo_ctx* ctx) {
     cudaMemPool_t pool = nullptr;
     if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) != cudaSuccess) {
@@ -834,6 +823,17 @@ static void pool_reset_mark(colo_ctx* ctx) {
     if (pool && cudaMemPoolSetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &zero) != cudaSuccess) cudaGetLastError();
 }
 
+// The stream-ordered pool keeps what it has mapped (its release threshold is
+// "everything"), but a mine whose blocks come and go in a different order than
+// the last one's may find no free block large enough and map more memory in
+// the middle of a step (about a millisecond per growth on the 20M-point
+// workload).  So after a mine that used more of the pool than any before it,
+// the pool gets one free block of twice that peak, the arrays laid out by bounds
+// (one block, held from the mine's start to its end) counted once, if the device has that
+// much to spare; later mines carve their blocks out of it.  (20 million points hold 5.9 GB;
+// with those arrays counted twice it was 10.8.)  The growth lands in the mine that set
+// the peak (a warm-up mine, typically), not in the next one.  The pool's
+// high-water mark is reset as a mine starts, so it measures that mine alone.
 static void pool_headroom(colo_ctx* ctx) {
     cudaMemPool_t pool = device_pool(ctx);
     if (!pool) return;
